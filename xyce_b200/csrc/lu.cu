@@ -15,7 +15,8 @@
 // (A destination written in a level is never read in it: M[i][k] being divided would need a pivot
 // of the same level to change column k, and U(k, j) being read would need one to change row k.)
 //
-// Circuit factors are deep and narrow: at 200k unknowns ~2,900 levels of a few pivots each, with a
+// This file serves the matrices that the elimination-tree plan (lutree.h) does not fit: wide fronts,
+// long thin paths. Circuit factors are deep and narrow: at 200k unknowns ~2,900 levels of a few pivots each, with a
 // few dozen levels holding half of the ~13M updates. The light levels are latency-bound, so runs of
 // them execute in ONE thread block with a block barrier after each step (the values written are
 // then visible to the whole block); a level with more work than one block turns over quickly runs
@@ -28,6 +29,8 @@
 #include <queue>
 #include <string>
 #include <vector>
+
+#include "lu_updates.cuh"
 
 int xd_internal_fail(int code, const std::string &msg);
 
@@ -46,37 +49,10 @@ __global__ void lu_scatter_kernel(int nnz_a, const int *__restrict__ a2m, const 
   if (k < nnz_a) mx[a2m[k]] = a[k];
 }
 
-__device__ __forceinline__ void lu_divide(int2 dv, double *mx) { mx[dv.x] = mx[dv.x] / mx[dv.y]; }
-
-// A destination's updates with the level's L factors already stored (after its division step).
-// ds = (destination, L(i, k), U(k, j), U(k, k)) for one update; (destination, first pair, count,
-// -1) for more, pairs (L(i, k), U(k, j), U(k, k), 0) in increasing k.
-__device__ __forceinline__ void lu_update(int4 ds, const int4 *__restrict__ pairs, double *mx) {
-  double acc = mx[ds.x];
-  if (ds.w >= 0) {
-    acc = acc - mx[ds.y] * mx[ds.z];
-  } else {
-    for (int p = ds.y; p < ds.y + ds.z; ++p) {
-      const int4 lu = pairs[p];
-      acc = acc - mx[lu.x] * mx[lu.y];
-    }
-  }
-  mx[ds.x] = acc;
-}
-
-// The same updates before the level's divisions: each L factor formed on the spot from the
-// undivided column entry and the pivot, the division the division step makes, so the same value.
-__device__ __forceinline__ void lu_update_divide(int4 ds, const int4 *__restrict__ pairs, double *mx) {
-  double acc = mx[ds.x];
-  if (ds.w >= 0) {
-    acc = acc - (mx[ds.y] / mx[ds.w]) * mx[ds.z];
-  } else {
-    for (int p = ds.y; p < ds.y + ds.z; ++p) {
-      const int4 lu = pairs[p];
-      acc = acc - (mx[lu.x] / mx[lu.z]) * mx[lu.y];
-    }
-  }
-  mx[ds.x] = acc;
+__global__ void lu_gather_kernel(int nnz, const int *__restrict__ pos, const double *__restrict__ v,
+                                 double *__restrict__ mx) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < nnz) mx[k] = v[pos[k]];
 }
 
 // Levels [l0, l1) in one block, one barrier per level: step l applies level l's updates, forming
@@ -207,6 +183,9 @@ int xd_lu_init(XdLu *lu, int n, int nnz_a, const int *rowptr_a, const int *colin
       const int *b = mi.data() + mp[i], *e = mi.data() + mp[i + 1];
       a2m[t] = (int)(std::lower_bound(b, e, j) - mi.data());
     }
+  lu->n = n;
+  lu->nnz = nnz;
+  lu->nnz_a = nnz_a;
   // Columns of the strict lower part (rows i > k with L(i, k)) and of the strict upper part (rows
   // k' < k with U(k', k)), both with their positions, in increasing row order.
   std::vector<int> lcp(n + 1, 0), ucp(n + 1, 0);
@@ -241,6 +220,28 @@ int xd_lu_init(XdLu *lu, int n, int nnz_a, const int *rowptr_a, const int *colin
     for (int t = ucp[k]; t < ucp[k + 1]; ++t) l = std::max(l, lev[uci[t]] + 1);
     lev[k] = l;
     nlev = std::max(nlev, l + 1);
+  }
+  lu->nlev = nlev;
+  for (int k = 0; k < n; ++k) lu->npairs += (long long)(lcp[k + 1] - lcp[k]) * (mp[k + 1] - diag[k] - 1);
+  cudaError_t e;
+  if ((e = upload(&lu->d_mp, mp)) != cudaSuccess || (e = upload(&lu->d_mi, mi)) != cudaSuccess ||
+      (e = cudaMalloc(&lu->d_mx, std::max(1, nnz) * sizeof(double))) != cudaSuccess) {
+    xd_lu_free(lu);
+    return xd_internal_fail(-3, std::string("LU set-up upload: ") + cudaGetErrorString(e));
+  }
+  // The elimination-tree plan where the structure allows it, else the level lists below.
+  XdTreePlan plan;
+  if (xd_tree_plan(n, mp, mi, diag, &plan)) {
+    for (int &m : a2m) m = plan.pos[m];
+    if ((e = upload(&lu->d_a2m, a2m)) != cudaSuccess || (e = upload(&lu->d_pos, plan.pos)) != cudaSuccess) {
+      xd_lu_free(lu);
+      return xd_internal_fail(-3, std::string("LU set-up upload: ") + cudaGetErrorString(e));
+    }
+    if (const int rc = xd_tree_upload(&lu->tree, plan)) {
+      xd_lu_free(lu);
+      return rc;
+    }
+    return 0;
   }
   std::vector<int> piv_start(nlev + 1, 0);
   for (int k = 0; k < n; ++k) ++piv_start[lev[k] + 1];
@@ -321,22 +322,11 @@ int xd_lu_init(XdLu *lu, int n, int nnz_a, const int *rowptr_a, const int *colin
     grid.push_back(0);
     l = e;
   }
-  long long npairs = (long long)pairs.size();
-  for (const int4 &d : dst)
-    if (d.w >= 0) ++npairs;
-  lu->n = n;
-  lu->nnz = nnz;
-  lu->nnz_a = nnz_a;
-  lu->nlev = nlev;
   lu->lev_div = lev_div;
   lu->lev_dst = lev_dst;
-  lu->npairs = npairs;
   lu->segments = segments;
   lu->segment_grid = grid;
-  cudaError_t e;
-  if ((e = upload(&lu->d_mp, mp)) != cudaSuccess || (e = upload(&lu->d_mi, mi)) != cudaSuccess ||
-      (e = cudaMalloc(&lu->d_mx, std::max(1, nnz) * sizeof(double))) != cudaSuccess ||
-      (e = upload(&lu->d_a2m, a2m)) != cudaSuccess || (e = upload(&lu->d_diag, diag)) != cudaSuccess ||
+  if ((e = upload(&lu->d_a2m, a2m)) != cudaSuccess || (e = upload(&lu->d_diag, diag)) != cudaSuccess ||
       (e = upload(&lu->d_lev_div, lev_div)) != cudaSuccess || (e = upload(&lu->d_lev_dst, lev_dst)) != cudaSuccess ||
       (e = upload(&lu->d_div, div)) != cudaSuccess || (e = upload(&lu->d_dst, dst)) != cudaSuccess ||
       (e = upload(&lu->d_pairs, pairs)) != cudaSuccess || (e = cudaMalloc(&lu->d_info, sizeof(int))) != cudaSuccess) {
@@ -358,11 +348,26 @@ void xd_lu_free(XdLu *lu) {
   cudaFree(lu->d_dst);
   cudaFree(lu->d_pairs);
   cudaFree(lu->d_info);
+  cudaFree(lu->d_pos);
+  xd_tree_free(&lu->tree);
   *lu = XdLu();
 }
 
 int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st) {
   cudaError_t e;
+  if (lu->tree.on) {
+    XdTree &t = lu->tree;
+    if ((e = cudaMemsetAsync(t.d_v, 0, std::max<long long>(1, t.nv) * sizeof(double), st)) != cudaSuccess ||
+        (e = cudaMemsetAsync(t.d_ctl, 0, (kTreeFlags + t.nchains) * sizeof(int), st)) != cudaSuccess)
+      return xd_internal_fail(-3, std::string("LU refactorization: ") + cudaGetErrorString(e));
+    if (lu->nnz_a > 0)
+      lu_scatter_kernel<<<(lu->nnz_a + 255) / 256, 256, 0, st>>>(lu->nnz_a, lu->d_a2m, d_vals_a, t.d_v);
+    if (const int rc = xd_tree_factor(&t, st)) return rc;
+    lu_gather_kernel<<<(lu->nnz + 255) / 256, 256, 0, st>>>(lu->nnz, lu->d_pos, t.d_v, lu->d_mx);
+    if ((e = cudaGetLastError()) != cudaSuccess)
+      return xd_internal_fail(-3, std::string("LU refactorization launch: ") + cudaGetErrorString(e));
+    return 0;
+  }
   if ((e = cudaMemsetAsync(lu->d_mx, 0, std::max(1, lu->nnz) * sizeof(double), st)) != cudaSuccess ||
       (e = cudaMemsetAsync(lu->d_info, 0x7f, sizeof(int), st)) != cudaSuccess)
     return xd_internal_fail(-3, std::string("LU refactorization: ") + cudaGetErrorString(e));
@@ -388,6 +393,15 @@ int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st) {
 }
 
 int xd_lu_info(XdLu *lu, cudaStream_t st, int *info) {
+  if (lu->tree.on) {
+    int c[2] = {0, 0};
+    cudaError_t e = cudaMemcpyAsync(c, lu->tree.d_ctl + kTreeInfo, sizeof(c), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return xd_internal_fail(-3, std::string("LU pivot report: ") + cudaGetErrorString(e));
+    if (c[kTreeExpired - kTreeInfo] != 0) return xd_internal_fail(-3, "LU refactorization: a wait between chains expired");
+    *info = c[0] == 0 ? 0 : lu->n - c[0] + 1;
+    return 0;
+  }
   int v = 0;
   cudaError_t e = cudaMemcpyAsync(&v, lu->d_info, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);

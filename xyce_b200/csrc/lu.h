@@ -6,6 +6,8 @@
 
 #include <vector>
 
+#include "lutree.h"
+
 // P A Q = L U with the pivot order and the fill pattern of one host factorization. The factors
 // are kept bundled as one CSR matrix M = L - I + U over P A Q's indices (columns sorted; L's unit
 // diagonal implicit, U's diagonal stored), the layout the triangular solves read.
@@ -34,6 +36,10 @@ struct XdLu {
   // than one block turns over quickly runs as its own grid-wide launches.
   std::vector<int2> segments;            // (first level, end level); end = first + 1 and heavy: grid-wide
   std::vector<char> segment_grid;
+  // A matrix with an elimination-tree plan (lutree.h) is factored by it instead: its values live in
+  // the plan's array and d_a2m points there.
+  XdTree tree;
+  int *d_pos = nullptr;                  // [nnz] position of each entry of M in the plan's array
   int *d_info = nullptr;                 // 1 + the first zero pivot's row, or kLuNoZeroPivot
 };
 

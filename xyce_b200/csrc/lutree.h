@@ -1,0 +1,97 @@
+// Elimination-tree plan of the sparse LU refactorization and of its triangular solves (internal to
+// the library).
+//
+// The pivots of P A Q form a tree: pivot k's updates reach only rows and columns of its front
+// struct(k) (the rows of L's column k and the columns of U's row k, closed under elimination), all
+// of which are ancestors of k. Two facts about circuit factors shape the plan:
+//   * the tree is a wide forest of small subtrees under a few long paths. At 200k unknowns (the
+//     placed 100k-MOSFET netlist) 4,374 subtrees of at most 36 levels hang off 61 paths, the
+//     longest of 2,890 pivots whose fronts have 24 to 64 variables;
+//   * a few pivots (a supply's branch equation and current) have an empty row of U or an empty
+//     column of L and so make no updates, however long their other side is; their adjacency must
+//     not be counted as a front (the rail's 90k-entry row would make one front of 90k variables).
+// So the pivots are split in two: the BOTTOM subtrees, of at most kTopWork updates each, are spread
+// over thread blocks that walk their levels independently; the TOP pivots are eliminated path by
+// path ("chains"), one thread block per chain, with the front held densely in registers
+// (lutree.cu). A matrix whose structure does not fit (frame over kMaxFrame, fill of the symmetrised
+// pattern, an update-free pivot that others wait for) has no plan, and the level-by-level
+// kernels of lu.cu and sptrsv.cu take it.
+#pragma once
+
+#include <vector>
+
+struct XdPos2 { int x, y; };
+struct XdPos4 { int x, y, z, w; };
+
+constexpr int kMaxFrame = 128;       // largest frame (slots) of a chain
+constexpr int kJoinNone = 255;       // a parent slot the child chain has no variable for
+constexpr int kBlockPivots = 8;      // pivots a chain eliminates at a time
+constexpr int kBlockInts = 12;       // a block's record: its pivots' slots (kNoPivot past the last), the
+                                     // frame's live slots, the first and last child chain that joins
+constexpr int kNoPivot = (int)0x80000000;
+
+// Host side of the plan. Values live in one array V: strict-lower entries whose column is a bottom
+// pivot row by row, upper entries of bottom rows row by row, bottom diagonals, and then one dense
+// panel of 2 * F values per top pivot: U's row by column slot (the pivot at its own slot), L's
+// column by row slot.
+struct XdTreePlan {
+  int n = 0, F = 0;                  // F: slots of a frame, a multiple of 16
+  int nbot = 0, ntop = 0;
+  std::vector<int> order;            // [n] bottom rows by (group, level, index), then top rows by panel
+  std::vector<int> lptr, lcol;       // strict-lower entries outside the panels, by position in order
+  std::vector<int> uptr, ucol;       // upper entries outside the panels, likewise
+  int u0 = 0, d0 = 0, p0 = 0;        // V offsets: upper entries, bottom diagonals, panels
+  long long nv = 0;                  // length of V
+  std::vector<int> pos;              // [nnz of M] position in V of each entry of M
+  std::vector<int> diag;             // [n] position in V of each pivot
+  // Bottom groups: group g has levels [glev[g], glev[g + 1]); level l its rows order[lrow[l] ..
+  // lrow[l + 1]), its divisions and its update destinations.
+  int ngroups = 0;
+  std::vector<int> glev, lrow, ldiv, ldst;
+  std::vector<XdPos2> div;           // (position of L(i, k), position of U(k, k))
+  std::vector<XdPos4> dst, pairs;    // as in lu.cu: one update inline, or a range of pairs
+  // Updates of top entries by bottom pivots: destination sdst[d], pairs (L, U) sptr[d] .. sptr[d + 1].
+  std::vector<int> sdst, sptr;
+  std::vector<XdPos2> spairs;
+  std::vector<XdPos2> tdiv;          // divisions of top pivots' entries outside their panels
+  std::vector<int> tail;             // positions in order of rows whose upper entries are solved last
+  // Chains, children before parents: chain c has panels [cptr[c], cptr[c + 1]), eliminated in blocks
+  // of kBlockPivots from the first: blocks [bptr[c], bptr[c + 1]), records in blocks. A variable has
+  // a slot from the first block whose pivots' fronts hold it to its own block.
+  int nchains = 0;
+  std::vector<int> cptr, bptr, blocks;
+  std::vector<int> jchild;           // child chains in the order they join
+  std::vector<unsigned char> jmap;   // [nchains * F] a chain's slot of each slot of its parent, or kJoinNone
+};
+
+// Builds the plan of M = L - I + U (CSR, columns ascending, closed under elimination; diag[k] the
+// position of the pivot). Returns false when the structure does not fit.
+bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi, const std::vector<int> &mdiag,
+                  XdTreePlan *plan);
+
+// ---- device side (lutree.cu) ---------------------------------------------------------------------
+#include <cuda_runtime.h>
+
+struct XdTree {
+  bool on = false;                   // the matrix has a plan
+  int n = 0, F = 0, ntop = 0, ngroups = 0, nchains = 0, nsd = 0, ntdiv = 0, p0 = 0;
+  long long nv = 0;
+  double *d_v = nullptr;             // V
+  int *d_diag = nullptr;             // [n]
+  int *d_glev = nullptr, *d_ldiv = nullptr, *d_ldst = nullptr;
+  int2 *d_div = nullptr;
+  int4 *d_dst = nullptr, *d_pairs = nullptr;
+  int *d_sdst = nullptr, *d_sptr = nullptr;
+  int2 *d_spairs = nullptr, *d_tdiv = nullptr;
+  int *d_cptr = nullptr, *d_bptr = nullptr, *d_blocks = nullptr, *d_jchild = nullptr;
+  unsigned char *d_jmap = nullptr;
+  double *d_jbuf = nullptr;          // [nchains][F * F] the fronts that chains hand to their parents
+  int *d_ctl = nullptr;              // zero pivots, expired waits, tickets, chain flags; zeroed by each call
+};
+
+int xd_tree_upload(XdTree *t, const XdTreePlan &p);
+void xd_tree_free(XdTree *t);
+// Eliminates V (holding P A Q, zeros elsewhere) in place; kTreeInfo of d_ctl holds n - k for the first
+// zero pivot k (0: none), kTreeExpired is nonzero when a wait between chains gave up.
+constexpr int kTreeInfo = 0, kTreeExpired = 1, kTreeTicket = 2, kTreeFlags = 4;
+int xd_tree_factor(XdTree *t, cudaStream_t st);
