@@ -237,7 +237,7 @@ int xd_lu_init(XdLu *lu, int n, int nnz_a, const int *rowptr_a, const int *colin
       xd_lu_free(lu);
       return xd_internal_fail(-3, std::string("LU set-up upload: ") + cudaGetErrorString(e));
     }
-    if (const int rc = xd_tree_upload(&lu->tree, plan)) {
+    if (const int rc = xd_tree_upload(&lu->tree, plan, p, q)) {
       xd_lu_free(lu);
       return rc;
     }
@@ -362,11 +362,7 @@ int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st) {
       return xd_internal_fail(-3, std::string("LU refactorization: ") + cudaGetErrorString(e));
     if (lu->nnz_a > 0)
       lu_scatter_kernel<<<(lu->nnz_a + 255) / 256, 256, 0, st>>>(lu->nnz_a, lu->d_a2m, d_vals_a, t.d_v);
-    if (const int rc = xd_tree_factor(&t, st)) return rc;
-    lu_gather_kernel<<<(lu->nnz + 255) / 256, 256, 0, st>>>(lu->nnz, lu->d_pos, t.d_v, lu->d_mx);
-    if ((e = cudaGetLastError()) != cudaSuccess)
-      return xd_internal_fail(-3, std::string("LU refactorization launch: ") + cudaGetErrorString(e));
-    return 0;
+    return xd_tree_factor(&t, st);
   }
   if ((e = cudaMemsetAsync(lu->d_mx, 0, std::max(1, lu->nnz) * sizeof(double), st)) != cudaSuccess ||
       (e = cudaMemsetAsync(lu->d_info, 0x7f, sizeof(int), st)) != cudaSuccess)
@@ -390,6 +386,16 @@ int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st) {
   if ((e = cudaGetLastError()) != cudaSuccess)
     return xd_internal_fail(-3, std::string("LU refactorization launch: ") + cudaGetErrorString(e));
   return 0;
+}
+
+int xd_lu_copy(XdLu *lu, double *h_vals) {
+  cudaError_t e = cudaSuccess;
+  if (lu->tree.on) {
+    lu_gather_kernel<<<(lu->nnz + 255) / 256, 256>>>(lu->nnz, lu->d_pos, lu->tree.d_v, lu->d_mx);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(h_vals, lu->d_mx, sizeof(double) * lu->nnz, cudaMemcpyDeviceToHost);
+  return e == cudaSuccess ? 0 : xd_internal_fail(-3, std::string("LU factors: ") + cudaGetErrorString(e));
 }
 
 int xd_lu_info(XdLu *lu, cudaStream_t st, int *info) {

@@ -52,5 +52,7 @@ void xd_lu_free(XdLu *lu);
 // Refactors with A's values d_vals_a (device, A's CSR order): M = P A Q scattered, then
 // eliminated in place. Stream-ordered; the zero-pivot report is left in d_info.
 int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st);
+// Copies M's values to host memory (nnz doubles, M's CSR order).
+int xd_lu_copy(XdLu *lu, double *h_vals);
 // Reads the zero-pivot report (synchronises the stream): 0, or 1 + the first row found.
 int xd_lu_info(XdLu *lu, cudaStream_t st, int *info);

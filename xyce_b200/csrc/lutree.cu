@@ -1,10 +1,12 @@
-// Sparse LU refactorization over an elimination-tree plan (lutree.h).
+// Sparse LU refactorization and triangular solves over an elimination-tree plan (lutree.h).
 //
-// What bounds it is the longest chain of dependent pivots, not arithmetic or bytes: at 200k unknowns
-// 12.6M updates (0.7 us of the FP64 pipe) and 15 MB of values, but 2,888 pivots in a row. On the
-// B200: 1.16 ms per refactorization there, of which the chains 0.8 ms (0.28 us a pivot), the bottom
-// subtrees 0.09 ms and their updates of top entries 0.03 ms; 0.31 ms at 41k unknowns. The level
-// lists of lu.cu, a barrier and a round trip to global memory per level, take 7.32 and 1.40 ms.
+// What bounds them is the longest chain of dependent pivots, not arithmetic or bytes: at 200k unknowns
+// 12.6M updates (0.7 us of the FP64 pipe) and 27 MB of values, but 2,888 pivots in a row. On the
+// B200, per refactorization there: 1.09 ms, of which the chains 0.95 ms (0.33 us a pivot), the bottom
+// subtrees 0.09 ms and their updates of top entries 0.03 ms; per solve 0.63 ms: the chains 0.22 ms
+// forward and 0.35 ms backward, the bottom subtrees 0.03 ms each way. At 41k unknowns 0.29 and 0.21
+// ms. The level lists of lu.cu and sptrsv.cu, with a barrier and a round trip to global memory per
+// level, take 7.32 and 7.25 ms, and 1.40 and 1.56 ms.
 #include <algorithm>
 #include <cfloat>
 #include <string>
@@ -193,13 +195,13 @@ __global__ void __launch_bounds__(kTopThreads) tree_top_kernel(int F, const int 
   for (int i = tid; i < F; i += kTopThreads) f.piv[i] = 0;
   __syncthreads();
   const int chain = s_chain, len = cptr[chain + 1] - cptr[chain], b0 = bptr[chain], nblk = bptr[chain + 1] - b0;
-  panels += (size_t)cptr[chain] * 2 * F;
+  const size_t stride = xd_panel_size(F);
+  panels += b0 * stride;
   auto fetch = [&](int t) {  // block t's panels and record
     if (t < nblk) {
-      const int units = min(kB, len - t * kB) * F;
       double *to = f.ring + (t & 1) * kB * 2 * F;
-      const double *from = panels + (size_t)t * kB * 2 * F;
-      for (int i = tid; i < units; i += kTopThreads) cp_async16(to + 2 * i, from + 2 * i);
+      const double *from = panels + t * stride;
+      for (int i = tid; i < kB * F; i += kTopThreads) cp_async16(to + 2 * i, from + 2 * i);
       if (tid < kBlockInts / 4)
         cp_async16(f.rec + (t & 1) * kBlockInts + 4 * tid, blocks + (size_t)(b0 + t) * kBlockInts + 4 * tid);
     }
@@ -236,14 +238,14 @@ __global__ void __launch_bounds__(kTopThreads) tree_top_kernel(int F, const int 
     const int me = lside ? tid : tid - half, m = min(me, R - 1);
     double x[kB];
     if (lside || uside) {
-      const double *base = lside ? f.a + m * ld : f.a + m, *pb = pan + (lside ? F + m : m);
+      const double *base = lside ? f.a + m * ld : f.a + m, *pb = pan + (lside ? kB * F + m : m);
       const int step = lside ? 1 : ld;
       double p[kB];
 #pragma unroll
       for (int j = 0; j < kB; ++j) {
         const int s = rec[j];
         x[j] = base[(s & 0xff) * step];
-        p[j] = pb[j * 2 * F];
+        p[j] = pb[j * F];
       }
 #pragma unroll
       for (int j = 0; j < kB; ++j) x[j] = j < nb && me < R ? x[j] + p[j] : 0.0;
@@ -251,7 +253,7 @@ __global__ void __launch_bounds__(kTopThreads) tree_top_kernel(int F, const int 
     if (tid >= kTopThreads - kB * kB) {
       const int i = (tid - (kTopThreads - kB * kB)) / kB, j = tid % kB;
       const int ti = rec[i] & 0xff, tj = rec[j] & 0xff;
-      const double v = f.a[ti * ld + tj], w = pan[j >= i ? i * 2 * F + tj : j * 2 * F + F + ti];
+      const double v = f.a[ti * ld + tj], w = pan[j >= i ? i * F + tj : (kB + j) * F + ti];
       f.sd[i * kB + j] = i < nb && j < nb ? v + w : (i == j ? 1.0 : 0.0);
     }
     if (tid < nb) f.piv[rec[tid]] = 1;
@@ -293,13 +295,20 @@ __global__ void __launch_bounds__(kTopThreads) tree_top_kernel(int F, const int 
         double *sx = (lside ? f.sl : f.su) + me * kLd;
 #pragma unroll
         for (int j = 0; j < kB; j += 2) *(double2 *)(sx + j) = make_double2(x[j], x[j + 1]);
-        double *to = panels + (size_t)t * kB * 2 * F + (lside ? F : 0) + me;
+        double *to = panels + t * stride + (lside ? kB * F : 0) + me;
 #pragma unroll
         for (int j = 0; j < kB; ++j)
-          if (j < nb) to[j * 2 * F] = x[j];
+          if (j < nb) to[j * F] = x[j];
       }
     }
     __syncthreads();
+    if (tid >= kTopThreads - kB * kB) {  // the factored diagonal part, for the solves
+      const int i = (tid - (kTopThreads - kB * kB)) / kB, j = tid % kB;
+      const double *row = (j >= i ? f.su : f.sl) + (rec[max(i, j)] & 0xff) * kLd;
+      double d = i == j ? 1.0 : 0.0;
+      if (i < nb && j < nb) d = i == j ? reciprocal(row[i]) : row[min(i, j)];
+      panels[t * stride + 2 * kB * F + i * kB + j] = d;
+    }
     for (int c0 = 0; c0 < R; c0 += 64) {
       const int nt = min(4, (R - c0 + 15) / 16);
       if (nt == 4)
@@ -333,6 +342,424 @@ __global__ void tree_finish_kernel(int nt, const int2 *__restrict__ tdiv, int n,
   }
 }
 
+// ---- solves --------------------------------------------------------------------------------------
+// Forward: the bottom subtrees' rows level by level, the top rows' sums over bottom columns in one
+// pass, then the chains; backward the other way round. As in the factorization, a chain's pivots
+// are the serial part: one warp per chain takes kB of them at a time, every lane solving the
+// block's small triangle redundantly in registers, so that consecutive pivots cost a
+// multiply-add's latency.
+
+constexpr int kSolveAhead = 4;        // blocks in flight in a chain's solve
+constexpr int kPassRows = 24 * 1024;  // rows of a group whose values fit shared memory
+constexpr int kTailChunk = 2048;      // entries a block sums of a row solved last
+static_assert(kB == 8, "the backward solve's reduction is written for blocks of eight pivots");
+
+__global__ void tree_rhs_kernel(int n, const int *__restrict__ bsrc, const double *__restrict__ b,
+                                double *__restrict__ y) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x < n) y[x] = b[bsrc[x]];
+}
+
+// One bottom group's passes (XdPasses): s[row] from the row's sum over already solved s. The group's
+// own solved values are kept in shared memory (the group's rows are [base, base + size); a group
+// with more than kPassRows keeps them in s), and what does not depend on them - columns and values of
+// a pass's first round, its rows and their right-hand sides, solved values of columns outside the
+// group - is loaded a pass ahead, so a level waits for shared memory alone. Forward: s[row] =
+// rhs[row] - sum, in place; backward: divided by the diagonal, and scattered to the solution.
+template <bool BACKWARD>
+__global__ void __launch_bounds__(kPassThreads) tree_pass_kernel(const int *__restrict__ gptr,
+                                                                 const int4 *__restrict__ pass,
+                                                                 const int *__restrict__ rows,
+                                                                 const int *__restrict__ col, int off0,
+                                                                 const double *__restrict__ v,
+                                                                 const double *__restrict__ vd, const double *rhs,
+                                                                 double *s, const int *__restrict__ xdst, double *out,
+                                                                 const int *__restrict__ grow) {
+  extern __shared__ __align__(16) double smem[];
+  const int tid = threadIdx.x, base = grow[blockIdx.x], size = grow[blockIdx.x + 1] - base;
+  const bool fits = size <= kPassRows;
+  double *loc = fits ? smem : s + base;
+  auto own = [&](int c) { return (unsigned)(c - base) < (unsigned)size; };
+  if (!BACKWARD && fits) {  // rows without entries keep their right-hand sides
+    for (int i = tid; i < size; i += kPassThreads) smem[i] = rhs[base + i];
+    __syncthreads();
+  }
+  // First what needs only the pass's record, two passes ahead; then what its column and row point to.
+  struct First {
+    int4 m;
+    int x, c;
+    double a;
+  };
+  struct Second {
+    double b, d, sv;
+    int to;
+  };
+  auto load_first = [&](int4 m) {
+    First f;
+    f.m = m;
+    f.x = f.c = -1;
+    f.a = 0.0;
+    const int lg = m.y >> 16 & 0xff;
+    if (tid < (m.y & 0xffff) << lg) {
+      f.c = col[m.z - off0 + tid];
+      f.a = v[m.z + tid];
+      if ((tid & ((1 << lg) - 1)) == 0) f.x = rows[m.x + (tid >> lg)];
+    }
+    return f;
+  };
+  auto load_second = [&](const First &f) {
+    Second q;
+    q.b = q.sv = 0.0;
+    q.d = 1.0;
+    q.to = 0;
+    if (f.c >= 0 && !own(f.c)) q.sv = s[f.c];
+    if (f.x >= 0) {
+      q.b = rhs[f.x];
+      if (BACKWARD) {
+        q.d = vd[f.x];
+        q.to = xdst[f.x];
+      }
+    }
+    return q;
+  };
+  const int p1 = gptr[blockIdx.x + 1];
+  int p = gptr[blockIdx.x];
+  if (p >= p1) return;
+  auto record = [&](int q) { return q < p1 ? pass[q] : make_int4(0, 0, 0, 0); };
+  int4 m2 = record(p + 1), m3 = record(p + 2);
+  First f0 = load_first(record(p)), f1 = load_first(m2);
+  Second q0 = load_second(f0);
+  m2 = m3;
+  m3 = record(p + 3);
+  for (; p < p1; ++p) {
+    const First f = f0;
+    const Second q = q0;
+    q0 = load_second(f1);
+    f0 = f1;
+    f1 = load_first(m2);
+    m2 = m3;
+    m3 = record(p + 4);
+    const int lg = f.m.y >> 16 & 0xff, width = (f.m.y & 0xffff) << lg;
+    double acc = f.c >= 0 ? f.a * (own(f.c) ? loc[f.c - base] : q.sv) : 0.0;
+    if (tid < width)
+      for (int k = 1; k < f.m.w; ++k) {
+        const int at = f.m.z + k * width + tid, c = col[at - off0];
+        if (c >= 0) acc += v[at] * (own(c) ? loc[c - base] : s[c]);
+      }
+    for (int o = 1 << lg >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (f.x >= 0) {
+      const double r = BACKWARD ? (q.b - acc) / q.d : q.b - acc;
+      s[f.x] = r;
+      if (fits) smem[f.x - base] = r;
+      if (BACKWARD) out[q.to] = r;
+    }
+    if (f.m.y >> 24) __syncthreads();
+  }
+}
+
+// Rows [x0, n): the top rows' sums over columns outside their panels, a warp each.
+__global__ void __launch_bounds__(256) tree_top_rows_kernel(int x0, int n, const int *__restrict__ lptr,
+                                                            const int *__restrict__ lcol, const double *v, double *y) {
+  const int r = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (x0 + r >= n) return;
+  const int b = lptr[r], end = lptr[r + 1];
+  double acc = 0.0;
+  for (int e = b + lane; e < end; e += 32) acc += v[e] * y[lcol[e]];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0 && end > b) y[x0 + r] -= acc;
+}
+
+__device__ __forceinline__ void cp_async8(void *s, const void *g) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(s);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sa), "l"(g) : "memory");
+}
+
+// A chain's solve in shared memory: per block in flight its panel half, its diagonal part, its
+// right-hand sides and its record; and what the threads exchange.
+struct SolveSmem {
+  double *ring, *diag, *rhs, *red;
+  int *rec;
+  static __host__ __device__ size_t bytes(int F) {
+    return sizeof(double) * (kSolveAhead * (kB * F + kB * kB + kB) + 2 * kB * (kMaxFrame / 32)) +
+           sizeof(int) * kSolveAhead * kBlockInts;
+  }
+  __device__ SolveSmem(double *s, int F) {
+    ring = s;
+    diag = ring + kSolveAhead * kB * F;
+    rhs = diag + kSolveAhead * kB * kB;
+    red = rhs + kSolveAhead * kB;
+    rec = (int *)(red + 2 * kB * (kMaxFrame / 32));
+  }
+  // Block t (of nblk, records and panels from the chain's first) by one warp; half 0: U, 1: L.
+  __device__ void fetch(int t, int nblk, int len, int F, int half, const double *panels, const int *blocks,
+                        const double *y, int lane) const {
+    if (t >= 0 && t < nblk) {
+      const int q = t % kSolveAhead, nb = min(kB, len - t * kB);
+      const double *from = panels + t * (size_t)xd_panel_size(F);
+      for (int i = lane; i < kB * F / 2; i += 32) cp_async16(ring + q * kB * F + 2 * i, from + half * kB * F + 2 * i);
+      cp_async16(diag + q * kB * kB + 2 * lane, from + 2 * kB * F + 2 * lane);
+      if (lane < kBlockInts / 4) cp_async16(rec + q * kBlockInts + 4 * lane, blocks + (size_t)t * kBlockInts + 4 * lane);
+      if (lane < nb) cp_async8(rhs + q * kB + lane, y + t * kB + lane);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+};
+
+// Waits (one thread) for a chain's flag; false when the wait gave up.
+__device__ __forceinline__ bool chain_wait(int *flag) {
+  int w = 0;
+  while (atomicAdd(flag, 0) == 0 && ++w < kSpinLimit) __nanosleep(32);
+  __threadfence();
+  return w < kSpinLimit;
+}
+
+// The value of the block's `mine`-th pivot from registers.
+__device__ __forceinline__ double pick(const double (&v)[kB], int mine) {
+  double x = v[0];
+#pragma unroll
+  for (int j = 1; j < kB; ++j) x = mine == j ? v[j] : x;
+  return x;
+}
+
+// This slot's pivot of the block, or -1.
+__device__ __forceinline__ int pivot_of(const int *rec, int r) {
+  int m = -1;
+#pragma unroll
+  for (int j = 0; j < kB; ++j)
+    if (rec[j] == r) m = j;
+  return m;
+}
+
+// What a chain's solve has in its registers of a block: the diagonal part, this slot's panel entries
+// and the right-hand sides.
+struct BlockRegs {
+  double d[kB][kB], pan[kB], rhs[kB];
+  __device__ void load(const SolveSmem &s, int q, int F, int r, int nb) {
+#pragma unroll
+    for (int i = 0; i < kB; ++i)
+#pragma unroll
+      for (int j = 0; j < kB; j += 2) {
+        const double2 t = *(const double2 *)(s.diag + q * kB * kB + i * kB + j);
+        d[i][j] = t.x;
+        d[i][j + 1] = t.y;
+      }
+#pragma unroll
+    for (int j = 0; j < kB; ++j) {
+      pan[j] = r < F ? s.ring[(q * kB + j) * F + r] : 0.0;
+      rhs[j] = j < nb ? s.rhs[q * kB + j] : 0.0;
+    }
+  }
+};
+
+// Forward chains: thread r holds slot r's sum (of L's entries times the solved values so far), the
+// last warp streams the blocks in. Per block: the threads of the pivots' slots publish their sums,
+// a barrier, and every thread solves the block's triangle and takes its entries times the block's
+// values. ticket, flags: zeroed by the caller.
+__global__ void __launch_bounds__(kMaxFrame + 32) tree_forward_chain_kernel(
+    int F, const int *__restrict__ cptr, const int *__restrict__ bptr, const int *__restrict__ blocks,
+    const int *__restrict__ jchild, const unsigned char *__restrict__ jmap, double *wbuf, const double *panels,
+    double *y, int *ticket, int *flags) {
+  extern __shared__ __align__(16) double smem[];
+  __shared__ int s_chain, s_ok;
+  const SolveSmem s(smem, F);
+  const int r = threadIdx.x, lane = r % 32;
+  const bool feeder = r >= (int)blockDim.x - 32;
+  if (r == 0) s_chain = atomicAdd(ticket, 1);
+  __syncthreads();
+  const int chain = s_chain, len = cptr[chain + 1] - cptr[chain], b0 = bptr[chain], nblk = bptr[chain + 1] - b0;
+  panels += b0 * (size_t)xd_panel_size(F);
+  blocks += (size_t)b0 * kBlockInts;
+  y += cptr[chain];
+  if (feeder) {
+    for (int t = 0; t < kSolveAhead - 1; ++t) s.fetch(t, nblk, len, F, 1, panels, blocks, y, lane);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kSolveAhead - 2) : "memory");
+  }
+  __syncthreads();
+  double w = 0.0;
+  for (int t = 0; t < nblk; ++t) {
+    const int q = t % kSolveAhead, nb = min(kB, len - t * kB);
+    const int *rec = s.rec + q * kBlockInts;
+    double *red = s.red + (t & 1) * kB;
+    for (int j = rec[kB + 1]; j < rec[kB + 2]; ++j) {
+      const int child = jchild[j];
+      if (r == 0) s_ok = chain_wait(flags + child);
+      __syncthreads();
+      if (r < F) {
+        const int m = jmap[(size_t)child * F + r];
+        if (m != kJoinNone) w += s_ok ? __ldcg(wbuf + (size_t)child * F + m) : __longlong_as_double(-1LL);
+      }
+      __syncthreads();
+    }
+    BlockRegs g;
+    int mine = -1;
+    if (!feeder) {
+      mine = pivot_of(rec, r);
+      if (mine >= 0) {
+        red[mine] = w;
+        w = 0.0;
+      }
+      g.load(s, q, F, r, nb);
+    } else {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kSolveAhead - 3) : "memory");
+    }
+    __syncthreads();
+    if (feeder) {
+      s.fetch(t + kSolveAhead - 1, nblk, len, F, 1, panels, blocks, y, lane);
+    } else {
+      double v[kB];
+#pragma unroll
+      for (int j = 0; j < kB; ++j) v[j] = j < nb ? g.rhs[j] + red[j] : 0.0;
+#pragma unroll
+      for (int j = 0; j < kB; ++j)
+#pragma unroll
+        for (int i = j + 1; i < kB; ++i) v[i] = i < nb ? fma(-g.d[i][j], v[j], v[i]) : 0.0;
+      double w2 = 0.0;
+#pragma unroll
+      for (int j = 0; j < kB; j += 2) {
+        w = fma(-g.pan[j], v[j], w);
+        w2 = fma(-g.pan[j + 1], v[j + 1], w2);
+      }
+      w += w2;
+      if (mine >= 0) {
+        w = 0.0;
+        y[t * kB + mine] = pick(v, mine);
+      }
+    }
+  }
+  if (r < F) __stcg(wbuf + (size_t)chain * F + r, w);
+  __threadfence();
+  __syncthreads();
+  if (r == 0) atomicExch(flags + chain, 1);
+}
+
+// Backward chains, parents first: thread r holds the solved value of slot r's variable. Per block:
+// the pivots' row sums over the front, reduced within warps by shuffles and across them through
+// shared memory, then the block's triangle.
+__global__ void __launch_bounds__(kMaxFrame + 32) tree_backward_chain_kernel(
+    int nchains, int F, const int *__restrict__ cptr, const int *__restrict__ bptr, const int *__restrict__ blocks,
+    const int *__restrict__ jchild, const int *__restrict__ border, const double *panels, const double *y, int x0,
+    double *x, const int *__restrict__ xdst, double *out, int *ticket, int *flags, const int *__restrict__ joined) {
+  extern __shared__ __align__(16) double smem[];
+  __shared__ int s_chain, s_ok;
+  const SolveSmem s(smem, F);
+  const int r = threadIdx.x, lane = r % 32, warps = (int)blockDim.x / 32 - 1;
+  const bool feeder = r >= (int)blockDim.x - 32;
+  if (r == 0) {
+    s_chain = nchains - 1 - atomicAdd(ticket, 1);
+    s_ok = joined[s_chain] ? chain_wait(flags + s_chain) : 1;
+  }
+  __syncthreads();
+  const int chain = s_chain, p0 = cptr[chain], len = cptr[chain + 1] - p0, b0 = bptr[chain];
+  const int nblk = bptr[chain + 1] - b0;
+  panels += b0 * (size_t)xd_panel_size(F);
+  blocks += (size_t)b0 * kBlockInts;
+  y += x0 + p0;
+  if (feeder) {
+    for (int t = nblk - 1; t > nblk - kSolveAhead; --t) s.fetch(t, nblk, len, F, 0, panels, blocks, y, lane);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kSolveAhead - 2) : "memory");
+  }
+  double w = 0.0;
+  if (r < F) {
+    const int at = border[(size_t)chain * F + r];
+    if (at >= 0) w = s_ok ? __ldcg(x + at) : __longlong_as_double(-1LL);
+  }
+  __syncthreads();
+  for (int t = nblk - 1; t >= 0; --t) {
+    const int q = t % kSolveAhead, nb = min(kB, len - t * kB);
+    const int *rec = s.rec + q * kBlockInts;
+    const int j0 = rec[kB + 1], j1 = rec[kB + 2];
+    double *red = s.red + (t & 1) * kB * (kMaxFrame / 32);
+    BlockRegs g;
+    int mine = -1;
+    if (!feeder) {
+      mine = pivot_of(rec, r);
+      if (mine >= 0) w = 0.0;  // the pivots' own slots: not solved yet
+      g.load(s, q, F, r, nb);
+      double acc[kB];
+#pragma unroll
+      for (int j = 0; j < kB; ++j) acc[j] = j < nb ? g.pan[j] * w : 0.0;
+      // Eight sums over 32 lanes: halve the values held while halving the lanes they come from.
+#pragma unroll
+      for (int h = 4; h > 0; h >>= 1) {
+        const int bit = h * 4;
+        const bool up = lane & bit;
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+          const double keep = up ? acc[j + h] : acc[j], give = up ? acc[j] : acc[j + h];
+          acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+      }
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+      if ((lane & 3) == 0) red[r / 32 * kB + (lane >> 4 & 1) * 4 + (lane >> 3 & 1) * 2 + (lane >> 2 & 1)] = acc[0];
+    } else {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kSolveAhead - 3) : "memory");
+    }
+    __syncthreads();
+    if (feeder) {
+      s.fetch(t - kSolveAhead + 1, nblk, len, F, 0, panels, blocks, y, lane);
+    } else {
+      double v[kB];
+#pragma unroll
+      for (int j = 0; j < kB; ++j) v[j] = g.rhs[j] - red[j];
+      for (int k = 1; k < warps; ++k)
+#pragma unroll
+        for (int j = 0; j < kB; ++j) v[j] -= red[k * kB + j];
+#pragma unroll
+      for (int j = kB - 1; j >= 0; --j) {
+        v[j] = j < nb ? v[j] * g.d[j][j] : 0.0;
+#pragma unroll
+        for (int i = 0; i < j; ++i) v[i] = fma(-g.d[i][j], v[j], v[i]);
+      }
+      if (mine >= 0) {
+        w = pick(v, mine);
+        const int at = x0 + p0 + t * kB + mine, to = xdst[at];
+        __stcg(x + at, w);
+        if (to >= 0) out[to] = w;
+      }
+    }
+    if (j0 < j1) {  // child chains start from here
+      __threadfence();
+      __syncthreads();
+      for (int j = j0 + r; j < j1; j += blockDim.x) atomicExch(flags + jchild[j], 1);
+    }
+  }
+}
+
+// Rows solved last (nobody reads their values, and one may hold an entry for every device of a
+// supply): a block per kTailChunk entries; the block that finishes a row's last chunk adds the
+// chunks' sums in order. A top row has its panel's part in xs already.
+__global__ void __launch_bounds__(256) tree_tail_kernel(const int4 *__restrict__ chunk, const int4 *__restrict__ tail,
+                                                        int nbot, const int *__restrict__ tcol, const double *vt,
+                                                        const double *v, const double *y, const double *xs,
+                                                        const int *__restrict__ xdst, double *part, int *done,
+                                                        double *out) {
+  __shared__ double red[8];
+  const int lane = threadIdx.x % 32;
+  const int4 c = chunk[blockIdx.x], row = tail[c.x];
+  double acc = 0.0;
+  for (int e = c.y + threadIdx.x; e < c.z; e += 256) acc += vt[e] * xs[tcol[e]];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) red[threadIdx.x / 32] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    acc = 0.0;
+    for (int w = 0; w < 8; ++w) acc += red[w];
+    if (row.w > 1) {
+      __stcg(part + row.z + c.w, acc);
+      __threadfence();
+      if (atomicAdd(done + c.x, 1) < row.w - 1) return;
+      __threadfence();
+      acc = 0.0;
+      for (int k = 0; k < row.w; ++k) acc += __ldcg(part + row.z + k);
+    }
+    const double p = v[row.y];
+    out[~xdst[row.x]] = row.x < nbot ? (y[row.x] - acc) / p : xs[row.x] - acc / p;
+  }
+}
+
 template <class D, class T>
 cudaError_t upload(D **d, const std::vector<T> &h) {
   static_assert(sizeof(D) == sizeof(T), "device and host records match");
@@ -343,7 +770,7 @@ cudaError_t upload(D **d, const std::vector<T> &h) {
 
 }  // namespace
 
-int xd_tree_upload(XdTree *t, const XdTreePlan &p) {
+int xd_tree_upload(XdTree *t, const XdTreePlan &p, const int *perm_p, const int *perm_q) {
   t->n = p.n;
   t->F = p.F;
   t->ntop = p.ntop;
@@ -353,8 +780,59 @@ int xd_tree_upload(XdTree *t, const XdTreePlan &p) {
   t->ntdiv = (int)p.tdiv.size();
   t->p0 = p.p0;
   t->nv = p.nv;
+  t->nbot = p.nbot;
+  t->ntail = (int)p.tail.size();
+  t->l0 = p.l0;
+  t->u0 = p.u0;
+  t->t0 = p.t0;
+  t->d0 = p.d0;
+  std::vector<int> bsrc(p.n), xdst(p.n), joined(std::max(1, p.nchains), 0);
+  for (int x = 0; x < p.n; ++x) {
+    bsrc[x] = perm_p[p.order[x]];
+    xdst[x] = perm_q[p.order[x]];
+  }
+  std::vector<int> grow(1, 0);
+  size_t most = 0;
+  for (int g = 0; g < p.ngroups; ++g) {
+    grow.push_back(p.lrow[p.glev[g + 1]]);
+    const size_t rows = grow[g + 1] - grow[g];
+    if (rows <= (size_t)kPassRows) most = std::max(most, rows);
+  }
+  t->pass_smem = sizeof(double) * most;
+  std::vector<XdPos4> tail, chunk;
+  for (int r = 0; r < t->ntail; ++r) {
+    const int x = p.tail[r], first = (int)chunk.size();
+    xdst[x] = ~xdst[x];
+    for (int e = p.tptr[r]; e < p.tptr[r + 1]; e += kTailChunk)
+      chunk.push_back({r, e, std::min(e + kTailChunk, p.tptr[r + 1]), (int)chunk.size() - first});
+    tail.push_back({x, p.diag[p.order[x]], first, (int)chunk.size() - first});
+  }
+  t->nchunk = (int)chunk.size();
+  for (int c : p.jchild) joined[c] = 1;
   cudaError_t e;
-  if ((e = cudaMalloc(&t->d_v, sizeof(double) * std::max<long long>(1, p.nv))) != cudaSuccess ||
+  auto upload_passes = [](XdTree::Passes &d, const XdPasses &h) {
+    cudaError_t e = upload(&d.gptr, h.gptr);
+    if (e == cudaSuccess) e = upload(&d.pass, h.pass);
+    if (e == cudaSuccess) e = upload(&d.rows, h.rows);
+    if (e == cudaSuccess) e = upload(&d.col, h.col);
+    return e;
+  };
+  if ((e = upload_passes(t->d_fwd, p.fwd)) != cudaSuccess || (e = upload_passes(t->d_bwd, p.bwd)) != cudaSuccess ||
+      (e = upload(&t->d_lptr, p.lptr)) != cudaSuccess || (e = upload(&t->d_lcol, p.lcol)) != cudaSuccess ||
+      (e = upload(&t->d_tcol, p.tcol)) != cudaSuccess || (e = upload(&t->d_chunk, chunk)) != cudaSuccess ||
+      (e = upload(&t->d_tail, tail)) != cudaSuccess || (e = upload(&t->d_bsrc, bsrc)) != cudaSuccess ||
+      (e = upload(&t->d_xdst, xdst)) != cudaSuccess || (e = upload(&t->d_joined, joined)) != cudaSuccess ||
+      (e = upload(&t->d_border, p.border)) != cudaSuccess || (e = upload(&t->d_grow, grow)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(tree_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(double) * kPassRows)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(tree_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(double) * kPassRows)) != cudaSuccess ||
+      (e = cudaMalloc(&t->d_y, sizeof(double) * std::max(1, p.n))) != cudaSuccess ||
+      (e = cudaMalloc(&t->d_x, sizeof(double) * std::max(1, p.n))) != cudaSuccess ||
+      (e = cudaMalloc(&t->d_wbuf, sizeof(double) * std::max<size_t>(1, (size_t)p.nchains * p.F))) != cudaSuccess ||
+      (e = cudaMalloc(&t->d_part, sizeof(double) * std::max(1, t->nchunk))) != cudaSuccess ||
+      (e = cudaMalloc(&t->d_sctl, sizeof(int) * (2 + 2 * p.nchains + t->ntail))) != cudaSuccess ||
+      (e = cudaMalloc(&t->d_v, sizeof(double) * std::max<long long>(1, p.nv))) != cudaSuccess ||
       (e = upload(&t->d_diag, p.diag)) != cudaSuccess || (e = upload(&t->d_glev, p.glev)) != cudaSuccess ||
       (e = upload(&t->d_ldiv, p.ldiv)) != cudaSuccess || (e = upload(&t->d_ldst, p.ldst)) != cudaSuccess ||
       (e = upload(&t->d_div, p.div)) != cudaSuccess || (e = upload(&t->d_dst, p.dst)) != cudaSuccess ||
@@ -366,6 +844,10 @@ int xd_tree_upload(XdTree *t, const XdTreePlan &p) {
       (e = cudaMalloc(&t->d_jbuf, sizeof(double) * std::max<size_t>(1, (size_t)p.nchains * p.F * p.F))) != cudaSuccess ||
       (e = cudaFuncSetAttribute(tree_top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)Frame::bytes(kMaxFrame))) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(tree_forward_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)SolveSmem::bytes(kMaxFrame))) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(tree_backward_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)SolveSmem::bytes(kMaxFrame))) != cudaSuccess ||
       (e = cudaMalloc(&t->d_ctl, sizeof(int) * (kTreeFlags + p.nchains))) != cudaSuccess) {
     xd_tree_free(t);
     return xd_internal_fail(-3, std::string("LU set-up upload: ") + cudaGetErrorString(e));
@@ -378,7 +860,12 @@ void xd_tree_free(XdTree *t) {
   for (void *p : {(void *)t->d_v, (void *)t->d_diag, (void *)t->d_glev, (void *)t->d_ldiv, (void *)t->d_ldst,
                   (void *)t->d_div, (void *)t->d_dst, (void *)t->d_pairs, (void *)t->d_sdst, (void *)t->d_sptr,
                   (void *)t->d_spairs, (void *)t->d_tdiv, (void *)t->d_cptr, (void *)t->d_bptr, (void *)t->d_blocks,
-                  (void *)t->d_jchild, (void *)t->d_jmap, (void *)t->d_jbuf, (void *)t->d_ctl})
+                  (void *)t->d_jchild, (void *)t->d_jmap, (void *)t->d_jbuf, (void *)t->d_ctl, (void *)t->d_fwd.gptr,
+                  (void *)t->d_fwd.pass, (void *)t->d_fwd.rows, (void *)t->d_fwd.col, (void *)t->d_bwd.gptr,
+                  (void *)t->d_bwd.pass, (void *)t->d_bwd.rows, (void *)t->d_bwd.col, (void *)t->d_lptr,
+                  (void *)t->d_lcol, (void *)t->d_tcol, (void *)t->d_chunk, (void *)t->d_tail, (void *)t->d_bsrc,
+                  (void *)t->d_xdst, (void *)t->d_joined, (void *)t->d_border, (void *)t->d_y, (void *)t->d_x,
+                  (void *)t->d_wbuf, (void *)t->d_part, (void *)t->d_sctl, (void *)t->d_grow})
     cudaFree(p);
   *t = XdTree();
 }
@@ -402,5 +889,39 @@ int xd_tree_factor(XdTree *t, cudaStream_t st) {
                                                              t->d_v, t->d_ctl);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return xd_internal_fail(-3, std::string("LU refactorization launch: ") + cudaGetErrorString(e));
+  return 0;
+}
+
+int xd_tree_solve(XdTree *t, double *d_x, cudaStream_t st) {
+  cudaError_t e;
+  const int n = t->n, nc = t->nchains;
+  const double *v = t->d_v;
+  if (nc + t->ntail > 0 &&
+      (e = cudaMemsetAsync(t->d_sctl, 0, sizeof(int) * (2 + 2 * nc + t->ntail), st)) != cudaSuccess)
+    return xd_internal_fail(-3, std::string("triangular solve: ") + cudaGetErrorString(e));
+  tree_rhs_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, t->d_bsrc, d_x, t->d_y);
+  if (t->ngroups > 0)
+    tree_pass_kernel<false><<<t->ngroups, kPassThreads, t->pass_smem, st>>>(t->d_fwd.gptr, t->d_fwd.pass, t->d_fwd.rows,
+                                                                 t->d_fwd.col, 0, v, nullptr, t->d_y, t->d_y, nullptr,
+                                                                 nullptr, t->d_grow);
+  if (nc > 0) {
+    const int threads = (t->F + 31) / 32 * 32 + 32;
+    tree_top_rows_kernel<<<(t->ntop + 7) / 8, 256, 0, st>>>(t->nbot, n, t->d_lptr, t->d_lcol, v + t->l0, t->d_y);
+    tree_forward_chain_kernel<<<nc, threads, SolveSmem::bytes(t->F), st>>>(
+        t->F, t->d_cptr, t->d_bptr, t->d_blocks, t->d_jchild, t->d_jmap, t->d_wbuf, v + t->p0, t->d_y + t->nbot,
+        t->d_sctl, t->d_sctl + 2);
+    tree_backward_chain_kernel<<<nc, threads, SolveSmem::bytes(t->F), st>>>(
+        nc, t->F, t->d_cptr, t->d_bptr, t->d_blocks, t->d_jchild, t->d_border, v + t->p0, t->d_y, t->nbot, t->d_x,
+        t->d_xdst, d_x, t->d_sctl + 1, t->d_sctl + 2 + nc, t->d_joined);
+  }
+  if (t->ngroups > 0)
+    tree_pass_kernel<true><<<t->ngroups, kPassThreads, t->pass_smem, st>>>(t->d_bwd.gptr, t->d_bwd.pass, t->d_bwd.rows,
+                                                                t->d_bwd.col, t->u0, v, v + t->d0, t->d_y, t->d_x,
+                                                                t->d_xdst, d_x, t->d_grow);
+  if (t->nchunk > 0)
+    tree_tail_kernel<<<t->nchunk, 256, 0, st>>>(t->d_chunk, t->d_tail, t->nbot, t->d_tcol, v + t->t0, v, t->d_y, t->d_x,
+                                                t->d_xdst, t->d_part, t->d_sctl + 2 + 2 * nc, d_x);
+  if ((e = cudaGetLastError()) != cudaSuccess)
+    return xd_internal_fail(-3, std::string("triangular solve launch: ") + cudaGetErrorString(e));
   return 0;
 }

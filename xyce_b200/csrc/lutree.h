@@ -29,18 +29,42 @@ constexpr int kBlockPivots = 8;      // pivots a chain eliminates at a time
 constexpr int kBlockInts = 12;       // a block's record: its pivots' slots (kNoPivot past the last), the
                                      // frame's live slots, the first and last child chain that joins
 constexpr int kNoPivot = (int)0x80000000;
+#ifdef __CUDACC__
+#define XD_TREE_FN __host__ __device__
+#else
+#define XD_TREE_FN
+#endif
+// Values per block of top pivots in V.
+XD_TREE_FN constexpr long long xd_panel_size(int F) { return 2LL * kBlockPivots * F + kBlockPivots * kBlockPivots; }
 
-// Host side of the plan. Values live in one array V: strict-lower entries whose column is a bottom
-// pivot row by row, upper entries of bottom rows row by row, bottom diagonals, and then one dense
-// panel of 2 * F values per top pivot: U's row by column slot (the pivot at its own slot), L's
-// column by row slot.
+// The bottom rows' sums of a triangular solve, as passes of a thread block: a pass is at most
+// kPassThreads / lanes rows of one level, `lanes` threads each; the entries of a pass sit in the
+// order its threads read them (round k, thread i at off + k * rows * lanes + i; absent ones have
+// column -1 and value 0), so a pass reads its columns and values in whole lines and needs no row
+// pointers.
+constexpr int kPassThreads = 512;
+struct XdPasses {
+  std::vector<int> gptr;             // group g's passes [gptr[g], gptr[g + 1])
+  std::vector<XdPos4> pass;          // (first row in rows, rows | log2 lanes << 16 | last of its level << 24, off, rounds)
+  std::vector<int> rows;             // positions in order
+  std::vector<int> col;              // column (position in order) of each entry slot, or -1
+};
+
+// Host side of the plan. Values live in one array V: the bottom rows' strict-lower entries by forward
+// pass, the top rows' strict-lower entries outside the panels row by row, the bottom rows' upper
+// entries by backward pass, the entries of rows that are solved last, bottom diagonals, and then per
+// block of top pivots a dense panel of 2 * kBlockPivots * F values, the pivots' U rows by column slot
+// (a pivot at its own slot) and their L columns by row slot, and the block's kBlockPivots x
+// kBlockPivots diagonal part once more with the pivots' reciprocals on its diagonal.
 struct XdTreePlan {
   int n = 0, F = 0;                  // F: slots of a frame, a multiple of 16
   int nbot = 0, ntop = 0;
   std::vector<int> order;            // [n] bottom rows by (group, level, index), then top rows by panel
-  std::vector<int> lptr, lcol;       // strict-lower entries outside the panels, by position in order
-  std::vector<int> uptr, ucol;       // upper entries outside the panels, likewise
-  int u0 = 0, d0 = 0, p0 = 0;        // V offsets: upper entries, bottom diagonals, panels
+  XdPasses fwd, bwd;
+  std::vector<int> lptr, lcol;       // top rows' lower entries outside the panels
+  std::vector<int> tail;             // positions in order of the rows that are solved last
+  std::vector<int> tptr, tcol;       // their upper entries outside the panels
+  int l0 = 0, u0 = 0, t0 = 0, d0 = 0, p0 = 0;  // V offsets: top rows, backward passes, last rows, diagonals, panels
   long long nv = 0;                  // length of V
   std::vector<int> pos;              // [nnz of M] position in V of each entry of M
   std::vector<int> diag;             // [n] position in V of each pivot
@@ -54,7 +78,6 @@ struct XdTreePlan {
   std::vector<int> sdst, sptr;
   std::vector<XdPos2> spairs;
   std::vector<XdPos2> tdiv;          // divisions of top pivots' entries outside their panels
-  std::vector<int> tail;             // positions in order of rows whose upper entries are solved last
   // Chains, children before parents: chain c has panels [cptr[c], cptr[c + 1]), eliminated in blocks
   // of kBlockPivots from the first: blocks [bptr[c], bptr[c + 1]), records in blocks. A variable has
   // a slot from the first block whose pivots' fronts hold it to its own block.
@@ -62,6 +85,7 @@ struct XdTreePlan {
   std::vector<int> cptr, bptr, blocks;
   std::vector<int> jchild;           // child chains in the order they join
   std::vector<unsigned char> jmap;   // [nchains * F] a chain's slot of each slot of its parent, or kJoinNone
+  std::vector<int> border;           // [nchains * F] position in order of the variable left in each slot, or -1
 };
 
 // Builds the plan of M = L - I + U (CSR, columns ascending, closed under elimination; diag[k] the
@@ -87,11 +111,32 @@ struct XdTree {
   unsigned char *d_jmap = nullptr;
   double *d_jbuf = nullptr;          // [nchains][F * F] the fronts that chains hand to their parents
   int *d_ctl = nullptr;              // zero pivots, expired waits, tickets, chain flags; zeroed by each call
+  // Solves: rows by position in the plan's order.
+  int nbot = 0, ntail = 0, nchunk = 0, l0 = 0, u0 = 0, t0 = 0, d0 = 0;
+  struct Passes {
+    int *gptr = nullptr, *rows = nullptr, *col = nullptr;
+    int4 *pass = nullptr;
+  } d_fwd, d_bwd;
+  int *d_grow = nullptr;             // [ngroups + 1] first row of each group
+  size_t pass_smem = 0;
+  int *d_lptr = nullptr, *d_lcol = nullptr, *d_tcol = nullptr;
+  int4 *d_chunk = nullptr;           // chunks of the rows solved last: (row, first entry, end, chunk of the row)
+  int4 *d_tail = nullptr;            // those rows: (position in order, V position of its pivot, first chunk, chunks)
+  int *d_bsrc = nullptr;             // [n] right-hand side index of each row
+  int *d_xdst = nullptr;             // [n] solution index, ~index for a row solved last
+  int *d_joined = nullptr, *d_border = nullptr;  // whether a chain has a parent; its border's rows
+  double *d_y = nullptr, *d_x = nullptr;  // [n] forward and backward solved values
+  double *d_wbuf = nullptr;          // [nchains][F] the sums that chains hand to their parents
+  double *d_part = nullptr;          // [nchunk]
+  int *d_sctl = nullptr;             // tickets, chain flags of both directions, finished chunks per last row
 };
 
-int xd_tree_upload(XdTree *t, const XdTreePlan &p);
+// p, q as in (P A Q)[i][j] = A[P[i]][Q[j]].
+int xd_tree_upload(XdTree *t, const XdTreePlan &plan, const int *p, const int *q);
 void xd_tree_free(XdTree *t);
 // Eliminates V (holding P A Q, zeros elsewhere) in place; kTreeInfo of d_ctl holds n - k for the first
 // zero pivot k (0: none), kTreeExpired is nonzero when a wait between chains gave up.
 constexpr int kTreeInfo = 0, kTreeExpired = 1, kTreeTicket = 2, kTreeFlags = 4;
 int xd_tree_factor(XdTree *t, cudaStream_t st);
+// Solves A x = b in place in d_x with V's factors. Stream-ordered.
+int xd_tree_solve(XdTree *t, double *d_x, cudaStream_t st);

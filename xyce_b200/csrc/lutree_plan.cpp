@@ -13,7 +13,7 @@ namespace {
 // / 3,000 / 10,000 / 30,000 / 100,000 updates: 106 / 95 / 99 / 120 / 183 us at 2.8k unknowns (74k
 // updates in all), 442 / 409 / 309 / 309 / 355 us at 41k (2M), 1.87 / 1.80 / 1.44 / 1.16 / 1.15 ms
 // at 200k (12.6M); a matrix with few updates has no use for tall subtrees.
-constexpr double kTopWork = 30000, kTopWorkSmall = 10000, kSmallMatrix = 300000;
+constexpr double kTopWork = 30000, kTopWorkSmall = 10000, kSmallMatrix = 300000, kNoPlan = 5000;
 constexpr int kTopHeight = 64;  // nor with more levels than this
 constexpr int kGroups = 296;  // two blocks per SM walk the bottom subtrees
 
@@ -93,6 +93,9 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
   double all = 0.0;
   for (int k = 0; k < n; ++k)
     if (parent[k] < 0) all += work[k];
+  // A few thousand updates in all: one block of level lists is as fast (1.1k unknowns, 2.2k updates:
+  // 58.6 + 42.2 us a refactorization and solve, 58.2 + 46.7 us over the plan).
+  if (all < kNoPlan) return false;
   const double top_work = all < kSmallMatrix ? kTopWorkSmall : kTopWork;
   for (int k = 0; k < n; ++k) {
     top[k] = work[k] > top_work || height[k] >= kTopHeight;
@@ -172,6 +175,8 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
   // to the end of its own block. slot[p]: the pivot's; sl[p]: those of struct(nodes[p]), aligned with it.
   std::vector<int> slot(t.ntop), where(n, -1);
   std::vector<std::vector<unsigned char>> sl(t.ntop);
+  std::vector<XdPos2> left;  // (slot, variable) of each chain's border
+  std::vector<int> left_ptr(1, 0);
   t.bptr.assign(1, 0);
   int frame = 0;
   for (int c = 0; c < t.nchains; ++c) {
@@ -213,7 +218,11 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
       }
       live.resize(kept);
     }
-    for (int j : live) where[j] = -1;
+    for (int j : live) {
+      left.push_back({where[j], j});
+      where[j] = -1;
+    }
+    left_ptr.push_back((int)left.size());
     t.bptr.push_back((int)t.blocks.size() / kBlockInts);
   }
   t.F = std::max(16, (frame + 15) / 16 * 16);
@@ -221,8 +230,8 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
   if (2.0 * t.F * t.ntop > 16.0 * nnz + 65536.0) return false;
   // Joins, at the start of the block that holds the child's parent pivot.
   t.jmap.assign((size_t)t.nchains * t.F, (unsigned char)kJoinNone);
+  auto block_of = [&](int p) { return t.bptr[chain_of[nodes[p]]] + (p - t.cptr[chain_of[nodes[p]]]) / kBlockPivots; };
   {
-    auto block_of = [&](int p) { return t.bptr[chain_of[nodes[p]]] + (p - t.cptr[chain_of[nodes[p]]]) / kBlockPivots; };
     const int nblocks = t.bptr[t.nchains];
     std::vector<int> jptr(nblocks + 1, 0);
     for (int c = 0; c < t.nchains; ++c)
@@ -254,6 +263,9 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
   // Positions in V.
   std::vector<int> place(n);
   for (int x = 0; x < n; ++x) place[t.order[x]] = x;
+  t.border.assign((size_t)t.nchains * t.F, -1);
+  for (int c = 0; c < t.nchains; ++c)
+    for (int x = left_ptr[c]; x < left_ptr[c + 1]; ++x) t.border[(size_t)c * t.F + left[x].x] = place[left[x].y];
   auto panel_slot = [&](int k, int j) {  // slot of j at pivot k, or -1 outside its front
     if (j == k) return slot[panel[k]];
     const size_t y = std::lower_bound(st[k].begin(), st[k].end(), j) - st[k].begin();
@@ -261,33 +273,86 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
   };
   t.pos.assign(nnz, -1);
   t.diag.assign(n, -1);
-  t.lptr.assign(1, 0);
-  t.uptr.assign(1, 0);
   const int *pi = mi.data();
-  std::vector<int> uent;  // M entries of the upper region in order
+  auto in_panel = [&](int i, int j) {
+    const int k = std::min(i, j);
+    return top[k] && panel_slot(k, std::max(i, j)) >= 0;
+  };
+  // Bottom rows' entries by pass: rows of a level by length, so that a pass's rows take about as many
+  // rounds; lanes a power of two near the rows' lengths, more where few rows are left.
+  auto build_passes = [&](XdPasses &ps, int off, bool upper) {
+    ps.gptr.assign(1, 0);
+    std::vector<std::vector<int>> ents(t.nbot);
+    for (int x = 0; x < t.nbot; ++x) {
+      const int i = t.order[x];
+      if (upper && last[i]) continue;
+      const int b = upper ? mdiag[i] + 1 : mp[i], e = upper ? mp[i + 1] : mdiag[i];
+      for (int k = b; k < e; ++k)
+        if (upper || !in_panel(i, pi[k])) ents[x].push_back(k);
+    }
+    for (int g = 0; g < t.ngroups; ++g) {
+      for (int s = 0; s < t.glev[g + 1] - t.glev[g]; ++s) {
+        const int l = upper ? t.glev[g + 1] - 1 - s : t.glev[g] + s;
+        std::vector<int> rows;
+        for (int x = t.lrow[l]; x < t.lrow[l + 1]; ++x)
+          if (upper ? !last[t.order[x]] : !ents[x].empty()) rows.push_back(x);
+        std::stable_sort(rows.begin(), rows.end(), [&](int a, int b) { return ents[a].size() < ents[b].size(); });
+        for (size_t r = 0; r < rows.size();) {
+          int lg = 0;
+          while (lg < 5 && (1u << lg) < ents[rows[r]].size()) ++lg;
+          size_t count = std::min(rows.size() - r, (size_t)(kPassThreads >> lg));
+          size_t most = ents[rows[r + count - 1]].size();
+          while (lg < 5 && most > (1u << lg) && (count << (lg + 1)) <= (size_t)kPassThreads) ++lg;
+          const int lanes = 1 << lg, rounds = std::max(1, (int)((most + lanes - 1) / lanes)), width = (int)count * lanes;
+          const bool end = r + count == rows.size();
+          ps.pass.push_back({(int)ps.rows.size(), (int)count | lg << 16 | (int)end << 24, off + (int)ps.col.size(), rounds});
+          const int base = (int)ps.col.size();
+          ps.col.resize(ps.col.size() + (size_t)rounds * width, -1);
+          for (size_t y = 0; y < count; ++y) {
+            const int x = rows[r + y];
+            ps.rows.push_back(x);
+            for (size_t z = 0; z < ents[x].size(); ++z) {
+              const int at = base + (int)(z / lanes) * width + (int)y * lanes + (int)(z % lanes);
+              ps.col[at] = place[pi[ents[x][z]]];
+              t.pos[ents[x][z]] = off + at;
+            }
+          }
+          r += count;
+        }
+      }
+      ps.gptr.push_back((int)ps.pass.size());
+    }
+    return off + (int)ps.col.size();
+  };
+  t.l0 = build_passes(t.fwd, 0, false);
+  t.lptr.assign(1, 0);
+  for (int x = t.nbot; x < n; ++x) {
+    const int i = t.order[x];
+    for (int e = mp[i]; e < mdiag[i]; ++e)
+      if (!in_panel(i, pi[e])) {
+        t.pos[e] = t.l0 + (int)t.lcol.size();
+        t.lcol.push_back(place[pi[e]]);
+      }
+    t.lptr.push_back((int)t.lcol.size());
+  }
+  t.u0 = t.l0 + (int)t.lcol.size();
+  t.t0 = build_passes(t.bwd, t.u0, true);
+  t.tptr.assign(1, 0);
   for (int x = 0; x < n; ++x) {
     const int i = t.order[x];
-    for (int e = mp[i]; e < mp[i + 1]; ++e) {
-      const int j = pi[e], k = std::min(i, j);
-      if (top[k] && panel_slot(k, std::max(i, j)) >= 0) continue;
-      if (j < i) {
-        t.pos[e] = (int)t.lcol.size();
-        t.lcol.push_back(place[j]);
-      } else if (j > i) {
-        uent.push_back(e);
-        t.ucol.push_back(place[j]);
+    if (!last[i]) continue;
+    t.tail.push_back(x);
+    for (int e = mdiag[i] + 1; e < mp[i + 1]; ++e)
+      if (!in_panel(i, pi[e])) {
+        t.pos[e] = t.t0 + (int)t.tcol.size();
+        t.tcol.push_back(place[pi[e]]);
       }
-    }
-    t.lptr.push_back((int)t.lcol.size());
-    t.uptr.push_back((int)t.ucol.size());
-    if (last[i]) t.tail.push_back(x);
+    t.tptr.push_back((int)t.tcol.size());
   }
-  t.u0 = (int)t.lcol.size();
-  t.d0 = t.u0 + (int)t.ucol.size();
+  t.d0 = t.t0 + (int)t.tcol.size();
   t.p0 = (t.d0 + t.nbot + 15) / 16 * 16;  // panels start on 128 bytes
-  t.nv = (long long)t.p0 + 2LL * t.F * t.ntop;
+  t.nv = (long long)t.p0 + xd_panel_size(t.F) * t.bptr[t.nchains];
   if (t.nv > INT_MAX) return false;
-  for (size_t x = 0; x < uent.size(); ++x) t.pos[uent[x]] = t.u0 + (int)x;
   for (int i = 0; i < n; ++i) {
     for (int e = mp[i]; e < mp[i + 1]; ++e) {
       if (t.pos[e] >= 0) continue;
@@ -296,7 +361,9 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
         t.pos[e] = t.d0 + place[i];
       } else {
         const int k = std::min(i, j), s = panel_slot(k, std::max(i, j));
-        t.pos[e] = t.p0 + 2 * t.F * panel[k] + (j >= i ? 0 : t.F) + s;
+        if (!top[k] || s < 0) return false;
+        const int p = panel[k], row = (p - t.cptr[chain_of[k]]) % kBlockPivots + (j >= i ? 0 : kBlockPivots);
+        t.pos[e] = t.p0 + (int)xd_panel_size(t.F) * block_of(p) + row * t.F + s;
       }
     }
     t.diag[i] = t.pos[mdiag[i]];

@@ -24,7 +24,7 @@ struct xd_rf {
   int *d_rowptr = nullptr, *d_colind = nullptr, *d_p = nullptr, *d_q = nullptr;
   double *d_temp = nullptr;
   XdLu lu;        // the refactorization
-  XdSptrsv tri;   // the triangular solves, over lu's bundled factors
+  XdSptrsv tri;   // the triangular solves over lu's bundled factors, where lu has no tree plan
   // The comparison library, created on first use from host copies of the set-up inputs.
   cusolverRfHandle_t h = nullptr;
   std::vector<int> ra, ca, rl, cl, ru, cu, hp, hq;
@@ -123,7 +123,7 @@ int xd_rf_create(int n, int nnz_a, const int *rowptr_a, const int *colind_a, con
     release(r);
     return rc;
   }
-  rc = xd_sptrsv_init(&r->tri, n, r->lu.nnz, r->lu.d_mp, r->lu.d_mi, p, q);
+  rc = xd_sptrsv_init(&r->tri, n, r->lu.nnz, r->lu.d_mp, r->lu.d_mi, p, q, r->lu.tree.on);
   if (rc != 0) {
     release(r);
     return rc;
@@ -164,7 +164,7 @@ int xd_rf_refactor(xd_rf *r, const double *d_vals_a) {
 int xd_rf_solve(xd_rf *r, double *d_x) {
   if (!r || !d_x) return xd_internal_fail(-1, "null refactorization argument");
   cudaSetDevice(r->device);
-  return xd_sptrsv_solve(&r->tri, r->lu.d_mx, d_x, 0);
+  return r->lu.tree.on ? xd_tree_solve(&r->lu.tree, d_x, 0) : xd_sptrsv_solve(&r->tri, r->lu.d_mx, d_x, 0);
 }
 
 int xd_rf_levels(const xd_rf *r, int *levels_l, int *levels_u) {
@@ -185,9 +185,7 @@ int xd_rf_stats(const xd_rf *r, int *nnz_factors, int *elimination_levels, long 
 int xd_rf_copy_factors(const xd_rf *r, double *h_vals) {
   if (!r || !h_vals) return xd_internal_fail(-1, "null argument");
   cudaSetDevice(r->device);
-  cudaError_t e = cudaMemcpy(h_vals, r->lu.d_mx, sizeof(double) * r->lu.nnz, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cu_fail(e, "xd_rf_copy_factors");
-  return 0;
+  return xd_lu_copy(const_cast<XdLu *>(&r->lu), h_vals);
 }
 
 }  // extern "C"

@@ -1,5 +1,6 @@
 // Forward and back substitution with the refactorization's factors (P A Q = L U, bundled by the
-// refactorization library as one CSR matrix M = L - I + U in the permuted index space).
+// refactorization library as one CSR matrix M = L - I + U in the permuted index space), for the
+// matrices that the elimination-tree plan (lutree.h) does not fit.
 //
 // Circuit factors are deep and narrow: the 200k-unknown placed netlist's L and U have 2,300-4,100
 // dependency levels each, a few dozen rows per level (plus one level of ~85k independent rows in
@@ -345,8 +346,9 @@ struct HostTri {
   int nlev = 0;            // dependency levels
 };
 
-void build_tri(int n, const std::vector<int> &mp, const std::vector<int> &mi, bool upper, HostTri &h) {
-  std::vector<int> lev(n, 0);
+// Dependency level of every row of a triangle; returns the number of levels.
+int row_levels(int n, const std::vector<int> &mp, const std::vector<int> &mi, bool upper, std::vector<int> &lev) {
+  lev.assign(n, 0);
   int nlev = 0;
   for (int t = 0; t < n; ++t) {
     const int r = upper ? n - 1 - t : t;
@@ -358,6 +360,12 @@ void build_tri(int n, const std::vector<int> &mp, const std::vector<int> &mi, bo
     lev[r] = d;
     nlev = std::max(nlev, d + 1);
   }
+  return nlev;
+}
+
+void build_tri(int n, const std::vector<int> &mp, const std::vector<int> &mi, bool upper, HostTri &h) {
+  std::vector<int> lev;
+  const int nlev = row_levels(n, mp, mi, upper, lev);
   // Buckets (level, length class): within a level the rows of at most kShortRow entries first, then
   // the longer ones, the rows longer than kBlockRow entries last.
   auto len = [&](int r) {
@@ -448,7 +456,8 @@ int upload(T **d, const std::vector<T> &h) {
 
 }  // namespace
 
-int xd_sptrsv_init(XdSptrsv *s, int n, int nnz_m, const int *d_mp, const int *d_mi, const int *p, const int *q) {
+int xd_sptrsv_init(XdSptrsv *s, int n, int nnz_m, const int *d_mp, const int *d_mi, const int *p, const int *q,
+                   bool levels_only) {
   std::vector<int> mp(n + 1), mi(std::max(1, nnz_m));
   cudaError_t e;
   if ((e = cudaMemcpy(mp.data(), d_mp, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost)) != cudaSuccess ||
@@ -459,6 +468,12 @@ int xd_sptrsv_init(XdSptrsv *s, int n, int nnz_m, const int *d_mp, const int *d_
     if (mp[r + 1] < mp[r]) return xd_internal_fail(-4, "unexpected bundled factor pattern");
   for (int k = 0; k < nnz_m; ++k)
     if (mi[k] < 0 || mi[k] >= n) return xd_internal_fail(-4, "unexpected bundled factor pattern");
+  if (levels_only) {
+    std::vector<int> lev;
+    s->n = n;
+    for (int u = 0; u < 2; ++u) s->nlev[u] = row_levels(n, mp, mi, u == 1, lev);
+    return 0;
+  }
   HostTri lo, up;
   build_tri(n, mp, mi, false, lo);
   build_tri(n, mp, mi, true, up);

@@ -25,8 +25,10 @@ struct XdSptrsv {
 };
 
 // Level order from the pattern of M = L - I + U (device CSR, read once to the host); p, q (host)
-// as in the refactorization: (P A Q)[i][j] = A[P[i]][Q[j]].
-int xd_sptrsv_init(XdSptrsv *s, int n, int nnz_m, const int *d_mp, const int *d_mi, const int *p, const int *q);
+// as in the refactorization: (P A Q)[i][j] = A[P[i]][Q[j]]. levels_only: only counts the triangles'
+// dependency levels (nlev), for factors that are solved otherwise.
+int xd_sptrsv_init(XdSptrsv *s, int n, int nnz_m, const int *d_mp, const int *d_mi, const int *p, const int *q,
+                   bool levels_only);
 void xd_sptrsv_free(XdSptrsv *s);
 // Solves A x = b in place in d_x with the current values d_mx of M (the pattern given to
 // xd_sptrsv_init). Stream-ordered.
