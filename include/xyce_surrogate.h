@@ -107,6 +107,29 @@ typedef struct xd_adam_args {
 int xd_adam(int rows, int cols, float *d_p, const float *d_grad, float *d_m, float *d_v, const xd_adam_args *a,
             void *d_p16, void *d_p16t, int ld16, int ld16t, void *stream);
 
+/* One whole training step of the surrogate network (5 layers: n_in -> 128 x 4 -> 16 padded outputs):
+ * forward, mean-squared-error gradient, backward and Adam, in two launches. The samples go through
+ * in tiles of 128 rows, the last one partly empty; results equal the layer-by-layer calls above up
+ * to the order of the FP32 sums over the batch. Arrays of layers 1..5 (index 0..4): master weights w
+ * ([128 x ldw1], 3 x [128 x 128], [16 x 128]) and biases b, their gradients gw, gb and moments mw, vw,
+ * mb, vb (FP32, in the weights' layouts), the weights' BF16 copies w16 and transposes w16t. z:
+ * scratch for the hidden layers' pre-activations, BF16 [rows rounded up to 128 x 128] each. x
+ * [n x ldx], t [n x n_out]; y [n x 16] receives the outputs, sq [n] the samples' squared errors. part:
+ * scratch of xd_mlp_train_part_size x its block count floats. 16-byte aligned w16, z, y and part. */
+typedef struct xd_mlp_train_args {
+  int n, n_in, n_out, ldx, ldw1;
+  float scale; /* of the output gradient: scale * (y - t) */
+  const float *x, *t;
+  float *w[5], *b[5], *gw[5], *gb[5], *mw[5], *vw[5], *mb[5], *vb[5];
+  void *w16[5], *w16t[5], *z[4];
+  float *y, *sq, *part;
+  int *err; /* device flag, set to 1 if an internal wait expired */
+  xd_adam_args adam;
+} xd_mlp_train_args;
+/* Floats per block of the step's scratch, and its blocks for n samples. */
+int xd_mlp_train_part_size(int n, int *blocks);
+int xd_mlp_train_step(const xd_mlp_train_args *args, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

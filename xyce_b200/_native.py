@@ -71,6 +71,16 @@ class XdAdamArgs(ctypes.Structure):
                 ("bias_corr1", ctypes.c_float), ("bias_corr2", ctypes.c_float)]
 
 
+class XdMlpTrainArgs(ctypes.Structure):
+    """Mirror of ``xd_mlp_train_args``."""
+
+    _fields_ = ([(k, ctypes.c_int) for k in ("n", "n_in", "n_out", "ldx", "ldw1")] + [("scale", ctypes.c_float)] +
+                [(k, ctypes.c_void_p) for k in ("x", "t")] +
+                [(k, ctypes.c_void_p * 5) for k in ("w", "b", "gw", "gb", "mw", "vw", "mb", "vb", "w16", "w16t")] +
+                [("z", ctypes.c_void_p * 4)] + [(k, ctypes.c_void_p) for k in ("y", "sq", "part", "err")] +
+                [("adam", XdAdamArgs)])
+
+
 # Every symbol the headers declare, with its ctypes signature.
 XD_DENSE_MAX_N = 160  # include/xyce_tia.h
 
@@ -162,6 +172,8 @@ SIGNATURES = {
     "xd_splitk_sum": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
     "xd_column_sum": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p,
                                      ctypes.c_void_p]),
+    "xd_mlp_train_part_size": (ctypes.c_int, [ctypes.c_int, _ip]),
+    "xd_mlp_train_step": (ctypes.c_int, [ctypes.POINTER(XdMlpTrainArgs), ctypes.c_void_p]),
     "xd_adam": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                ctypes.c_void_p, ctypes.POINTER(XdAdamArgs), ctypes.c_void_p, ctypes.c_void_p,
                                ctypes.c_int, ctypes.c_int, ctypes.c_void_p]),

@@ -620,6 +620,415 @@ __global__ void __launch_bounds__(kFusedThreads, 1) mlp_forward_fused_kernel(xd_
   if (warp == 0) tmem_free(tmem, kHid);
 }
 
+// ---- fused training step ------------------------------------------------------------------------
+// One 128-sample tile at a time through the whole network and back in one kernel: the activations
+// of the four hidden layers stay in shared memory (a layer's is overwritten by its gradient once
+// the next layer's weight gradient has read it), the weights pass through two buffers, and the
+// weight gradients of the three 128 x 128 layers accumulate in tensor memory over the block's tiles.
+// Every product runs from the same row-major tiles: a weight gradient dZ^T H and a backward product
+// dZ W read them as MN-major operands, so nothing is transposed. Pre-activations go through global
+// memory (BF16, as the layer-by-layer path rounds them). A second kernel sums the blocks' partial
+// gradients in block order and applies Adam. The layer-by-layer path is ~60 launches and writes and
+// reads every activation and its transpose: a step on 16,384 samples takes 929 us that way, 98 us
+// fused (with the copies of the batch; 5 GFLOP, so either is bound by latencies: a tile's eight
+// layer steps follow one another).
+
+constexpr int kTileBytes = kHid * kHid * 2;
+constexpr int kPartW5 = 3 * kHid * kHid;                 // partials: W2..W4, W5 (transposed), W1, biases
+constexpr int kPartW1 = kPartW5 + kHid * kOutPad;
+constexpr int kPartB = kPartW1 + kHid * 8;
+constexpr int kPartSize = kPartB + 4 * kHid + kOutPad;
+
+struct TrainSmem {
+  unsigned char h[4][kTileBytes];        // activations, then gradients, of the hidden layers
+  unsigned char w[2][kTileBytes];        // W2 / W4, W3
+  unsigned char w5[kOutPad * kHid * 2];
+  unsigned char dy[kTileM * kOutPad * 2];  // output gradient, 8 x 8 core matrices, row groups 256 B apart
+  float w1[kHid * 8];
+  float b[4 * kHid + kOutPad];
+  float x[kTileM * 8];
+  uint64_t bar;
+  uint32_t tmem;
+};
+static_assert(sizeof(TrainSmem) <= 227 * 1024, "one block's shared memory");
+
+// MN-major operand flags of the instruction descriptor (A: bit 15, B: bit 16).
+constexpr uint32_t kMnA = 1u << 15, kMnB = 1u << 16;
+
+__device__ __forceinline__ void stage_weights(unsigned char *dst, const void *src, int tid) {
+  const __nv_bfloat16 *W = static_cast<const __nv_bfloat16 *>(src);
+  for (int i = tid; i < kHid * 16; i += kFusedThreads) {
+    const int r = i >> 4, kc = i & 15;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + off128(r, kc))),
+                 "l"(W + (size_t)r * kHid + kc * 8)
+                 : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// Sums over the tile's rows of a gradient tile's columns, each row times its weight: warp w takes
+// rows 16 w .. 16 w + 15, lane i & 7 one row of each group of eight; per 8-column group the eight lanes' sums
+// are exchanged so that each lane keeps one column. acc[k]: column (4 k + lane / 8) * 8 + col(lane).
+__device__ __forceinline__ void column_sums(const unsigned char *tile, float w0, float w1, int warp, int lane,
+                                            float (&acc)[4]) {
+  const int i = lane & 7, q = lane >> 3;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int kc = 4 * k + q;
+    float s[8];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(tile + (2 * warp + c) * 2048 + kc * 128 + i * 16);
+      const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
+      const float w = c ? w1 : w0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(h[j]);
+        s[2 * j] = c ? s[2 * j] + w * f.x : w * f.x;
+        s[2 * j + 1] = c ? s[2 * j + 1] + w * f.y : w * f.y;
+      }
+    }
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1) {
+      const bool up = i & h;
+#pragma unroll
+      for (int j = 0; j < h; ++j) {
+        const float keep = up ? s[j + h] : s[j], give = up ? s[j] : s[j + h];
+        s[j] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+      }
+    }
+    acc[k] += s[0];
+  }
+}
+__device__ __forceinline__ int column_of(int k, int lane) { return (4 * k + (lane >> 3)) * 8 + (lane & 7); }
+
+__global__ void __launch_bounds__(kFusedThreads, 1) mlp_train_kernel(xd_mlp_train_args a, int tiles) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  TrainSmem &S = *reinterpret_cast<TrainSmem *>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  stage_weights(S.w[0], a.w16[1], tid);
+  stage_weights(S.w[1], a.w16[2], tid);
+  {
+    const __nv_bfloat16 *W = static_cast<const __nv_bfloat16 *>(a.w16[4]);
+    for (int i = tid; i < kOutPad * 16; i += kFusedThreads) {
+      const int r = i >> 4, kc = i & 15;
+      *reinterpret_cast<uint4 *>(S.w5 + off128(r, kc)) = *reinterpret_cast<const uint4 *>(W + (size_t)r * kHid + kc * 8);
+    }
+  }
+  for (int i = tid; i < kHid * 8; i += kFusedThreads) S.w1[i] = i % 8 < a.n_in ? a.w[0][(i / 8) * a.ldw1 + i % 8] : 0.0f;
+  for (int i = tid; i < 4 * kHid + kOutPad; i += kFusedThreads) {
+    const int l = i / kHid, u = i % kHid;
+    S.b[i] = l < 4 ? a.b[l][u] : a.b[4][i - 4 * kHid];
+  }
+  if (warp == 0) tmem_alloc(&S.tmem, 512);
+  if (tid == 0) {
+    mbar_init(&S.bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = S.tmem;
+  const int quarter = warp & 3, half = warp >> 2, row = quarter * 32 + lane;
+  const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
+  uint32_t phase = 0;
+  bool ok = true;
+  float gb[4][4] = {}, gw1[5][4] = {}, gb5 = 0.0f, g5[8] = {};  // sums over the block's tiles
+  float gwx[3][4] = {};                                         // first-layer inputs 6 to 8
+  // Everything written to shared memory is visible to the tensor core and the last reads of tensor
+  // memory are done; one thread issues, all wait.
+  auto begin = [&]() {
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+  };
+  auto finish = [&]() {
+    ok = __syncthreads_and(mbar_wait(&S.bar, phase)) != 0;
+    phase ^= 1u;
+    tc_fence_after();
+  };
+  // D[128 x N] (+)= A B over `steps` K steps of 16; an operand advances sa / sb bytes per step.
+  auto product = [&](uint32_t d, uint32_t A, uint32_t la, uint32_t ssa, uint32_t sa, uint32_t B, uint32_t lb, uint32_t ssb,
+                     uint32_t sb, uint32_t idesc, int steps, bool add) {
+    for (int s = 0; s < steps; ++s)
+      mma_bf16(tmem + d, smem_desc(A + s * sa, la, ssa), smem_desc(B + s * sb, lb, ssb), idesc, add || s > 0 ? 1u : 0u);
+  };
+  const uint32_t kFwd = instr_desc_bf16(kTileM, kHid), kOut = instr_desc_bf16(kTileM, kOutPad);
+  bool first = true;
+  for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, first = false) {
+    const int g = tile * kTileM + row;
+    for (int i = tid; i < kTileM * 8; i += kFusedThreads) {
+      const int r = tile * kTileM + i / 8;
+      S.x[i] = i % 8 < a.n_in && r < a.n ? a.x[(size_t)r * a.ldx + i % 8] : 0.0f;
+    }
+    __syncthreads();
+    // Layer 1 on the CUDA cores (FP32).
+    {
+      float xi[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) xi[i] = S.x[row * 8 + i];
+      __nv_bfloat16 *Z = static_cast<__nv_bfloat16 *>(a.z[0]) + (size_t)g * kHid;
+      for (int c8 = 0; c8 < 8; ++c8) {
+        __align__(16) __nv_bfloat16 z8[8], h8[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int u = half * 64 + c8 * 8 + j;
+          float z = S.b[u];
+          for (int i = 0; i < a.n_in; ++i) z += S.w1[u * 8 + i] * xi[i];
+          z8[j] = __float2bfloat16(z);
+          h8[j] = __float2bfloat16(silu(z));
+        }
+        *reinterpret_cast<uint4 *>(S.h[0] + off128(row, half * 8 + c8)) = *reinterpret_cast<uint4 *>(h8);
+        *reinterpret_cast<uint4 *>(Z + half * 64 + c8 * 8) = *reinterpret_cast<uint4 *>(z8);
+      }
+    }
+    // Layers 2..4: W2 in buffer 0, W3 in buffer 1, then W4 in buffer 0.
+    for (int l = 1; l < 4 && ok; ++l) {
+      if (l == 3) asm volatile("cp.async.wait_group 0;" ::: "memory");
+      begin();
+      if (tid == 0) {
+        product(0, smem_u32(S.h[l - 1]), 128, 2048, 256, smem_u32(S.w[(l - 1) & 1]), 128, 2048, 256, kFwd, 8, false);
+        mma_commit(&S.bar);
+      }
+      finish();
+      if (!ok) break;
+      if (l == 1) stage_weights(S.w[0], a.w16[3], tid);
+      __nv_bfloat16 *Z = static_cast<__nv_bfloat16 *>(a.z[l]) + (size_t)g * kHid;
+#pragma unroll
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        float v[32];
+        tmem_ld32(lane_base + half * 64 + c0, v);
+#pragma unroll
+        for (int c8 = 0; c8 < 4; ++c8) {
+          __align__(16) __nv_bfloat16 z8[8], h8[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float z = v[c8 * 8 + j] + S.b[l * kHid + half * 64 + c0 + c8 * 8 + j];
+            z8[j] = __float2bfloat16(z);
+            h8[j] = __float2bfloat16(silu(z));
+          }
+          const int kc = (half * 64 + c0) / 8 + c8;
+          *reinterpret_cast<uint4 *>(S.h[l] + off128(row, kc)) = *reinterpret_cast<uint4 *>(h8);
+          *reinterpret_cast<uint4 *>(Z + kc * 8) = *reinterpret_cast<uint4 *>(z8);
+        }
+      }
+    }
+    if (!ok) break;
+    // Output layer, squared error and its gradient.
+    begin();
+    if (tid == 0) {
+      product(0, smem_u32(S.h[3]), 128, 2048, 256, smem_u32(S.w5), 128, 2048, 256, kOut, 8, false);
+      mma_commit(&S.bar);
+    }
+    finish();
+    if (!ok) break;
+    if (half == 0) {
+      float v[16];
+      tmem_ld16(lane_base, v);
+      float sq = 0.0f, d[16];
+      __align__(16) __nv_bfloat16 d8[16];
+#pragma unroll
+      for (int j = 0; j < kOutPad; ++j) {
+        v[j] += S.b[4 * kHid + j];
+        d[j] = 0.0f;
+        if (j < a.n_out && g < a.n) {
+          const float e = v[j] - a.t[(size_t)g * a.n_out + j];
+          sq += e * e;
+          d[j] = a.scale * e;
+        }
+        d8[j] = __float2bfloat16(d[j]);
+        d[j] = __bfloat162float(d8[j]);
+      }
+      *reinterpret_cast<uint4 *>(S.dy + (row >> 3) * 256 + (row & 7) * 16) = *reinterpret_cast<uint4 *>(d8);
+      *reinterpret_cast<uint4 *>(S.dy + (row >> 3) * 256 + 128 + (row & 7) * 16) = *reinterpret_cast<uint4 *>(d8 + 8);
+      if (g < a.n) {
+        a.sq[g] = sq;
+#pragma unroll
+        for (int j = 0; j < kOutPad; j += 4)
+          *reinterpret_cast<float4 *>(a.y + (size_t)g * kOutPad + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+      }
+      // Sixteen sums over 32 lanes: lane keeps output (lane / 2 with its bits as exchanged).
+#pragma unroll
+      for (int h = 8; h > 0; h >>= 1) {
+        const bool up = lane & (2 * h);
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+          const float keep = up ? d[j + h] : d[j], give = up ? d[j] : d[j + h];
+          d[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+        }
+      }
+      gb5 += d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);
+    }
+    // W5's gradient, transposed: H4^T dY, 128 x 16, added up in registers.
+    begin();
+    if (tid == 0) {
+      product(0, smem_u32(S.h[3]), 2048, 128, 4096, smem_u32(S.dy), 256, 128, 512, kOut | kMnA | kMnB, 8, false);
+      mma_commit(&S.bar);
+    }
+    finish();
+    if (!ok) break;
+    {
+      float v[16];
+      tmem_ld16(lane_base, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g5[j] += half ? v[j + 8] : v[j];
+    }
+    // Backward through layers 4..1: dH_l = dZ_{l+1} W_{l+1} (and layer l + 1's weight gradient beside it),
+    // dZ_l = dH_l silu'(z_l) in the place of H_l.
+    for (int l = 3; l >= 0 && ok; --l) {
+      if (l == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
+      begin();
+      if (tid == 0) {
+        if (l == 3) {
+          product(0, smem_u32(S.dy), 128, 256, 256, smem_u32(S.w5), 2048, 128, 4096, kFwd | kMnB, 1, false);
+        } else {
+          product(0, smem_u32(S.h[l + 1]), 128, 2048, 256, smem_u32(S.w[l & 1]), 2048, 128, 4096, kFwd | kMnB, 8, false);
+          product(128 + l * 128, smem_u32(S.h[l + 1]), 2048, 128, 4096, smem_u32(S.h[l]), 2048, 128, 4096,
+                  kFwd | kMnA | kMnB, 8, !first);
+        }
+        mma_commit(&S.bar);
+      }
+      // Meanwhile: this thread's pre-activations, and the column sums of layer l + 1's gradient.
+      uint4 zq[8];
+      const uint4 *Z = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(a.z[l]) + (size_t)g * kHid +
+                                                       half * 64);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) zq[i] = Z[i];
+      if (l < 3) column_sums(S.h[l + 1], 1.0f, 1.0f, warp, lane, gb[l + 1]);
+      finish();
+      if (!ok) break;
+      if (l == 2) stage_weights(S.w[0], a.w16[1], tid);  // W4 has been read: W2 for the last product and the next tile
+#pragma unroll
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        float v[32];
+        tmem_ld32(lane_base + half * 64 + c0, v);
+#pragma unroll
+        for (int c8 = 0; c8 < 4; ++c8) {
+          const __nv_bfloat16 *z8 = reinterpret_cast<const __nv_bfloat16 *>(&zq[c0 / 8 + c8]);
+          __align__(16) __nv_bfloat16 d8[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            d8[j] = __float2bfloat16(v[c8 * 8 + j] * silu_grad(__bfloat162float(z8[j])));
+          *reinterpret_cast<uint4 *>(S.h[l] + off128(row, (half * 64 + c0) / 8 + c8)) = *reinterpret_cast<uint4 *>(d8);
+        }
+      }
+    }
+    if (!ok) break;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    column_sums(S.h[0], 1.0f, 1.0f, warp, lane, gb[0]);
+    const float *x0 = S.x + (16 * warp + (lane & 7)) * 8, *x1 = x0 + 64;
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+      if (i < a.n_in) column_sums(S.h[0], x0[i], x1[i], warp, lane, gw1[i]);
+#pragma unroll
+    for (int i = 5; i < 8; ++i)
+      if (i < a.n_in) column_sums(S.h[0], x0[i], x1[i], warp, lane, gwx[i - 5]);
+    __syncthreads();
+  }
+  if (!ok) {
+    if (tid == 0) atomicExch(a.err, 1);
+    mbar_wait(&S.bar, phase ^ 1u);
+  } else {
+    // The block's partial gradients.
+    float *P = a.part + (size_t)blockIdx.x * kPartSize;
+    for (int l = 0; l < 3; ++l)
+#pragma unroll
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        float v[32];
+        tmem_ld32(lane_base + 128 + l * 128 + half * 64 + c0, v);
+        float4 *to = reinterpret_cast<float4 *>(P + l * kHid * kHid + row * kHid + half * 64 + c0);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) to[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) P[kPartW5 + row * kOutPad + half * 8 + j] = g5[j];
+    // Across the warps, in order, through shared memory (the activations' place).
+    float *red = reinterpret_cast<float *>(S.h[0]);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = column_of(k, lane);
+#pragma unroll
+      for (int l = 0; l < 4; ++l) red[(warp * 12 + l) * kHid + c] = gb[l][k];
+#pragma unroll
+      for (int i = 0; i < 5; ++i) red[(warp * 12 + 4 + i) * kHid + c] = gw1[i][k];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) red[(warp * 12 + 9 + i) * kHid + c] = gwx[i][k];
+    }
+    float *red5 = red + 8 * 12 * kHid;
+    if (half == 0 && (lane & 1) == 0) red5[warp * kOutPad + (lane >> 1)] = gb5;
+    __syncthreads();
+    for (int i = tid; i < 12 * kHid; i += kFusedThreads) {
+      float s = 0.0f;
+      for (int w = 0; w < 8; ++w) s += red[w * 12 * kHid + i];
+      const int q = i / kHid, c = i % kHid;
+      if (q < 4)
+        P[kPartB + q * kHid + c] = s;
+      else
+        P[kPartW1 + c * 8 + q - 4] = s;
+    }
+    if (tid < kOutPad) {
+      float s = 0.0f;
+      for (int w = 0; w < 4; ++w) s += red5[w * kOutPad + tid];
+      P[kPartB + 4 * kHid + tid] = s;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 0) tmem_free(tmem, 512);
+}
+
+// Adds the blocks' partial gradients in block order and applies Adam, one thread per parameter; the
+// padding (inputs from n_in, outputs from n_out on) stays zero.
+__global__ void __launch_bounds__(256) mlp_apply_kernel(xd_mlp_train_args a, int blocks) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= kPartSize) return;
+  float gr = 0.0f;
+#pragma unroll 8
+  for (int k = 0; k < blocks; ++k) gr += a.part[(size_t)k * kPartSize + i];
+  int l, r, c = 0;
+  bool bias = false, pad = false;
+  if (i < kPartW5) {
+    l = 1 + i / (kHid * kHid);
+    r = i / kHid % kHid;
+    c = i % kHid;
+  } else if (i < kPartW1) {
+    l = 4;
+    r = (i - kPartW5) % kOutPad;
+    c = (i - kPartW5) / kOutPad;
+    pad = r >= a.n_out;
+  } else if (i < kPartB) {
+    l = 0;
+    r = (i - kPartW1) / 8;
+    c = (i - kPartW1) % 8;
+    if (c >= a.n_in) return;
+  } else {
+    bias = true;
+    l = min((i - kPartB) / kHid, 4);
+    r = i - kPartB - l * kHid;
+    pad = l == 4 && r >= a.n_out;
+  }
+  if (pad) gr = 0.0f;
+  const int ld = l == 0 ? a.ldw1 : kHid, at = bias ? r : r * ld + c;
+  float *p = bias ? a.b[l] : a.w[l], *m = bias ? a.mb[l] : a.mw[l], *v = bias ? a.vb[l] : a.vw[l];
+  (bias ? a.gb[l] : a.gw[l])[at] = gr;
+  const float mi = a.adam.beta1 * m[at] + (1.0f - a.adam.beta1) * gr;
+  const float vi = a.adam.beta2 * v[at] + (1.0f - a.adam.beta2) * gr * gr;
+  m[at] = mi;
+  v[at] = vi;
+  const float pi = pad ? 0.0f : p[at] - a.adam.lr * (mi / a.adam.bias_corr1) / (sqrtf(vi / a.adam.bias_corr2) + a.adam.eps);
+  p[at] = pi;
+  if (!bias) {
+    static_cast<__nv_bfloat16 *>(a.w16[l])[at] = __float2bfloat16(pi);
+    static_cast<__nv_bfloat16 *>(a.w16t[l])[(size_t)c * (l == 4 ? kOutPad : kHid) + r] = __float2bfloat16(pi);
+  }
+}
+
 int cuda_err(cudaError_t e, const char *where) {
   return xd_internal_fail(-3, std::string("CUDA error in ") + where + ": " + cudaGetErrorString(e));
 }
@@ -763,6 +1172,40 @@ int xd_adam(int rows, int cols, float *d_p, const float *d_grad, float *d_m, flo
       (__nv_bfloat16 *)d_p16, (__nv_bfloat16 *)d_p16t, ld16, ld16t);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_err(e, "adam_kernel");
+}
+
+int xd_mlp_train_part_size(int n, int *blocks) {
+  if (n <= 0 || !blocks) return xd_internal_fail(-1, "bad training-step arguments");
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int tiles = (n + kTileM - 1) / kTileM;
+  *blocks = tiles < sms ? tiles : sms;
+  return kPartSize;
+}
+
+int xd_mlp_train_step(const xd_mlp_train_args *a, void *stream) {
+  if (!a || a->n <= 0 || a->n_in < 1 || a->n_in > 8 || a->n_out < 1 || a->n_out > kOutPad || a->ldx < a->n_in ||
+      a->ldw1 < a->n_in || !a->x || !a->t || !a->y || !a->sq || !a->part || !a->err)
+    return xd_internal_fail(-1, "bad training-step arguments");
+  uintptr_t align = reinterpret_cast<uintptr_t>(a->y) | reinterpret_cast<uintptr_t>(a->part);
+  for (int l = 0; l < 5; ++l) {
+    if (!a->w[l] || !a->b[l] || !a->gw[l] || !a->gb[l] || !a->mw[l] || !a->vw[l] || !a->mb[l] || !a->vb[l] ||
+        !a->w16[l] || !a->w16t[l] || (l < 4 && !a->z[l]))
+      return xd_internal_fail(-1, "null training-step buffer");
+    align |= reinterpret_cast<uintptr_t>(a->w16[l]);
+    if (l < 4) align |= reinterpret_cast<uintptr_t>(a->z[l]);
+  }
+  if (align & 15) return xd_internal_fail(-1, "training-step buffers must be 16-byte aligned");
+  int blocks = 0;
+  xd_mlp_train_part_size(a->n, &blocks);
+  const size_t smem = sizeof(TrainSmem);
+  cudaError_t e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return cuda_err(e, "cudaFuncSetAttribute(mlp_train_kernel)");
+  cudaStream_t st = (cudaStream_t)stream;
+  mlp_train_kernel<<<blocks, kFusedThreads, smem, st>>>(*a, (a->n + kTileM - 1) / kTileM);
+  mlp_apply_kernel<<<(kPartSize + 255) / 256, 256, 0, st>>>(*a, blocks);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : cuda_err(e, "mlp_train_kernel");
 }
 
 }  // extern "C"

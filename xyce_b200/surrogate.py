@@ -155,6 +155,7 @@ class SurrogateMLP:
         self.sq = torch.zeros(B, **f32)
         self.T = torch.zeros(B, N_OUT, **f32)
         self.splits = 64
+        self._part = None
         self.part = torch.zeros(self.splits * N_HID * N_HID, **f32)
         self.gW = [torch.zeros_like(w) for w in self.W]
         self.gb = [torch.zeros_like(b) for b in self.b]
@@ -271,12 +272,33 @@ class SurrogateMLP:
     def train_step(self, X, T, cfg: AdamConfig):
         """One Adam step on a batch (X [n, 5], T [n, 10] in scaled space); returns the loss tensor."""
         torch = self.torch
-        n, Bp = self._load_inputs(X)
+        n, _ = self._load_inputs(X)
         self.T[:n] = torch.as_tensor(T, dtype=torch.float32, device=self.dev)
-        self._forward(Bp)
-        self.backward(n, Bp)
-        self.adam_step(cfg)
+        self.step_count += 1
+        t = self.step_count
+        a = self._train_args()
+        a.n, a.scale = n, 2.0 / (n * N_OUT)
+        a.adam = _native.XdAdamArgs(cfg.lr, cfg.beta1, cfg.beta2, cfg.eps, 1 - cfg.beta1 ** t, 1 - cfg.beta2 ** t)
+        _native.check(self.k.lib.xd_mlp_train_step(ctypes.byref(a), self.k.stream()), "xd_mlp_train_step")
         return self.sq[:n].mean() / N_OUT
+
+    def _train_args(self):
+        """The fused training step's argument record on this network's buffers as they are now."""
+        a = _native.XdMlpTrainArgs()
+        if self._part is None:  # scratch of the largest batch, kept until the batch buffers grow
+            blocks = ctypes.c_int()
+            with self.torch.cuda.device(self.dev):
+                size = self.k.lib.xd_mlp_train_part_size(self.max_batch, ctypes.byref(blocks))
+            self._part = self.torch.zeros(size * blocks.value, dtype=self.torch.float32, device=self.dev)
+        a.n_in, a.n_out, a.ldx, a.ldw1 = N_IN, N_OUT, PAD_IN, PAD_IN
+        a.x, a.t, a.y, a.sq = (v.data_ptr() for v in (self.X32, self.T, self.Y, self.sq))
+        a.part, a.err = self._part.data_ptr(), self.k.err.data_ptr()
+        for name, ts in (("w", self.W), ("b", self.b), ("gw", self.gW), ("gb", self.gb), ("mw", self.mW),
+                         ("vw", self.vW), ("mb", self.mb), ("vb", self.vb), ("w16", self.W16), ("w16t", self.W16T),
+                         ("z", self.Z)):
+            for l, v in enumerate(ts):
+                getattr(a, name)[l] = v.data_ptr()
+        return a
 
     def parameters_numpy(self):
         """(W, b) per layer as float64 arrays, unpadded: the FP32 first layer, the BF16 weights the
