@@ -487,137 +487,181 @@ __device__ __forceinline__ uint32_t off128(int r, int kc) {
   return (uint32_t)((r >> 3) * 2048 + kc * 128 + (r & 7) * 16);
 }
 
+// A block works on kFwdGroups tiles at a time, a group of kFusedThreads threads each with its own
+// activation tile, tensor-memory columns and barriers over the shared weights: one group's tensor-core
+// products and waits run under the other's epilogues, whose exponentials and reciprocals (two of the
+// 16-a-clock special-function operations per activation, 55 us for 250k samples on 148 SMs) are
+// the bound. 250k samples take 120 us, 1M 398 us (two groups: 131 and 459; one group, without the
+// next tile's inputs and the weights' copies in flight: 297 us and 1.85 ms).
+constexpr int kFwdGroups = 3;
 struct FusedSmem {
   unsigned char w[3][kHid * kHid * 2];   // hidden layers 2..4, [out][in] K-major
   unsigned char w5[kOutPad * kHid * 2];  // output layer, 16 x 128
-  unsigned char act[kHid * kHid * 2];    // activation tile (A operand), 128 x 128
+  unsigned char act[kFwdGroups][kHid * kHid * 2];  // activation tiles (A operands), 128 x 128
   float w1[kHid * 8];                    // first layer, FP32, 128 x n_in (n_in <= 8)
   float b[4 * kHid + kOutPad];           // biases of layers 1..5
-  uint64_t bar;
+  uint64_t bar[kFwdGroups];
   uint32_t tmem;
+  int failed[kFwdGroups];                // a wait of the group expired
 };
+static_assert(sizeof(FusedSmem) <= 227 * 1024, "one block's shared memory");
 
-__global__ void __launch_bounds__(kFusedThreads, 1) mlp_forward_fused_kernel(xd_mlp_net net, int n, const float *x,
-                                                                            int ldx, float *y, int ldy, int *err) {
+// First layer of eight hidden units from u on, on the CUDA cores (FP32, inputs added in order).
+template <int NIN>
+__device__ __forceinline__ void first_layer8(const float *w1, const float *b, const float (&xi)[8], int n_in, bool on,
+                                             __nv_bfloat16 (&h8)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float z = b[j];
+    float w[8];
+    *reinterpret_cast<float4 *>(w) = *reinterpret_cast<const float4 *>(w1 + j * 8);
+    *reinterpret_cast<float4 *>(w + 4) = *reinterpret_cast<const float4 *>(w1 + j * 8 + 4);
+    if constexpr (NIN > 0) {
+#pragma unroll
+      for (int i = 0; i < NIN; ++i) z += w[i] * xi[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < n_in) z += w[i] * xi[i];
+    }
+    h8[j] = __float2bfloat16(on ? silu(z) : 0.0f);
+  }
+}
+
+template <int NIN>
+__global__ void __launch_bounds__(kFwdGroups *kFusedThreads, 1) mlp_forward_fused_kernel(xd_mlp_net net, int n,
+                                                                                        const float *x, int ldx,
+                                                                                        float *y, int ldy, int *err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   FusedSmem &S = *reinterpret_cast<FusedSmem *>(smem_raw);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // Stage the weights once per CTA.
-  for (int l = 0; l < 3; ++l) {
-    const __nv_bfloat16 *W = static_cast<const __nv_bfloat16 *>(net.w[l]);
-    for (int i = tid; i < kHid * 16; i += kFusedThreads) {
+  constexpr int kAll = kFwdGroups * kFusedThreads;
+  const int group = threadIdx.x / kFusedThreads, tid = threadIdx.x % kFusedThreads, warp = tid >> 5, lane = tid & 31;
+  // Stage the weights once per CTA, under the first tiles' first layer.
+  auto stage = [&](unsigned char *dst, const void *src, int rows) {
+    const __nv_bfloat16 *W = static_cast<const __nv_bfloat16 *>(src);
+    for (int i = threadIdx.x; i < rows * 16; i += kAll) {
       const int r = i >> 4, kc = i & 15;
-      *reinterpret_cast<uint4 *>(S.w[l] + off128(r, kc)) =
-          *reinterpret_cast<const uint4 *>(W + (size_t)r * kHid + kc * 8);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + off128(r, kc))),
+                   "l"(W + (size_t)r * kHid + kc * 8)
+                   : "memory");
     }
-  }
-  {
-    const __nv_bfloat16 *W = static_cast<const __nv_bfloat16 *>(net.w5);
-    for (int i = tid; i < kOutPad * 16; i += kFusedThreads) {
-      const int r = i >> 4, kc = i & 15;
-      *reinterpret_cast<uint4 *>(S.w5 + off128(r, kc)) = *reinterpret_cast<const uint4 *>(W + (size_t)r * kHid + kc * 8);
-    }
-  }
-  for (int i = tid; i < kHid * net.n_in; i += kFusedThreads) S.w1[(i / net.n_in) * 8 + i % net.n_in] =
-      net.w1[(i / net.n_in) * net.ldw1 + i % net.n_in];
-  for (int i = tid; i < 4 * kHid + kOutPad; i += kFusedThreads) {
+  };
+  for (int l = 0; l < 3; ++l) stage(S.w[l], net.w[l], kHid);
+  stage(S.w5, net.w5, kOutPad);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int i = threadIdx.x; i < kHid * 8; i += kAll)
+    S.w1[i] = i % 8 < net.n_in ? net.w1[(i / 8) * net.ldw1 + i % 8] : 0.0f;
+  for (int i = threadIdx.x; i < 4 * kHid + kOutPad; i += kAll) {
     const int l = i / kHid, u = i % kHid;
     S.b[i] = (l < 4) ? net.b[l][u] : net.b[4][i - 4 * kHid];
   }
-  if (warp == 0) tmem_alloc(&S.tmem, kHid);
-  if (tid == 0) {
-    mbar_init(&S.bar, 1);
+  if (threadIdx.x < 32) tmem_alloc(&S.tmem, 512);
+  if (threadIdx.x < kFwdGroups) {
+    mbar_init(&S.bar[threadIdx.x], 1);
+    S.failed[threadIdx.x] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = S.tmem;
+  const uint32_t tmem = S.tmem + group * kHid;
   const uint32_t idesc_h = instr_desc_bf16(kTileM, kHid);
   const uint32_t idesc_o = instr_desc_bf16(kTileM, kOutPad);
-  const uint32_t act_a = smem_u32(S.act);
+  unsigned char *act = S.act[group];
+  uint64_t *bar = &S.bar[group];
   const int quarter = warp & 3;           // tensor-memory lanes 32q .. 32q + 31
   const int half = warp >> 2;             // columns [64 half, 64 half + 64)
   const int row = quarter * 32 + lane;    // the tile row this thread owns in the epilogues
   const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
   uint32_t phase = 0;
   bool ok = true;
-  const int tiles = (n + kTileM - 1) / kTileM;
-  for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kFusedThreads) : "memory"); };
+  const int tiles = (n + kTileM - 1) / kTileM, stride = gridDim.x * kFwdGroups;
+  bool staged = false;
+  float xi[8];
+  auto load_x = [&](int tile) {
     const int g = tile * kTileM + row;
-    // Layer 1 on the CUDA cores (FP32): this thread's 64 hidden units of its row.
-    {
-      float xi[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) xi[i] = (i < net.n_in && g < n) ? x[(size_t)g * ldx + i] : 0.0f;
-      for (int c8 = 0; c8 < 8; ++c8) {
-        __align__(16) __nv_bfloat16 h8[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int u = half * 64 + c8 * 8 + j;
-          float z = S.b[u];
-          for (int i = 0; i < net.n_in; ++i) z += S.w1[u * 8 + i] * xi[i];
-          h8[j] = __float2bfloat16(g < n ? silu(z) : 0.0f);
-        }
-        *reinterpret_cast<uint4 *>(S.act + off128(row, half * 8 + c8)) = *reinterpret_cast<uint4 *>(h8);
-      }
+    for (int i = 0; i < 8; ++i) xi[i] = (i < net.n_in && g < n) ? x[(size_t)g * ldx + i] : 0.0f;
+  };
+  int tile = group * gridDim.x + blockIdx.x;
+  load_x(tile);
+  for (; tile < tiles && ok; tile += stride) {
+    const int g = tile * kTileM + row;
+    for (int c8 = 0; c8 < 8; ++c8) {
+      const int u = half * 64 + c8 * 8;
+      __align__(16) __nv_bfloat16 h8[8];
+      first_layer8<NIN>(S.w1 + u * 8, S.b + u, xi, net.n_in, g < n, h8);
+      *reinterpret_cast<uint4 *>(act + off128(row, half * 8 + c8)) = *reinterpret_cast<uint4 *>(h8);
+    }
+    load_x(tile + stride);  // the next tile's inputs, under this one's layers
+    if (!staged) {
+      // All groups' copies; a group without a tile meets the others below.
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      fence_proxy_async_smem();
+      asm volatile("bar.sync 0;" ::: "memory");
+      staged = true;
     }
     // Layers 2..5 on the tensor cores.
-    for (int l = 0; l < 4 && ok; ++l) {
+    for (int l = 0; l < 4; ++l) {
       fence_proxy_async_smem();
       tc_fence_before();
-      __syncthreads();
+      group_sync();
       tc_fence_after();
+      ok = *(volatile int *)&S.failed[group] == 0;
+      if (!ok) break;
       const bool last = (l == 3);
       if (tid == 0) {
-        const uint32_t wb = last ? smem_u32(S.w5) : smem_u32(S.w[l]);
+        const uint32_t wb = last ? smem_u32(S.w5) : smem_u32(S.w[l]), ab = smem_u32(act);
         for (int s = 0; s < 8; ++s)
-          mma_bf16(tmem, smem_desc(act_a + s * 256, 128, 2048), smem_desc(wb + s * 256, 128, 2048),
+          mma_bf16(tmem, smem_desc(ab + s * 256, 128, 2048), smem_desc(wb + s * 256, 128, 2048),
                    last ? idesc_o : idesc_h, s > 0 ? 1u : 0u);
-        mma_commit(&S.bar);
+        mma_commit(bar);
       }
-      ok = __syncthreads_and(mbar_wait(&S.bar, phase)) != 0;
+      if (!mbar_wait(bar, phase)) S.failed[group] = 1;
       phase ^= 1u;
       tc_fence_after();
-      if (!ok) break;
       if (!last) {
         // Epilogue: bias + SiLU, written back as the next layer's operand.
 #pragma unroll
         for (int c0 = 0; c0 < 64; c0 += 32) {
           float v[32];
+          __syncwarp();
           tmem_ld32(lane_base + half * 64 + c0, v);
 #pragma unroll
           for (int c8 = 0; c8 < 4; ++c8) {
+            const float *b = S.b + (l + 1) * kHid + half * 64 + c0 + c8 * 8;
             __align__(16) __nv_bfloat16 h8[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int u = half * 64 + c0 + c8 * 8 + j;
-              h8[j] = __float2bfloat16(silu(v[c8 * 8 + j] + S.b[(l + 1) * kHid + u]));
-            }
-            *reinterpret_cast<uint4 *>(S.act + off128(row, (half * 64 + c0) / 8 + c8)) =
-                *reinterpret_cast<uint4 *>(h8);
+            for (int j = 0; j < 8; ++j) h8[j] = __float2bfloat16(silu(v[c8 * 8 + j] + b[j]));
+            *reinterpret_cast<uint4 *>(act + off128(row, (half * 64 + c0) / 8 + c8)) = *reinterpret_cast<uint4 *>(h8);
           }
         }
       } else if (half == 0) {
         float v[16];
+        __syncwarp();
         tmem_ld16(lane_base, v);
         if (g < n) {
 #pragma unroll
           for (int j = 0; j < kOutPad; ++j) y[(size_t)g * ldy + j] = v[j] + S.b[4 * kHid + j];
         }
       }
-      tc_fence_before();
     }
-    __syncthreads();
   }
-  if (!ok) {
+  if (!staged) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    fence_proxy_async_smem();
+    asm volatile("bar.sync 0;" ::: "memory");
+  }
+  group_sync();
+  if (S.failed[group]) {  // an expired wait: record it and drain (bounded) before tensor memory goes
     if (tid == 0) atomicExch(err, 1);
-    mbar_wait(&S.bar, phase ^ 1u);
+    mbar_wait(bar, phase ^ 1u);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) tmem_free(tmem, kHid);
+  if (threadIdx.x < 32) tmem_free(S.tmem, 512);
 }
 
 // ---- fused training step ------------------------------------------------------------------------
@@ -1126,9 +1170,10 @@ int xd_mlp_forward(const xd_mlp_net *net, int n, const float *d_x, int ldx, floa
   int grid = tiles < sms ? tiles : sms;
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
   const size_t smem = sizeof(FusedSmem);
-  cudaError_t e = cudaFuncSetAttribute(mlp_forward_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kernel = net->n_in == 5 ? mlp_forward_fused_kernel<5> : mlp_forward_fused_kernel<0>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_err(e, "cudaFuncSetAttribute(mlp_forward_fused_kernel)");
-  mlp_forward_fused_kernel<<<grid, kFusedThreads, smem, (cudaStream_t)stream>>>(*net, n, d_x, ldx, d_y, ldy, d_err);
+  kernel<<<grid, kFwdGroups * kFusedThreads, smem, (cudaStream_t)stream>>>(*net, n, d_x, ldx, d_y, ldy, d_err);
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_err(e, "mlp_forward_fused_kernel");
 }
