@@ -240,6 +240,10 @@ int xd_eval_variant_general(int v);
 int xd_get_eval_variant(const xd_ctx *ctx);
 int xd_set_eval_variant(xd_ctx *ctx, int v);
 int xd_probe_fp64_fma(double *d_out, int blocks, int iters, void *stream);
+/* xd_probe_quot: the device models' quotients a[i] / b[i], then a[i] / 3, a[i] / 12 and a[i] / 0.25, as the
+ * evaluation kernels form them, into d_out [4 * n] (d_a, d_b: [n]); correctly rounded except where
+ * csrc/quot.h says. */
+int xd_probe_quot(const double *d_a, const double *d_b, double *d_out, int n, void *stream);
 
 /* Allocation-free load (no counterpart in the reference: it is for callers of this library).
  *

@@ -161,15 +161,15 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       gbs = gmin;
       cbs = gbs * vbs;
     } else if (P(ijth) == 0.0) {
-      const double evbs = exp(vbs / Nvtm);
-      gbs = SourceSatCurrent * evbs / Nvtm + gmin;
+      const double evbs = exp(quot(vbs, Nvtm));
+      gbs = quot(SourceSatCurrent * evbs, Nvtm) + gmin;
       cbs = SourceSatCurrent * (evbs - 1.0) + gmin * vbs;
     } else if (vbs < P(vjsm)) {
-      const double evbs = exp(vbs / Nvtm);
-      gbs = SourceSatCurrent * evbs / Nvtm + gmin;
+      const double evbs = exp(quot(vbs, Nvtm));
+      gbs = quot(SourceSatCurrent * evbs, Nvtm) + gmin;
       cbs = SourceSatCurrent * (evbs - 1.0) + gmin * vbs;
     } else {
-      const double T0 = P(IsEvjsm) / Nvtm;
+      const double T0 = quot(P(IsEvjsm), Nvtm);
       gbs = T0 + gmin;
       cbs = P(IsEvjsm) - SourceSatCurrent + T0 * (vbs - P(vjsm)) + gmin * vbs;
     }
@@ -178,15 +178,15 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       gbd = gmin;
       cbd = gbd * vbd;
     } else if (P(ijth) == 0.0) {
-      const double evbd = exp(vbd / Nvtm);
-      gbd = DrainSatCurrent * evbd / Nvtm + gmin;
+      const double evbd = exp(quot(vbd, Nvtm));
+      gbd = quot(DrainSatCurrent * evbd, Nvtm) + gmin;
       cbd = DrainSatCurrent * (evbd - 1.0) + gmin * vbd;
     } else if (vbd < P(vjdm)) {
-      const double evbd = exp(vbd / Nvtm);
-      gbd = DrainSatCurrent * evbd / Nvtm + gmin;
+      const double evbd = exp(quot(vbd, Nvtm));
+      gbd = quot(DrainSatCurrent * evbd, Nvtm) + gmin;
       cbd = DrainSatCurrent * (evbd - 1.0) + gmin * vbd;
     } else {
-      const double T0 = P(IsEvjdm) / Nvtm;
+      const double T0 = quot(P(IsEvjdm), Nvtm);
       gbd = T0 + gmin;
       cbd = P(IsEvjdm) - DrainSatCurrent + T0 * (vbd - P(vjdm)) + gmin * vbd;
     }
@@ -214,23 +214,23 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   T0 = Vbs - vbsc - 0.001;
   T1 = sqrt(T0 * T0 - 0.004 * vbsc);
   double Vbseff = vbsc + 0.5 * (T0 + T1);
-  double dVbseff_dVb = 0.5 * (1.0 + T0 / T1);
+  double dVbseff_dVb = 0.5 * (1.0 + quot(T0, T1));
   if (Vbseff < Vbs) Vbseff = Vbs;
   double Phis, dPhis_dVb, sqrtPhis, dsqrtPhis_dVb;
   if (Vbseff > 0.0) {
-    T0 = phi / (phi + Vbseff);
+    T0 = quot(phi, phi + Vbseff);
     Phis = phi * T0;
     dPhis_dVb = -T0 * T0;
-    sqrtPhis = P(phis3) / (phi + 0.5 * Vbseff);
-    dsqrtPhis_dVb = -0.5 * sqrtPhis * sqrtPhis / P(phis3);
+    sqrtPhis = quot(P(phis3), phi + 0.5 * Vbseff);
+    dsqrtPhis_dVb = quot(-0.5 * sqrtPhis * sqrtPhis, P(phis3));
   } else {
     Phis = phi - Vbseff;
     dPhis_dVb = -1.0;
     sqrtPhis = sqrt(Phis);
-    dsqrtPhis_dVb = -0.5 / sqrtPhis;
+    dsqrtPhis_dVb = quot(-0.5, sqrtPhis);
   }
-  const double Xdep = P(Xdep0) * sqrtPhis / sqrtPhi;
-  const double dXdep_dVb = (P(Xdep0) / sqrtPhi) * dsqrtPhis_dVb;
+  const double Xdep = quot(P(Xdep0) * sqrtPhis, sqrtPhi);
+  const double dXdep_dVb = (quot(P(Xdep0), sqrtPhi)) * dsqrtPhis_dVb;
   const double Leff = P(leff);
   const double Vtm = P(vtm);
   const double factor1 = P(factor1);
@@ -243,29 +243,29 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
     T1 = 1.0 + T0;
     T2 = P(dvt2);
   } else {
-    T4 = 1.0 / (3.0 + 8.0 * T0);
+    T4 = quot(1.0, 3.0 + 8.0 * T0);
     T1 = (1.0 + 3.0 * T0) * T4;
     T2 = P(dvt2) * T4 * T4;
   }
   const double lt1 = factor1 * T3 * T1;
-  const double dlt1_dVb = factor1 * (0.5 / T3 * T1 * dXdep_dVb + T3 * T2);
+  const double dlt1_dVb = factor1 * (quot(0.5, T3) * T1 * dXdep_dVb + T3 * T2);
   T0 = P(dvt2w) * Vbseff;
   if (T0 >= -0.5) {
     T1 = 1.0 + T0;
     T2 = P(dvt2w);
   } else {
-    T4 = 1.0 / (3.0 + 8.0 * T0);
+    T4 = quot(1.0, 3.0 + 8.0 * T0);
     T1 = (1.0 + 3.0 * T0) * T4;
     T2 = P(dvt2w) * T4 * T4;
   }
   const double ltw = factor1 * T3 * T1;
-  const double dltw_dVb = factor1 * (0.5 / T3 * T1 * dXdep_dVb + T3 * T2);
+  const double dltw_dVb = factor1 * (quot(0.5, T3) * T1 * dXdep_dVb + T3 * T2);
   double Theta0, dTheta0_dVb;
-  T0 = -0.5 * P(dvt1) * Leff / lt1;
+  T0 = quot(-0.5 * P(dvt1) * Leff, lt1);
   if (T0 > -CONSTEXP_THRESHOLD) {
     T1 = exp(T0);
     Theta0 = T1 * (1.0 + 2.0 * T1);
-    dT1_dVb = -T0 / lt1 * T1 * dlt1_dVb;
+    dT1_dVb = quot(-T0, lt1) * T1 * dlt1_dVb;
     dTheta0_dVb = (1.0 + 4.0 * T1) * dT1_dVb;
   } else {
     T1 = CONSTMIN_EXP;
@@ -275,11 +275,11 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   const double thetavth = P(dvt0) * Theta0;
   const double Delt_vth = thetavth * V0;
   const double dDelt_vth_dVb = P(dvt0) * dTheta0_dVb * V0;
-  T0 = -0.5 * P(dvt1w) * P(weff) * Leff / ltw;
+  T0 = quot(-0.5 * P(dvt1w) * P(weff) * Leff, ltw);
   if (T0 > -CONSTEXP_THRESHOLD) {
     T1 = exp(T0);
     T2 = T1 * (1.0 + 2.0 * T1);
-    dT1_dVb = -T0 / ltw * T1 * dltw_dVb;
+    dT1_dVb = quot(-T0, ltw) * T1 * dltw_dVb;
     dT2_dVb = (1.0 + 4.0 * T1) * dT1_dVb;
   } else {
     T1 = CONSTMIN_EXP;
@@ -290,12 +290,12 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   T2 = T0 * V0;
   dT2_dVb = P(dvt0w) * dT2_dVb * V0;
   const double TempRatio = P(TempRatio);
-  T0 = sqrt(1.0 + P(nlx) / Leff);
-  T1 = P(k1ox) * (T0 - 1.0) * sqrtPhi + (P(kt1) + P(kt1l) / Leff + P(kt2) * Vbseff) * TempRatio;
-  tmp2 = P(tox) * phi / (P(weff) + P(w0));
+  T0 = sqrt(1.0 + quot(P(nlx), Leff));
+  T1 = P(k1ox) * (T0 - 1.0) * sqrtPhi + (P(kt1) + quot(P(kt1l), Leff) + P(kt2) * Vbseff) * TempRatio;
+  tmp2 = quot(P(tox) * phi, P(weff) + P(w0));
   T3 = P(eta0) + P(etab) * Vbseff;
   if (T3 < 1.0e-4) {
-    T9 = 1.0 / (3.0 - 2.0e4 * T3);
+    T9 = quot(1.0, 3.0 - 2.0e4 * T3);
     T3 = (2.0e-4 - T3) * T9;
     T4 = T9 * T9;
   } else {
@@ -313,34 +313,34 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   // Subthreshold swing factor n (:5291-5312).
   const double cox = P(cox);
   double n, dn_dVb, dn_dVd;
-  tmp2 = P(nfactor) * CONSTEPSSI / Xdep;
+  tmp2 = quot(P(nfactor) * CONSTEPSSI, Xdep);
   tmp3 = P(cdsc) + P(cdscb) * Vbseff + P(cdscd) * Vds;
-  tmp4 = (tmp2 + tmp3 * Theta0 + P(cit)) / cox;
+  tmp4 = quot((tmp2 + tmp3 * Theta0 + P(cit)), cox);
   if (tmp4 >= -0.5) {
     n = 1.0 + tmp4;
-    dn_dVb = (-tmp2 / Xdep * dXdep_dVb + tmp3 * dTheta0_dVb + P(cdscb) * Theta0) / cox;
-    dn_dVd = P(cdscd) * Theta0 / cox;
+    dn_dVb = quot((quot(-tmp2, Xdep) * dXdep_dVb + tmp3 * dTheta0_dVb + P(cdscb) * Theta0), cox);
+    dn_dVd = quot(P(cdscd) * Theta0, cox);
   } else {
-    T0 = 1.0 / (3.0 + 8.0 * tmp4);
+    T0 = quot(1.0, 3.0 + 8.0 * tmp4);
     n = (1.0 + 3.0 * tmp4) * T0;
     T0 *= T0;
-    dn_dVb = (-tmp2 / Xdep * dXdep_dVb + tmp3 * dTheta0_dVb + P(cdscb) * Theta0) / cox * T0;
-    dn_dVd = P(cdscd) * Theta0 / cox * T0;
+    dn_dVb = quot((quot(-tmp2, Xdep) * dXdep_dVb + tmp3 * dTheta0_dVb + P(cdscb) * Theta0), cox) * T0;
+    dn_dVd = quot(P(cdscd) * Theta0, cox) * T0;
   }
 
   // Poly-gate depletion (:5313-5335).
   double Vgs_eff, dVgs_eff_dVg;
   T0 = P(vfb) + phi;
   if ((P(ngate) > 1.e18) && (P(ngate) < 1.e25) && (Vgs > T0)) {
-    T1 = 1.0e6 * CONSTQ * CONSTEPSSI * P(ngate) / (cox * cox);
-    T4 = sqrt(1.0 + 2.0 * (Vgs - T0) / T1);
+    T1 = quot(1.0e6 * CONSTQ * CONSTEPSSI * P(ngate), cox * cox);
+    T4 = sqrt(1.0 + quot(2.0 * (Vgs - T0), T1));
     T2 = T1 * (T4 - 1.0);
-    T3 = 0.5 * T2 * T2 / T1;
+    T3 = quot(0.5 * T2 * T2, T1);
     T7 = 1.12 - T3 - 0.05;
     T6 = sqrt(T7 * T7 + 0.224);
     T5 = 1.12 - 0.5 * (T7 + T6);
     Vgs_eff = Vgs - T5;
-    dVgs_eff_dVg = 1.0 - (0.5 - 0.5 / T4) * (1.0 + T7 / T6);
+    dVgs_eff_dVg = 1.0 - (0.5 - quot(0.5, T4)) * (1.0 + quot(T7, T6));
   } else {
     Vgs_eff = Vgs;
     dVgs_eff_dVg = 1.0;
@@ -350,36 +350,36 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   // Effective Vgst (Vgsteff) for I-V (:5336-5380).
   double Vgsteff, dVgsteff_dVg, dVgsteff_dVd, dVgsteff_dVb;
   T10 = 2.0 * n * Vtm;
-  double VgstNVt = Vgst / T10;
-  const double ExpArg = (2.0 * P(voff) - Vgst) / T10;
+  double VgstNVt = quot(Vgst, T10);
+  const double ExpArg = quot((2.0 * P(voff) - Vgst), T10);
   if (VgstNVt > CONSTEXP_THRESHOLD) {
     Vgsteff = Vgst;
     dVgsteff_dVg = dVgs_eff_dVg;
     dVgsteff_dVd = -dVth_dVd;
     dVgsteff_dVb = -dVth_dVb;
   } else if (ExpArg > CONSTEXP_THRESHOLD) {
-    T0 = (Vgst - P(voff)) / (n * Vtm);
+    T0 = quot((Vgst - P(voff)), n * Vtm);
     const double ExpVgst = exp(T0);
-    Vgsteff = Vtm * P(cdep0) / cox * ExpVgst;
-    dVgsteff_dVg = Vgsteff / (n * Vtm);
+    Vgsteff = quot(Vtm * P(cdep0), cox) * ExpVgst;
+    dVgsteff_dVg = quot(Vgsteff, n * Vtm);
     dVgsteff_dVd = -dVgsteff_dVg * (dVth_dVd + T0 * Vtm * dn_dVd);
     dVgsteff_dVb = -dVgsteff_dVg * (dVth_dVb + T0 * Vtm * dn_dVb);
     dVgsteff_dVg *= dVgs_eff_dVg;
   } else {
     const double ExpVgst = exp(VgstNVt);
     T1 = T10 * log(1.0 + ExpVgst);
-    dT1_dVg = ExpVgst / (1.0 + ExpVgst);
-    dT1_dVb = -dT1_dVg * (dVth_dVb + Vgst / n * dn_dVb) + T1 / n * dn_dVb;
-    dT1_dVd = -dT1_dVg * (dVth_dVd + Vgst / n * dn_dVd) + T1 / n * dn_dVd;
-    dT2_dVg = -cox / (Vtm * P(cdep0)) * exp(ExpArg);
+    dT1_dVg = quot(ExpVgst, 1.0 + ExpVgst);
+    dT1_dVb = -dT1_dVg * (dVth_dVb + quot(Vgst, n) * dn_dVb) + quot(T1, n) * dn_dVb;
+    dT1_dVd = -dT1_dVg * (dVth_dVd + quot(Vgst, n) * dn_dVd) + quot(T1, n) * dn_dVd;
+    dT2_dVg = quot(-cox, Vtm * P(cdep0)) * exp(ExpArg);
     T2 = 1.0 - T10 * dT2_dVg;
-    dT2_dVd = -dT2_dVg * (dVth_dVd - 2.0 * Vtm * ExpArg * dn_dVd) + (T2 - 1.0) / n * dn_dVd;
-    dT2_dVb = -dT2_dVg * (dVth_dVb - 2.0 * Vtm * ExpArg * dn_dVb) + (T2 - 1.0) / n * dn_dVb;
-    Vgsteff = T1 / T2;
+    dT2_dVd = -dT2_dVg * (dVth_dVd - 2.0 * Vtm * ExpArg * dn_dVd) + quot((T2 - 1.0), n) * dn_dVd;
+    dT2_dVb = -dT2_dVg * (dVth_dVb - 2.0 * Vtm * ExpArg * dn_dVb) + quot((T2 - 1.0), n) * dn_dVb;
+    Vgsteff = quot(T1, T2);
     T3 = T2 * T2;
-    dVgsteff_dVg = (T2 * dT1_dVg - T1 * dT2_dVg) / T3 * dVgs_eff_dVg;
-    dVgsteff_dVd = (T2 * dT1_dVd - T1 * dT2_dVd) / T3;
-    dVgsteff_dVb = (T2 * dT1_dVb - T1 * dT2_dVb) / T3;
+    dVgsteff_dVg = quot((T2 * dT1_dVg - T1 * dT2_dVg), T3) * dVgs_eff_dVg;
+    dVgsteff_dVd = quot((T2 * dT1_dVd - T1 * dT2_dVd), T3);
+    dVgsteff_dVb = quot((T2 * dT1_dVb - T1 * dT2_dVb), T3);
   }
 
   // Effective width and source/drain resistance (:5381-5410).
@@ -388,7 +388,7 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   double dWeff_dVg = -2.0 * P(dwg);
   double dWeff_dVb = -2.0 * P(dwb) * dsqrtPhis_dVb;
   if (Weff < 2.0e-8) {
-    T0 = 1.0 / (6.0e-8 - 2.0 * Weff);
+    T0 = quot(1.0, 6.0e-8 - 2.0 * Weff);
     Weff = 2.0e-8 * (4.0e-8 - Weff) * T0;
     T0 *= T0 * 4.0e-16;
     dWeff_dVg *= T0;
@@ -402,7 +402,7 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
     dRds_dVg = rds0 * P(prwg);
     dRds_dVb = rds0 * P(prwb) * dsqrtPhis_dVb;
   } else {
-    T1 = 1.0 / (17.0 + 20.0 * T0);
+    T1 = quot(1.0, 17.0 + 20.0 * T0);
     Rds = rds0 * (0.8 + T0) * T1;
     T1 *= T1;
     dRds_dVg = rds0 * P(prwg) * T1;
@@ -410,16 +410,16 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   }
 
   // Bulk charge factor Abulk (:5411-5460).
-  T1 = 0.5 * P(k1ox) / sqrtPhis;
-  dT1_dVb = -T1 / sqrtPhis * dsqrtPhis_dVb;
+  T1 = quot(0.5 * P(k1ox), sqrtPhis);
+  dT1_dVb = quot(-T1, sqrtPhis) * dsqrtPhis_dVb;
   T9 = sqrt(P(xj) * Xdep);
   tmp1 = Leff + 2.0 * T9;
-  T5 = Leff / tmp1;
+  T5 = quot(Leff, tmp1);
   tmp2 = P(a0) * T5;
   tmp3 = P(weff) + P(b1);
-  tmp4 = P(b0) / tmp3;
+  tmp4 = quot(P(b0), tmp3);
   T2 = tmp2 + tmp4;
-  dT2_dVb = -T9 / tmp1 / Xdep * dXdep_dVb;
+  dT2_dVb = quot(quot(-T9, tmp1), Xdep) * dXdep_dVb;
   T6 = T5 * T5;
   T7 = T5 * T6;
   double Abulk0 = 1.0 + T1 * T2;
@@ -429,12 +429,12 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   double Abulk = Abulk0 + dAbulk_dVg * Vgsteff;
   double dAbulk_dVb = dAbulk0_dVb - T8 * Vgsteff * (dT1_dVb + 3.0 * T1 * dT2_dVb);
   if (Abulk0 < 0.1) {
-    T9 = 1.0 / (3.0 - 20.0 * Abulk0);
+    T9 = quot(1.0, 3.0 - 20.0 * Abulk0);
     Abulk0 = (0.2 - Abulk0) * T9;
     dAbulk0_dVb *= T9 * T9;
   }
   if (Abulk < 0.1) {
-    T9 = 1.0 / (3.0 - 20.0 * Abulk);
+    T9 = quot(1.0, 3.0 - 20.0 * Abulk);
     Abulk = (0.2 - Abulk) * T9;
     T10 = T9 * T9;
     dAbulk_dVb *= T10;
@@ -442,10 +442,10 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   }
   T2 = P(keta) * Vbseff;
   if (T2 >= -0.9) {
-    T0 = 1.0 / (1.0 + T2);
+    T0 = quot(1.0, 1.0 + T2);
     dT0_dVb = -P(keta) * T0 * T0;
   } else {
-    T1 = 1.0 / (0.8 + T2);
+    T1 = quot(1.0, 0.8 + T2);
     T0 = (17.0 + 20.0 * T2) * T1;
     dT0_dVb = -P(keta) * T1 * T1;
   }
@@ -462,38 +462,38 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   if (mobMod == 1) {
     T0 = Vgsteff + Vth + Vth;
     T2 = P(ua) + P(uc) * Vbseff;
-    T3 = T0 / tox;
+    T3 = quot(T0, tox);
     T5 = T3 * (T2 + P(ub) * T3);
-    dDenomi_dVg = (T2 + 2.0 * P(ub) * T3) / tox;
+    dDenomi_dVg = quot((T2 + 2.0 * P(ub) * T3), tox);
     dDenomi_dVd = dDenomi_dVg * 2.0 * dVth_dVd;
     dDenomi_dVb = dDenomi_dVg * 2.0 * dVth_dVb + P(uc) * T3;
   } else if (mobMod == 2) {
-    T5 = Vgsteff / tox * (P(ua) + P(uc) * Vbseff + P(ub) * Vgsteff / tox);
-    dDenomi_dVg = (P(ua) + P(uc) * Vbseff + 2.0 * P(ub) * Vgsteff / tox) / tox;
+    T5 = quot(Vgsteff, tox) * (P(ua) + P(uc) * Vbseff + quot(P(ub) * Vgsteff, tox));
+    dDenomi_dVg = quot((P(ua) + P(uc) * Vbseff + quot(2.0 * P(ub) * Vgsteff, tox)), tox);
     dDenomi_dVd = 0.0;
-    dDenomi_dVb = Vgsteff * P(uc) / tox;
+    dDenomi_dVb = quot(Vgsteff * P(uc), tox);
   } else {
     T0 = Vgsteff + Vth + Vth;
     T2 = 1.0 + P(uc) * Vbseff;
-    T3 = T0 / tox;
+    T3 = quot(T0, tox);
     T4 = T3 * (P(ua) + P(ub) * T3);
     T5 = T4 * T2;
-    dDenomi_dVg = (P(ua) + 2.0 * P(ub) * T3) * T2 / tox;
+    dDenomi_dVg = quot((P(ua) + 2.0 * P(ub) * T3) * T2, tox);
     dDenomi_dVd = dDenomi_dVg * 2.0 * dVth_dVd;
     dDenomi_dVb = dDenomi_dVg * 2.0 * dVth_dVb + P(uc) * T4;
   }
   if (T5 >= -0.8) {
     Denomi = 1.0 + T5;
   } else {
-    T9 = 1.0 / (7.0 + 10.0 * T5);
+    T9 = quot(1.0, 7.0 + 10.0 * T5);
     Denomi = (0.6 + T5) * T9;
     T9 *= T9;
     dDenomi_dVg *= T9;
     dDenomi_dVd *= T9;
     dDenomi_dVb *= T9;
   }
-  const double ueff = P(u0temp) / Denomi;
-  T9 = -ueff / Denomi;
+  const double ueff = quot(P(u0temp), Denomi);
+  T9 = quot(-ueff, Denomi);
   const double dueff_dVg = T9 * dDenomi_dVg;
   const double dueff_dVd = T9 * dDenomi_dVd;
   const double dueff_dVb = T9 * dDenomi_dVb;
@@ -502,9 +502,9 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   const double vsattemp = P(vsattemp);
   const double WVCox = Weff * vsattemp * cox;
   const double WVCoxRds = WVCox * Rds;
-  const double Esat = 2.0 * vsattemp / ueff;
+  const double Esat = quot(2.0 * vsattemp, ueff);
   const double EsatL = Esat * Leff;
-  T0 = -EsatL / ueff;
+  T0 = quot(-EsatL, ueff);
   const double dEsatL_dVg = T0 * dueff_dVg;
   const double dEsatL_dVd = T0 * dueff_dVd;
   const double dEsatL_dVb = T0 * dueff_dVb;
@@ -518,24 +518,24 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
     T1 = T0 - P(a1) * Vgsteff - 0.0001;
     T2 = sqrt(T1 * T1 + 0.0004 * T0);
     Lambda = P(a2) + T0 - 0.5 * (T1 + T2);
-    dLambda_dVg = 0.5 * P(a1) * (1.0 + T1 / T2);
+    dLambda_dVg = 0.5 * P(a1) * (1.0 + quot(T1, T2));
   } else {
     T1 = P(a2) + P(a1) * Vgsteff - 0.0001;
     T2 = sqrt(T1 * T1 + 0.0004 * P(a2));
     Lambda = 0.5 * (T1 + T2);
-    dLambda_dVg = 0.5 * P(a1) * (1.0 + T1 / T2);
+    dLambda_dVg = 0.5 * P(a1) * (1.0 + quot(T1, T2));
   }
   const double Vgst2Vtm = Vgsteff + 2.0 * Vtm;
   if (Rds > 0) {
-    tmp2 = dRds_dVg / Rds + dWeff_dVg / Weff;
-    tmp3 = dRds_dVb / Rds + dWeff_dVb / Weff;
+    tmp2 = quot(dRds_dVg, Rds) + quot(dWeff_dVg, Weff);
+    tmp3 = quot(dRds_dVb, Rds) + quot(dWeff_dVb, Weff);
   } else {
-    tmp2 = dWeff_dVg / Weff;
-    tmp3 = dWeff_dVb / Weff;
+    tmp2 = quot(dWeff_dVg, Weff);
+    tmp3 = quot(dWeff_dVb, Weff);
   }
   double Vdsat, dVdsat_dVg, dVdsat_dVd, dVdsat_dVb;
   if ((Rds == 0.0) && (Lambda == 1.0)) {
-    T0 = 1.0 / (Abulk * EsatL + Vgst2Vtm);
+    T0 = quot(1.0, Abulk * EsatL + Vgst2Vtm);
     tmp1 = 0.0;
     T1 = T0 * T0;
     T2 = Vgst2Vtm * T0;
@@ -548,17 +548,17 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
     dVdsat_dVd = T3 * dT0_dVd + T2 * dEsatL_dVd;
     dVdsat_dVb = T3 * dT0_dVb + T2 * dEsatL_dVb;
   } else {
-    tmp1 = dLambda_dVg / (Lambda * Lambda);
+    tmp1 = quot(dLambda_dVg, Lambda * Lambda);
     T9 = Abulk * WVCoxRds;
     T8 = Abulk * T9;
     T7 = Vgst2Vtm * T9;
     T6 = Vgst2Vtm * WVCoxRds;
-    T0 = 2.0 * Abulk * (T9 - 1.0 + 1.0 / Lambda);
-    dT0_dVg = 2.0 * (T8 * tmp2 - Abulk * tmp1 + (2.0 * T9 + 1.0 / Lambda - 1.0) * dAbulk_dVg);
-    dT0_dVb = 2.0 * (T8 * (2.0 / Abulk * dAbulk_dVb + tmp3) + (1.0 / Lambda - 1.0) * dAbulk_dVb);
+    T0 = 2.0 * Abulk * (T9 - 1.0 + quot(1.0, Lambda));
+    dT0_dVg = 2.0 * (T8 * tmp2 - Abulk * tmp1 + (2.0 * T9 + quot(1.0, Lambda) - 1.0) * dAbulk_dVg);
+    dT0_dVb = 2.0 * (T8 * (quot(2.0, Abulk) * dAbulk_dVb + tmp3) + (quot(1.0, Lambda) - 1.0) * dAbulk_dVb);
     dT0_dVd = 0.0;
-    T1 = Vgst2Vtm * (2.0 / Lambda - 1.0) + Abulk * EsatL + 3.0 * T7;
-    dT1_dVg = (2.0 / Lambda - 1.0) - 2.0 * Vgst2Vtm * tmp1 + Abulk * dEsatL_dVg + EsatL * dAbulk_dVg +
+    T1 = Vgst2Vtm * (quot(2.0, Lambda) - 1.0) + Abulk * EsatL + 3.0 * T7;
+    dT1_dVg = (quot(2.0, Lambda) - 1.0) - 2.0 * Vgst2Vtm * tmp1 + Abulk * dEsatL_dVg + EsatL * dAbulk_dVg +
               3.0 * (T9 + T7 * tmp2 + T6 * dAbulk_dVg);
     dT1_dVb = Abulk * dEsatL_dVb + EsatL * dAbulk_dVb + 3.0 * (T6 * dAbulk_dVb + T7 * tmp3);
     dT1_dVd = Abulk * dEsatL_dVd;
@@ -567,16 +567,16 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
     dT2_dVb = Vgst2Vtm * (dEsatL_dVb + 2.0 * T6 * tmp3);
     dT2_dVd = Vgst2Vtm * dEsatL_dVd;
     T3 = sqrt(T1 * T1 - 2.0 * T0 * T2);
-    Vdsat = (T1 - T3) / T0;
-    dT3_dVg = (T1 * dT1_dVg - 2.0 * (T0 * dT2_dVg + T2 * dT0_dVg)) / T3;
-    dT3_dVd = (T1 * dT1_dVd - 2.0 * (T0 * dT2_dVd + T2 * dT0_dVd)) / T3;
-    dT3_dVb = (T1 * dT1_dVb - 2.0 * (T0 * dT2_dVb + T2 * dT0_dVb)) / T3;
+    Vdsat = quot((T1 - T3), T0);
+    dT3_dVg = quot((T1 * dT1_dVg - 2.0 * (T0 * dT2_dVg + T2 * dT0_dVg)), T3);
+    dT3_dVd = quot((T1 * dT1_dVd - 2.0 * (T0 * dT2_dVd + T2 * dT0_dVd)), T3);
+    dT3_dVb = quot((T1 * dT1_dVb - 2.0 * (T0 * dT2_dVb + T2 * dT0_dVb)), T3);
     (void)dT3_dVg;
     (void)dT3_dVd;
     (void)dT3_dVb;
-    dVdsat_dVg = (dT1_dVg - (T1 * dT1_dVg - dT0_dVg * T2 - T0 * dT2_dVg) / T3 - Vdsat * dT0_dVg) / T0;
-    dVdsat_dVb = (dT1_dVb - (T1 * dT1_dVb - dT0_dVb * T2 - T0 * dT2_dVb) / T3 - Vdsat * dT0_dVb) / T0;
-    dVdsat_dVd = (dT1_dVd - (T1 * dT1_dVd - T0 * dT2_dVd) / T3) / T0;
+    dVdsat_dVg = quot((dT1_dVg - quot((T1 * dT1_dVg - dT0_dVg * T2 - T0 * dT2_dVg), T3) - Vdsat * dT0_dVg), T0);
+    dVdsat_dVb = quot((dT1_dVb - quot((T1 * dT1_dVb - dT0_dVb * T2 - T0 * dT2_dVb), T3) - Vdsat * dT0_dVb), T0);
+    dVdsat_dVd = quot((dT1_dVd - quot((T1 * dT1_dVd - T0 * dT2_dVd), T3)), T0);
   }
 
   // Effective Vds (:5641-5665).
@@ -586,8 +586,8 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   dT1_dVd = dVdsat_dVd - 1.0;
   dT1_dVb = dVdsat_dVb;
   T2 = sqrt(T1 * T1 + 4.0 * delta * Vdsat);
-  T0 = T1 / T2;
-  T3 = 2.0 * delta / T2;
+  T0 = quot(T1, T2);
+  T3 = quot(2.0 * delta, T2);
   dT2_dVg = T0 * dT1_dVg + T3 * dVdsat_dVg;
   dT2_dVd = T0 * dT1_dVd + T3 * dVdsat_dVd;
   dT2_dVb = T0 * dT1_dVb + T3 * dVdsat_dVb;
@@ -602,37 +602,37 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   }
 
   // Vasat (:5666-5700).
-  tmp4 = 1.0 - 0.5 * Abulk * Vdsat / Vgst2Vtm;
+  tmp4 = 1.0 - quot(0.5 * Abulk * Vdsat, Vgst2Vtm);
   T9 = WVCoxRds * Vgsteff;
-  T8 = T9 / Vgst2Vtm;
+  T8 = quot(T9, Vgst2Vtm);
   T0 = EsatL + Vdsat + 2.0 * T9 * tmp4;
   T7 = 2.0 * WVCoxRds * tmp4;
   dT0_dVg = dEsatL_dVg + dVdsat_dVg + T7 * (1.0 + tmp2 * Vgsteff) -
-            T8 * (Abulk * dVdsat_dVg - Abulk * Vdsat / Vgst2Vtm + Vdsat * dAbulk_dVg);
+            T8 * (Abulk * dVdsat_dVg - quot(Abulk * Vdsat, Vgst2Vtm) + Vdsat * dAbulk_dVg);
   dT0_dVb = dEsatL_dVb + dVdsat_dVb + T7 * tmp3 * Vgsteff - T8 * (dAbulk_dVb * Vdsat + Abulk * dVdsat_dVb);
   dT0_dVd = dEsatL_dVd + dVdsat_dVd - T8 * Abulk * dVdsat_dVd;
   T9 = WVCoxRds * Abulk;
-  T1 = 2.0 / Lambda - 1.0 + T9;
+  T1 = quot(2.0, Lambda) - 1.0 + T9;
   dT1_dVg = -2.0 * tmp1 + WVCoxRds * (Abulk * tmp2 + dAbulk_dVg);
   dT1_dVb = dAbulk_dVb * WVCoxRds + T9 * tmp3;
-  const double Vasat = T0 / T1;
-  const double dVasat_dVg = (dT0_dVg - Vasat * dT1_dVg) / T1;
-  const double dVasat_dVb = (dT0_dVb - Vasat * dT1_dVb) / T1;
-  const double dVasat_dVd = dT0_dVd / T1;
+  const double Vasat = quot(T0, T1);
+  const double dVasat_dVg = quot((dT0_dVg - Vasat * dT1_dVg), T1);
+  const double dVasat_dVb = quot((dT0_dVb - Vasat * dT1_dVb), T1);
+  const double dVasat_dVd = quot(dT0_dVd, T1);
   if (Vdseff > Vds) Vdseff = Vds;
   const double diffVds = Vds - Vdseff;
 
   // Channel-length modulation, DIBL, pvag, SCBE (:5701-5860).
   double VACLM, dVACLM_dVg, dVACLM_dVd, dVACLM_dVb;
   if ((P(pclm) > 0.0) && (diffVds > 1.0e-10)) {
-    T0 = 1.0 / (P(pclm) * Abulk * P(litl));
-    dT0_dVb = -T0 / Abulk * dAbulk_dVb;
-    dT0_dVg = -T0 / Abulk * dAbulk_dVg;
-    T2 = Vgsteff / EsatL;
+    T0 = quot(1.0, P(pclm) * Abulk * P(litl));
+    dT0_dVb = quot(-T0, Abulk) * dAbulk_dVb;
+    dT0_dVg = quot(-T0, Abulk) * dAbulk_dVg;
+    T2 = quot(Vgsteff, EsatL);
     T1 = Leff * (Abulk + T2);
-    dT1_dVg = Leff * ((1.0 - T2 * dEsatL_dVg) / EsatL + dAbulk_dVg);
-    dT1_dVb = Leff * (dAbulk_dVb - T2 * dEsatL_dVb / EsatL);
-    dT1_dVd = -T2 * dEsatL_dVd / Esat;
+    dT1_dVg = Leff * (quot((1.0 - T2 * dEsatL_dVg), EsatL) + dAbulk_dVg);
+    dT1_dVb = Leff * (dAbulk_dVb - quot(T2 * dEsatL_dVb, EsatL));
+    dT1_dVd = quot(-T2 * dEsatL_dVd, Esat);
     T9 = T0 * T1;
     VACLM = T9 * diffVds;
     dVACLM_dVg = T0 * dT1_dVg * diffVds - T9 * dVdseff_dVg + T1 * diffVds * dT0_dVg;
@@ -655,19 +655,19 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
     dT1_dVd = Abulk * dVdsat_dVd;
     T9 = T1 * T1;
     T2 = P(thetaRout);
-    VADIBL = (Vgst2Vtm - T0 / T1) / T2;
-    dVADIBL_dVg = (1.0 - dT0_dVg / T1 + T0 * dT1_dVg / T9) / T2;
-    dVADIBL_dVb = (-dT0_dVb / T1 + T0 * dT1_dVb / T9) / T2;
-    dVADIBL_dVd = (-dT0_dVd / T1 + T0 * dT1_dVd / T9) / T2;
+    VADIBL = quot((Vgst2Vtm - quot(T0, T1)), T2);
+    dVADIBL_dVg = quot((1.0 - quot(dT0_dVg, T1) + quot(T0 * dT1_dVg, T9)), T2);
+    dVADIBL_dVb = quot((quot(-dT0_dVb, T1) + quot(T0 * dT1_dVb, T9)), T2);
+    dVADIBL_dVd = quot((quot(-dT0_dVd, T1) + quot(T0 * dT1_dVd, T9)), T2);
     T7 = P(pdiblb) * Vbseff;
     if (T7 >= -0.9) {
-      T3 = 1.0 / (1.0 + T7);
+      T3 = quot(1.0, 1.0 + T7);
       VADIBL *= T3;
       dVADIBL_dVg *= T3;
       dVADIBL_dVb = (dVADIBL_dVb - VADIBL * P(pdiblb)) * T3;
       dVADIBL_dVd *= T3;
     } else {
-      T4 = 1.0 / (0.8 + T7);
+      T4 = quot(1.0, 0.8 + T7);
       T3 = (17.0 + 20.0 * T7) * T4;
       dVADIBL_dVg *= T3;
       dVADIBL_dVb = dVADIBL_dVb * T3 - VADIBL * P(pdiblb) * T4 * T4;
@@ -678,45 +678,45 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
     VADIBL = CONSTMAX_EXP;
     dVADIBL_dVd = dVADIBL_dVg = dVADIBL_dVb = 0.0;
   }
-  T8 = P(pvag) / EsatL;
+  T8 = quot(P(pvag), EsatL);
   T9 = T8 * Vgsteff;
   if (T9 > -0.9) {
     T0 = 1.0 + T9;
-    dT0_dVg = T8 * (1.0 - Vgsteff * dEsatL_dVg / EsatL);
-    dT0_dVb = -T9 * dEsatL_dVb / EsatL;
-    dT0_dVd = -T9 * dEsatL_dVd / EsatL;
+    dT0_dVg = T8 * (1.0 - quot(Vgsteff * dEsatL_dVg, EsatL));
+    dT0_dVb = quot(-T9 * dEsatL_dVb, EsatL);
+    dT0_dVd = quot(-T9 * dEsatL_dVd, EsatL);
   } else {
-    T1 = 1.0 / (17.0 + 20.0 * T9);
+    T1 = quot(1.0, 17.0 + 20.0 * T9);
     T0 = (0.8 + T9) * T1;
     T1 *= T1;
-    dT0_dVg = T8 * (1.0 - Vgsteff * dEsatL_dVg / EsatL) * T1;
-    T9 *= T1 / EsatL;
+    dT0_dVg = T8 * (1.0 - quot(Vgsteff * dEsatL_dVg, EsatL)) * T1;
+    T9 *= quot(T1, EsatL);
     dT0_dVb = -T9 * dEsatL_dVb;
     dT0_dVd = -T9 * dEsatL_dVd;
   }
   tmp1 = VACLM * VACLM;
   tmp2 = VADIBL * VADIBL;
   tmp3 = VACLM + VADIBL;
-  T1 = VACLM * VADIBL / tmp3;
+  T1 = quot(VACLM * VADIBL, tmp3);
   tmp3 *= tmp3;
-  dT1_dVg = (tmp1 * dVADIBL_dVg + tmp2 * dVACLM_dVg) / tmp3;
-  dT1_dVd = (tmp1 * dVADIBL_dVd + tmp2 * dVACLM_dVd) / tmp3;
-  dT1_dVb = (tmp1 * dVADIBL_dVb + tmp2 * dVACLM_dVb) / tmp3;
+  dT1_dVg = quot((tmp1 * dVADIBL_dVg + tmp2 * dVACLM_dVg), tmp3);
+  dT1_dVd = quot((tmp1 * dVADIBL_dVd + tmp2 * dVACLM_dVd), tmp3);
+  dT1_dVb = quot((tmp1 * dVADIBL_dVb + tmp2 * dVACLM_dVb), tmp3);
   const double Va = Vasat + T0 * T1;
   const double dVa_dVg = dVasat_dVg + T1 * dT0_dVg + T0 * dT1_dVg;
   const double dVa_dVd = dVasat_dVd + T1 * dT0_dVd + T0 * dT1_dVd;
   const double dVa_dVb = dVasat_dVb + T1 * dT0_dVb + T0 * dT1_dVb;
   double VASCBE, dVASCBE_dVg, dVASCBE_dVd, dVASCBE_dVb;
   if (P(pscbe2) > 0.0) {
-    if (diffVds > P(pscbe1) * P(litl) / CONSTEXP_THRESHOLD) {
-      T0 = P(pscbe1) * P(litl) / diffVds;
-      VASCBE = Leff * exp(T0) / P(pscbe2);
-      T1 = T0 * VASCBE / diffVds;
+    if (diffVds > quot(P(pscbe1) * P(litl), CONSTEXP_THRESHOLD)) {
+      T0 = quot(P(pscbe1) * P(litl), diffVds);
+      VASCBE = quot(Leff * exp(T0), P(pscbe2));
+      T1 = quot(T0 * VASCBE, diffVds);
       dVASCBE_dVg = T1 * dVdseff_dVg;
       dVASCBE_dVd = -T1 * (1.0 - dVdseff_dVd);
       dVASCBE_dVb = T1 * dVdseff_dVb;
     } else {
-      VASCBE = CONSTMAX_EXP * Leff / P(pscbe2);
+      VASCBE = quot(CONSTMAX_EXP * Leff, P(pscbe2));
       dVASCBE_dVg = dVASCBE_dVd = dVASCBE_dVb = 0.0;
     }
   } else {
@@ -725,46 +725,46 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   }
 
   // Drain current (:5861-5935).
-  const double CoxWovL = cox * Weff / Leff;
+  const double CoxWovL = quot(cox * Weff, Leff);
   const double beta = ueff * CoxWovL;
-  const double dbeta_dVg = CoxWovL * dueff_dVg + beta * dWeff_dVg / Weff;
+  const double dbeta_dVg = CoxWovL * dueff_dVg + quot(beta * dWeff_dVg, Weff);
   const double dbeta_dVd = CoxWovL * dueff_dVd;
-  const double dbeta_dVb = CoxWovL * dueff_dVb + beta * dWeff_dVb / Weff;
-  T0 = 1.0 - 0.5 * Abulk * Vdseff / Vgst2Vtm;
-  dT0_dVg = -0.5 * (Abulk * dVdseff_dVg - Abulk * Vdseff / Vgst2Vtm + Vdseff * dAbulk_dVg) / Vgst2Vtm;
-  dT0_dVd = -0.5 * Abulk * dVdseff_dVd / Vgst2Vtm;
-  dT0_dVb = -0.5 * (Abulk * dVdseff_dVb + dAbulk_dVb * Vdseff) / Vgst2Vtm;
+  const double dbeta_dVb = CoxWovL * dueff_dVb + quot(beta * dWeff_dVb, Weff);
+  T0 = 1.0 - quot(0.5 * Abulk * Vdseff, Vgst2Vtm);
+  dT0_dVg = quot(-0.5 * (Abulk * dVdseff_dVg - quot(Abulk * Vdseff, Vgst2Vtm) + Vdseff * dAbulk_dVg), Vgst2Vtm);
+  dT0_dVd = quot(-0.5 * Abulk * dVdseff_dVd, Vgst2Vtm);
+  dT0_dVb = quot(-0.5 * (Abulk * dVdseff_dVb + dAbulk_dVb * Vdseff), Vgst2Vtm);
   const double fgche1 = Vgsteff * T0;
   const double dfgche1_dVg = Vgsteff * dT0_dVg + T0;
   const double dfgche1_dVd = Vgsteff * dT0_dVd;
   const double dfgche1_dVb = Vgsteff * dT0_dVb;
-  T9 = Vdseff / EsatL;
+  T9 = quot(Vdseff, EsatL);
   const double fgche2 = 1.0 + T9;
-  const double dfgche2_dVg = (dVdseff_dVg - T9 * dEsatL_dVg) / EsatL;
-  const double dfgche2_dVd = (dVdseff_dVd - T9 * dEsatL_dVd) / EsatL;
-  const double dfgche2_dVb = (dVdseff_dVb - T9 * dEsatL_dVb) / EsatL;
-  const double gche = beta * fgche1 / fgche2;
-  const double dgche_dVg = (beta * dfgche1_dVg + fgche1 * dbeta_dVg - gche * dfgche2_dVg) / fgche2;
-  const double dgche_dVd = (beta * dfgche1_dVd + fgche1 * dbeta_dVd - gche * dfgche2_dVd) / fgche2;
-  const double dgche_dVb = (beta * dfgche1_dVb + fgche1 * dbeta_dVb - gche * dfgche2_dVb) / fgche2;
+  const double dfgche2_dVg = quot((dVdseff_dVg - T9 * dEsatL_dVg), EsatL);
+  const double dfgche2_dVd = quot((dVdseff_dVd - T9 * dEsatL_dVd), EsatL);
+  const double dfgche2_dVb = quot((dVdseff_dVb - T9 * dEsatL_dVb), EsatL);
+  const double gche = quot(beta * fgche1, fgche2);
+  const double dgche_dVg = quot((beta * dfgche1_dVg + fgche1 * dbeta_dVg - gche * dfgche2_dVg), fgche2);
+  const double dgche_dVd = quot((beta * dfgche1_dVd + fgche1 * dbeta_dVd - gche * dfgche2_dVd), fgche2);
+  const double dgche_dVb = quot((beta * dfgche1_dVb + fgche1 * dbeta_dVb - gche * dfgche2_dVb), fgche2);
   T0 = 1.0 + gche * Rds;
-  T9 = Vdseff / T0;
+  T9 = quot(Vdseff, T0);
   const double Idl = gche * T9;
-  const double dIdl_dVg = (gche * dVdseff_dVg + T9 * dgche_dVg) / T0 - Idl * gche / T0 * dRds_dVg;
-  const double dIdl_dVd = (gche * dVdseff_dVd + T9 * dgche_dVd) / T0;
-  const double dIdl_dVb = (gche * dVdseff_dVb + T9 * dgche_dVb - Idl * dRds_dVb * gche) / T0;
-  T9 = diffVds / Va;
+  const double dIdl_dVg = quot((gche * dVdseff_dVg + T9 * dgche_dVg), T0) - quot(Idl * gche, T0) * dRds_dVg;
+  const double dIdl_dVd = quot((gche * dVdseff_dVd + T9 * dgche_dVd), T0);
+  const double dIdl_dVb = quot((gche * dVdseff_dVb + T9 * dgche_dVb - Idl * dRds_dVb * gche), T0);
+  T9 = quot(diffVds, Va);
   T0 = 1.0 + T9;
   const double Idsa = Idl * T0;
-  const double dIdsa_dVg = T0 * dIdl_dVg - Idl * (dVdseff_dVg + T9 * dVa_dVg) / Va;
-  const double dIdsa_dVd = T0 * dIdl_dVd + Idl * (1.0 - dVdseff_dVd - T9 * dVa_dVd) / Va;
-  const double dIdsa_dVb = T0 * dIdl_dVb - Idl * (dVdseff_dVb + T9 * dVa_dVb) / Va;
-  T9 = diffVds / VASCBE;
+  const double dIdsa_dVg = T0 * dIdl_dVg - quot(Idl * (dVdseff_dVg + T9 * dVa_dVg), Va);
+  const double dIdsa_dVd = T0 * dIdl_dVd + quot(Idl * (1.0 - dVdseff_dVd - T9 * dVa_dVd), Va);
+  const double dIdsa_dVb = T0 * dIdl_dVb - quot(Idl * (dVdseff_dVb + T9 * dVa_dVb), Va);
+  T9 = quot(diffVds, VASCBE);
   T0 = 1.0 + T9;
   const double Ids = Idsa * T0;
-  double Gm = T0 * dIdsa_dVg - Idsa * (dVdseff_dVg + T9 * dVASCBE_dVg) / VASCBE;
-  double Gds = T0 * dIdsa_dVd + Idsa * (1.0 - dVdseff_dVd - T9 * dVASCBE_dVd) / VASCBE;
-  double Gmb = T0 * dIdsa_dVb - Idsa * (dVdseff_dVb + T9 * dVASCBE_dVb) / VASCBE;
+  double Gm = T0 * dIdsa_dVg - quot(Idsa * (dVdseff_dVg + T9 * dVASCBE_dVg), VASCBE);
+  double Gds = T0 * dIdsa_dVd + quot(Idsa * (1.0 - dVdseff_dVd - T9 * dVASCBE_dVd), VASCBE);
+  double Gmb = T0 * dIdsa_dVb - quot(Idsa * (dVdseff_dVb + T9 * dVASCBE_dVb), VASCBE);
   Gds += Gm * dVgsteff_dVd;
   Gmb += Gm * dVgsteff_dVb;
   Gm *= dVgsteff_dVg;
@@ -776,11 +776,11 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
   if ((tmp <= 0.0) || (P(beta0) <= 0.0)) {
     Isub = Gbd = Gbb = Gbg = 0.0;
   } else {
-    T2 = tmp / Leff;
-    if (diffVds > P(beta0) / CONSTEXP_THRESHOLD) {
-      T0 = -P(beta0) / diffVds;
+    T2 = quot(tmp, Leff);
+    if (diffVds > quot(P(beta0), CONSTEXP_THRESHOLD)) {
+      T0 = quot(-P(beta0), diffVds);
       T1 = T2 * diffVds * exp(T0);
-      T3 = T1 / diffVds * (T0 - 1.0);
+      T3 = quot(T1, diffVds) * (T0 - 1.0);
       dT1_dVg = T3 * dVdseff_dVg;
       dT1_dVd = T3 * (dVdseff_dVd - 1.0);
       dT1_dVb = T3 * dVdseff_dVb;
@@ -833,7 +833,7 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
     const double dnoff_dVb = P(noff) * dn_dVb;
     T0 = Vtm * noff;
     const double voffcv = P(voffcv);
-    VgstNVt = (Vgst - voffcv) / T0;
+    VgstNVt = quot((Vgst - voffcv), T0);
     if (VgstNVt > CONSTEXP_THRESHOLD) {
       Vgsteff = Vgst - voffcv;
       dVgsteff_dVg = dVgs_eff_dVg;
@@ -842,15 +842,15 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
     } else if (VgstNVt < -CONSTEXP_THRESHOLD) {
       Vgsteff = T0 * log(1.0 + CONSTMIN_EXP);
       dVgsteff_dVg = 0.0;
-      dVgsteff_dVd = Vgsteff / noff;
+      dVgsteff_dVd = quot(Vgsteff, noff);
       dVgsteff_dVb = dVgsteff_dVd * dnoff_dVb;
       dVgsteff_dVd *= dnoff_dVd;
     } else {
       const double ExpVgst = exp(VgstNVt);
       Vgsteff = T0 * log(1.0 + ExpVgst);
-      dVgsteff_dVg = ExpVgst / (1.0 + ExpVgst);
-      dVgsteff_dVd = -dVgsteff_dVg * (dVth_dVd + (Vgst - voffcv) / noff * dnoff_dVd) + Vgsteff / noff * dnoff_dVd;
-      dVgsteff_dVb = -dVgsteff_dVg * (dVth_dVb + (Vgst - voffcv) / noff * dnoff_dVb) + Vgsteff / noff * dnoff_dVb;
+      dVgsteff_dVg = quot(ExpVgst, 1.0 + ExpVgst);
+      dVgsteff_dVd = -dVgsteff_dVg * (dVth_dVd + quot((Vgst - voffcv), noff) * dnoff_dVd) + quot(Vgsteff, noff) * dnoff_dVd;
+      dVgsteff_dVb = -dVgsteff_dVg * (dVth_dVb + quot((Vgst - voffcv), noff) * dnoff_dVb) + quot(Vgsteff, noff) * dnoff_dVb;
       dVgsteff_dVg *= dVgs_eff_dVg;
     }
     double Cgg, Cgd, Cgb, Cbg, Cbd, Cbb, Csg, Csd, Csb;
@@ -872,7 +872,7 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       } else {
         T0 = 0.5 * k1ox;
         T1 = sqrt(T0 * T0 + Arg1);
-        T2 = CoxWL * T0 / T1;
+        T2 = quot(CoxWL * T0, T1);
         qgate = CoxWL * k1ox * (T1 - T0);
         Cgg = T2 * (dVgs_eff_dVg - dVgsteff_dVg);
         Cgd = -T2 * dVgsteff_dVd;
@@ -882,17 +882,17 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       Cbg = -Cgg;
       Cbd = -Cgd;
       Cbb = -Cgb;
-      const double One_Third_CoxWL = CoxWL / 3.0;
+      const double One_Third_CoxWL = quot_by_constant(CoxWL, 3.0);
       const double Two_Third_CoxWL = 2.0 * One_Third_CoxWL;
       AbulkCV = Abulk0 * P(abulkCVfactor);
       dAbulkCV_dVb = P(abulkCVfactor) * dAbulk0_dVb;
-      VdsatCV = Vgsteff / AbulkCV;
+      VdsatCV = quot(Vgsteff, AbulkCV);
       if (VdsatCV < Vds) {
-        const double dVdsatCV_dVg = 1.0 / AbulkCV;
-        const double dVdsatCV_dVb = -VdsatCV * dAbulkCV_dVb / AbulkCV;
-        T0 = Vgsteff - VdsatCV / 3.0;
-        dT0_dVg = 1.0 - dVdsatCV_dVg / 3.0;
-        dT0_dVb = -dVdsatCV_dVb / 3.0;
+        const double dVdsatCV_dVg = quot(1.0, AbulkCV);
+        const double dVdsatCV_dVb = quot(-VdsatCV * dAbulkCV_dVb, AbulkCV);
+        T0 = Vgsteff - quot_by_constant(VdsatCV, 3.0);
+        dT0_dVg = 1.0 - quot_by_constant(dVdsatCV_dVg, 3.0);
+        dT0_dVb = quot_by_constant(-dVdsatCV_dVb, 3.0);
         qgate += CoxWL * T0;
         Cgg1 = CoxWL * dT0_dVg;
         Cgb1 = CoxWL * dT0_dVb + Cgg1 * dVgsteff_dVb;
@@ -925,10 +925,10 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       } else {
         T0 = AbulkCV * Vds;
         T1 = 12.0 * (Vgsteff - 0.5 * T0 + 1.e-20);
-        T2 = Vds / T1;
+        T2 = quot(Vds, T1);
         T3 = T0 * T2;
         dT3_dVg = -12.0 * T2 * T2 * AbulkCV;
-        dT3_dVd = 6.0 * T0 * (4.0 * Vgsteff - T0) / T1 / T1 - 0.5;
+        dT3_dVd = quot(quot(6.0 * T0 * (4.0 * Vgsteff - T0), T1), T1) - 0.5;
         dT3_dVb = 12.0 * T2 * T2 * dAbulkCV_dVb * Vgsteff;
         qgate += CoxWL * (Vgsteff - 0.5 * Vds + T3);
         Cgg1 = CoxWL * (1.0 + dT3_dVg);
@@ -948,21 +948,21 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
         Cbd += Cbd1;
         if (xpart > 0.5) {  // 0/100
           T1 = T1 + T1;
-          qsrc = -CoxWL * (0.5 * Vgsteff + 0.25 * T0 - T0 * T0 / T1);
-          Csg = -CoxWL * (0.5 + 24.0 * T0 * Vds / T1 / T1 * AbulkCV);
-          Csb = -CoxWL * (0.25 * Vds * dAbulkCV_dVb - 12.0 * T0 * Vds / T1 / T1 * (4.0 * Vgsteff - T0) * dAbulkCV_dVb) +
+          qsrc = -CoxWL * (0.5 * Vgsteff + 0.25 * T0 - quot(T0 * T0, T1));
+          Csg = -CoxWL * (0.5 + quot(quot(24.0 * T0 * Vds, T1), T1) * AbulkCV);
+          Csb = -CoxWL * (0.25 * Vds * dAbulkCV_dVb - quot(quot(12.0 * T0 * Vds, T1), T1) * (4.0 * Vgsteff - T0) * dAbulkCV_dVb) +
                 Csg * dVgsteff_dVb;
-          Csd = -CoxWL * (0.25 * AbulkCV - 12.0 * AbulkCV * T0 / T1 / T1 * (4.0 * Vgsteff - T0)) + Csg * dVgsteff_dVd;
+          Csd = -CoxWL * (0.25 * AbulkCV - quot(quot(12.0 * AbulkCV * T0, T1), T1) * (4.0 * Vgsteff - T0)) + Csg * dVgsteff_dVd;
           Csg *= dVgsteff_dVg;
         } else if (xpart < 0.5) {  // 40/60
-          T1 = T1 / 12.0;
-          T2 = 0.5 * CoxWL / (T1 * T1);
-          T3 = Vgsteff * (2.0 * T0 * T0 / 3.0 + Vgsteff * (Vgsteff - 4.0 * T0 / 3.0)) - 2.0 * T0 * T0 * T0 / 15.0;
+          T1 = quot_by_constant(T1, 12.0);
+          T2 = quot(0.5 * CoxWL, T1 * T1);
+          T3 = Vgsteff * (quot_by_constant(2.0 * T0 * T0, 3.0) + Vgsteff * (Vgsteff - quot_by_constant(4.0 * T0, 3.0))) - quot_by_constant(2.0 * T0 * T0 * T0, 15.0);
           qsrc = -T2 * T3;
-          T4 = 4.0 / 3.0 * Vgsteff * (Vgsteff - T0) + 0.4 * T0 * T0;
-          Csg = -2.0 * qsrc / T1 - T2 * (Vgsteff * (3.0 * Vgsteff - 8.0 * T0 / 3.0) + 2.0 * T0 * T0 / 3.0);
-          Csb = (qsrc / T1 * Vds + T2 * T4 * Vds) * dAbulkCV_dVb + Csg * dVgsteff_dVb;
-          Csd = (qsrc / T1 + T2 * T4) * AbulkCV + Csg * dVgsteff_dVd;
+          T4 = quot_by_constant(4.0, 3.0) * Vgsteff * (Vgsteff - T0) + 0.4 * T0 * T0;
+          Csg = quot(-2.0 * qsrc, T1) - T2 * (Vgsteff * (3.0 * Vgsteff - quot_by_constant(8.0 * T0, 3.0)) + quot_by_constant(2.0 * T0 * T0, 3.0));
+          Csb = (quot(qsrc, T1) * Vds + T2 * T4 * Vds) * dAbulkCV_dVb + Csg * dVgsteff_dVb;
+          Csd = (quot(qsrc, T1) + T2 * T4) * AbulkCV + Csg * dVgsteff_dVd;
           Csg *= dVgsteff_dVg;
         } else {  // 50/50
           qsrc = -0.5 * (qgate + qbulk);
@@ -977,12 +977,12 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       V3 = Vfb - Vgs_eff + VbseffCV - CONSTDELTA_3;
       if (Vfb <= 0.0) {
         T0 = sqrt(V3 * V3 - 4.0 * CONSTDELTA_3 * Vfb);
-        T2 = -CONSTDELTA_3 / T0;
+        T2 = quot(-CONSTDELTA_3, T0);
       } else {
         T0 = sqrt(V3 * V3 + 4.0 * CONSTDELTA_3 * Vfb);
-        T2 = CONSTDELTA_3 / T0;
+        T2 = quot(CONSTDELTA_3, T0);
       }
-      T1 = 0.5 * (1.0 + V3 / T0);
+      T1 = 0.5 * (1.0 + quot(V3, T0));
       Vfbeff = Vfb - 0.5 * (V3 + T0);
       dVfbeff_dVg = T1 * dVgs_eff_dVg;
       dVfbeff_dVb = -T1 * dVbseffCV_dVb;
@@ -995,11 +995,11 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
         T1 = 0.0;
         T2 = 0.0;
       } else if (T3 < 0.0) {
-        T1 = T0 + T3 / k1ox;
+        T1 = T0 + quot(T3, k1ox);
         T2 = CoxWL;
       } else {
         T1 = sqrt(T0 * T0 + T3);
-        T2 = CoxWL * T0 / T1;
+        T2 = quot(CoxWL * T0, T1);
       }
       Qsub0 = CoxWL * k1ox * (T1 - T0);
       dQsub0_dVg = T2 * (dVgs_eff_dVg - dVfbeff_dVg - dVgsteff_dVg);
@@ -1007,13 +1007,13 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       dQsub0_dVb = -T2 * (dVfbeff_dVb + dVbseffCV_dVb + dVgsteff_dVb);
       AbulkCV = Abulk0 * P(abulkCVfactor);
       dAbulkCV_dVb = P(abulkCVfactor) * dAbulk0_dVb;
-      VdsatCV = Vgsteff / AbulkCV;
+      VdsatCV = quot(Vgsteff, AbulkCV);
       V4 = VdsatCV - Vds - CONSTDELTA_4;
       T0 = sqrt(V4 * V4 + 4.0 * CONSTDELTA_4 * VdsatCV);
       VdseffCV = VdsatCV - 0.5 * (V4 + T0);
-      T1 = 0.5 * (1.0 + V4 / T0);
-      T2 = CONSTDELTA_4 / T0;
-      T3 = (1.0 - T1 - T2) / AbulkCV;
+      T1 = 0.5 * (1.0 + quot(V4, T0));
+      T2 = quot(CONSTDELTA_4, T0);
+      T3 = quot((1.0 - T1 - T2), AbulkCV);
       dVdseffCV_dVg = T3;
       dVdseffCV_dVd = T1;
       dVdseffCV_dVb = -T3 * VdsatCV * dAbulkCV_dVb;
@@ -1024,10 +1024,10 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       }
       T0 = AbulkCV * VdseffCV;
       T1 = 12.0 * (Vgsteff - 0.5 * T0 + 1e-20);
-      T2 = VdseffCV / T1;
+      T2 = quot(VdseffCV, T1);
       T3 = T0 * T2;
       T4 = (1.0 - 12.0 * T2 * T2 * AbulkCV);
-      T5 = (6.0 * T0 * (4.0 * Vgsteff - T0) / (T1 * T1) - 0.5);
+      T5 = (quot(6.0 * T0 * (4.0 * Vgsteff - T0), T1 * T1) - 0.5);
       T6 = 12.0 * T2 * T2 * Vgsteff;
       qgate = CoxWL * (Vgsteff - 0.5 * VdseffCV + T3);
       Cgg1 = CoxWL * (T4 + T5 * dVdseffCV_dVg);
@@ -1045,9 +1045,9 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       Cbg1 *= dVgsteff_dVg;
       if (xpart > 0.5) {
         T1 = T1 + T1;
-        qsrc = -CoxWL * (0.5 * Vgsteff + 0.25 * T0 - T0 * T0 / T1);
-        T7 = (4.0 * Vgsteff - T0) / (T1 * T1);
-        T4 = -(0.5 + 24.0 * T0 * T0 / (T1 * T1));
+        qsrc = -CoxWL * (0.5 * Vgsteff + 0.25 * T0 - quot(T0 * T0, T1));
+        T7 = quot((4.0 * Vgsteff - T0), T1 * T1);
+        T4 = -(0.5 + quot(24.0 * T0 * T0, T1 * T1));
         T5 = -(0.25 * AbulkCV - 12.0 * AbulkCV * T0 * T7);
         T6 = -(0.25 * VdseffCV - 12.0 * T0 * VdseffCV * T7);
         Csg = CoxWL * (T4 + T5 * dVdseffCV_dVg);
@@ -1055,14 +1055,14 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
         Csb = CoxWL * (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Csg * dVgsteff_dVb;
         Csg *= dVgsteff_dVg;
       } else if (xpart < 0.5) {
-        T1 = T1 / 12.0;
-        T2 = 0.5 * CoxWL / (T1 * T1);
-        T3 = Vgsteff * (2.0 * T0 * T0 / 3.0 + Vgsteff * (Vgsteff - 4.0 * T0 / 3.0)) - 2.0 * T0 * T0 * T0 / 15.0;
+        T1 = quot_by_constant(T1, 12.0);
+        T2 = quot(0.5 * CoxWL, T1 * T1);
+        T3 = Vgsteff * (quot_by_constant(2.0 * T0 * T0, 3.0) + Vgsteff * (Vgsteff - quot_by_constant(4.0 * T0, 3.0))) - quot_by_constant(2.0 * T0 * T0 * T0, 15.0);
         qsrc = -T2 * T3;
-        T7 = 4.0 / 3.0 * Vgsteff * (Vgsteff - T0) + 0.4 * T0 * T0;
-        T4 = -2.0 * qsrc / T1 - T2 * (Vgsteff * (3.0 * Vgsteff - 8.0 * T0 / 3.0) + 2.0 * T0 * T0 / 3.0);
-        T5 = (qsrc / T1 + T2 * T7) * AbulkCV;
-        T6 = (qsrc / T1 * VdseffCV + T2 * T7 * VdseffCV);
+        T7 = quot_by_constant(4.0, 3.0) * Vgsteff * (Vgsteff - T0) + 0.4 * T0 * T0;
+        T4 = quot(-2.0 * qsrc, T1) - T2 * (Vgsteff * (3.0 * Vgsteff - quot_by_constant(8.0 * T0, 3.0)) + quot_by_constant(2.0 * T0 * T0, 3.0));
+        T5 = (quot(qsrc, T1) + T2 * T7) * AbulkCV;
+        T6 = (quot(qsrc, T1) * VdseffCV + T2 * T7 * VdseffCV);
         Csg = (T4 + T5 * dVdseffCV_dVg);
         Csd = T5 * dVdseffCV_dVd + Csg * dVgsteff_dVd;
         Csb = (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Csg * dVgsteff_dVb;
@@ -1087,20 +1087,20 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       V3 = vfbzb - Vgs_eff + VbseffCV - CONSTDELTA_3;
       if (vfbzb <= 0.0) {
         T0 = sqrt(V3 * V3 - 4.0 * CONSTDELTA_3 * vfbzb);
-        T2 = -CONSTDELTA_3 / T0;
+        T2 = quot(-CONSTDELTA_3, T0);
       } else {
         T0 = sqrt(V3 * V3 + 4.0 * CONSTDELTA_3 * vfbzb);
-        T2 = CONSTDELTA_3 / T0;
+        T2 = quot(CONSTDELTA_3, T0);
       }
-      T1 = 0.5 * (1.0 + V3 / T0);
+      T1 = 0.5 * (1.0 + quot(V3, T0));
       Vfbeff = vfbzb - 0.5 * (V3 + T0);
       dVfbeff_dVg = T1 * dVgs_eff_dVg;
       dVfbeff_dVb = -T1 * dVbseffCV_dVb;
       const double Cox = cox;
       double Tox = 1.0e8 * tox;
-      T0 = (Vgs_eff - VbseffCV - vfbzb) / Tox;
-      dT0_dVg = dVgs_eff_dVg / Tox;
-      dT0_dVb = -dVbseffCV_dVb / Tox;
+      T0 = quot((Vgs_eff - VbseffCV - vfbzb), Tox);
+      dT0_dVg = quot(dVgs_eff_dVg, Tox);
+      dT0_dVb = quot(-dVbseffCV_dVb, Tox);
       tmp = T0 * P(acde);
       double Tcen, dTcen_dVg, dTcen_dVd, dTcen_dVb;
       const double ldeb = P(ldeb);
@@ -1120,19 +1120,19 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       V3 = ldeb - Tcen - LINK;
       V4 = sqrt(V3 * V3 + 4.0 * LINK * ldeb);
       Tcen = ldeb - 0.5 * (V3 + V4);
-      T1 = 0.5 * (1.0 + V3 / V4);
+      T1 = 0.5 * (1.0 + quot(V3, V4));
       dTcen_dVg *= T1;
       dTcen_dVb *= T1;
-      double Ccen = CONSTEPSSI / Tcen;
-      T2 = Cox / (Cox + Ccen);
+      double Ccen = quot(CONSTEPSSI, Tcen);
+      T2 = quot(Cox, Cox + Ccen);
       double Coxeff = T2 * Ccen;
-      T3 = -Ccen / Tcen;
+      T3 = quot(-Ccen, Tcen);
       double dCoxeff_dVg = T2 * T2 * T3;
       double dCoxeff_dVb = dCoxeff_dVg * dTcen_dVb;
       dCoxeff_dVg *= dTcen_dVg;
-      double CoxWLcen = CoxWL * Coxeff / Cox;
+      double CoxWLcen = quot(CoxWL * Coxeff, Cox);
       Qac0 = CoxWLcen * (Vfbeff - vfbzb);
-      double QovCox = Qac0 / Coxeff;
+      double QovCox = quot(Qac0, Coxeff);
       dQac0_dVg = CoxWLcen * dVfbeff_dVg + QovCox * dCoxeff_dVg;
       dQac0_dVb = CoxWLcen * dVfbeff_dVb + QovCox * dCoxeff_dVb;
       T0 = 0.5 * k1ox;
@@ -1141,14 +1141,14 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
         T1 = 0.0;
         T2 = 0.0;
       } else if (T3 < 0.0) {
-        T1 = T0 + T3 / k1ox;
+        T1 = T0 + quot(T3, k1ox);
         T2 = CoxWLcen;
       } else {
         T1 = sqrt(T0 * T0 + T3);
-        T2 = CoxWLcen * T0 / T1;
+        T2 = quot(CoxWLcen * T0, T1);
       }
       Qsub0 = CoxWLcen * k1ox * (T1 - T0);
-      QovCox = Qsub0 / Coxeff;
+      QovCox = quot(Qsub0, Coxeff);
       dQsub0_dVg = T2 * (dVgs_eff_dVg - dVfbeff_dVg - dVgsteff_dVg) + QovCox * dCoxeff_dVg;
       dQsub0_dVd = -T2 * dVgsteff_dVd;
       dQsub0_dVb = -T2 * (dVfbeff_dVb + dVbseffCV_dVb + dVgsteff_dVb) + QovCox * dCoxeff_dVb;
@@ -1161,46 +1161,46 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
         T0 = k1ox * sqrtPhi;
       }
       T1 = 2.0 * T0 + Vgsteff;
-      const double DeltaPhi = Vtm * log(1.0 + T1 * Vgsteff / DenomiQ);
-      const double dDeltaPhi_dVg = 2.0 * Vtm * (T1 - T0) / (DenomiQ + T1 * Vgsteff);
+      const double DeltaPhi = Vtm * log(1.0 + quot(T1 * Vgsteff, DenomiQ));
+      const double dDeltaPhi_dVg = quot(2.0 * Vtm * (T1 - T0), DenomiQ + T1 * Vgsteff);
       T3 = 4.0 * (Vth - vfbzb - phi);
       Tox += Tox;
       if (T3 >= 0.0) {
-        T0 = (Vgsteff + T3) / Tox;
-        dT0_dVd = (dVgsteff_dVd + 4.0 * dVth_dVd) / Tox;
-        dT0_dVb = (dVgsteff_dVb + 4.0 * dVth_dVb) / Tox;
+        T0 = quot((Vgsteff + T3), Tox);
+        dT0_dVd = quot((dVgsteff_dVd + 4.0 * dVth_dVd), Tox);
+        dT0_dVb = quot((dVgsteff_dVb + 4.0 * dVth_dVb), Tox);
       } else {
-        T0 = (Vgsteff + 1.0e-20) / Tox;
-        dT0_dVd = dVgsteff_dVd / Tox;
-        dT0_dVb = dVgsteff_dVb / Tox;
+        T0 = quot((Vgsteff + 1.0e-20), Tox);
+        dT0_dVd = quot(dVgsteff_dVd, Tox);
+        dT0_dVb = quot(dVgsteff_dVb, Tox);
       }
       tmp = exp(0.7 * log(T0));
       T1 = 1.0 + tmp;
-      T2 = 0.7 * tmp / (T0 * Tox);
-      Tcen = 1.9e-9 / T1;
-      dTcen_dVg = -1.9e-9 * T2 / T1 / T1;
+      T2 = quot(0.7 * tmp, T0 * Tox);
+      Tcen = quot(1.9e-9, T1);
+      dTcen_dVg = quot(quot(-1.9e-9 * T2, T1), T1);
       dTcen_dVd = Tox * dTcen_dVg;
       dTcen_dVb = dTcen_dVd * dT0_dVb;
       dTcen_dVd *= dT0_dVd;
       dTcen_dVg *= dVgsteff_dVg;
-      Ccen = CONSTEPSSI / Tcen;
-      T0 = Cox / (Cox + Ccen);
+      Ccen = quot(CONSTEPSSI, Tcen);
+      T0 = quot(Cox, Cox + Ccen);
       Coxeff = T0 * Ccen;
-      T1 = -Ccen / Tcen;
+      T1 = quot(-Ccen, Tcen);
       dCoxeff_dVg = T0 * T0 * T1;
       const double dCoxeff_dVd = dCoxeff_dVg * dTcen_dVd;
       dCoxeff_dVb = dCoxeff_dVg * dTcen_dVb;
       dCoxeff_dVg *= dTcen_dVg;
-      CoxWLcen = CoxWL * Coxeff / Cox;
+      CoxWLcen = quot(CoxWL * Coxeff, Cox);
       AbulkCV = Abulk0 * P(abulkCVfactor);
       dAbulkCV_dVb = P(abulkCVfactor) * dAbulk0_dVb;
-      VdsatCV = (Vgsteff - DeltaPhi) / AbulkCV;
+      VdsatCV = quot((Vgsteff - DeltaPhi), AbulkCV);
       V4 = VdsatCV - Vds - CONSTDELTA_4;
       T0 = sqrt(V4 * V4 + 4.0 * CONSTDELTA_4 * VdsatCV);
       VdseffCV = VdsatCV - 0.5 * (V4 + T0);
-      T1 = 0.5 * (1.0 + V4 / T0);
-      T2 = CONSTDELTA_4 / T0;
-      T3 = (1.0 - T1 - T2) / AbulkCV;
+      T1 = 0.5 * (1.0 + quot(V4, T0));
+      T2 = quot(CONSTDELTA_4, T0);
+      T3 = quot((1.0 - T1 - T2), AbulkCV);
       T4 = T3 * (1.0 - dDeltaPhi_dVg);
       dVdseffCV_dVg = T4;
       dVdseffCV_dVd = T1;
@@ -1213,35 +1213,35 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       T0 = AbulkCV * VdseffCV;
       T1 = Vgsteff - DeltaPhi;
       T2 = 12.0 * (T1 - 0.5 * T0 + 1.0e-20);
-      T3 = T0 / T2;
+      T3 = quot(T0, T2);
       T4 = 1.0 - 12.0 * T3 * T3;
-      T5 = AbulkCV * (6.0 * T0 * (4.0 * T1 - T0) / (T2 * T2) - 0.5);
-      T6 = T5 * VdseffCV / AbulkCV;
+      T5 = AbulkCV * (quot(6.0 * T0 * (4.0 * T1 - T0), T2 * T2) - 0.5);
+      T6 = quot(T5 * VdseffCV, AbulkCV);
       qgate = CoxWLcen * (T1 - T0 * (0.5 - T3));
-      QovCox = qgate / Coxeff;
+      QovCox = quot(qgate, Coxeff);
       Cgg1 = CoxWLcen * (T4 * (1.0 - dDeltaPhi_dVg) + T5 * dVdseffCV_dVg);
       Cgd1 = CoxWLcen * T5 * dVdseffCV_dVd + Cgg1 * dVgsteff_dVd + QovCox * dCoxeff_dVd;
       Cgb1 = CoxWLcen * (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Cgg1 * dVgsteff_dVb + QovCox * dCoxeff_dVb;
       Cgg1 = Cgg1 * dVgsteff_dVg + QovCox * dCoxeff_dVg;
       T7 = 1.0 - AbulkCV;
       T8 = T2 * T2;
-      T9 = 12.0 * T7 * T0 * T0 / (T8 * AbulkCV);
+      T9 = quot(12.0 * T7 * T0 * T0, T8 * AbulkCV);
       T10 = T9 * (1.0 - dDeltaPhi_dVg);
-      T11 = -T7 * T5 / AbulkCV;
-      T12 = -(T9 * T1 / AbulkCV + VdseffCV * (0.5 - T0 / T2));
-      qbulk = CoxWLcen * T7 * (0.5 * VdseffCV - T0 * VdseffCV / T2);
-      QovCox = qbulk / Coxeff;
+      T11 = quot(-T7 * T5, AbulkCV);
+      T12 = -(quot(T9 * T1, AbulkCV) + VdseffCV * (0.5 - quot(T0, T2)));
+      qbulk = CoxWLcen * T7 * (0.5 * VdseffCV - quot(T0 * VdseffCV, T2));
+      QovCox = quot(qbulk, Coxeff);
       Cbg1 = CoxWLcen * (T10 + T11 * dVdseffCV_dVg);
       Cbd1 = CoxWLcen * T11 * dVdseffCV_dVd + Cbg1 * dVgsteff_dVd + QovCox * dCoxeff_dVd;
       Cbb1 = CoxWLcen * (T11 * dVdseffCV_dVb + T12 * dAbulkCV_dVb) + Cbg1 * dVgsteff_dVb + QovCox * dCoxeff_dVb;
       Cbg1 = Cbg1 * dVgsteff_dVg + QovCox * dCoxeff_dVg;
       if (xpart > 0.5) {
-        qsrc = -CoxWLcen * (T1 / 2.0 + T0 / 4.0 - 0.5 * T0 * T0 / T2);
-        QovCox = qsrc / Coxeff;
+        qsrc = -CoxWLcen * (quot_by_constant(T1, 2.0) + quot_by_constant(T0, 4.0) - quot(0.5 * T0 * T0, T2));
+        QovCox = quot(qsrc, Coxeff);
         T2 += T2;
         T3 = T2 * T2;
-        T7 = -(0.25 - 12.0 * T0 * (4.0 * T1 - T0) / T3);
-        T4 = -(0.5 + 24.0 * T0 * T0 / T3) * (1.0 - dDeltaPhi_dVg);
+        T7 = -(0.25 - quot(12.0 * T0 * (4.0 * T1 - T0), T3));
+        T4 = -(0.5 + quot(24.0 * T0 * T0, T3)) * (1.0 - dDeltaPhi_dVg);
         T5 = T7 * AbulkCV;
         T6 = T7 * VdseffCV;
         Csg = CoxWLcen * (T4 + T5 * dVdseffCV_dVg);
@@ -1249,15 +1249,15 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
         Csb = CoxWLcen * (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Csg * dVgsteff_dVb + QovCox * dCoxeff_dVb;
         Csg = Csg * dVgsteff_dVg + QovCox * dCoxeff_dVg;
       } else if (xpart < 0.5) {
-        T2 = T2 / 12.0;
-        T3 = 0.5 * CoxWLcen / (T2 * T2);
-        T4 = T1 * (2.0 * T0 * T0 / 3.0 + T1 * (T1 - 4.0 * T0 / 3.0)) - 2.0 * T0 * T0 * T0 / 15.0;
+        T2 = quot_by_constant(T2, 12.0);
+        T3 = quot(0.5 * CoxWLcen, T2 * T2);
+        T4 = T1 * (quot_by_constant(2.0 * T0 * T0, 3.0) + T1 * (T1 - quot_by_constant(4.0 * T0, 3.0))) - quot_by_constant(2.0 * T0 * T0 * T0, 15.0);
         qsrc = -T3 * T4;
-        QovCox = qsrc / Coxeff;
-        T8 = 4.0 / 3.0 * T1 * (T1 - T0) + 0.4 * T0 * T0;
-        T5 = -2.0 * qsrc / T2 - T3 * (T1 * (3.0 * T1 - 8.0 * T0 / 3.0) + 2.0 * T0 * T0 / 3.0);
-        T6 = AbulkCV * (qsrc / T2 + T3 * T8);
-        T7 = T6 * VdseffCV / AbulkCV;
+        QovCox = quot(qsrc, Coxeff);
+        T8 = quot_by_constant(4.0, 3.0) * T1 * (T1 - T0) + 0.4 * T0 * T0;
+        T5 = quot(-2.0 * qsrc, T2) - T3 * (T1 * (3.0 * T1 - quot_by_constant(8.0 * T0, 3.0)) + quot_by_constant(2.0 * T0 * T0, 3.0));
+        T6 = AbulkCV * (quot(qsrc, T2) + T3 * T8);
+        T7 = quot(T6 * VdseffCV, AbulkCV);
         Csg = T5 * (1.0 - dDeltaPhi_dVg) + T6 * dVdseffCV_dVg;
         Csd = Csg * dVgsteff_dVd + T6 * dVdseffCV_dVd + QovCox * dCoxeff_dVd;
         Csb = Csg * dVgsteff_dVb + T6 * dVdseffCV_dVb + T7 * dAbulkCV_dVb + QovCox * dCoxeff_dVb;
@@ -1308,38 +1308,38 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       capbs = czbs + czbssw + czbsswg;
     } else if (vbs < 0.0) {
       if (czbs > 0.0) {
-        arg = 1.0 - vbs / PhiBTemp;
+        arg = 1.0 - quot(vbs, PhiBTemp);
         if (MJ == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJ * log(arg));
-        qbs = PhiBTemp * czbs * (1.0 - arg * sarg) / (1.0 - MJ);
+        qbs = quot(PhiBTemp * czbs * (1.0 - arg * sarg), 1.0 - MJ);
         capbs = czbs * sarg;
       } else {
         qbs = 0.0;
         capbs = 0.0;
       }
       if (czbssw > 0.0) {
-        arg = 1.0 - vbs / PhiBSWTemp;
+        arg = 1.0 - quot(vbs, PhiBSWTemp);
         if (MJSW == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJSW * log(arg));
-        qbs += PhiBSWTemp * czbssw * (1.0 - arg * sarg) / (1.0 - MJSW);
+        qbs += quot(PhiBSWTemp * czbssw * (1.0 - arg * sarg), 1.0 - MJSW);
         capbs += czbssw * sarg;
       }
       if (czbsswg > 0.0) {
-        arg = 1.0 - vbs / PhiBSWGTemp;
+        arg = 1.0 - quot(vbs, PhiBSWGTemp);
         if (MJSWG == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJSWG * log(arg));
-        qbs += PhiBSWGTemp * czbsswg * (1.0 - arg * sarg) / (1.0 - MJSWG);
+        qbs += quot(PhiBSWGTemp * czbsswg * (1.0 - arg * sarg), 1.0 - MJSWG);
         capbs += czbsswg * sarg;
       }
     } else {
       T0 = czbs + czbssw + czbsswg;
-      T1 = vbs * (czbs * MJ / PhiBTemp + czbssw * MJSW / PhiBSWTemp + czbsswg * MJSWG / PhiBSWGTemp);
+      T1 = vbs * (quot(czbs * MJ, PhiBTemp) + quot(czbssw * MJSW, PhiBSWTemp) + quot(czbsswg * MJSWG, PhiBSWGTemp));
       qbs = vbs * (T0 + 0.5 * T1);
       capbs = T0 + T1;
     }
@@ -1348,38 +1348,38 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       capbd = czbd + czbdsw + czbdswg;
     } else if (vbd < 0.0) {
       if (czbd > 0.0) {
-        arg = 1.0 - vbd / PhiBTemp;
+        arg = 1.0 - quot(vbd, PhiBTemp);
         if (MJ == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJ * log(arg));
-        qbd = PhiBTemp * czbd * (1.0 - arg * sarg) / (1.0 - MJ);
+        qbd = quot(PhiBTemp * czbd * (1.0 - arg * sarg), 1.0 - MJ);
         capbd = czbd * sarg;
       } else {
         qbd = 0.0;
         capbd = 0.0;
       }
       if (czbdsw > 0.0) {
-        arg = 1.0 - vbd / PhiBSWTemp;
+        arg = 1.0 - quot(vbd, PhiBSWTemp);
         if (MJSW == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJSW * log(arg));
-        qbd += PhiBSWTemp * czbdsw * (1.0 - arg * sarg) / (1.0 - MJSW);
+        qbd += quot(PhiBSWTemp * czbdsw * (1.0 - arg * sarg), 1.0 - MJSW);
         capbd += czbdsw * sarg;
       }
       if (czbdswg > 0.0) {
-        arg = 1.0 - vbd / PhiBSWGTemp;
+        arg = 1.0 - quot(vbd, PhiBSWGTemp);
         if (MJSWG == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJSWG * log(arg));
-        qbd += PhiBSWGTemp * czbdswg * (1.0 - arg * sarg) / (1.0 - MJSWG);
+        qbd += quot(PhiBSWGTemp * czbdswg * (1.0 - arg * sarg), 1.0 - MJSWG);
         capbd += czbdswg * sarg;
       }
     } else {
       T0 = czbd + czbdsw + czbdswg;
-      T1 = vbd * (czbd * MJ / PhiBTemp + czbdsw * MJSW / PhiBSWTemp + czbdswg * MJSWG / PhiBSWGTemp);
+      T1 = vbd * (quot(czbd * MJ, PhiBTemp) + quot(czbdsw * MJSW, PhiBSWTemp) + quot(czbdswg * MJSWG, PhiBSWGTemp));
       qbd = vbd * (T0 + 0.5 * T1);
       capbd = T0 + T1;
     }
@@ -1393,16 +1393,16 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       qgso = P(cgso) * vgs;
     } else if ((int)P(capMod) == 1) {
       if (vgd < 0.0) {
-        T1 = sqrt(1.0 - 4.0 * vgd / ckappa);
-        cgdo = P(cgdo) + weffCV * P(cgdl) / T1;
+        T1 = sqrt(1.0 - quot(4.0 * vgd, ckappa));
+        cgdo = P(cgdo) + quot(weffCV * P(cgdl), T1);
         qgdo = P(cgdo) * vgd - weffCV * 0.5 * P(cgdl) * ckappa * (T1 - 1.0);
       } else {
         cgdo = P(cgdo) + weffCV * P(cgdl);
         qgdo = (weffCV * P(cgdl) + P(cgdo)) * vgd;
       }
       if (vgs < 0.0) {
-        T1 = sqrt(1.0 - 4.0 * vgs / ckappa);
-        cgso = P(cgso) + weffCV * P(cgsl) / T1;
+        T1 = sqrt(1.0 - quot(4.0 * vgs, ckappa));
+        cgso = P(cgso) + quot(weffCV * P(cgsl), T1);
         qgso = P(cgso) * vgs - weffCV * 0.5 * P(cgsl) * ckappa * (T1 - 1.0);
       } else {
         cgso = P(cgso) + weffCV * P(cgsl);
@@ -1413,15 +1413,15 @@ XD_HD void bsim3_load(const RV &P_, const double V[4], const double *sto_old, co
       T1 = sqrt(T0 * T0 + 4.0 * CONSTDELTA_1);
       T2 = 0.5 * (T0 - T1);
       T3 = weffCV * P(cgdl);
-      T4 = sqrt(1.0 - 4.0 * T2 / ckappa);
-      cgdo = P(cgdo) + T3 - T3 * (1.0 - 1.0 / T4) * (0.5 - 0.5 * T0 / T1);
+      T4 = sqrt(1.0 - quot(4.0 * T2, ckappa));
+      cgdo = P(cgdo) + T3 - T3 * (1.0 - quot(1.0, T4)) * (0.5 - quot(0.5 * T0, T1));
       qgdo = (P(cgdo) + T3) * vgd - T3 * (T2 + 0.5 * ckappa * (T4 - 1.0));
       T0 = vgs + CONSTDELTA_1;
       T1 = sqrt(T0 * T0 + 4.0 * CONSTDELTA_1);
       T2 = 0.5 * (T0 - T1);
       T3 = weffCV * P(cgsl);
-      T4 = sqrt(1.0 - 4.0 * T2 / ckappa);
-      cgso = P(cgso) + T3 - T3 * (1.0 - 1.0 / T4) * (0.5 - 0.5 * T0 / T1);
+      T4 = sqrt(1.0 - quot(4.0 * T2, ckappa));
+      cgso = P(cgso) + T3 - T3 * (1.0 - quot(1.0, T4)) * (0.5 - quot(0.5 * T0, T1));
       qgso = (P(cgso) + T3) * vgs - T3 * (T2 + 0.5 * ckappa * (T4 - 1.0));
     }
     // setupCapacitors_oldDAE (charge bookkeeping only, nqsMod = 0).

@@ -21,6 +21,7 @@
 #pragma once
 
 #include "bsim4_fields.h"
+#include "quot.h"
 #include "xd_consts.h"
 #include "mos_cv.h"
 
@@ -129,16 +130,16 @@ struct RecPtr {
 XD_HD void poly_depletion(double phi, double ngate, double epsgate, double coxe, double Vgs_arg, double &Vgs_eff,
                           double &dVgs_eff_dVg) {
   if ((ngate > 1.0e18) && (ngate < 1.0e25) && (Vgs_arg > phi) && (epsgate != 0)) {
-    double T1 = 1.0e6 * xdc::CONSTQ * epsgate * ngate / (coxe * coxe);
+    double T1 = quot(1.0e6 * xdc::CONSTQ * epsgate * ngate, coxe * coxe);
     double T8 = Vgs_arg - phi;
-    double T4 = sqrt(1.0 + 2.0 * T8 / T1);
-    double T2 = 2.0 * T8 / (T4 + 1.0);
-    double T3 = 0.5 * T2 * T2 / T1;
+    double T4 = sqrt(1.0 + quot(2.0 * T8, T1));
+    double T2 = quot(2.0 * T8, T4 + 1.0);
+    double T3 = quot(0.5 * T2 * T2, T1);
     double T7 = 1.12 - T3 - 0.05;
     double T6 = sqrt(T7 * T7 + 0.224);
     double T5 = 1.12 - 0.5 * (T7 + T6);
     Vgs_eff = Vgs_arg - T5;
-    dVgs_eff_dVg = 1.0 - (0.5 - 0.5 / T4) * (1.0 + T7 / T6);
+    dVgs_eff_dVg = 1.0 - (0.5 - quot(0.5, T4)) * (1.0 + quot(T7, T6));
   } else {
     Vgs_eff = Vgs_arg;
     dVgs_eff_dVg = 1.0;
@@ -354,7 +355,7 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
   const double Phis = phi - Vbseff;
   const double dPhis_dVb = -1.0;
   const double sqrtPhis = sqrt(Phis);
-  const double dsqrtPhis_dVb = -0.5 / sqrtPhis;
+  const double dsqrtPhis_dVb = quot(-0.5, sqrtPhis);
   const double Vtm = P(vtm);
   const double k1ox = P(k1ox);
   const double coxe = P(coxe);
@@ -412,7 +413,7 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       const double dnoff_dVb = P(noff) * dn_dVb;
       T0 = Vtm * noff;
       const double voffcv = P(voffcv);
-      const double VgstNVt = (Vgst - voffcv) / T0;
+      const double VgstNVt = quot((Vgst - voffcv), T0);
       if (VgstNVt > CONSTEXP_THRESHOLD) {
         Vgsteff = Vgst - voffcv;
         dVgsteff_dVg = dVgs_eff_dVg;
@@ -421,22 +422,22 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       } else if (VgstNVt < -CONSTEXP_THRESHOLD) {
         Vgsteff = T0 * log(1.0 + CONSTMIN_EXP);
         dVgsteff_dVg = 0.0;
-        dVgsteff_dVd = Vgsteff / noff;
+        dVgsteff_dVd = quot(Vgsteff, noff);
         dVgsteff_dVb = dVgsteff_dVd * dnoff_dVb;
         dVgsteff_dVd *= dnoff_dVd;
       } else {
         const double ExpVgst = exp(VgstNVt);
         Vgsteff = T0 * log(1.0 + ExpVgst);
-        dVgsteff_dVg = ExpVgst / (1.0 + ExpVgst);
-        dVgsteff_dVd = -dVgsteff_dVg * (dVth_dVd + (Vgst - voffcv) / noff * dnoff_dVd) + Vgsteff / noff * dnoff_dVd;
-        dVgsteff_dVb = -dVgsteff_dVg * (dVth_dVb + (Vgst - voffcv) / noff * dnoff_dVb) + Vgsteff / noff * dnoff_dVb;
+        dVgsteff_dVg = quot(ExpVgst, 1.0 + ExpVgst);
+        dVgsteff_dVd = -dVgsteff_dVg * (dVth_dVd + quot((Vgst - voffcv), noff) * dnoff_dVd) + quot(Vgsteff, noff) * dnoff_dVd;
+        dVgsteff_dVb = -dVgsteff_dVg * (dVth_dVb + quot((Vgst - voffcv), noff) * dnoff_dVb) + quot(Vgsteff, noff) * dnoff_dVb;
         dVgsteff_dVg *= dVgs_eff_dVg;
       }
     } else {
       const double mstarcv = P(mstarcv);
       T0 = n * Vtm;
       T1 = mstarcv * Vgst;
-      T2 = T1 / T0;
+      T2 = quot(T1, T0);
       if (T2 > CONSTEXP_THRESHOLD) {
         T10 = T1;
         dT10_dVg = mstarcv * dVgs_eff_dVg;
@@ -452,41 +453,41 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
         const double ExpVgst = exp(T2);
         T3 = Vtm * log(1.0 + ExpVgst);
         T10 = n * T3;
-        dT10_dVg = mstarcv * ExpVgst / (1.0 + ExpVgst);
-        dT10_dVb = T3 * dn_dVb - dT10_dVg * (dVth_dVb + Vgst * dn_dVb / n);
-        dT10_dVd = T3 * dn_dVd - dT10_dVg * (dVth_dVd + Vgst * dn_dVd / n);
+        dT10_dVg = quot(mstarcv * ExpVgst, 1.0 + ExpVgst);
+        dT10_dVb = T3 * dn_dVb - dT10_dVg * (dVth_dVb + quot(Vgst * dn_dVb, n));
+        dT10_dVd = T3 * dn_dVd - dT10_dVg * (dVth_dVd + quot(Vgst * dn_dVd, n));
         dT10_dVg *= dVgs_eff_dVg;
       }
       T1 = P(voffcbncv) - (1.0 - mstarcv) * Vgst;
-      T2 = T1 / T0;
+      T2 = quot(T1, T0);
       if (T2 < -CONSTEXP_THRESHOLD) {
-        T3 = coxe * CONSTMIN_EXP / P(cdep0);
+        T3 = quot(coxe * CONSTMIN_EXP, P(cdep0));
         T9 = mstarcv + T3 * n;
         dT9_dVg = 0.0;
         dT9_dVd = dn_dVd * T3;
         dT9_dVb = dn_dVb * T3;
       } else if (T2 > CONSTEXP_THRESHOLD) {
-        T3 = coxe * CONSTMAX_EXP / P(cdep0);
+        T3 = quot(coxe * CONSTMAX_EXP, P(cdep0));
         T9 = mstarcv + T3 * n;
         dT9_dVg = 0.0;
         dT9_dVd = dn_dVd * T3;
         dT9_dVb = dn_dVb * T3;
       } else {
         const double ExpVgst = exp(T2);
-        T3 = coxe / P(cdep0);
+        T3 = quot(coxe, P(cdep0));
         T4 = T3 * ExpVgst;
-        T5 = T1 * T4 / T0;
+        T5 = quot(T1 * T4, T0);
         T9 = mstarcv + n * T4;
-        dT9_dVg = T3 * (mstarcv - 1.0) * ExpVgst / Vtm;
+        dT9_dVg = quot(T3 * (mstarcv - 1.0) * ExpVgst, Vtm);
         dT9_dVb = T4 * dn_dVb - dT9_dVg * dVth_dVb - T5 * dn_dVb;
         dT9_dVd = T4 * dn_dVd - dT9_dVg * dVth_dVd - T5 * dn_dVd;
         dT9_dVg *= dVgs_eff_dVg;
       }
-      Vgsteff = T10 / T9;
+      Vgsteff = quot(T10, T9);
       T11 = T9 * T9;
-      dVgsteff_dVg = (T9 * dT10_dVg - T10 * dT9_dVg) / T11;
-      dVgsteff_dVd = (T9 * dT10_dVd - T10 * dT9_dVd) / T11;
-      dVgsteff_dVb = (T9 * dT10_dVb - T10 * dT9_dVb) / T11;
+      dVgsteff_dVg = quot((T9 * dT10_dVg - T10 * dT9_dVg), T11);
+      dVgsteff_dVd = quot((T9 * dT10_dVd - T10 * dT9_dVd), T11);
+      dVgsteff_dVb = quot((T9 * dT10_dVb - T10 * dT9_dVb), T11);
     }
     if (capMod == 1) {
       // capMod = 1 (:11139-11319): accumulation and depletion charges Qac0 / Qsub0 with the
@@ -497,7 +498,7 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
         T0 = sqrt(V3 * V3 - 4.0 * CONSTDELTA_3 * Vfb1);
       else
         T0 = sqrt(V3 * V3 + 4.0 * CONSTDELTA_3 * Vfb1);
-      T1 = 0.5 * (1.0 + V3 / T0);
+      T1 = 0.5 * (1.0 + quot(V3, T0));
       const double Vfbeff = Vfb1 - 0.5 * (V3 + T0);
       const double dVfbeff_dVg = T1 * dVgs_eff_dVg;
       const double dVfbeff_dVb = -T1 * dVbseffCV_dVb;
@@ -511,11 +512,11 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
         T1 = 0.0;
         T2 = 0.0;
       } else if (T3 < 0.0) {
-        T1 = T0 + T3 / k1ox1;
+        T1 = T0 + quot(T3, k1ox1);
         T2 = CoxWL;
       } else {
         T1 = sqrt(T0 * T0 + T3);
-        T2 = CoxWL * T0 / T1;
+        T2 = quot(CoxWL * T0, T1);
       }
       const double Qsub0 = CoxWL * k1ox1 * (T1 - T0);
       const double dQsub0_dVg = T2 * (dVgs_eff_dVg - dVfbeff_dVg - dVgsteff_dVg);
@@ -523,13 +524,13 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       const double dQsub0_dVb = -T2 * (dVfbeff_dVb + dVbseffCV_dVb + dVgsteff_dVb);
       const double AbulkCV = Abulk0 * P(abulkCVfactor);
       const double dAbulkCV_dVb = P(abulkCVfactor) * dAbulk0_dVb;
-      const double VdsatCV = Vgsteff / AbulkCV;
+      const double VdsatCV = quot(Vgsteff, AbulkCV);
       T0 = VdsatCV - Vds - CONSTDELTA_4;
-      dT0_dVg = 1.0 / AbulkCV;
-      dT0_dVb = -VdsatCV * dAbulkCV_dVb / AbulkCV;
+      dT0_dVg = quot(1.0, AbulkCV);
+      dT0_dVb = quot(-VdsatCV * dAbulkCV_dVb, AbulkCV);
       T1 = sqrt(T0 * T0 + 4.0 * CONSTDELTA_4 * VdsatCV);
-      dT1_dVg = (T0 + CONSTDELTA_4 + CONSTDELTA_4) / T1;
-      dT1_dVd = -T0 / T1;
+      dT1_dVg = quot((T0 + CONSTDELTA_4 + CONSTDELTA_4), T1);
+      dT1_dVd = quot(-T0, T1);
       dT1_dVb = dT1_dVg * dT0_dVb;
       dT1_dVg *= dT0_dVg;
       double VdseffCV, dVdseffCV_dVg, dVdseffCV_dVd, dVdseffCV_dVb;
@@ -539,9 +540,9 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
         dVdseffCV_dVd = 0.5 * (1.0 - dT1_dVd);
         dVdseffCV_dVb = 0.5 * (dT0_dVb - dT1_dVb);
       } else {
-        T3 = (CONSTDELTA_4 + CONSTDELTA_4) / (T1 - T0);
+        T3 = quot((CONSTDELTA_4 + CONSTDELTA_4), T1 - T0);
         T4 = 1.0 - T3;
-        T5 = VdsatCV * T3 / (T1 - T0);
+        T5 = quot(VdsatCV * T3, T1 - T0);
         VdseffCV = VdsatCV * T4;
         dVdseffCV_dVg = dT0_dVg * T4 + T5 * (dT1_dVg - dT0_dVg);
         dVdseffCV_dVd = T5 * (dT1_dVd + 1.0);
@@ -554,10 +555,10 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       }
       T0 = AbulkCV * VdseffCV;
       T1 = 12.0 * (Vgsteff - 0.5 * T0 + 1.0e-20);
-      T2 = VdseffCV / T1;
+      T2 = quot(VdseffCV, T1);
       T3 = T0 * T2;
       T4 = (1.0 - 12.0 * T2 * T2 * AbulkCV);
-      T5 = (6.0 * T0 * (4.0 * Vgsteff - T0) / (T1 * T1) - 0.5);
+      T5 = (quot(6.0 * T0 * (4.0 * Vgsteff - T0), T1 * T1) - 0.5);
       T6 = 12.0 * T2 * T2 * Vgsteff;
       qgate = CoxWL * (Vgsteff - 0.5 * VdseffCV + T3);
       double Cgg1 = CoxWL * (T4 + T5 * dVdseffCV_dVg);
@@ -577,9 +578,9 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       const double xpart = P(xpart);
       if (xpart > 0.5) {  // 0/100
         T1 = T1 + T1;
-        qsrc = -CoxWL * (0.5 * Vgsteff + 0.25 * T0 - T0 * T0 / T1);
-        T7 = (4.0 * Vgsteff - T0) / (T1 * T1);
-        T4 = -(0.5 + 24.0 * T0 * T0 / (T1 * T1));
+        qsrc = -CoxWL * (0.5 * Vgsteff + 0.25 * T0 - quot(T0 * T0, T1));
+        T7 = quot((4.0 * Vgsteff - T0), T1 * T1);
+        T4 = -(0.5 + quot(24.0 * T0 * T0, T1 * T1));
         T5 = -(0.25 * AbulkCV - 12.0 * AbulkCV * T0 * T7);
         T6 = -(0.25 * VdseffCV - 12.0 * T0 * VdseffCV * T7);
         Csg = CoxWL * (T4 + T5 * dVdseffCV_dVg);
@@ -587,14 +588,14 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
         Csb = CoxWL * (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Csg * dVgsteff_dVb;
         Csg *= dVgsteff_dVg;
       } else if (xpart < 0.5) {  // 40/60
-        T1 = T1 / 12.0;
-        T2 = 0.5 * CoxWL / (T1 * T1);
-        T3 = Vgsteff * (2.0 * T0 * T0 / 3.0 + Vgsteff * (Vgsteff - 4.0 * T0 / 3.0)) - 2.0 * T0 * T0 * T0 / 15.0;
+        T1 = quot_by_constant(T1, 12.0);
+        T2 = quot(0.5 * CoxWL, T1 * T1);
+        T3 = Vgsteff * (quot_by_constant(2.0 * T0 * T0, 3.0) + Vgsteff * (Vgsteff - quot_by_constant(4.0 * T0, 3.0))) - quot_by_constant(2.0 * T0 * T0 * T0, 15.0);
         qsrc = -T2 * T3;
-        T7 = 4.0 / 3.0 * Vgsteff * (Vgsteff - T0) + 0.4 * T0 * T0;
-        T4 = -2.0 * qsrc / T1 - T2 * (Vgsteff * (3.0 * Vgsteff - 8.0 * T0 / 3.0) + 2.0 * T0 * T0 / 3.0);
-        T5 = (qsrc / T1 + T2 * T7) * AbulkCV;
-        T6 = (qsrc / T1 * VdseffCV + T2 * T7 * VdseffCV);
+        T7 = quot_by_constant(4.0, 3.0) * Vgsteff * (Vgsteff - T0) + 0.4 * T0 * T0;
+        T4 = quot(-2.0 * qsrc, T1) - T2 * (Vgsteff * (3.0 * Vgsteff - quot_by_constant(8.0 * T0, 3.0)) + quot_by_constant(2.0 * T0 * T0, 3.0));
+        T5 = (quot(qsrc, T1) + T2 * T7) * AbulkCV;
+        T6 = (quot(qsrc, T1) * VdseffCV + T2 * T7 * VdseffCV);
         Csg = (T4 + T5 * dVdseffCV_dVg);
         Csd = T5 * dVdseffCV_dVd + Csg * dVgsteff_dVd;
         Csb = (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Csg * dVgsteff_dVb;
@@ -634,15 +635,15 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       T0 = sqrt(V3 * V3 - 4.0 * CONSTDELTA_3 * vfbzb);
     else
       T0 = sqrt(V3 * V3 + 4.0 * CONSTDELTA_3 * vfbzb);
-    T1 = 0.5 * (1.0 + V3 / T0);
+    T1 = 0.5 * (1.0 + quot(V3, T0));
     const double Vfbeff = vfbzb - 0.5 * (V3 + T0);
     const double dVfbeff_dVg = T1 * dVgs_eff_dVg;
     const double dVfbeff_dVb = -T1 * dVbseffCV_dVb;
     const double Cox = coxp;
     double Tox = 1.0e8 * P(toxp);
-    T0 = (Vgs_eff - VbseffCV - vfbzb) / Tox;
-    dT0_dVg = dVgs_eff_dVg / Tox;
-    dT0_dVb = -dVbseffCV_dVb / Tox;
+    T0 = quot((Vgs_eff - VbseffCV - vfbzb), Tox);
+    dT0_dVg = quot(dVgs_eff_dVg, Tox);
+    dT0_dVb = quot(-dVbseffCV_dVb, Tox);
     tmp = T0 * P(acde);
     const double ldeb = P(ldeb);
     double dTcen_dVb, dTcen_dVd;
@@ -662,19 +663,19 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
     V3 = ldeb - Tcen - LINK;
     const double V4 = sqrt(V3 * V3 + 4.0 * LINK * ldeb);
     Tcen = ldeb - 0.5 * (V3 + V4);
-    T1 = 0.5 * (1.0 + V3 / V4);
+    T1 = 0.5 * (1.0 + quot(V3, V4));
     dTcen_dVg *= T1;
     dTcen_dVb *= T1;
-    double Ccen = epssub / Tcen;
-    T2 = Cox / (Cox + Ccen);
+    double Ccen = quot(epssub, Tcen);
+    T2 = quot(Cox, Cox + Ccen);
     Coxeff = T2 * Ccen;
-    T3 = -Ccen / Tcen;
+    T3 = quot(-Ccen, Tcen);
     dCoxeff_dVg = T2 * T2 * T3;
     double dCoxeff_dVb = dCoxeff_dVg * dTcen_dVb;
     dCoxeff_dVg *= dTcen_dVg;
-    double CoxWLcen = CoxWL * Coxeff / coxe;
+    double CoxWLcen = quot(CoxWL * Coxeff, coxe);
     const double Qac0 = CoxWLcen * (Vfbeff - vfbzb);
-    double QovCox = Qac0 / Coxeff;
+    double QovCox = quot(Qac0, Coxeff);
     const double dQac0_dVg = CoxWLcen * dVfbeff_dVg + QovCox * dCoxeff_dVg;
     const double dQac0_dVb = CoxWLcen * dVfbeff_dVb + QovCox * dCoxeff_dVb;
     T0 = 0.5 * k1ox;
@@ -683,14 +684,14 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       T1 = 0.0;
       T2 = 0.0;
     } else if (T3 < 0.0) {
-      T1 = T0 + T3 / k1ox;
+      T1 = T0 + quot(T3, k1ox);
       T2 = CoxWLcen;
     } else {
       T1 = sqrt(T0 * T0 + T3);
-      T2 = CoxWLcen * T0 / T1;
+      T2 = quot(CoxWLcen * T0, T1);
     }
     const double Qsub0 = CoxWLcen * k1ox * (T1 - T0);
-    QovCox = Qsub0 / Coxeff;
+    QovCox = quot(Qsub0, Coxeff);
     const double dQsub0_dVg = T2 * (dVgs_eff_dVg - dVfbeff_dVg - dVgsteff_dVg) + QovCox * dCoxeff_dVg;
     const double dQsub0_dVd = -T2 * dVgsteff_dVd;
     const double dQsub0_dVb = -T2 * (dVfbeff_dVb + dVbseffCV_dVb + dVgsteff_dVb) + QovCox * dCoxeff_dVb;
@@ -702,41 +703,41 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       T0 = k1ox * sqrtPhi_p;
     }
     T1 = 2.0 * T0 + Vgsteff;
-    const double DeltaPhi = Vtm * log(1.0 + T1 * Vgsteff / Denomi);
-    const double dDeltaPhi_dVg = 2.0 * Vtm * (T1 - T0) / (Denomi + T1 * Vgsteff);
+    const double DeltaPhi = Vtm * log(1.0 + quot(T1 * Vgsteff, Denomi));
+    const double dDeltaPhi_dVg = quot(2.0 * Vtm * (T1 - T0), Denomi + T1 * Vgsteff);
     T0 = Vgsteff - DeltaPhi - 0.001;
     dT0_dVg = 1.0 - dDeltaPhi_dVg;
     T1 = sqrt(T0 * T0 + Vgsteff * 0.004);
     const double VgDP = 0.5 * (T0 + T1);
-    const double dVgDP_dVg = 0.5 * (dT0_dVg + (T0 * dT0_dVg + 0.002) / T1);
+    const double dVgDP_dVg = 0.5 * (dT0_dVg + quot((T0 * dT0_dVg + 0.002), T1));
     Tox += Tox;
-    T0 = (Vgsteff + P(vtfbphi2)) / Tox;
+    T0 = quot((Vgsteff + P(vtfbphi2)), Tox);
     tmp = exp(P(bdos) * 0.7 * log(T0));
     T1 = 1.0 + tmp;
-    T2 = P(bdos) * 0.7 * tmp / (T0 * Tox);
-    Tcen = P(ados) * 1.9e-9 / T1;
-    dTcen_dVg = -Tcen * T2 / T1;
+    T2 = quot(P(bdos) * 0.7 * tmp, T0 * Tox);
+    Tcen = quot(P(ados) * 1.9e-9, T1);
+    dTcen_dVg = quot(-Tcen * T2, T1);
     dTcen_dVd = dTcen_dVg * dVgsteff_dVd;
     dTcen_dVb = dTcen_dVg * dVgsteff_dVb;
     dTcen_dVg *= dVgsteff_dVg;
-    Ccen = epssub / Tcen;
-    T0 = Cox / (Cox + Ccen);
+    Ccen = quot(epssub, Tcen);
+    T0 = quot(Cox, Cox + Ccen);
     Coxeff = T0 * Ccen;
-    T1 = -Ccen / Tcen;
+    T1 = quot(-Ccen, Tcen);
     dCoxeff_dVg = T0 * T0 * T1;
     const double dCoxeff_dVd = dCoxeff_dVg * dTcen_dVd;
     dCoxeff_dVb = dCoxeff_dVg * dTcen_dVb;
     dCoxeff_dVg *= dTcen_dVg;
-    CoxWLcen = CoxWL * Coxeff / coxe;
+    CoxWLcen = quot(CoxWL * Coxeff, coxe);
     const double AbulkCV = Abulk0 * P(abulkCVfactor);
     const double dAbulkCV_dVb = P(abulkCVfactor) * dAbulk0_dVb;
-    const double VdsatCV = VgDP / AbulkCV;
+    const double VdsatCV = quot(VgDP, AbulkCV);
     T0 = VdsatCV - Vds - CONSTDELTA_4;
-    dT0_dVg = dVgDP_dVg / AbulkCV;
-    dT0_dVb = -VdsatCV * dAbulkCV_dVb / AbulkCV;
+    dT0_dVg = quot(dVgDP_dVg, AbulkCV);
+    dT0_dVb = quot(-VdsatCV * dAbulkCV_dVb, AbulkCV);
     T1 = sqrt(T0 * T0 + 4.0 * CONSTDELTA_4 * VdsatCV);
-    dT1_dVg = (T0 + CONSTDELTA_4 + CONSTDELTA_4) / T1;
-    dT1_dVd = -T0 / T1;
+    dT1_dVg = quot((T0 + CONSTDELTA_4 + CONSTDELTA_4), T1);
+    dT1_dVd = quot(-T0, T1);
     dT1_dVb = dT1_dVg * dT0_dVb;
     dT1_dVg *= dT0_dVg;
     double VdseffCV, dVdseffCV_dVg, dVdseffCV_dVd, dVdseffCV_dVb;
@@ -746,9 +747,9 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       dVdseffCV_dVd = 0.5 * (1.0 - dT1_dVd);
       dVdseffCV_dVb = 0.5 * (dT0_dVb - dT1_dVb);
     } else {
-      T3 = (CONSTDELTA_4 + CONSTDELTA_4) / (T1 - T0);
+      T3 = quot((CONSTDELTA_4 + CONSTDELTA_4), T1 - T0);
       T4 = 1.0 - T3;
-      T5 = VdsatCV * T3 / (T1 - T0);
+      T5 = quot(VdsatCV * T3, T1 - T0);
       VdseffCV = VdsatCV * T4;
       dVdseffCV_dVg = dT0_dVg * T4 + T5 * (dT1_dVg - dT0_dVg);
       dVdseffCV_dVd = T5 * (dT1_dVd + 1.0);
@@ -762,24 +763,24 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
     T0 = AbulkCV * VdseffCV;
     T1 = VgDP;
     T2 = 12.0 * (T1 - 0.5 * T0 + 1.0e-20);
-    T3 = T0 / T2;
+    T3 = quot(T0, T2);
     T4 = 1.0 - 12.0 * T3 * T3;
-    T5 = AbulkCV * (6.0 * T0 * (4.0 * T1 - T0) / (T2 * T2) - 0.5);
-    T6 = T5 * VdseffCV / AbulkCV;
+    T5 = AbulkCV * (quot(6.0 * T0 * (4.0 * T1 - T0), T2 * T2) - 0.5);
+    T6 = quot(T5 * VdseffCV, AbulkCV);
     qgate = CoxWLcen * (T1 - T0 * (0.5 - T3));
-    QovCox = qgate / Coxeff;
+    QovCox = quot(qgate, Coxeff);
     double Cgg1 = CoxWLcen * (T4 * dVgDP_dVg + T5 * dVdseffCV_dVg);
     const double Cgd1 = CoxWLcen * T5 * dVdseffCV_dVd + Cgg1 * dVgsteff_dVd + QovCox * dCoxeff_dVd;
     const double Cgb1 = CoxWLcen * (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Cgg1 * dVgsteff_dVb + QovCox * dCoxeff_dVb;
     Cgg1 = Cgg1 * dVgsteff_dVg + QovCox * dCoxeff_dVg;
     T7 = 1.0 - AbulkCV;
     T8 = T2 * T2;
-    T9 = 12.0 * T7 * T0 * T0 / (T8 * AbulkCV);
+    T9 = quot(12.0 * T7 * T0 * T0, T8 * AbulkCV);
     T10 = T9 * dVgDP_dVg;
-    T11 = -T7 * T5 / AbulkCV;
-    T12 = -(T9 * T1 / AbulkCV + VdseffCV * (0.5 - T0 / T2));
-    qbulk = CoxWLcen * T7 * (0.5 * VdseffCV - T0 * VdseffCV / T2);
-    QovCox = qbulk / Coxeff;
+    T11 = quot(-T7 * T5, AbulkCV);
+    T12 = -(quot(T9 * T1, AbulkCV) + VdseffCV * (0.5 - quot(T0, T2)));
+    qbulk = CoxWLcen * T7 * (0.5 * VdseffCV - quot(T0 * VdseffCV, T2));
+    QovCox = quot(qbulk, Coxeff);
     double Cbg1 = CoxWLcen * (T10 + T11 * dVdseffCV_dVg);
     const double Cbd1 = CoxWLcen * T11 * dVdseffCV_dVd + Cbg1 * dVgsteff_dVd + QovCox * dCoxeff_dVd;
     const double Cbb1 = CoxWLcen * (T11 * dVdseffCV_dVb + T12 * dAbulkCV_dVb) + Cbg1 * dVgsteff_dVb + QovCox * dCoxeff_dVb;
@@ -787,12 +788,12 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
     double Csg, Csd, Csb;
     const double xpart = P(xpart);
     if (xpart > 0.5) {
-      qsrc = -CoxWLcen * (T1 / 2.0 + T0 / 4.0 - 0.5 * T0 * T0 / T2);
-      QovCox = qsrc / Coxeff;
+      qsrc = -CoxWLcen * (quot_by_constant(T1, 2.0) + quot_by_constant(T0, 4.0) - quot(0.5 * T0 * T0, T2));
+      QovCox = quot(qsrc, Coxeff);
       T2 += T2;
       T3 = T2 * T2;
-      T7 = -(0.25 - 12.0 * T0 * (4.0 * T1 - T0) / T3);
-      T4 = -(0.5 + 24.0 * T0 * T0 / T3) * dVgDP_dVg;
+      T7 = -(0.25 - quot(12.0 * T0 * (4.0 * T1 - T0), T3));
+      T4 = -(0.5 + quot(24.0 * T0 * T0, T3)) * dVgDP_dVg;
       T5 = T7 * AbulkCV;
       T6 = T7 * VdseffCV;
       Csg = CoxWLcen * (T4 + T5 * dVdseffCV_dVg);
@@ -800,15 +801,15 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       Csb = CoxWLcen * (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Csg * dVgsteff_dVb + QovCox * dCoxeff_dVb;
       Csg = Csg * dVgsteff_dVg + QovCox * dCoxeff_dVg;
     } else if (xpart < 0.5) {
-      T2 = T2 / 12.0;
-      T3 = 0.5 * CoxWLcen / (T2 * T2);
-      T4 = T1 * (2.0 * T0 * T0 / 3.0 + T1 * (T1 - 4.0 * T0 / 3.0)) - 2.0 * T0 * T0 * T0 / 15.0;
+      T2 = quot_by_constant(T2, 12.0);
+      T3 = quot(0.5 * CoxWLcen, T2 * T2);
+      T4 = T1 * (quot_by_constant(2.0 * T0 * T0, 3.0) + T1 * (T1 - quot_by_constant(4.0 * T0, 3.0))) - quot_by_constant(2.0 * T0 * T0 * T0, 15.0);
       qsrc = -T3 * T4;
-      QovCox = qsrc / Coxeff;
-      T8 = 4.0 / 3.0 * T1 * (T1 - T0) + 0.4 * T0 * T0;
-      T5 = -2.0 * qsrc / T2 - T3 * (T1 * (3.0 * T1 - 8.0 * T0 / 3.0) + 2.0 * T0 * T0 / 3.0);
-      T6 = AbulkCV * (qsrc / T2 + T3 * T8);
-      T7 = T6 * VdseffCV / AbulkCV;
+      QovCox = quot(qsrc, Coxeff);
+      T8 = quot_by_constant(4.0, 3.0) * T1 * (T1 - T0) + 0.4 * T0 * T0;
+      T5 = quot(-2.0 * qsrc, T2) - T3 * (T1 * (3.0 * T1 - quot_by_constant(8.0 * T0, 3.0)) + quot_by_constant(2.0 * T0 * T0, 3.0));
+      T6 = AbulkCV * (quot(qsrc, T2) + T3 * T8);
+      T7 = quot(T6 * VdseffCV, AbulkCV);
       Csg = T5 * dVgDP_dVg + T6 * dVdseffCV_dVg;
       Csd = Csg * dVgsteff_dVd + T6 * dVdseffCV_dVd + QovCox * dCoxeff_dVd;
       Csb = Csg * dVgsteff_dVb + T6 * dVdseffCV_dVb + T7 * dAbulkCV_dVb + QovCox * dCoxeff_dVb;
@@ -856,7 +857,7 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
     cqsb = -(cgsb + cbsb);
     cqbb = -(cqgb + cqdb + cqsb);
     CoxWL = P(coxe) * P(weffCV) * nf * P(leffCV);
-    gtau = m.v[m_gcrg] / CoxWL * ScalingFactor;
+    gtau = quot(m.v[m_gcrg], CoxWL) * ScalingFactor;
   }
   double qcheq = qchqs;
 
@@ -881,38 +882,38 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       capbs = czbs + czbssw + czbsswg;
     } else if (vbs_jct < 0.0) {
       if (czbs > 0.0) {
-        arg = 1.0 - vbs_jct / P(PhiBS);
+        arg = 1.0 - quot(vbs_jct, P(PhiBS));
         if (MJS == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJS * log(arg));
-        qbs = P(PhiBS) * czbs * (1.0 - arg * sarg) / (1.0 - MJS);
+        qbs = quot(P(PhiBS) * czbs * (1.0 - arg * sarg), 1.0 - MJS);
         capbs = czbs * sarg;
       } else {
         qbs = 0.0;
         capbs = 0.0;
       }
       if (czbssw > 0.0) {
-        arg = 1.0 - vbs_jct / P(PhiBSWS);
+        arg = 1.0 - quot(vbs_jct, P(PhiBSWS));
         if (MJSWS == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJSWS * log(arg));
-        qbs += P(PhiBSWS) * czbssw * (1.0 - arg * sarg) / (1.0 - MJSWS);
+        qbs += quot(P(PhiBSWS) * czbssw * (1.0 - arg * sarg), 1.0 - MJSWS);
         capbs += czbssw * sarg;
       }
       if (czbsswg > 0.0) {
-        arg = 1.0 - vbs_jct / P(PhiBSWGS);
+        arg = 1.0 - quot(vbs_jct, P(PhiBSWGS));
         if (MJSWGS == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJSWGS * log(arg));
-        qbs += P(PhiBSWGS) * czbsswg * (1.0 - arg * sarg) / (1.0 - MJSWGS);
+        qbs += quot(P(PhiBSWGS) * czbsswg * (1.0 - arg * sarg), 1.0 - MJSWGS);
         capbs += czbsswg * sarg;
       }
     } else {
       T0 = czbs + czbssw + czbsswg;
-      T1 = vbs_jct * (czbs * MJS / P(PhiBS) + czbssw * MJSWS / P(PhiBSWS) + czbsswg * MJSWGS / P(PhiBSWGS));
+      T1 = vbs_jct * (quot(czbs * MJS, P(PhiBS)) + quot(czbssw * MJSWS, P(PhiBSWS)) + quot(czbsswg * MJSWGS, P(PhiBSWGS)));
       qbs = vbs_jct * (T0 + 0.5 * T1);
       capbs = T0 + T1;
     }
@@ -921,38 +922,38 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       capbd = czbd + czbdsw + czbdswg;
     } else if (vbd_jct < 0.0) {
       if (czbd > 0.0) {
-        arg = 1.0 - vbd_jct / P(PhiBD);
+        arg = 1.0 - quot(vbd_jct, P(PhiBD));
         if (MJD == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJD * log(arg));
-        qbd = P(PhiBD) * czbd * (1.0 - arg * sarg) / (1.0 - MJD);
+        qbd = quot(P(PhiBD) * czbd * (1.0 - arg * sarg), 1.0 - MJD);
         capbd = czbd * sarg;
       } else {
         qbd = 0.0;
         capbd = 0.0;
       }
       if (czbdsw > 0.0) {
-        arg = 1.0 - vbd_jct / P(PhiBSWD);
+        arg = 1.0 - quot(vbd_jct, P(PhiBSWD));
         if (MJSWD == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJSWD * log(arg));
-        qbd += P(PhiBSWD) * czbdsw * (1.0 - arg * sarg) / (1.0 - MJSWD);
+        qbd += quot(P(PhiBSWD) * czbdsw * (1.0 - arg * sarg), 1.0 - MJSWD);
         capbd += czbdsw * sarg;
       }
       if (czbdswg > 0.0) {
-        arg = 1.0 - vbd_jct / P(PhiBSWGD);
+        arg = 1.0 - quot(vbd_jct, P(PhiBSWGD));
         if (MJSWGD == 0.5)
-          sarg = 1.0 / sqrt(arg);
+          sarg = quot(1.0, sqrt(arg));
         else
           sarg = exp(-MJSWGD * log(arg));
-        qbd += P(PhiBSWGD) * czbdswg * (1.0 - arg * sarg) / (1.0 - MJSWGD);
+        qbd += quot(P(PhiBSWGD) * czbdswg * (1.0 - arg * sarg), 1.0 - MJSWGD);
         capbd += czbdswg * sarg;
       }
     } else {
       T0 = czbd + czbdsw + czbdswg;
-      T1 = vbd_jct * (czbd * MJD / P(PhiBD) + czbdsw * MJSWD / P(PhiBSWD) + czbdswg * MJSWGD / P(PhiBSWGD));
+      T1 = vbd_jct * (quot(czbd * MJD, P(PhiBD)) + quot(czbdsw * MJSWD, P(PhiBSWD)) + quot(czbdswg * MJSWGD, P(PhiBSWGD)));
       qbd = vbd_jct * (T0 + 0.5 * T1);
       capbd = T0 + T1;
     }
@@ -984,15 +985,15 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
     T1 = sqrt(T0 * T0 + 4.0 * CONSTDELTA_1);
     T2 = 0.5 * (T0 - T1);
     T3 = P(weffCV) * P(cgdl);
-    T4 = sqrt(1.0 - 4.0 * T2 / P(ckappad));
-    cgdo = P(cgdo) + T3 - T3 * (1.0 - 1.0 / T4) * (0.5 - 0.5 * T0 / T1);
+    T4 = sqrt(1.0 - quot(4.0 * T2, P(ckappad)));
+    cgdo = P(cgdo) + T3 - T3 * (1.0 - quot(1.0, T4)) * (0.5 - quot(0.5 * T0, T1));
     qgdo = (P(cgdo) + T3) * vgdx - T3 * (T2 + 0.5 * P(ckappad) * (T4 - 1.0));
     T0 = vgsx + CONSTDELTA_1;
     T1 = sqrt(T0 * T0 + 4.0 * CONSTDELTA_1);
     T2 = 0.5 * (T0 - T1);
     T3 = P(weffCV) * P(cgsl);
-    T4 = sqrt(1.0 - 4.0 * T2 / P(ckappas));
-    cgso = P(cgso) + T3 - T3 * (1.0 - 1.0 / T4) * (0.5 - 0.5 * T0 / T1);
+    T4 = sqrt(1.0 - quot(4.0 * T2, P(ckappas)));
+    cgso = P(cgso) + T3 - T3 * (1.0 - quot(1.0, T4)) * (0.5 - quot(0.5 * T0, T1));
     qgso = (P(cgso) + T3) * vgsx - T3 * (T2 + 0.5 * P(ckappas) * (T4 - 1.0));
   }
   if (nf != 1.0) {
@@ -1016,7 +1017,7 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
   const double ag0 = (!fl.dcop && fl.init_tran && fl.newton_iter == 0) ? 0.0 : fl.pdt;
   if (trnqsMod) {
     qcheq = qchqs;
-    const double T0q = qdef * ScalingFactor / CoxWL;
+    const double T0q = quot(qdef * ScalingFactor, CoxWL);
     const double gcg = m.v[m_gcrgg], gcd = m.v[m_gcrgd], gcs = m.v[m_gcrgs], gcb = m.v[m_gcrgb];
     ggtg = T0q * gcg;
     ggtd = T0q * (mode > 0 ? gcd : gcs);
@@ -1028,13 +1029,13 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       if (fabs(qcheq) <= 1.0e-5 * CoxWL) {
         dxpart = (xpart < 0.5) ? 0.4 : (xpart > 0.5) ? 0.0 : 0.5;
       } else {
-        dxpart = qdrn / qcheq;
+        dxpart = quot(qdrn, qcheq);
         const double Cdd = cddb, Csd = -(cgdb + cddb + cbdb);
-        ddxpart_dVd = (Cdd - dxpart * (Cdd + Csd)) / qcheq;
+        ddxpart_dVd = quot((Cdd - dxpart * (Cdd + Csd)), qcheq);
         const double Cdg = cdgb, Csg = -(cggb + cdgb + cbgb);
-        ddxpart_dVg = (Cdg - dxpart * (Cdg + Csg)) / qcheq;
+        ddxpart_dVg = quot((Cdg - dxpart * (Cdg + Csg)), qcheq);
         const double Cds = cdsb, Css = -(cgsb + cdsb + cbsb);
-        ddxpart_dVs = (Cds - dxpart * (Cds + Css)) / qcheq;
+        ddxpart_dVs = quot((Cds - dxpart * (Cds + Css)), qcheq);
         ddxpart_dVb = -(ddxpart_dVd + ddxpart_dVg + ddxpart_dVs);
       }
       sxpart = 1.0 - dxpart;
@@ -1046,13 +1047,13 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
       if (fabs(qcheq) <= 1.0e-5 * CoxWL) {
         sxpart = (xpart < 0.5) ? 0.4 : (xpart > 0.5) ? 0.0 : 0.5;
       } else {
-        sxpart = qdrn / qcheq;
+        sxpart = quot(qdrn, qcheq);
         const double Css = cddb, Cds = -(cgdb + cddb + cbdb);
-        dsxpart_dVs = (Css - sxpart * (Css + Cds)) / qcheq;
+        dsxpart_dVs = quot((Css - sxpart * (Css + Cds)), qcheq);
         const double Csg = cdgb, Cdg = -(cggb + cdgb + cbgb);
-        dsxpart_dVg = (Csg - sxpart * (Csg + Cdg)) / qcheq;
+        dsxpart_dVg = quot((Csg - sxpart * (Csg + Cdg)), qcheq);
         const double Csd = cdsb, Cdd = -(cgsb + cdsb + cbsb);
-        dsxpart_dVd = (Csd - sxpart * (Csd + Cdd)) / qcheq;
+        dsxpart_dVd = quot((Csd - sxpart * (Csd + Cdd)), qcheq);
         dsxpart_dVb = -(dsxpart_dVd + dsxpart_dVg + dsxpart_dVs);
       }
       dxpart = 1.0 - sxpart;
@@ -1639,7 +1640,7 @@ XD_HD void bsim4_finish(const RV &P_, const double *V, const LoadFlags &fl, doub
         sxpart = (1.0 - (dxpart = (mode > 0) ? 0.4 : 0.6));
         ddxpart_dVd = ddxpart_dVg = ddxpart_dVb = ddxpart_dVs = 0.0;
         dsxpart_dVd = dsxpart_dVg = dsxpart_dVb = dsxpart_dVs = 0.0;
-        gtau = gcrg / CoxWL * ScalingFactor;
+        gtau = quot(gcrg, CoxWL) * ScalingFactor;
       }
     }
     const double sgn = dtype > 0 ? 1.0 : -1.0;
@@ -2231,23 +2232,23 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     } else {
       switch (dioMod) {
         case 0: {
-          double evbs = exp(vbs_jct / Nvtms);
-          T1 = P(xjbvs) * exp(-(P(bvs) + vbs_jct) / Nvtms);
-          gbs = SourceSatCurrent * (evbs + T1) / Nvtms + gmin;
+          double evbs = exp(quot(vbs_jct, Nvtms));
+          T1 = P(xjbvs) * exp(quot(-(P(bvs) + vbs_jct), Nvtms));
+          gbs = quot(SourceSatCurrent * (evbs + T1), Nvtms) + gmin;
           cbs = SourceSatCurrent * (evbs + P(XExpBVS) - T1 - 1.0) + gmin * vbs_jct;
           break;
         }
         case 1:
-          T2 = vbs_jct / Nvtms;
+          T2 = quot(vbs_jct, Nvtms);
           if (T2 < -CONSTEXP_THRESHOLD) {
             gbs = gmin;
             cbs = SourceSatCurrent * (CONSTMIN_EXP - 1.0) + gmin * vbs_jct;
           } else if (vbs_jct <= P(vjsmFwd)) {
             double evbs = exp(T2);
-            gbs = SourceSatCurrent * evbs / Nvtms + gmin;
+            gbs = quot(SourceSatCurrent * evbs, Nvtms) + gmin;
             cbs = SourceSatCurrent * (evbs - 1.0) + gmin * vbs_jct;
           } else {
-            T0 = P(IVjsmFwd) / Nvtms;
+            T0 = quot(P(IVjsmFwd), Nvtms);
             gbs = T0 + gmin;
             cbs = P(IVjsmFwd) - SourceSatCurrent + T0 * (vbs_jct - P(vjsmFwd)) + gmin * vbs_jct;
           }
@@ -2255,34 +2256,34 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
         default: {
           double evbs, devbs_dvb;
           if (vbs_jct < P(vjsmRev)) {
-            T0 = vbs_jct / Nvtms;
+            T0 = quot(vbs_jct, Nvtms);
             if (T0 < -CONSTEXP_THRESHOLD) {
               evbs = CONSTMIN_EXP;
               devbs_dvb = 0.0;
             } else {
               evbs = exp(T0);
-              devbs_dvb = evbs / Nvtms;
+              devbs_dvb = quot(evbs, Nvtms);
             }
             T1 = evbs - 1.0;
             T2 = P(IVjsmRev) + P(SslpRev) * (vbs_jct - P(vjsmRev));
             gbs = devbs_dvb * T2 + T1 * P(SslpRev) + gmin;
             cbs = T1 * T2 + gmin * vbs_jct;
           } else if (vbs_jct <= P(vjsmFwd)) {
-            T0 = vbs_jct / Nvtms;
+            T0 = quot(vbs_jct, Nvtms);
             if (T0 < -CONSTEXP_THRESHOLD) {
               evbs = CONSTMIN_EXP;
               devbs_dvb = 0.0;
             } else {
               evbs = exp(T0);
-              devbs_dvb = evbs / Nvtms;
+              devbs_dvb = quot(evbs, Nvtms);
             }
-            T1 = (P(bvs) + vbs_jct) / Nvtms;
+            T1 = quot((P(bvs) + vbs_jct), Nvtms);
             if (T1 > CONSTEXP_THRESHOLD) {
               T2 = CONSTMIN_EXP;
               T3 = 0.0;
             } else {
               T2 = exp(-T1);
-              T3 = -T2 / Nvtms;
+              T3 = quot(-T2, Nvtms);
             }
             gbs = SourceSatCurrent * (devbs_dvb - P(xjbvs) * T3) + gmin;
             cbs = SourceSatCurrent * (evbs + P(XExpBVS) - 1.0 - P(xjbvs) * T2) + gmin * vbs_jct;
@@ -2307,23 +2308,23 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     } else {
       switch (dioMod) {
         case 0: {
-          double evbd = exp(vbd_jct / Nvtmd);
-          T1 = P(xjbvd) * exp(-(P(bvd) + vbd_jct) / Nvtmd);
-          gbd = DrainSatCurrent * (evbd + T1) / Nvtmd + gmin;
+          double evbd = exp(quot(vbd_jct, Nvtmd));
+          T1 = P(xjbvd) * exp(quot(-(P(bvd) + vbd_jct), Nvtmd));
+          gbd = quot(DrainSatCurrent * (evbd + T1), Nvtmd) + gmin;
           cbd = DrainSatCurrent * (evbd + P(XExpBVD) - T1 - 1.0) + gmin * vbd_jct;
           break;
         }
         case 1:
-          T2 = vbd_jct / Nvtmd;
+          T2 = quot(vbd_jct, Nvtmd);
           if (T2 < -CONSTEXP_THRESHOLD) {
             gbd = gmin;
             cbd = DrainSatCurrent * (CONSTMIN_EXP - 1.0) + gmin * vbd_jct;
           } else if (vbd_jct <= P(vjdmFwd)) {
             double evbd = exp(T2);
-            gbd = DrainSatCurrent * evbd / Nvtmd + gmin;
+            gbd = quot(DrainSatCurrent * evbd, Nvtmd) + gmin;
             cbd = DrainSatCurrent * (evbd - 1.0) + gmin * vbd_jct;
           } else {
-            T0 = P(IVjdmFwd) / Nvtmd;
+            T0 = quot(P(IVjdmFwd), Nvtmd);
             gbd = T0 + gmin;
             cbd = P(IVjdmFwd) - DrainSatCurrent + T0 * (vbd_jct - P(vjdmFwd)) + gmin * vbd_jct;
           }
@@ -2331,34 +2332,34 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
         default: {
           double evbd, devbd_dvb;
           if (vbd_jct < P(vjdmRev)) {
-            T0 = vbd_jct / Nvtmd;
+            T0 = quot(vbd_jct, Nvtmd);
             if (T0 < -CONSTEXP_THRESHOLD) {
               evbd = CONSTMIN_EXP;
               devbd_dvb = 0.0;
             } else {
               evbd = exp(T0);
-              devbd_dvb = evbd / Nvtmd;
+              devbd_dvb = quot(evbd, Nvtmd);
             }
             T1 = evbd - 1.0;
             T2 = P(IVjdmRev) + P(DslpRev) * (vbd_jct - P(vjdmRev));
             gbd = devbd_dvb * T2 + T1 * P(DslpRev) + gmin;
             cbd = T1 * T2 + gmin * vbd_jct;
           } else if (vbd_jct <= P(vjdmFwd)) {
-            T0 = vbd_jct / Nvtmd;
+            T0 = quot(vbd_jct, Nvtmd);
             if (T0 < -CONSTEXP_THRESHOLD) {
               evbd = CONSTMIN_EXP;
               devbd_dvb = 0.0;
             } else {
               evbd = exp(T0);
-              devbd_dvb = evbd / Nvtmd;
+              devbd_dvb = quot(evbd, Nvtmd);
             }
-            T1 = (P(bvd) + vbd_jct) / Nvtmd;
+            T1 = quot((P(bvd) + vbd_jct), Nvtmd);
             if (T1 > CONSTEXP_THRESHOLD) {
               T2 = CONSTMIN_EXP;
               T3 = 0.0;
             } else {
               T2 = exp(-T1);
-              T3 = -T2 / Nvtmd;
+              T3 = quot(-T2, Nvtmd);
             }
             gbd = DrainSatCurrent * (devbd_dvb - P(xjbvd) * T3) + gmin;
             cbd = DrainSatCurrent * (evbd + P(XExpBVD) - 1.0 - P(xjbvd) * T2) + gmin * vbd_jct;
@@ -2385,40 +2386,40 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     const double vtss = P(vtss), vtsd = P(vtsd), vtssws = P(vtssws), vtsswd = P(vtsswd), vtsswgs = P(vtsswgs),
                  vtsswgd = P(vtsswgd);
     if ((vtss - vbs_jct) < (vtss * 1e-3)) {
-      T9 = 1.0e3; T0 = -vbs_jct / Nvtmrss * T9; dexp(T0, e1, T10); d1 = T10 / Nvtmrss * T9;
+      T9 = 1.0e3; T0 = quot(-vbs_jct, Nvtmrss) * T9; dexp(T0, e1, T10); d1 = quot(T10, Nvtmrss) * T9;
     } else {
-      T9 = 1.0 / (vtss - vbs_jct); T0 = -vbs_jct / Nvtmrss * vtss * T9;
-      dT0_dVb = vtss / Nvtmrss * (T9 + vbs_jct * T9 * T9); dexp(T0, e1, T10); d1 = T10 * dT0_dVb;
+      T9 = quot(1.0, vtss - vbs_jct); T0 = quot(-vbs_jct, Nvtmrss) * vtss * T9;
+      dT0_dVb = quot(vtss, Nvtmrss) * (T9 + vbs_jct * T9 * T9); dexp(T0, e1, T10); d1 = T10 * dT0_dVb;
     }
     if ((vtsd - vbd_jct) < (vtsd * 1e-3)) {
-      T9 = 1.0e3; T0 = -vbd_jct / Nvtmrsd * T9; dexp(T0, e2, T10); d2 = T10 / Nvtmrsd * T9;
+      T9 = 1.0e3; T0 = quot(-vbd_jct, Nvtmrsd) * T9; dexp(T0, e2, T10); d2 = quot(T10, Nvtmrsd) * T9;
     } else {
-      T9 = 1.0 / (vtsd - vbd_jct); T0 = -vbd_jct / Nvtmrsd * vtsd * T9;
-      dT0_dVb = vtsd / Nvtmrsd * (T9 + vbd_jct * T9 * T9); dexp(T0, e2, T10); d2 = T10 * dT0_dVb;
+      T9 = quot(1.0, vtsd - vbd_jct); T0 = quot(-vbd_jct, Nvtmrsd) * vtsd * T9;
+      dT0_dVb = quot(vtsd, Nvtmrsd) * (T9 + vbd_jct * T9 * T9); dexp(T0, e2, T10); d2 = T10 * dT0_dVb;
     }
     if ((vtssws - vbs_jct) < (vtssws * 1e-3)) {
-      T9 = 1.0e3; T0 = -vbs_jct / Nvtmrssws * T9; dexp(T0, e3, T10); d3 = T10 / Nvtmrssws * T9;
+      T9 = 1.0e3; T0 = quot(-vbs_jct, Nvtmrssws) * T9; dexp(T0, e3, T10); d3 = quot(T10, Nvtmrssws) * T9;
     } else {
-      T9 = 1.0 / (vtssws - vbs_jct); T0 = -vbs_jct / Nvtmrssws * vtssws * T9;
-      dT0_dVb = vtssws / Nvtmrssws * (T9 + vbs_jct * T9 * T9); dexp(T0, e3, T10); d3 = T10 * dT0_dVb;
+      T9 = quot(1.0, vtssws - vbs_jct); T0 = quot(-vbs_jct, Nvtmrssws) * vtssws * T9;
+      dT0_dVb = quot(vtssws, Nvtmrssws) * (T9 + vbs_jct * T9 * T9); dexp(T0, e3, T10); d3 = T10 * dT0_dVb;
     }
     if ((vtsswd - vbd_jct) < (vtsswd * 1e-3)) {
-      T9 = 1.0e3; T0 = -vbd_jct / Nvtmrsswd * T9; dexp(T0, e4, T10); d4 = T10 / Nvtmrsswd * T9;
+      T9 = 1.0e3; T0 = quot(-vbd_jct, Nvtmrsswd) * T9; dexp(T0, e4, T10); d4 = quot(T10, Nvtmrsswd) * T9;
     } else {
-      T9 = 1.0 / (vtsswd - vbd_jct); T0 = -vbd_jct / Nvtmrsswd * vtsswd * T9;
-      dT0_dVb = vtsswd / Nvtmrsswd * (T9 + vbd_jct * T9 * T9); dexp(T0, e4, T10); d4 = T10 * dT0_dVb;
+      T9 = quot(1.0, vtsswd - vbd_jct); T0 = quot(-vbd_jct, Nvtmrsswd) * vtsswd * T9;
+      dT0_dVb = quot(vtsswd, Nvtmrsswd) * (T9 + vbd_jct * T9 * T9); dexp(T0, e4, T10); d4 = T10 * dT0_dVb;
     }
     if ((vtsswgs - vbs_jct) < (vtsswgs * 1e-3)) {
-      T9 = 1.0e3; T0 = -vbs_jct / Nvtmrsswgs * T9; dexp(T0, e5, T10); d5 = T10 / Nvtmrsswgs * T9;
+      T9 = 1.0e3; T0 = quot(-vbs_jct, Nvtmrsswgs) * T9; dexp(T0, e5, T10); d5 = quot(T10, Nvtmrsswgs) * T9;
     } else {
-      T9 = 1.0 / (vtsswgs - vbs_jct); T0 = -vbs_jct / Nvtmrsswgs * vtsswgs * T9;
-      dT0_dVb = vtsswgs / Nvtmrsswgs * (T9 + vbs_jct * T9 * T9); dexp(T0, e5, T10); d5 = T10 * dT0_dVb;
+      T9 = quot(1.0, vtsswgs - vbs_jct); T0 = quot(-vbs_jct, Nvtmrsswgs) * vtsswgs * T9;
+      dT0_dVb = quot(vtsswgs, Nvtmrsswgs) * (T9 + vbs_jct * T9 * T9); dexp(T0, e5, T10); d5 = T10 * dT0_dVb;
     }
     if ((vtsswgd - vbd_jct) < (vtsswgd * 1e-3)) {
-      T9 = 1.0e3; T0 = -vbd_jct / Nvtmrsswgd * T9; dexp(T0, e6, T10); d6 = T10 / Nvtmrsswgd * T9;
+      T9 = 1.0e3; T0 = quot(-vbd_jct, Nvtmrsswgd) * T9; dexp(T0, e6, T10); d6 = quot(T10, Nvtmrsswgd) * T9;
     } else {
-      T9 = 1.0 / (vtsswgd - vbd_jct); T0 = -vbd_jct / Nvtmrsswgd * vtsswgd * T9;
-      dT0_dVb = vtsswgd / Nvtmrsswgd * (T9 + vbd_jct * T9 * T9); dexp(T0, e6, T10); d6 = T10 * dT0_dVb;
+      T9 = quot(1.0, vtsswgd - vbd_jct); T0 = quot(-vbd_jct, Nvtmrsswgd) * vtsswgd * T9;
+      dT0_dVb = quot(vtsswgd, Nvtmrsswgd) * (T9 + vbd_jct * T9 * T9); dexp(T0, e6, T10); d6 = T10 * dT0_dVb;
     }
     gbs += P(SjctTempRevSatCur) * d1 + P(SswTempRevSatCur) * d3 + P(SswgTempRevSatCur) * d5;
     cbs -= P(SjctTempRevSatCur) * (e1 - 1.0) + P(SswTempRevSatCur) * (e3 - 1.0) + P(SswgTempRevSatCur) * (e5 - 1.0);
@@ -2453,24 +2454,24 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   T1 = sqrt(T0 * T0 - 0.004 * vbsc);
   if (T0 >= 0.0) {
     Vbseff = vbsc + 0.5 * (T0 + T1);
-    dVbseff_dVb = 0.5 * (1.0 + T0 / T1);
+    dVbseff_dVb = 0.5 * (1.0 + quot(T0, T1));
   } else {
-    T2 = -0.002 / (T1 - T0);
+    T2 = quot(-0.002, T1 - T0);
     Vbseff = vbsc * (1.0 + T2);
-    dVbseff_dVb = T2 * vbsc / T1;
+    dVbseff_dVb = quot(T2 * vbsc, T1);
   }
   const double phi = P(phi), sqrtPhi_p = P(sqrtPhi);
   T9 = 0.95 * phi;
   T0 = T9 - Vbseff - 0.001;
   T1 = sqrt(T0 * T0 + 0.004 * T9);
   Vbseff = T9 - 0.5 * (T0 + T1);
-  dVbseff_dVb *= 0.5 * (1.0 + T0 / T1);
+  dVbseff_dVb *= 0.5 * (1.0 + quot(T0, T1));
   const double Phis = phi - Vbseff;
   const double dPhis_dVb = -1.0;
   const double sqrtPhis = sqrt(Phis);
-  const double dsqrtPhis_dVb = -0.5 / sqrtPhis;
-  const double Xdep = P(Xdep0) * sqrtPhis / sqrtPhi_p;
-  const double dXdep_dVb = (P(Xdep0) / sqrtPhi_p) * dsqrtPhis_dVb;
+  const double dsqrtPhis_dVb = quot(-0.5, sqrtPhis);
+  const double Xdep = quot(P(Xdep0) * sqrtPhis, sqrtPhi_p);
+  const double dXdep_dVb = (quot(P(Xdep0), sqrtPhi_p)) * dsqrtPhis_dVb;
   const double Leff = P(leff);
   const double Vtm = P(vtm);
   const double Vtm0 = P(vtm0);
@@ -2481,65 +2482,65 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     T1 = 1.0 + T0;
     T2 = P(dvt2);
   } else {
-    T4 = 1.0 / (3.0 + 8.0 * T0);
+    T4 = quot(1.0, 3.0 + 8.0 * T0);
     T1 = (1.0 + 3.0 * T0) * T4;
     T2 = P(dvt2) * T4 * T4;
   }
   const double factor1 = P(factor1);
   const double lt1 = factor1 * T3 * T1;
-  const double dlt1_dVb = factor1 * (0.5 / T3 * T1 * dXdep_dVb + T3 * T2);
+  const double dlt1_dVb = factor1 * (quot(0.5, T3) * T1 * dXdep_dVb + T3 * T2);
   T0 = P(dvt2w) * Vbseff;
   if (T0 >= -0.5) {
     T1 = 1.0 + T0;
     T2 = P(dvt2w);
   } else {
-    T4 = 1.0 / (3.0 + 8.0 * T0);
+    T4 = quot(1.0, 3.0 + 8.0 * T0);
     T1 = (1.0 + 3.0 * T0) * T4;
     T2 = P(dvt2w) * T4 * T4;
   }
   const double ltw = factor1 * T3 * T1;
-  const double dltw_dVb = factor1 * (0.5 / T3 * T1 * dXdep_dVb + T3 * T2);
+  const double dltw_dVb = factor1 * (quot(0.5, T3) * T1 * dXdep_dVb + T3 * T2);
   double Theta0, dTheta0_dVb;
-  T0 = P(dvt1) * Leff / lt1;
+  T0 = quot(P(dvt1) * Leff, lt1);
   if (T0 < CONSTEXP_THRESHOLD) {
     T1 = exp(T0);
     T2 = T1 - 1.0;
     T3 = T2 * T2;
     T4 = T3 + 2.0 * T1 * CONSTMIN_EXP;
-    Theta0 = T1 / T4;
-    dT1_dVb = -T0 * T1 * dlt1_dVb / lt1;
-    dTheta0_dVb = dT1_dVb * (T4 - 2.0 * T1 * (T2 + CONSTMIN_EXP)) / T4 / T4;
+    Theta0 = quot(T1, T4);
+    dT1_dVb = quot(-T0 * T1 * dlt1_dVb, lt1);
+    dTheta0_dVb = quot(quot(dT1_dVb * (T4 - 2.0 * T1 * (T2 + CONSTMIN_EXP)), T4), T4);
   } else {
-    Theta0 = 1.0 / (CONSTMAX_EXP - 2.0);
+    Theta0 = quot(1.0, CONSTMAX_EXP - 2.0);
     dTheta0_dVb = 0.0;
   }
   const double thetavth = P(dvt0) * Theta0;
   const double Delt_vth = thetavth * V0;
   const double dDelt_vth_dVb = P(dvt0) * dTheta0_dVb * V0;
-  T0 = P(dvt1w) * P(weff) * Leff / ltw;
+  T0 = quot(P(dvt1w) * P(weff) * Leff, ltw);
   if (T0 < CONSTEXP_THRESHOLD) {
     T1 = exp(T0);
     T2 = T1 - 1.0;
     T3 = T2 * T2;
     T4 = T3 + 2.0 * T1 * CONSTMIN_EXP;
-    T5 = T1 / T4;
-    dT1_dVb = -T0 * T1 * dltw_dVb / ltw;
-    dT5_dVb = dT1_dVb * (T4 - 2.0 * T1 * (T2 + CONSTMIN_EXP)) / T4 / T4;
+    T5 = quot(T1, T4);
+    dT1_dVb = quot(-T0 * T1 * dltw_dVb, ltw);
+    dT5_dVb = quot(quot(dT1_dVb * (T4 - 2.0 * T1 * (T2 + CONSTMIN_EXP)), T4), T4);
   } else {
-    T5 = 1.0 / (CONSTMAX_EXP - 2.0);
+    T5 = quot(1.0, CONSTMAX_EXP - 2.0);
     dT5_dVb = 0.0;
   }
   T0 = P(dvt0w) * T5;
   T2 = T0 * V0;
   dT2_dVb = P(dvt0w) * dT5_dVb * V0;
-  const double TempRatio = P(temp) / P(tnom) - 1.0;
-  T0 = sqrt(1.0 + P(lpe0) / Leff);
+  const double TempRatio = quot(P(temp), P(tnom)) - 1.0;
+  T0 = sqrt(1.0 + quot(P(lpe0), Leff));
   const double k1ox = P(k1ox);
-  T1 = k1ox * (T0 - 1.0) * sqrtPhi_p + (P(kt1) + P(kt1l) / Leff + P(kt2) * Vbseff) * TempRatio;
-  const double Vth_NarrowW = toxe * phi / (P(weff) + P(w0));
+  T1 = k1ox * (T0 - 1.0) * sqrtPhi_p + (P(kt1) + quot(P(kt1l), Leff) + P(kt2) * Vbseff) * TempRatio;
+  const double Vth_NarrowW = quot(toxe * phi, P(weff) + P(w0));
   T3 = P(eta0) + P(etab) * Vbseff;
   if (T3 < 1.0e-4) {
-    T9 = 1.0 / (3.0 - 2.0e4 * T3);
+    T9 = quot(1.0, 3.0 - 2.0e4 * T3);
     T3 = (2.0e-4 - T3) * T9;
     T4 = T9 * T9;
   } else {
@@ -2547,7 +2548,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   }
   const double dDIBL_Sft_dVd = T3 * P(theta0vb0);
   const double DIBL_Sft = dDIBL_Sft_dVd * Vds;
-  const double Lpe_Vb = sqrt(1.0 + P(lpeb) / Leff);
+  const double Lpe_Vb = sqrt(1.0 + quot(P(lpeb), Leff));
   const double k2ox = P(k2ox);
   double Vth = dtype * vth0 + (k1ox * sqrtPhis - P(k1) * sqrtPhi_p) * Lpe_Vb - k2ox * Vbseff - Delt_vth - T2 +
                (P(k3) + P(k3b) * Vbseff) * Vth_NarrowW + T1 - DIBL_Sft;
@@ -2555,21 +2556,21 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
                     P(etab) * Vds * P(theta0vb0) * T4 + P(kt2) * TempRatio;
   double dVth_dVd = -dDIBL_Sft_dVd;
   const double coxe = P(coxe);
-  tmp1 = epssub / Xdep;
+  tmp1 = quot(epssub, Xdep);
   tmp2 = P(nfactor) * tmp1;
   tmp3 = P(cdsc) + P(cdscb) * Vbseff + P(cdscd) * Vds;
-  tmp4 = (tmp2 + tmp3 * Theta0 + P(cit)) / coxe;
+  tmp4 = quot((tmp2 + tmp3 * Theta0 + P(cit)), coxe);
   double n, dn_dVb, dn_dVd;
   if (tmp4 >= -0.5) {
     n = 1.0 + tmp4;
-    dn_dVb = (-tmp2 / Xdep * dXdep_dVb + tmp3 * dTheta0_dVb + P(cdscb) * Theta0) / coxe;
-    dn_dVd = P(cdscd) * Theta0 / coxe;
+    dn_dVb = quot((quot(-tmp2, Xdep) * dXdep_dVb + tmp3 * dTheta0_dVb + P(cdscb) * Theta0), coxe);
+    dn_dVd = quot(P(cdscd) * Theta0, coxe);
   } else {
-    T0 = 1.0 / (3.0 + 8.0 * tmp4);
+    T0 = quot(1.0, 3.0 + 8.0 * tmp4);
     n = (1.0 + 3.0 * tmp4) * T0;
     T0 *= T0;
-    dn_dVb = (-tmp2 / Xdep * dXdep_dVb + tmp3 * dTheta0_dVb + P(cdscb) * Theta0) / coxe * T0;
-    dn_dVd = P(cdscd) * Theta0 / coxe * T0;
+    dn_dVb = quot((quot(-tmp2, Xdep) * dXdep_dVb + tmp3 * dTheta0_dVb + P(cdscb) * Theta0), coxe) * T0;
+    dn_dVd = quot(P(cdscd) * Theta0, coxe) * T0;
   }
   if (P(dvtp0) > 0.0) {
     T0 = -P(dvtp1) * Vds;
@@ -2583,11 +2584,11 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     T3 = Leff + P(dvtp0) * (1.0 + T2);
     dT3_dVd = P(dvtp0) * dT2_dVd;
     if (tempMod < 2) {
-      T4 = Vtm * log(Leff / T3);
-      dT4_dVd = -Vtm * dT3_dVd / T3;
+      T4 = Vtm * log(quot(Leff, T3));
+      dT4_dVd = quot(-Vtm * dT3_dVd, T3);
     } else {
-      T4 = Vtm0 * log(Leff / T3);
-      dT4_dVd = -Vtm0 * dT3_dVd / T3;
+      T4 = Vtm0 * log(quot(Leff, T3));
+      dT4_dVd = quot(-Vtm0 * dT3_dVd, T3);
     }
     const double dDITS_Sft_dVd = dn_dVd * T4 + n * dT4_dVd;
     const double dDITS_Sft_dVb = T4 * dn_dVb;
@@ -2617,7 +2618,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   const double mstar = P(mstar);
   T0 = n * Vtm;
   T1 = mstar * Vgst;
-  T2 = T1 / T0;
+  T2 = quot(T1, T0);
   if (T2 > CONSTEXP_THRESHOLD) {
     T10 = T1;
     dT10_dVg = mstar * dVgs_eff_dVg;
@@ -2633,41 +2634,41 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     const double ExpVgst = exp(T2);
     T3 = Vtm * log(1.0 + ExpVgst);
     T10 = n * T3;
-    dT10_dVg = mstar * ExpVgst / (1.0 + ExpVgst);
-    dT10_dVb = T3 * dn_dVb - dT10_dVg * (dVth_dVb + Vgst * dn_dVb / n);
-    dT10_dVd = T3 * dn_dVd - dT10_dVg * (dVth_dVd + Vgst * dn_dVd / n);
+    dT10_dVg = quot(mstar * ExpVgst, 1.0 + ExpVgst);
+    dT10_dVb = T3 * dn_dVb - dT10_dVg * (dVth_dVb + quot(Vgst * dn_dVb, n));
+    dT10_dVd = T3 * dn_dVd - dT10_dVg * (dVth_dVd + quot(Vgst * dn_dVd, n));
     dT10_dVg *= dVgs_eff_dVg;
   }
   T1 = P(voffcbn) - (1.0 - mstar) * Vgst;
-  T2 = T1 / T0;
+  T2 = quot(T1, T0);
   if (T2 < -CONSTEXP_THRESHOLD) {
-    T3 = coxe * CONSTMIN_EXP / P(cdep0);
+    T3 = quot(coxe * CONSTMIN_EXP, P(cdep0));
     T9 = mstar + T3 * n;
     dT9_dVg = 0.0;
     dT9_dVd = dn_dVd * T3;
     dT9_dVb = dn_dVb * T3;
   } else if (T2 > CONSTEXP_THRESHOLD) {
-    T3 = coxe * CONSTMAX_EXP / P(cdep0);
+    T3 = quot(coxe * CONSTMAX_EXP, P(cdep0));
     T9 = mstar + T3 * n;
     dT9_dVg = 0.0;
     dT9_dVd = dn_dVd * T3;
     dT9_dVb = dn_dVb * T3;
   } else {
     const double ExpVgst = exp(T2);
-    T3 = coxe / P(cdep0);
+    T3 = quot(coxe, P(cdep0));
     T4 = T3 * ExpVgst;
-    T5 = T1 * T4 / T0;
+    T5 = quot(T1 * T4, T0);
     T9 = mstar + n * T4;
-    dT9_dVg = T3 * (mstar - 1.0) * ExpVgst / Vtm;
+    dT9_dVg = quot(T3 * (mstar - 1.0) * ExpVgst, Vtm);
     dT9_dVb = T4 * dn_dVb - dT9_dVg * dVth_dVb - T5 * dn_dVb;
     dT9_dVd = T4 * dn_dVd - dT9_dVg * dVth_dVd - T5 * dn_dVd;
     dT9_dVg *= dVgs_eff_dVg;
   }
-  double Vgsteff = T10 / T9;
+  double Vgsteff = quot(T10, T9);
   T11 = T9 * T9;
-  double dVgsteff_dVg = (T9 * dT10_dVg - T10 * dT9_dVg) / T11;
-  double dVgsteff_dVd = (T9 * dT10_dVd - T10 * dT9_dVd) / T11;
-  double dVgsteff_dVb = (T9 * dT10_dVb - T10 * dT9_dVb) / T11;
+  double dVgsteff_dVg = quot((T9 * dT10_dVg - T10 * dT9_dVg), T11);
+  double dVgsteff_dVd = quot((T9 * dT10_dVd - T10 * dT9_dVd), T11);
+  double dVgsteff_dVb = quot((T9 * dT10_dVb - T10 * dT9_dVb), T11);
 
   // Effective width and source/drain series resistance (:9155-9200).
   T9 = sqrtPhis - sqrtPhi_p;
@@ -2675,7 +2676,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   double dWeff_dVg = -2.0 * P(dwg);
   double dWeff_dVb = -2.0 * P(dwb) * dsqrtPhis_dVb;
   if (Weff < 2.0e-8) {
-    T0 = 1.0 / (6.0e-8 - 2.0 * Weff);
+    T0 = quot(1.0, 6.0e-8 - 2.0 * Weff);
     Weff = 2.0e-8 * (4.0e-8 - Weff) * T0;
     T0 *= T0 * 4.0e-16;
     dWeff_dVg *= T0;
@@ -2686,12 +2687,12 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     Rds = dRds_dVg = dRds_dVb = 0.0;
   } else {
     T0 = 1.0 + P(prwg) * Vgsteff;
-    dT0_dVg = -P(prwg) / T0 / T0;
+    dT0_dVg = quot(quot(-P(prwg), T0), T0);
     T1 = P(prwb) * T9;
     dT1_dVb = P(prwb) * dsqrtPhis_dVb;
-    T2 = 1.0 / T0 + T1;
+    T2 = quot(1.0, T0) + T1;
     T3 = T2 + sqrt(T2 * T2 + 0.01);
-    dT3_dVg = 1.0 + T2 / (T3 - T2);
+    dT3_dVg = 1.0 + quot(T2, T3 - T2);
     dT3_dVb = dT3_dVg * dT1_dVb;
     dT3_dVg *= dT0_dVg;
     T4 = P(rds0) * 0.5;
@@ -2701,17 +2702,17 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   }
 
   // Bulk charge factor Abulk (:9201-9260).
-  T9 = 0.5 * k1ox * Lpe_Vb / sqrtPhis;
+  T9 = quot(0.5 * k1ox * Lpe_Vb, sqrtPhis);
   T1 = T9 + k2ox - P(k3b) * Vth_NarrowW;
-  dT1_dVb = -T9 / sqrtPhis * dsqrtPhis_dVb;
+  dT1_dVb = quot(-T9, sqrtPhis) * dsqrtPhis_dVb;
   T9 = sqrt(P(xj) * Xdep);
   tmp1 = Leff + 2.0 * T9;
-  T5 = Leff / tmp1;
+  T5 = quot(Leff, tmp1);
   tmp2 = P(a0) * T5;
   tmp3 = P(weff) + P(b1);
-  tmp4 = P(b0) / tmp3;
+  tmp4 = quot(P(b0), tmp3);
   T2 = tmp2 + tmp4;
-  dT2_dVb = -T9 / tmp1 / Xdep * dXdep_dVb;
+  dT2_dVb = quot(quot(-T9, tmp1), Xdep) * dXdep_dVb;
   T6 = T5 * T5;
   T7 = T5 * T6;
   double Abulk0 = 1.0 + T1 * T2;
@@ -2721,12 +2722,12 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   double Abulk = Abulk0 + dAbulk_dVg * Vgsteff;
   double dAbulk_dVb = dAbulk0_dVb - T8 * Vgsteff * (dT1_dVb + 3.0 * T1 * dT2_dVb);
   if (Abulk0 < 0.1) {
-    T9 = 1.0 / (3.0 - 20.0 * Abulk0);
+    T9 = quot(1.0, 3.0 - 20.0 * Abulk0);
     Abulk0 = (0.2 - Abulk0) * T9;
     dAbulk0_dVb *= T9 * T9;
   }
   if (Abulk < 0.1) {
-    T9 = 1.0 / (3.0 - 20.0 * Abulk);
+    T9 = quot(1.0, 3.0 - 20.0 * Abulk);
     Abulk = (0.2 - Abulk) * T9;
     T10 = T9 * T9;
     dAbulk_dVb *= T10;
@@ -2734,10 +2735,10 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   }
   T2 = P(keta) * Vbseff;
   if (T2 >= -0.9) {
-    T0 = 1.0 / (1.0 + T2);
+    T0 = quot(1.0, 1.0 + T2);
     dT0_dVb = -P(keta) * T0 * T0;
   } else {
-    T1 = 1.0 / (0.8 + T2);
+    T1 = quot(1.0, 0.8 + T2);
     T0 = (17.0 + 20.0 * T2) * T1;
     dT0_dVb = -P(keta) * T1 * T1;
   }
@@ -2753,16 +2754,16 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   if (mobMod == 0) {
     T0 = Vgsteff + Vth + Vth - T14;
     T2 = P(ua) + P(uc) * Vbseff;
-    T3 = T0 / toxe;
+    T3 = quot(T0, toxe);
     T12 = sqrt(Vth * Vth + 0.0001);
-    T9 = 1.0 / (Vgsteff + 2 * T12);
+    T9 = quot(1.0, Vgsteff + 2 * T12);
     T10 = T9 * toxe;
     T8 = P(ud) * T10 * T10 * Vth;
     T6 = T8 * Vth;
     T5 = T3 * (T2 + P(ub) * T3) + T6;
     T7 = -2.0 * T6 * T9;
-    T11 = T7 * Vth / T12;
-    dDenomi_dVg = (T2 + 2.0 * P(ub) * T3) / toxe;
+    T11 = quot(T7 * Vth, T12);
+    dDenomi_dVg = quot((T2 + 2.0 * P(ub) * T3), toxe);
     T13 = 2.0 * (dDenomi_dVg + T11 + T8);
     dDenomi_dVd = T13 * dVth_dVd;
     dDenomi_dVb = T13 * dVth_dVb + P(uc) * T3;
@@ -2770,35 +2771,35 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   } else if (mobMod == 1) {
     T0 = Vgsteff + Vth + Vth - T14;
     T2 = 1.0 + P(uc) * Vbseff;
-    T3 = T0 / toxe;
+    T3 = quot(T0, toxe);
     T4 = T3 * (P(ua) + P(ub) * T3);
     T12 = sqrt(Vth * Vth + 0.0001);
-    T9 = 1.0 / (Vgsteff + 2 * T12);
+    T9 = quot(1.0, Vgsteff + 2 * T12);
     T10 = T9 * toxe;
     T8 = P(ud) * T10 * T10 * Vth;
     T6 = T8 * Vth;
     T5 = T4 * T2 + T6;
     T7 = -2.0 * T6 * T9;
-    T11 = T7 * Vth / T12;
-    dDenomi_dVg = (P(ua) + 2.0 * P(ub) * T3) * T2 / toxe;
+    T11 = quot(T7 * Vth, T12);
+    dDenomi_dVg = quot((P(ua) + 2.0 * P(ub) * T3) * T2, toxe);
     T13 = 2.0 * (dDenomi_dVg + T11 + T8);
     dDenomi_dVd = T13 * dVth_dVd;
     dDenomi_dVb = T13 * dVth_dVb + P(uc) * T4;
     dDenomi_dVg += T7;
   } else {
-    T0 = (Vgsteff + P(vtfbphi1)) / toxe;
+    T0 = quot((Vgsteff + P(vtfbphi1)), toxe);
     T1 = exp(P(eu) * log(T0));
-    dT1_dVg = T1 * P(eu) / T0 / toxe;
+    dT1_dVg = quot(quot(T1 * P(eu), T0), toxe);
     T2 = P(ua) + P(uc) * Vbseff;
-    T3 = T0 / toxe;
+    T3 = quot(T0, toxe);
     T12 = sqrt(Vth * Vth + 0.0001);
-    T9 = 1.0 / (Vgsteff + 2 * T12);
+    T9 = quot(1.0, Vgsteff + 2 * T12);
     T10 = T9 * toxe;
     T8 = P(ud) * T10 * T10 * Vth;
     T6 = T8 * Vth;
     T5 = T1 * T2 + T6;
     T7 = -2.0 * T6 * T9;
-    T11 = T7 * Vth / T12;
+    T11 = quot(T7 * Vth, T12);
     dDenomi_dVg = T2 * dT1_dVg + T7;
     T13 = 2.0 * (T11 + T8);
     dDenomi_dVd = T13 * dVth_dVd;
@@ -2807,15 +2808,15 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   if (T5 >= -0.8) {
     Denomi = 1.0 + T5;
   } else {
-    T9 = 1.0 / (7.0 + 10.0 * T5);
+    T9 = quot(1.0, 7.0 + 10.0 * T5);
     Denomi = (0.6 + T5) * T9;
     T9 *= T9;
     dDenomi_dVg *= T9;
     dDenomi_dVd *= T9;
     dDenomi_dVb *= T9;
   }
-  const double ueff = P(u0temp) / Denomi;
-  T9 = -ueff / Denomi;
+  const double ueff = quot(P(u0temp), Denomi);
+  T9 = quot(-ueff, Denomi);
   const double dueff_dVg = T9 * dDenomi_dVg;
   const double dueff_dVd = T9 * dDenomi_dVd;
   const double dueff_dVb = T9 * dDenomi_dVb;
@@ -2824,9 +2825,9 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   const double vsattemp = P(vsattemp);
   const double WVCox = Weff * vsattemp * coxe;
   const double WVCoxRds = WVCox * Rds;
-  const double Esat = 2.0 * vsattemp / ueff;
+  const double Esat = quot(2.0 * vsattemp, ueff);
   double EsatL = Esat * Leff;
-  T0 = -EsatL / ueff;
+  T0 = quot(-EsatL, ueff);
   double dEsatL_dVg = T0 * dueff_dVg;
   double dEsatL_dVd = T0 * dueff_dVd;
   double dEsatL_dVb = T0 * dueff_dVb;
@@ -2840,24 +2841,24 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     T1 = T0 - a1 * Vgsteff - 0.0001;
     T2 = sqrt(T1 * T1 + 0.0004 * T0);
     Lambda = P(a2) + T0 - 0.5 * (T1 + T2);
-    dLambda_dVg = 0.5 * a1 * (1.0 + T1 / T2);
+    dLambda_dVg = 0.5 * a1 * (1.0 + quot(T1, T2));
   } else {
     T1 = P(a2) + a1 * Vgsteff - 0.0001;
     T2 = sqrt(T1 * T1 + 0.0004 * P(a2));
     Lambda = 0.5 * (T1 + T2);
-    dLambda_dVg = 0.5 * a1 * (1.0 + T1 / T2);
+    dLambda_dVg = 0.5 * a1 * (1.0 + quot(T1, T2));
   }
   const double Vgst2Vtm = Vgsteff + 2.0 * Vtm;
   if (Rds > 0) {
-    tmp2 = dRds_dVg / Rds + dWeff_dVg / Weff;
-    tmp3 = dRds_dVb / Rds + dWeff_dVb / Weff;
+    tmp2 = quot(dRds_dVg, Rds) + quot(dWeff_dVg, Weff);
+    tmp3 = quot(dRds_dVb, Rds) + quot(dWeff_dVb, Weff);
   } else {
-    tmp2 = dWeff_dVg / Weff;
-    tmp3 = dWeff_dVb / Weff;
+    tmp2 = quot(dWeff_dVg, Weff);
+    tmp3 = quot(dWeff_dVb, Weff);
   }
   double Vdsat, dVdsat_dVg, dVdsat_dVd, dVdsat_dVb;
   if ((Rds == 0.0) && (Lambda == 1.0)) {
-    T0 = 1.0 / (Abulk * EsatL + Vgst2Vtm);
+    T0 = quot(1.0, Abulk * EsatL + Vgst2Vtm);
     tmp1 = 0.0;
     T1 = T0 * T0;
     T2 = Vgst2Vtm * T0;
@@ -2870,17 +2871,17 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     dVdsat_dVd = T3 * dT0_dVd + T2 * dEsatL_dVd;
     dVdsat_dVb = T3 * dT0_dVb + T2 * dEsatL_dVb;
   } else {
-    tmp1 = dLambda_dVg / (Lambda * Lambda);
+    tmp1 = quot(dLambda_dVg, Lambda * Lambda);
     T9 = Abulk * WVCoxRds;
     T8 = Abulk * T9;
     T7 = Vgst2Vtm * T9;
     T6 = Vgst2Vtm * WVCoxRds;
-    T0 = 2.0 * Abulk * (T9 - 1.0 + 1.0 / Lambda);
-    dT0_dVg = 2.0 * (T8 * tmp2 - Abulk * tmp1 + (2.0 * T9 + 1.0 / Lambda - 1.0) * dAbulk_dVg);
-    dT0_dVb = 2.0 * (T8 * (2.0 / Abulk * dAbulk_dVb + tmp3) + (1.0 / Lambda - 1.0) * dAbulk_dVb);
+    T0 = 2.0 * Abulk * (T9 - 1.0 + quot(1.0, Lambda));
+    dT0_dVg = 2.0 * (T8 * tmp2 - Abulk * tmp1 + (2.0 * T9 + quot(1.0, Lambda) - 1.0) * dAbulk_dVg);
+    dT0_dVb = 2.0 * (T8 * (quot(2.0, Abulk) * dAbulk_dVb + tmp3) + (quot(1.0, Lambda) - 1.0) * dAbulk_dVb);
     dT0_dVd = 0.0;
-    T1 = Vgst2Vtm * (2.0 / Lambda - 1.0) + Abulk * EsatL + 3.0 * T7;
-    dT1_dVg = (2.0 / Lambda - 1.0) - 2.0 * Vgst2Vtm * tmp1 + Abulk * dEsatL_dVg + EsatL * dAbulk_dVg +
+    T1 = Vgst2Vtm * (quot(2.0, Lambda) - 1.0) + Abulk * EsatL + 3.0 * T7;
+    dT1_dVg = (quot(2.0, Lambda) - 1.0) - 2.0 * Vgst2Vtm * tmp1 + Abulk * dEsatL_dVg + EsatL * dAbulk_dVg +
               3.0 * (T9 + T7 * tmp2 + T6 * dAbulk_dVg);
     dT1_dVb = Abulk * dEsatL_dVb + EsatL * dAbulk_dVb + 3.0 * (T6 * dAbulk_dVb + T7 * tmp3);
     dT1_dVd = Abulk * dEsatL_dVd;
@@ -2889,10 +2890,10 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     dT2_dVb = Vgst2Vtm * (dEsatL_dVb + 2.0 * T6 * tmp3);
     dT2_dVd = Vgst2Vtm * dEsatL_dVd;
     T3 = sqrt(T1 * T1 - 2.0 * T0 * T2);
-    Vdsat = (T1 - T3) / T0;
-    dVdsat_dVg = (dT1_dVg - (T1 * dT1_dVg - dT0_dVg * T2 - T0 * dT2_dVg) / T3 - Vdsat * dT0_dVg) / T0;
-    dVdsat_dVb = (dT1_dVb - (T1 * dT1_dVb - dT0_dVb * T2 - T0 * dT2_dVb) / T3 - Vdsat * dT0_dVb) / T0;
-    dVdsat_dVd = (dT1_dVd - (T1 * dT1_dVd - T0 * dT2_dVd) / T3) / T0;
+    Vdsat = quot((T1 - T3), T0);
+    dVdsat_dVg = quot((dT1_dVg - quot((T1 * dT1_dVg - dT0_dVg * T2 - T0 * dT2_dVg), T3) - Vdsat * dT0_dVg), T0);
+    dVdsat_dVb = quot((dT1_dVb - quot((T1 * dT1_dVb - dT0_dVb * T2 - T0 * dT2_dVb), T3) - Vdsat * dT0_dVb), T0);
+    dVdsat_dVd = quot((dT1_dVd - quot((T1 * dT1_dVd - T0 * dT2_dVd), T3)), T0);
   }
 
   // Effective Vds (:9461-9500).
@@ -2902,9 +2903,9 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   dT1_dVd = dVdsat_dVd - 1.0;
   dT1_dVb = dVdsat_dVb;
   T2 = sqrt(T1 * T1 + 4.0 * delta * Vdsat);
-  T0 = T1 / T2;
+  T0 = quot(T1, T2);
   T9 = 2.0 * delta;
-  T3 = T9 / T2;
+  T3 = quot(T9, T2);
   dT2_dVg = T0 * dT1_dVg + T3 * dVdsat_dVg;
   dT2_dVd = T0 * dT1_dVd + T3 * dVdsat_dVd;
   dT2_dVb = T0 * dT1_dVb + T3 * dVdsat_dVb;
@@ -2915,9 +2916,9 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     dVdseff_dVd = dVdsat_dVd - 0.5 * (dT1_dVd + dT2_dVd);
     dVdseff_dVb = dVdsat_dVb - 0.5 * (dT1_dVb + dT2_dVb);
   } else {
-    T4 = T9 / (T2 - T1);
+    T4 = quot(T9, T2 - T1);
     T5 = 1.0 - T4;
-    T6 = Vdsat * T4 / (T2 - T1);
+    T6 = quot(Vdsat * T4, T2 - T1);
     Vdseff = Vdsat * T5;
     dVdseff_dVg = dVdsat_dVg * T5 + T6 * (dT2_dVg - dT1_dVg);
     dVdseff_dVd = dVdsat_dVd * T5 + T6 * (dT2_dVd - dT1_dVd);
@@ -2934,13 +2935,13 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   // Velocity overshoot (lambda) (:9501-9545).
   if ((P(lambdaGiven) != 0.0) && (P(lambda_m) > 0.0)) {
     T1 = Leff * ueff;
-    T2 = P(lambda) / T1;
-    T3 = -T2 / T1 * Leff;
+    T2 = quot(P(lambda), T1);
+    T3 = quot(-T2, T1) * Leff;
     dT2_dVd = T3 * dueff_dVd;
     dT2_dVg = T3 * dueff_dVg;
     dT2_dVb = T3 * dueff_dVb;
-    T5 = 1.0 / (Esat * P(litl));
-    T4 = -T5 / EsatL;
+    T5 = quot(1.0, Esat * P(litl));
+    T4 = quot(-T5, EsatL);
     dT5_dVg = dEsatL_dVg * T4;
     dT5_dVd = dEsatL_dVd * T4;
     dT5_dVb = dEsatL_dVb * T4;
@@ -2948,7 +2949,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     dT6_dVg = dT5_dVg * diffVds - dVdseff_dVg * T5;
     dT6_dVd = dT5_dVd * diffVds + (1.0 - dVdseff_dVd) * T5;
     dT6_dVb = dT5_dVb * diffVds - dVdseff_dVb * T5;
-    T7 = 2.0 / (T6 * T6 + 1.0);
+    T7 = quot(2.0, T6 * T6 + 1.0);
     T8 = 1.0 - T7;
     T9 = T6 * T7 * T7;
     dT8_dVg = T9 * dT6_dVg;
@@ -2969,67 +2970,67 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   }
 
   // Vasat (:9546-9565).
-  tmp4 = 1.0 - 0.5 * Abulk * Vdsat / Vgst2Vtm;
+  tmp4 = 1.0 - quot(0.5 * Abulk * Vdsat, Vgst2Vtm);
   T9 = WVCoxRds * Vgsteff;
-  T8 = T9 / Vgst2Vtm;
+  T8 = quot(T9, Vgst2Vtm);
   T0 = EsatL + Vdsat + 2.0 * T9 * tmp4;
   T7 = 2.0 * WVCoxRds * tmp4;
   dT0_dVg = dEsatL_dVg + dVdsat_dVg + T7 * (1.0 + tmp2 * Vgsteff) -
-            T8 * (Abulk * dVdsat_dVg - Abulk * Vdsat / Vgst2Vtm + Vdsat * dAbulk_dVg);
+            T8 * (Abulk * dVdsat_dVg - quot(Abulk * Vdsat, Vgst2Vtm) + Vdsat * dAbulk_dVg);
   dT0_dVb = dEsatL_dVb + dVdsat_dVb + T7 * tmp3 * Vgsteff - T8 * (dAbulk_dVb * Vdsat + Abulk * dVdsat_dVb);
   dT0_dVd = dEsatL_dVd + dVdsat_dVd - T8 * Abulk * dVdsat_dVd;
   T9 = WVCoxRds * Abulk;
-  T1 = 2.0 / Lambda - 1.0 + T9;
+  T1 = quot(2.0, Lambda) - 1.0 + T9;
   dT1_dVg = -2.0 * tmp1 + WVCoxRds * (Abulk * tmp2 + dAbulk_dVg);
   dT1_dVb = dAbulk_dVb * WVCoxRds + T9 * tmp3;
-  const double Vasat = T0 / T1;
-  const double dVasat_dVg = (dT0_dVg - Vasat * dT1_dVg) / T1;
-  const double dVasat_dVb = (dT0_dVb - Vasat * dT1_dVb) / T1;
-  const double dVasat_dVd = dT0_dVd / T1;
+  const double Vasat = quot(T0, T1);
+  const double dVasat_dVg = quot((dT0_dVg - Vasat * dT1_dVg), T1);
+  const double dVasat_dVb = quot((dT0_dVb - Vasat * dT1_dVb), T1);
+  const double dVasat_dVd = quot(dT0_dVd, T1);
 
   // Quantum-mechanical effective oxide capacitance and beta (:9566-9590).
   tmp1 = P(vtfbphi2);
   tmp2 = 2.0e8 * P(toxp);
-  dT0_dVg = 1.0 / tmp2;
+  dT0_dVg = quot(1.0, tmp2);
   T0 = (Vgsteff + tmp1) * dT0_dVg;
   tmp3 = exp(P(bdos) * 0.7 * log(T0));
   T1 = 1.0 + tmp3;
-  T2 = P(bdos) * 0.7 * tmp3 / T0;
-  double Tcen = P(ados) * 1.9e-9 / T1;
-  double dTcen_dVg = -Tcen * T2 * dT0_dVg / T1;
+  T2 = quot(P(bdos) * 0.7 * tmp3, T0);
+  double Tcen = quot(P(ados) * 1.9e-9, T1);
+  double dTcen_dVg = quot(-Tcen * T2 * dT0_dVg, T1);
   const double coxp = P(coxp);
-  double Coxeff = epssub * coxp / (epssub + coxp * Tcen);
-  double dCoxeff_dVg = -Coxeff * Coxeff * dTcen_dVg / epssub;
-  const double CoxeffWovL = Coxeff * Weff / Leff;
+  double Coxeff = quot(epssub * coxp, epssub + coxp * Tcen);
+  double dCoxeff_dVg = quot(-Coxeff * Coxeff * dTcen_dVg, epssub);
+  const double CoxeffWovL = quot(Coxeff * Weff, Leff);
   const double beta = ueff * CoxeffWovL;
-  T3 = ueff / Leff;
+  T3 = quot(ueff, Leff);
   const double dbeta_dVg = CoxeffWovL * dueff_dVg + T3 * (Weff * dCoxeff_dVg + Coxeff * dWeff_dVg);
   const double dbeta_dVd = CoxeffWovL * dueff_dVd;
   const double dbeta_dVb = CoxeffWovL * dueff_dVb + T3 * Coxeff * dWeff_dVb;
   (void)dbeta_dVd; (void)dbeta_dVb;
 
   // Linear-region current Idl (:9591-9640).
-  const double AbovVgst2Vtm = Abulk / Vgst2Vtm;
+  const double AbovVgst2Vtm = quot(Abulk, Vgst2Vtm);
   T0 = 1.0 - 0.5 * Vdseff * AbovVgst2Vtm;
-  dT0_dVg = -0.5 * (Abulk * dVdseff_dVg - Abulk * Vdseff / Vgst2Vtm + Vdseff * dAbulk_dVg) / Vgst2Vtm;
-  dT0_dVd = -0.5 * Abulk * dVdseff_dVd / Vgst2Vtm;
-  dT0_dVb = -0.5 * (Abulk * dVdseff_dVb + dAbulk_dVb * Vdseff) / Vgst2Vtm;
+  dT0_dVg = quot(-0.5 * (Abulk * dVdseff_dVg - quot(Abulk * Vdseff, Vgst2Vtm) + Vdseff * dAbulk_dVg), Vgst2Vtm);
+  dT0_dVd = quot(-0.5 * Abulk * dVdseff_dVd, Vgst2Vtm);
+  dT0_dVb = quot(-0.5 * (Abulk * dVdseff_dVb + dAbulk_dVb * Vdseff), Vgst2Vtm);
   const double fgche1 = Vgsteff * T0;
   const double dfgche1_dVg = Vgsteff * dT0_dVg + T0;
   const double dfgche1_dVd = Vgsteff * dT0_dVd;
   const double dfgche1_dVb = Vgsteff * dT0_dVb;
-  T9 = Vdseff / EsatL;
+  T9 = quot(Vdseff, EsatL);
   const double fgche2 = 1.0 + T9;
-  const double dfgche2_dVg = (dVdseff_dVg - T9 * dEsatL_dVg) / EsatL;
-  const double dfgche2_dVd = (dVdseff_dVd - T9 * dEsatL_dVd) / EsatL;
-  const double dfgche2_dVb = (dVdseff_dVb - T9 * dEsatL_dVb) / EsatL;
-  const double gche = beta * fgche1 / fgche2;
-  const double dgche_dVg = (beta * dfgche1_dVg + fgche1 * dbeta_dVg - gche * dfgche2_dVg) / fgche2;
-  const double dgche_dVd = (beta * dfgche1_dVd + fgche1 * dbeta_dVd - gche * dfgche2_dVd) / fgche2;
-  const double dgche_dVb = (beta * dfgche1_dVb + fgche1 * dbeta_dVb - gche * dfgche2_dVb) / fgche2;
+  const double dfgche2_dVg = quot((dVdseff_dVg - T9 * dEsatL_dVg), EsatL);
+  const double dfgche2_dVd = quot((dVdseff_dVd - T9 * dEsatL_dVd), EsatL);
+  const double dfgche2_dVb = quot((dVdseff_dVb - T9 * dEsatL_dVb), EsatL);
+  const double gche = quot(beta * fgche1, fgche2);
+  const double dgche_dVg = quot((beta * dfgche1_dVg + fgche1 * dbeta_dVg - gche * dfgche2_dVg), fgche2);
+  const double dgche_dVd = quot((beta * dfgche1_dVd + fgche1 * dbeta_dVd - gche * dfgche2_dVd), fgche2);
+  const double dgche_dVb = quot((beta * dfgche1_dVb + fgche1 * dbeta_dVb - gche * dfgche2_dVb), fgche2);
   T0 = 1.0 + gche * Rds;
-  const double Idl = gche / T0;
-  T1 = (1.0 - Idl * Rds) / T0;
+  const double Idl = quot(gche, T0);
+  T1 = quot((1.0 - Idl * Rds), T0);
   T2 = Idl * Idl;
   const double dIdl_dVg = T1 * dgche_dVg - T2 * dRds_dVg;
   const double dIdl_dVd = T1 * dgche_dVd;
@@ -3041,24 +3042,24 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     FP = 1.0;
     dFP_dVg = 0.0;
   } else {
-    T9 = P(fprout) * sqrt(Leff) / Vgst2Vtm;
-    FP = 1.0 / (1.0 + T9);
-    dFP_dVg = FP * FP * T9 / Vgst2Vtm;
+    T9 = quot(P(fprout) * sqrt(Leff), Vgst2Vtm);
+    FP = quot(1.0, 1.0 + T9);
+    dFP_dVg = quot(FP * FP * T9, Vgst2Vtm);
   }
   double PvagTerm, dPvagTerm_dVg, dPvagTerm_dVb, dPvagTerm_dVd;
-  T8 = P(pvag) / EsatL;
+  T8 = quot(P(pvag), EsatL);
   T9 = T8 * Vgsteff;
   if (T9 > -0.9) {
     PvagTerm = 1.0 + T9;
-    dPvagTerm_dVg = T8 * (1.0 - Vgsteff * dEsatL_dVg / EsatL);
-    dPvagTerm_dVb = -T9 * dEsatL_dVb / EsatL;
-    dPvagTerm_dVd = -T9 * dEsatL_dVd / EsatL;
+    dPvagTerm_dVg = T8 * (1.0 - quot(Vgsteff * dEsatL_dVg, EsatL));
+    dPvagTerm_dVb = quot(-T9 * dEsatL_dVb, EsatL);
+    dPvagTerm_dVd = quot(-T9 * dEsatL_dVd, EsatL);
   } else {
-    T4 = 1.0 / (17.0 + 20.0 * T9);
+    T4 = quot(1.0, 17.0 + 20.0 * T9);
     PvagTerm = (0.8 + T9) * T4;
     T4 *= T4;
-    dPvagTerm_dVg = T8 * (1.0 - Vgsteff * dEsatL_dVg / EsatL) * T4;
-    T9 *= T4 / EsatL;
+    dPvagTerm_dVg = T8 * (1.0 - quot(Vgsteff * dEsatL_dVg, EsatL)) * T4;
+    T9 *= quot(T4, EsatL);
     dPvagTerm_dVb = -T9 * dEsatL_dVb;
     dPvagTerm_dVd = -T9 * dEsatL_dVd;
   }
@@ -3068,15 +3069,15 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     dT0_dVg = dRds_dVg * Idl + Rds * dIdl_dVg;
     dT0_dVd = Rds * dIdl_dVd;
     dT0_dVb = dRds_dVb * Idl + Rds * dIdl_dVb;
-    T2 = Vdsat / Esat;
+    T2 = quot(Vdsat, Esat);
     T1 = Leff + T2;
-    dT1_dVg = (dVdsat_dVg - T2 * dEsatL_dVg / Leff) / Esat;
-    dT1_dVd = (dVdsat_dVd - T2 * dEsatL_dVd / Leff) / Esat;
-    dT1_dVb = (dVdsat_dVb - T2 * dEsatL_dVb / Leff) / Esat;
-    Cclm = FP * PvagTerm * T0 * T1 / (P(pclm) * P(litl));
-    dCclm_dVg = Cclm * (dFP_dVg / FP + dPvagTerm_dVg / PvagTerm + dT0_dVg / T0 + dT1_dVg / T1);
-    dCclm_dVb = Cclm * (dPvagTerm_dVb / PvagTerm + dT0_dVb / T0 + dT1_dVb / T1);
-    dCclm_dVd = Cclm * (dPvagTerm_dVd / PvagTerm + dT0_dVd / T0 + dT1_dVd / T1);
+    dT1_dVg = quot((dVdsat_dVg - quot(T2 * dEsatL_dVg, Leff)), Esat);
+    dT1_dVd = quot((dVdsat_dVd - quot(T2 * dEsatL_dVd, Leff)), Esat);
+    dT1_dVb = quot((dVdsat_dVb - quot(T2 * dEsatL_dVb, Leff)), Esat);
+    Cclm = quot(FP * PvagTerm * T0 * T1, P(pclm) * P(litl));
+    dCclm_dVg = Cclm * (quot(dFP_dVg, FP) + quot(dPvagTerm_dVg, PvagTerm) + quot(dT0_dVg, T0) + quot(dT1_dVg, T1));
+    dCclm_dVb = Cclm * (quot(dPvagTerm_dVb, PvagTerm) + quot(dT0_dVb, T0) + quot(dT1_dVb, T1));
+    dCclm_dVd = Cclm * (quot(dPvagTerm_dVd, PvagTerm) + quot(dT0_dVd, T0) + quot(dT1_dVd, T1));
     VACLM = Cclm * diffVds;
     dVACLM_dVg = dCclm_dVg * diffVds - dVdseff_dVg * Cclm;
     dVACLM_dVb = dCclm_dVb * diffVds - dVdseff_dVb * Cclm;
@@ -3099,19 +3100,19 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     dT1_dVd = Abulk * dVdsat_dVd;
     T9 = T1 * T1;
     T2 = P(thetaRout);
-    VADIBL = (Vgst2Vtm - T0 / T1) / T2;
-    dVADIBL_dVg = (1.0 - dT0_dVg / T1 + T0 * dT1_dVg / T9) / T2;
-    dVADIBL_dVb = (-dT0_dVb / T1 + T0 * dT1_dVb / T9) / T2;
-    dVADIBL_dVd = (-dT0_dVd / T1 + T0 * dT1_dVd / T9) / T2;
+    VADIBL = quot((Vgst2Vtm - quot(T0, T1)), T2);
+    dVADIBL_dVg = quot((1.0 - quot(dT0_dVg, T1) + quot(T0 * dT1_dVg, T9)), T2);
+    dVADIBL_dVb = quot((quot(-dT0_dVb, T1) + quot(T0 * dT1_dVb, T9)), T2);
+    dVADIBL_dVd = quot((quot(-dT0_dVd, T1) + quot(T0 * dT1_dVd, T9)), T2);
     T7 = P(pdiblb) * Vbseff;
     if (T7 >= -0.9) {
-      T3 = 1.0 / (1.0 + T7);
+      T3 = quot(1.0, 1.0 + T7);
       VADIBL *= T3;
       dVADIBL_dVg *= T3;
       dVADIBL_dVb = (dVADIBL_dVb - VADIBL * P(pdiblb)) * T3;
       dVADIBL_dVd *= T3;
     } else {
-      T4 = 1.0 / (0.8 + T7);
+      T4 = quot(1.0, 0.8 + T7);
       T3 = (17.0 + 20.0 * T7) * T4;
       dVADIBL_dVg *= T3;
       dVADIBL_dVb = dVADIBL_dVb * T3 - VADIBL * P(pdiblb) * T4 * T4;
@@ -3141,9 +3142,9 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   double VADITS, dVADITS_dVg, dVADITS_dVd;
   if (P(pdits) > CONSTMIN_EXP) {
     T2 = 1.0 + P(pditsl) * Leff;
-    VADITS = (1.0 + T2 * T1) / P(pdits);
+    VADITS = quot((1.0 + T2 * T1), P(pdits));
     dVADITS_dVg = VADITS * dFP_dVg;
-    dVADITS_dVd = FP * T2 * dT1_dVd / P(pdits);
+    dVADITS_dVd = quot(FP * T2 * dT1_dVd, P(pdits));
     VADITS *= FP;
   } else {
     VADITS = CONSTMAX_EXP;
@@ -3151,15 +3152,15 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   }
   double VASCBE, dVASCBE_dVg, dVASCBE_dVd, dVASCBE_dVb;
   if (P(pscbe2) > 0.0) {
-    if (diffVds > P(pscbe1) * P(litl) / CONSTEXP_THRESHOLD) {
-      T0 = P(pscbe1) * P(litl) / diffVds;
-      VASCBE = Leff * exp(T0) / P(pscbe2);
-      T1 = T0 * VASCBE / diffVds;
+    if (diffVds > quot(P(pscbe1) * P(litl), CONSTEXP_THRESHOLD)) {
+      T0 = quot(P(pscbe1) * P(litl), diffVds);
+      VASCBE = quot(Leff * exp(T0), P(pscbe2));
+      T1 = quot(T0 * VASCBE, diffVds);
       dVASCBE_dVg = T1 * dVdseff_dVg;
       dVASCBE_dVd = -T1 * (1.0 - dVdseff_dVd);
       dVASCBE_dVb = T1 * dVdseff_dVb;
     } else {
-      VASCBE = CONSTMAX_EXP * Leff / P(pscbe2);
+      VASCBE = quot(CONSTMAX_EXP * Leff, P(pscbe2));
       dVASCBE_dVg = dVASCBE_dVd = dVASCBE_dVb = 0.0;
     }
   } else {
@@ -3168,27 +3169,27 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   }
 
   // Drain current with CLM, DIBL, DITS, SCBE (:9801-9870).
-  T9 = diffVds / VADIBL;
+  T9 = quot(diffVds, VADIBL);
   T0 = 1.0 + T9;
   double Idsa = Idl * T0;
-  double dIdsa_dVg = T0 * dIdl_dVg - Idl * (dVdseff_dVg + T9 * dVADIBL_dVg) / VADIBL;
-  double dIdsa_dVd = T0 * dIdl_dVd + Idl * (1.0 - dVdseff_dVd - T9 * dVADIBL_dVd) / VADIBL;
-  double dIdsa_dVb = T0 * dIdl_dVb - Idl * (dVdseff_dVb + T9 * dVADIBL_dVb) / VADIBL;
-  T9 = diffVds / VADITS;
+  double dIdsa_dVg = T0 * dIdl_dVg - quot(Idl * (dVdseff_dVg + T9 * dVADIBL_dVg), VADIBL);
+  double dIdsa_dVd = T0 * dIdl_dVd + quot(Idl * (1.0 - dVdseff_dVd - T9 * dVADIBL_dVd), VADIBL);
+  double dIdsa_dVb = T0 * dIdl_dVb - quot(Idl * (dVdseff_dVb + T9 * dVADIBL_dVb), VADIBL);
+  T9 = quot(diffVds, VADITS);
   T0 = 1.0 + T9;
-  dIdsa_dVg = T0 * dIdsa_dVg - Idsa * (dVdseff_dVg + T9 * dVADITS_dVg) / VADITS;
-  dIdsa_dVd = T0 * dIdsa_dVd + Idsa * (1.0 - dVdseff_dVd - T9 * dVADITS_dVd) / VADITS;
-  dIdsa_dVb = T0 * dIdsa_dVb - Idsa * dVdseff_dVb / VADITS;
+  dIdsa_dVg = T0 * dIdsa_dVg - quot(Idsa * (dVdseff_dVg + T9 * dVADITS_dVg), VADITS);
+  dIdsa_dVd = T0 * dIdsa_dVd + quot(Idsa * (1.0 - dVdseff_dVd - T9 * dVADITS_dVd), VADITS);
+  dIdsa_dVb = T0 * dIdsa_dVb - quot(Idsa * dVdseff_dVb, VADITS);
   Idsa *= T0;
-  T0 = log(Va / Vasat);
-  dT0_dVg = dVa_dVg / Va - dVasat_dVg / Vasat;
-  dT0_dVb = dVa_dVb / Va - dVasat_dVb / Vasat;
-  dT0_dVd = dVa_dVd / Va - dVasat_dVd / Vasat;
-  T1 = T0 / Cclm;
+  T0 = log(quot(Va, Vasat));
+  dT0_dVg = quot(dVa_dVg, Va) - quot(dVasat_dVg, Vasat);
+  dT0_dVb = quot(dVa_dVb, Va) - quot(dVasat_dVb, Vasat);
+  dT0_dVd = quot(dVa_dVd, Va) - quot(dVasat_dVd, Vasat);
+  T1 = quot(T0, Cclm);
   T9 = 1.0 + T1;
-  dT9_dVg = (dT0_dVg - T1 * dCclm_dVg) / Cclm;
-  dT9_dVb = (dT0_dVb - T1 * dCclm_dVb) / Cclm;
-  dT9_dVd = (dT0_dVd - T1 * dCclm_dVd) / Cclm;
+  dT9_dVg = quot((dT0_dVg - T1 * dCclm_dVg), Cclm);
+  dT9_dVb = quot((dT0_dVb - T1 * dCclm_dVb), Cclm);
+  dT9_dVd = quot((dT0_dVd - T1 * dCclm_dVd), Cclm);
   dIdsa_dVg = dIdsa_dVg * T9 + Idsa * dT9_dVg;
   dIdsa_dVb = dIdsa_dVb * T9 + Idsa * dT9_dVb;
   dIdsa_dVd = dIdsa_dVd * T9 + Idsa * dT9_dVd;
@@ -3200,11 +3201,11 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   if ((tmp <= 0.0) || (P(beta0) <= 0.0)) {
     Isub = Gbd = Gbb = Gbg = 0.0;
   } else {
-    T2 = tmp / Leff;
-    if (diffVds > P(beta0) / CONSTEXP_THRESHOLD) {
-      T0 = -P(beta0) / diffVds;
+    T2 = quot(tmp, Leff);
+    if (diffVds > quot(P(beta0), CONSTEXP_THRESHOLD)) {
+      T0 = quot(-P(beta0), diffVds);
       T1 = T2 * diffVds * exp(T0);
-      T3 = T1 / diffVds * (T0 - 1.0);
+      T3 = quot(T1, diffVds) * (T0 - 1.0);
       dT1_dVg = T3 * dVdseff_dVg;
       dT1_dVd = T3 * (dVdseff_dVd - 1.0);
       dT1_dVb = T3 * dVdseff_dVb;
@@ -3228,12 +3229,12 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   double csub = Isub, gbbs = Gbb, gbgs = Gbg, gbds = Gbd;
 
   // Drain current and conductances (:9911-9990).
-  T9 = diffVds / VASCBE;
+  T9 = quot(diffVds, VASCBE);
   T0 = 1.0 + T9;
   const double Ids = Idsa * T0;
-  double Gm = T0 * dIdsa_dVg - Idsa * (dVdseff_dVg + T9 * dVASCBE_dVg) / VASCBE;
-  double Gds = T0 * dIdsa_dVd + Idsa * (1.0 - dVdseff_dVd - T9 * dVASCBE_dVd) / VASCBE;
-  double Gmb = T0 * dIdsa_dVb - Idsa * (dVdseff_dVb + T9 * dVASCBE_dVb) / VASCBE;
+  double Gm = T0 * dIdsa_dVg - quot(Idsa * (dVdseff_dVg + T9 * dVASCBE_dVg), VASCBE);
+  double Gds = T0 * dIdsa_dVd + quot(Idsa * (1.0 - dVdseff_dVd - T9 * dVASCBE_dVd), VASCBE);
+  double Gmb = T0 * dIdsa_dVb - quot(Idsa * (dVdseff_dVb + T9 * dVASCBE_dVb), VASCBE);
   tmp1 = Gds + Gm * dVgsteff_dVd;
   tmp2 = Gmb + Gm * dVgsteff_dVb;
   tmp3 = Gm;
@@ -3242,24 +3243,24 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   Gmb = (Ids * (dVdseff_dVb + dVdseff_dVg * dVgsteff_dVb) + Vdseff * tmp2) * dVbseff_dVb;
   double cdrain = Ids * Vdseff;
   if ((P(vtlGiven) != 0.0) && (P(vtl_m) > 0.0)) {
-    T12 = 1.0 / Leff / CoxeffWovL;
-    T11 = T12 / Vgsteff;
-    T10 = -T11 / Vgsteff;
+    T12 = quot(quot(1.0, Leff), CoxeffWovL);
+    T11 = quot(T12, Vgsteff);
+    T10 = quot(-T11, Vgsteff);
     const double vs = cdrain * T11;
     const double dvs_dVg = Gm * T11 + cdrain * T10 * dVgsteff_dVg;
     const double dvs_dVd = Gds * T11 + cdrain * T10 * dVgsteff_dVd;
     const double dvs_dVb = Gmb * T11 + cdrain * T10 * dVgsteff_dVb;
     T0 = 2 * CONSTMM;
-    T1 = vs / (P(vtl) * P(tfactor));
+    T1 = quot(vs, P(vtl) * P(tfactor));
     double Fsevl, dFsevl_dVg, dFsevl_dVd, dFsevl_dVb;
     if (T1 > 0.0) {
       T2 = 1.0 + exp(T0 * log(T1));
-      T3 = (T2 - 1.0) * T0 / vs;
-      Fsevl = 1.0 / exp(log(T2) / T0);
+      T3 = quot((T2 - 1.0) * T0, vs);
+      Fsevl = quot(1.0, exp(quot(log(T2), T0)));
       dT2_dVg = T3 * dvs_dVg;
       dT2_dVd = T3 * dvs_dVd;
       dT2_dVb = T3 * dvs_dVb;
-      T4 = -1.0 / T0 * Fsevl / T2;
+      T4 = quot(quot(-1.0, T0) * Fsevl, T2);
       dFsevl_dVg = T4 * dT2_dVg;
       dFsevl_dVd = T4 * dT2_dVd;
       dFsevl_dVb = T4 * dT2_dVb;
@@ -3300,8 +3301,8 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     if (rgateMod == 2) {
       T10 = P(grgeltd) * P(grgeltd);
       T11 = P(grgeltd) + gcrg;
-      gcrg = P(grgeltd) * gcrg / T11;
-      T12 = T10 / T11 / T11;
+      gcrg = quot(P(grgeltd) * gcrg, T11);
+      T12 = quot(quot(T10, T11), T11);
       gcrgg *= T12;
       gcrgd *= T12;
       gcrgb *= T12;
@@ -3317,14 +3318,14 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     T0 = vgs - P(vfbsd);
     T1 = sqrt(T0 * T0 + 1.0e-4);
     vgs_eff = 0.5 * (T0 + T1);
-    dvgs_eff_dvg = vgs_eff / T1;
+    dvgs_eff_dvg = quot(vgs_eff, T1);
     T0 = 1.0 + P(prwg) * vgs_eff;
-    double dT0_dvg = -P(prwg) / T0 / T0 * dvgs_eff_dvg;
+    double dT0_dvg = quot(quot(-P(prwg), T0), T0) * dvgs_eff_dvg;
     T1 = -P(prwb) * vbs;
     double dT1_dvb = -P(prwb);
-    T2 = 1.0 / T0 + T1;
+    T2 = quot(1.0, T0) + T1;
     T3 = T2 + sqrt(T2 * T2 + 0.01);
-    double dT3_dvg = T3 / (T3 - T2);
+    double dT3_dvg = quot(T3, T3 - T2);
     double dT3_dvb = dT3_dvg * dT1_dvb;
     dT3_dvg *= dT0_dvg;
     T4 = P(rs0) * 0.5;
@@ -3332,7 +3333,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     const double dRs_dvg = T4 * dT3_dvg;
     const double dRs_dvb = T4 * dT3_dvb;
     T0 = 1.0 + P(sourceConductance) * Rs;
-    gstot = P(sourceConductance) / T0;
+    gstot = quot(P(sourceConductance), T0);
     T0 = -gstot * gstot;
     const double dgstot_dvd = 0.0;
     const double dgstot_dvg = T0 * dRs_dvg;
@@ -3341,14 +3342,14 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     T0 = vgd - P(vfbsd);
     T1 = sqrt(T0 * T0 + 1.0e-4);
     vgd_eff = 0.5 * (T0 + T1);
-    dvgd_eff_dvg = vgd_eff / T1;
+    dvgd_eff_dvg = quot(vgd_eff, T1);
     T0 = 1.0 + P(prwg) * vgd_eff;
-    dT0_dvg = -P(prwg) / T0 / T0 * dvgd_eff_dvg;
+    dT0_dvg = quot(quot(-P(prwg), T0), T0) * dvgd_eff_dvg;
     T1 = -P(prwb) * vbd;
     dT1_dvb = -P(prwb);
-    T2 = 1.0 / T0 + T1;
+    T2 = quot(1.0, T0) + T1;
     T3 = T2 + sqrt(T2 * T2 + 0.01);
-    dT3_dvg = T3 / (T3 - T2);
+    dT3_dvg = quot(T3, T3 - T2);
     dT3_dvb = dT3_dvg * dT1_dvb;
     dT3_dvg *= dT0_dvg;
     T4 = P(rd0) * 0.5;
@@ -3356,7 +3357,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     const double dRd_dvg = T4 * dT3_dvg;
     const double dRd_dvb = T4 * dT3_dvb;
     T0 = 1.0 + P(drainConductance) * Rd;
-    gdtot = P(drainConductance) / T0;
+    gdtot = quot(P(drainConductance), T0);
     T0 = -gdtot * gdtot;
     const double dgdtot_dvs = 0.0;
     const double dgdtot_dvg = T0 * dRd_dvg;
@@ -3376,17 +3377,17 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
   // GIDL and GISL (:10063-10180). vgs_eff / vgd_eff here are the poly-depleted gate voltages
   // (rdsMod 0) or the S/D-resistance ones (rdsMod 1).
   T0 = 3.0 * toxe;
-  T1 = (vds - vgs_eff - P(egidl)) / T0;
+  T1 = quot((vds - vgs_eff - P(egidl)), T0);
   double Igidl, Ggidld, Ggidlg, Ggidlb;
   if ((P(agidl) <= 0.0) || (P(bgidl) <= 0.0) || (T1 <= 0.0) || (P(cgidl) <= 0.0) || (vbd > 0.0)) {
     Igidl = Ggidld = Ggidlg = Ggidlb = 0.0;
   } else {
-    dT1_dVd = 1.0 / T0;
+    dT1_dVd = quot(1.0, T0);
     dT1_dVg = -dvgs_eff_dvg * dT1_dVd;
-    T2 = P(bgidl) / T1;
+    T2 = quot(P(bgidl), T1);
     if (T2 < 100.0) {
       Igidl = P(agidl) * weffCJ * T1 * exp(-T2);
-      T3 = Igidl * (1.0 + T2) / T1;
+      T3 = quot(Igidl * (1.0 + T2), T1);
       Ggidld = T3 * dT1_dVd;
       Ggidlg = T3 * dT1_dVg;
     } else {
@@ -3398,25 +3399,25 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     T4 = vbd * vbd;
     T5 = -vbd * T4;
     T6 = P(cgidl) + T5;
-    T7 = T5 / T6;
-    T8 = 3.0 * P(cgidl) * T4 / T6 / T6;
+    T7 = quot(T5, T6);
+    T8 = quot(quot(3.0 * P(cgidl) * T4, T6), T6);
     Ggidld = Ggidld * T7 + Igidl * T8;
     Ggidlg = Ggidlg * T7;
     Ggidlb = -Igidl * T8;
     Igidl *= T7;
   }
   double ggidld = Ggidld, ggidlg = Ggidlg, ggidlb = Ggidlb;
-  T1 = (-vds - vgd_eff - P(egisl)) / T0;
+  T1 = quot((-vds - vgd_eff - P(egisl)), T0);
   double Igisl, Ggisls, Ggislg, Ggislb;
   if ((P(agisl) <= 0.0) || (P(bgisl) <= 0.0) || (T1 <= 0.0) || (P(cgisl) <= 0.0) || (vbs > 0.0)) {
     Igisl = Ggisls = Ggislg = Ggislb = 0.0;
   } else {
-    dT1_dVd = 1.0 / T0;
+    dT1_dVd = quot(1.0, T0);
     dT1_dVg = -dvgd_eff_dvg * dT1_dVd;
-    T2 = P(bgisl) / T1;
+    T2 = quot(P(bgisl), T1);
     if (T2 < 100.0) {
       Igisl = P(agisl) * weffCJ * T1 * exp(-T2);
-      T3 = Igisl * (1.0 + T2) / T1;
+      T3 = quot(Igisl * (1.0 + T2), T1);
       Ggisls = T3 * dT1_dVd;
       Ggislg = T3 * dT1_dVg;
     } else {
@@ -3428,8 +3429,8 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     T4 = vbs * vbs;
     T5 = -vbs * T4;
     T6 = P(cgisl) + T5;
-    T7 = T5 / T6;
-    T8 = 3.0 * P(cgisl) * T4 / T6 / T6;
+    T7 = quot(T5, T6);
+    T8 = quot(quot(3.0 * P(cgisl) * T4, T6), T6);
     Ggisls = Ggisls * T7 + Igisl * T8;
     Ggislg = Ggislg * T7;
     Ggislb = -Igisl * T8;
@@ -3453,7 +3454,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
         T0 = sqrt(V3 * V3 - 4.0 * CONSTDELTA_3 * Vfb_g);
       else
         T0 = sqrt(V3 * V3 + 4.0 * CONSTDELTA_3 * Vfb_g);
-      T1 = 0.5 * (1.0 + V3 / T0);
+      T1 = 0.5 * (1.0 + quot(V3, T0));
       const double Vfbeff = Vfb_g - 0.5 * (V3 + T0);
       const double dVfbeff_dVg = T1 * dVgs_eff_dVg;
       const double dVfbeff_dVb = -T1;
@@ -3475,7 +3476,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
         dVoxdepinv_dVb = dVfbeff_dVb + 1.0 + dVgsteff_dVb;
       } else {
         T1 = sqrt(T0 * T0 + T3);
-        T2 = T0 / T1;
+        T2 = quot(T0, T1);
         Voxdepinv = k1ox * (T1 - T0);
         dVoxdepinv_dVg = T2 * (dVgs_eff_dVg - dVfbeff_dVg - dVgsteff_dVg);
         dVoxdepinv_dVd = -T2 * dVgsteff_dVd;
@@ -3491,7 +3492,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     if (igcMod) {
       T0 = vtmg * P(nigc);
       if (igcMod == 1) {
-        VxNVt = (Vgs_eff - dtype * vth0) / T0;
+        VxNVt = quot((Vgs_eff - dtype * vth0), T0);
         if (VxNVt > CONSTEXP_THRESHOLD) {
           Vaux = Vgs_eff - dtype * vth0;
           dVaux_dVg = dVgs_eff_dVg;
@@ -3499,7 +3500,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
           dVaux_dVb = 0.0;
         }
       } else {
-        VxNVt = (Vgs_eff - von) / T0;
+        VxNVt = quot((Vgs_eff - von), T0);
         if (VxNVt > CONSTEXP_THRESHOLD) {
           Vaux = Vgs_eff - von;
           dVaux_dVg = dVgs_eff_dVg;
@@ -3513,7 +3514,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
       } else if ((VxNVt >= -CONSTEXP_THRESHOLD) && (VxNVt <= CONSTEXP_THRESHOLD)) {
         const double ExpVxNVt = exp(VxNVt);
         Vaux = T0 * log(1.0 + ExpVxNVt);
-        dVaux_dVg = ExpVxNVt / (1.0 + ExpVxNVt);
+        dVaux_dVg = quot(ExpVxNVt, 1.0 + ExpVxNVt);
         if (igcMod == 1) {
           dVaux_dVd = 0.0;
           dVaux_dVb = 0.0;
@@ -3556,10 +3557,10 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
       } else {
         T11 = P(Bechvb) * toxe;
         T12 = Vgsteff + 1.0e-20;
-        T13 = T11 / T12 / T12;
-        T14 = -T13 / T12;
-        Pigcd = T13 * (1.0 - 0.5 * Vdseff / T12);
-        dPigcd_dVg = T14 * (2.0 + 0.5 * (dVdseff_dVg - 3.0 * Vdseff / T12));
+        T13 = quot(quot(T11, T12), T12);
+        T14 = quot(-T13, T12);
+        Pigcd = T13 * (1.0 - quot(0.5 * Vdseff, T12));
+        dPigcd_dVg = T14 * (2.0 + 0.5 * (dVdseff_dVg - quot(3.0 * Vdseff, T12)));
         dPigcd_dVd = 0.5 * T14 * dVdseff_dVd;
         dPigcd_dVb = 0.5 * T14 * dVdseff_dVb;
       }
@@ -3588,19 +3589,19 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
       }
       T0 = T8 * T8;
       T1 = T9 - 1.0 + 1.0e-4;
-      T10 = (T1 - T7) / T8;
-      dT10_dVg = (dT9_dVg - dT7_dVg - T10 * dT8_dVg) / T8;
-      dT10_dVd = (dT9_dVd - dT7_dVd - T10 * dT8_dVd) / T8;
-      dT10_dVb = (dT9_dVb - dT7_dVb - T10 * dT8_dVb) / T8;
+      T10 = quot((T1 - T7), T8);
+      dT10_dVg = quot((dT9_dVg - dT7_dVg - T10 * dT8_dVg), T8);
+      dT10_dVd = quot((dT9_dVd - dT7_dVd - T10 * dT8_dVd), T8);
+      dT10_dVb = quot((dT9_dVb - dT7_dVb - T10 * dT8_dVb), T8);
       Igcs = Igc * T10;
       const double dIgcs_dVg = dIgc_dVg * T10 + Igc * dT10_dVg;
       const double dIgcs_dVd = dIgc_dVd * T10 + Igc * dT10_dVd;
       const double dIgcs_dVb = dIgc_dVb * T10 + Igc * dT10_dVb;
       T1 = T9 - 1.0 - 1.0e-4;
-      T10 = (T7 * T9 - T1) / T8;
-      dT10_dVg = (dT7_dVg * T9 + (T7 - 1.0) * dT9_dVg - T10 * dT8_dVg) / T8;
-      dT10_dVd = (dT7_dVd * T9 + (T7 - 1.0) * dT9_dVd - T10 * dT8_dVd) / T8;
-      dT10_dVb = (dT7_dVb * T9 + (T7 - 1.0) * dT9_dVb - T10 * dT8_dVb) / T8;
+      T10 = quot((T7 * T9 - T1), T8);
+      dT10_dVg = quot((dT7_dVg * T9 + (T7 - 1.0) * dT9_dVg - T10 * dT8_dVg), T8);
+      dT10_dVd = quot((dT7_dVd * T9 + (T7 - 1.0) * dT9_dVd - T10 * dT8_dVd), T8);
+      dT10_dVb = quot((dT7_dVb * T9 + (T7 - 1.0) * dT9_dVb - T10 * dT8_dVb), T8);
       Igcd = Igc * T10;
       const double dIgcd_dVg = dIgc_dVg * T10 + Igc * dT10_dVg;
       const double dIgcd_dVd = dIgc_dVd * T10 + Igc * dT10_dVd;
@@ -3615,7 +3616,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
       const double vfbsd_t = P(vfbsd) + P(vfbsdoff);
       T0 = vgs - vfbsd_t;
       double vgx_eff = sqrt(T0 * T0 + 1.0e-4);
-      double dvgx_eff_dvg = T0 / vgx_eff;
+      double dvgx_eff_dvg = quot(T0, vgx_eff);
       T2 = vgs * vgx_eff;
       dT2_dVg = vgs * dvgx_eff_dvg + vgx_eff;
       T11 = P(AechvbEdgeS);
@@ -3638,7 +3639,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
       const double dIgs_dVs = -dIgs_dVg;
       T0 = vgd - vfbsd_t;
       vgx_eff = sqrt(T0 * T0 + 1.0e-4);
-      dvgx_eff_dvg = T0 / vgx_eff;
+      dvgx_eff_dvg = quot(T0, vgx_eff);
       T2 = vgd * vgx_eff;
       dT2_dVg = vgd * dvgx_eff_dvg + vgx_eff;
       T11 = P(AechvbEdgeD);
@@ -3666,7 +3667,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
     if (igbMod) {
       T0 = vtmg * P(nigbacc);
       T1 = -Vgs_eff + Vbseff + Vfb_g;
-      VxNVt = T1 / T0;
+      VxNVt = quot(T1, T0);
       if (VxNVt > CONSTEXP_THRESHOLD) {
         Vaux = T1;
         dVaux_dVg = -dVgs_eff_dVg;
@@ -3677,7 +3678,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
       } else {
         const double ExpVxNVt = exp(VxNVt);
         Vaux = T0 * log(1.0 + ExpVxNVt);
-        dVaux_dVb = ExpVxNVt / (1.0 + ExpVxNVt);
+        dVaux_dVb = quot(ExpVxNVt, 1.0 + ExpVxNVt);
         dVaux_dVg = -dVaux_dVb * dVgs_eff_dVg;
       }
       T2 = (Vgs_eff - Vbseff) * Vaux;
@@ -3705,7 +3706,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
       const double dIgbacc_dVb = T11 * (T2 * dT6_dVb + T6 * dT2_dVb);
       T0 = vtmg * P(nigbinv);
       T1 = Voxdepinv - P(eigbinv);
-      VxNVt = T1 / T0;
+      VxNVt = quot(T1, T0);
       if (VxNVt > CONSTEXP_THRESHOLD) {
         Vaux = T1;
         dVaux_dVg = dVoxdepinv_dVg;
@@ -3717,7 +3718,7 @@ XD_HD void bsim4_load(const RV &P_, const double *V, const double *sto_old, cons
       } else {
         const double ExpVxNVt = exp(VxNVt);
         Vaux = T0 * log(1.0 + ExpVxNVt);
-        dVaux_dVg = ExpVxNVt / (1.0 + ExpVxNVt);
+        dVaux_dVg = quot(ExpVxNVt, 1.0 + ExpVxNVt);
         dVaux_dVd = dVaux_dVg * dVoxdepinv_dVd;
         dVaux_dVb = dVaux_dVg * dVoxdepinv_dVb;
         dVaux_dVg *= dVoxdepinv_dVg;

@@ -686,6 +686,17 @@ void free_map(GatherMap &m) {
   m = GatherMap();
 }
 
+// The models' quotient (quot.h) of each pair, and of each numerator by the constants 3, 12 and 0.25.
+__global__ void quot_probe_kernel(int n, const double *__restrict__ a, const double *__restrict__ b,
+                                  double *__restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  out[i] = quot(a[i], b[i]);
+  out[(size_t)n + i] = quot_by_constant(a[i], 3.0);
+  out[(size_t)2 * n + i] = quot_by_constant(a[i], 12.0);
+  out[(size_t)3 * n + i] = quot_by_constant(a[i], 0.25);
+}
+
 // FP64 FMA throughput probe: 8 independent accumulator chains x 8 FMAs per iteration per thread.
 __global__ void __launch_bounds__(256) fma_probe_kernel(double *out, int iters) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1634,6 +1645,14 @@ int xd_probe_fp64_fma(double *d_out, int blocks, int iters, void *stream) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "fma_probe_kernel launch");
   return 0;
+}
+
+int xd_probe_quot(const double *d_a, const double *d_b, double *d_out, int n, void *stream) {
+  if (n < 0 || (n > 0 && (!d_a || !d_b || !d_out))) return fail(-1, "bad quotient probe arguments");
+  if (n == 0) return 0;
+  quot_probe_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(n, d_a, d_b, d_out);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : cuda_fail(e, "quot_probe_kernel");
 }
 
 int xd_num_stage_slots(const xd_ctx *ctx) { return ctx ? ctx->stage_slots : -1; }

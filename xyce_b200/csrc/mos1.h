@@ -64,29 +64,29 @@ XD_HD void qmeyer(double vgs, double vgd, double vgb, double von, double vdsat, 
   (void)vgb;
   const double vgst = vgs - von;
   if (vgst <= -phi) {
-    capgb = cox / 2;
+    capgb = quot_by_constant(cox, 2);
     capgs = 0;
     capgd = 0;
-  } else if (vgst <= -phi / 2) {
-    capgb = -vgst * cox / (2 * phi);
+  } else if (vgst <= quot_by_constant(-phi, 2)) {
+    capgb = quot(-vgst * cox, 2 * phi);
     capgs = 0;
     capgd = 0;
   } else if (vgst <= 0) {
-    capgb = -vgst * cox / (2 * phi);
-    capgs = vgst * cox / (1.5 * phi) + cox / 3;
+    capgb = quot(-vgst * cox, 2 * phi);
+    capgs = quot(vgst * cox, 1.5 * phi) + quot_by_constant(cox, 3);
     capgd = 0;
   } else {
     const double vds = vgs - vgd;
     if (vdsat <= vds) {
-      capgs = cox / 3;
+      capgs = quot_by_constant(cox, 3);
       capgd = 0;
       capgb = 0;
     } else {
       const double vddif = 2.0 * vdsat - vds;
       const double vddif1 = vdsat - vds;
       const double vddif2 = vddif * vddif;
-      capgd = cox * (1.0 - vdsat * vdsat / vddif2) / 3;
-      capgs = cox * (1.0 - vddif1 * vddif1 / vddif2) / 3;
+      capgd = quot_by_constant(cox * (1.0 - quot(vdsat * vdsat, vddif2)), 3);
+      capgs = quot_by_constant(cox * (1.0 - quot(vddif1 * vddif1, vddif2)), 3);
       capgb = 0;
     }
   }
@@ -175,21 +175,21 @@ XD_HD void mos1_load(const RV &P_, const double V[4], const double *sto_old, con
   if (vgs_orig != vgs || vds_orig != vds || vbs_orig != vbs || vbd_orig != vbd || vgd_orig != vgd) origFlag = 0;
   double gbs, cbs, gbd, cbd;
   if (vbs <= 0) {
-    gbs = SourceSatCur / vt;
+    gbs = quot(SourceSatCur, vt);
     gbs += gmin;
     cbs = gbs * vbs;
   } else {
-    const double evbs = exp(dmin(CONSTMAX_EXP_ARG, vbs / vt));
-    gbs = (SourceSatCur * evbs / vt + gmin);
+    const double evbs = exp(dmin(CONSTMAX_EXP_ARG, quot(vbs, vt)));
+    gbs = (quot(SourceSatCur * evbs, vt) + gmin);
     cbs = (SourceSatCur * (evbs - 1) + gmin * vbs);
   }
   if (vbd <= 0) {
-    gbd = DrainSatCur / vt;
+    gbd = quot(DrainSatCur, vt);
     gbd += gmin;
     cbd = gbd * vbd;
   } else {
-    const double evbd = exp(dmin(CONSTMAX_EXP_ARG, vbd / vt));
-    gbd = (DrainSatCur * evbd / vt + gmin);
+    const double evbd = exp(dmin(CONSTMAX_EXP_ARG, quot(vbd, vt)));
+    gbd = (quot(DrainSatCur * evbd, vt) + gmin);
     cbd = (DrainSatCur * (evbd - 1) + gmin * vbd);
   }
   const int mode = (vds >= 0) ? 1 : -1;
@@ -203,13 +203,13 @@ XD_HD void mos1_load(const RV &P_, const double V[4], const double *sto_old, con
       sarg = sqrt(tPhi - vbx);
     } else {
       sarg = sqrt(tPhi);
-      sarg = sarg - vbx / (sarg + sarg);
+      sarg = sarg - quot(vbx, sarg + sarg);
       sarg = dmax(0.0, sarg);
     }
     Von = (P(tVbi) * dtype) + gamma * sarg;
     const double vgst = (mode == 1 ? vgs : vgd) - Von;
     Vdsat = dmax(vgst, 0.0);
-    const double arg = (sarg <= 0) ? 0 : gamma / (sarg + sarg);
+    const double arg = (sarg <= 0) ? 0 : quot(gamma, sarg + sarg);
     if (vgst <= 0) {
       cdrain = 0;
       gm = 0;
@@ -237,27 +237,27 @@ XD_HD void mos1_load(const RV &P_, const double V[4], const double *sto_old, con
   double qbs, capbs, qbd, capbd;
   if (Cbs != 0 || Cbssw != 0) {
     if (vbs < tDepCap) {
-      const double arg = 1 - vbs / tBulkPot;
+      const double arg = 1 - quot(vbs, tBulkPot);
       double sarg, sargsw;
       if (MJ == MJSW) {
         if (MJ == .5)
-          sarg = sargsw = 1 / sqrt(arg);
+          sarg = sargsw = quot(1, sqrt(arg));
         else
           sarg = sargsw = exp(-MJ * log(arg));
       } else {
         if (MJ == .5)
-          sarg = 1 / sqrt(arg);
+          sarg = quot(1, sqrt(arg));
         else
           sarg = exp(-MJ * log(arg));
         if (MJSW == .5)
-          sargsw = 1 / sqrt(arg);
+          sargsw = quot(1, sqrt(arg));
         else
           sargsw = exp(-MJSW * log(arg));
       }
-      qbs = tBulkPot * (Cbs * (1 - arg * sarg) / (1 - MJ) + Cbssw * (1 - arg * sargsw) / (1 - MJSW));
+      qbs = tBulkPot * (quot(Cbs * (1 - arg * sarg), 1 - MJ) + quot(Cbssw * (1 - arg * sargsw), 1 - MJSW));
       capbs = Cbs * sarg + Cbssw * sargsw;
     } else {
-      qbs = P(f4s) + vbs * (P(f2s) + vbs * (P(f3s) / 2));
+      qbs = P(f4s) + vbs * (P(f2s) + vbs * (quot_by_constant(P(f3s), 2)));
       capbs = P(f2s) + P(f3s) * vbs;
     }
   } else {
@@ -266,24 +266,24 @@ XD_HD void mos1_load(const RV &P_, const double V[4], const double *sto_old, con
   }
   if (Cbd != 0 || Cbdsw != 0) {
     if (vbd < tDepCap) {
-      const double arg = 1 - vbd / tBulkPot;
+      const double arg = 1 - quot(vbd, tBulkPot);
       double sarg, sargsw;
       if (MJ == .5 && MJSW == .5) {
-        sarg = sargsw = 1 / sqrt(arg);
+        sarg = sargsw = quot(1, sqrt(arg));
       } else {
         if (MJ == .5)
-          sarg = 1 / sqrt(arg);
+          sarg = quot(1, sqrt(arg));
         else
           sarg = exp(-MJ * log(arg));
         if (MJSW == .5)
-          sargsw = 1 / sqrt(arg);
+          sargsw = quot(1, sqrt(arg));
         else
           sargsw = exp(-MJSW * log(arg));
       }
-      qbd = tBulkPot * (Cbd * (1 - arg * sarg) / (1 - MJ) + Cbdsw * (1 - arg * sargsw) / (1 - MJSW));
+      qbd = tBulkPot * (quot(Cbd * (1 - arg * sarg), 1 - MJ) + quot(Cbdsw * (1 - arg * sargsw), 1 - MJSW));
       capbd = Cbd * sarg + Cbdsw * sargsw;
     } else {
-      qbd = P(f4d) + vbd * (P(f2d) + vbd * P(f3d) / 2);
+      qbd = P(f4d) + vbd * (P(f2d) + quot_by_constant(vbd * P(f3d), 2));
       capbd = P(f2d) + vbd * P(f3d);
     }
   } else {

@@ -11,6 +11,7 @@
 
 #include <cmath>
 
+#include "quot.h"
 #include "xd_consts.h"
 
 namespace xdc {
@@ -58,7 +59,7 @@ XD_HD void cv_simple(double Vbseff, double Vbs, double phi, double Phis, double 
     c.qgate = CoxWL * k1ox0 * (T2 - T1);
     c.qbulk = -c.qgate;
     c.qdrn = 0.0;
-    T0 = CoxWL * T1 / T2;
+    T0 = quot(CoxWL * T1, T2);
     c.cggb = T0 * dVgs_eff_dVg;
     c.cgdb = 0.0;
     c.cgsb = T0 * (dVbs0_dVb - dVgs_eff_dVg);
@@ -69,17 +70,17 @@ XD_HD void cv_simple(double Vbseff, double Vbs, double phi, double Phis, double 
     c.cbdb = 0.0;
     c.cbsb = -c.cgsb;
   } else {  // inversion
-    const double One_Third_CoxWL = CoxWL / 3.0;
+    const double One_Third_CoxWL = quot_by_constant(CoxWL, 3.0);
     const double Two_Third_CoxWL = 2.0 * One_Third_CoxWL;
     const double AbulkCV = Abulk0 * abulkCVfactor;
     const double dAbulkCV_dVb = abulkCVfactor * dAbulk0_dVb;
-    const double Vdsat0 = Vgst0 / AbulkCV;
-    const double dVdsat_dVg = dVgs_eff_dVg / AbulkCV;
-    const double dVdsat_dVb = -(Vdsat0 * dAbulkCV_dVb + dVth0_dVb) / AbulkCV;
+    const double Vdsat0 = quot(Vgst0, AbulkCV);
+    const double dVdsat_dVg = quot(dVgs_eff_dVg, AbulkCV);
+    const double dVdsat_dVb = quot(-(Vdsat0 * dAbulkCV_dVb + dVth0_dVb), AbulkCV);
     const double xpart = xpart_;
     const bool sat = (xpart > 0.5) ? (Vdsat0 <= Vds) : (Vds >= Vdsat0);
     if (sat) {
-      T1 = Vdsat0 / 3.0;
+      T1 = quot_by_constant(Vdsat0, 3.0);
       c.qgate = CoxWL * (Vgs_eff - Vfb0 - phi - T1);
       T2 = -Two_Third_CoxWL * Vgst0;
       c.qbulk = -(c.qgate + T2);
@@ -110,9 +111,9 @@ XD_HD void cv_simple(double Vbseff, double Vbs, double phi, double Phis, double 
       c.cbsb = -(c.cbgb + T3);
       c.cbdb = 0.0;
     } else {  // linear region
-      const double Alphaz = Vgst0 / Vdsat0;
+      const double Alphaz = quot(Vgst0, Vdsat0);
       T1 = 2.0 * Vdsat0 - Vds;
-      T2 = Vds / (3.0 * T1);
+      T2 = quot(Vds, 3.0 * T1);
       T3 = T2 * Vds;
       T9 = 0.25 * CoxWL;
       T4 = T9 * Alphaz;
@@ -126,7 +127,7 @@ XD_HD void cv_simple(double Vbseff, double Vbs, double phi, double Phis, double 
         c.qdrn = T4 * T7;
         c.qbulk = -(c.qgate + c.qdrn + T10);
       }
-      T5 = T3 / T1;
+      T5 = quot(T3, T1);
       c.cggb = CoxWL * (1.0 - T5 * dVdsat_dVg) * dVgs_eff_dVg;
       if (xpart > 0.5) {
         T11 = -CoxWL * T5 * dVdsat_dVb;
@@ -137,7 +138,7 @@ XD_HD void cv_simple(double Vbseff, double Vbs, double phi, double Phis, double 
         c.cgdb = CoxWL * (T2 - 0.5 + 0.5 * T5);
         c.cgsb = -(c.cggb + c.cgdb + tmp);
       }
-      T6 = 1.0 / Vdsat0;
+      T6 = quot(1.0, Vdsat0);
       const double dAlphaz_dVg = T6 * (1.0 - Alphaz * dVdsat_dVg);
       const double dAlphaz_dVb = -T6 * (dVth0_dVb + Alphaz * dVdsat_dVb);
       if (xpart > 0.5) {  // 0/100
@@ -158,15 +159,15 @@ XD_HD void cv_simple(double Vbseff, double Vbs, double phi, double Phis, double 
         c.cbsb = -(c.cgsb + c.cdsb + T0);
       } else if (xpart < 0.5) {  // 40/60
         T6 = 8.0 * Vdsat0 * Vdsat0 - 6.0 * Vdsat0 * Vds + 1.2 * Vds * Vds;
-        T8 = T2 / T1;
+        T8 = quot(T2, T1);
         T7 = Vds - T1 - T8 * T6;
         c.qdrn = T4 * T7;
         T7 *= T9;
-        tmp = T8 / T1;
+        tmp = quot(T8, T1);
         tmp1 = T4 * (2.0 - 4.0 * tmp * T6 + T8 * (16.0 * Vdsat0 - 6.0 * Vds));
         c.cdgb = (T7 * dAlphaz_dVg - tmp1 * dVdsat_dVg) * dVgs_eff_dVg;
         T10 = T7 * dAlphaz_dVb - tmp1 * dVdsat_dVb;
-        c.cddb = T4 * (2.0 - (1.0 / (3.0 * T1 * T1) + 2.0 * tmp) * T6 + T8 * (6.0 * Vdsat0 - 2.4 * Vds));
+        c.cddb = T4 * (2.0 - (quot(1.0, 3.0 * T1 * T1) + 2.0 * tmp) * T6 + T8 * (6.0 * Vdsat0 - 2.4 * Vds));
         c.cdsb = -(c.cdgb + T10 + c.cddb);
         T7 = 2.0 * (T1 + T3);
         c.qbulk = -(c.qgate - T4 * T7);
