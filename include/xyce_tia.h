@@ -141,7 +141,7 @@ int xd_tia_residual_norm(xd_tia *t, const double *d_rhs, const int *d_flag, doub
  * A + A^T (rows and columns alike), factors one matrix on the host in that order with row pivoting
  * that keeps the diagonal unless it is below 0.1 of its column's largest entry, and keeps the
  * orders and the fill pattern; xd_slu_solve eliminates each later matrix in those orders over the
- * pattern alone (no pivot search), on one warp. A pivot smaller than tol times an entry below it
+ * pattern alone (no pivot search), on one block, independent steps side by side. A pivot smaller than tol times an entry below it
  * (the threshold test of circuit solvers; 1e-3 as KLU's default) stops the solve with *d_info =
  * k + 1 for step k and leaves d_x unwritten; xd_tia_dense_solve_fallback queued after it then
  * solves that system with partial pivoting, so the pair is one stream-ordered, capturable solve.
@@ -154,6 +154,10 @@ int xd_slu_solve(xd_slu *s, const double *d_vals, const double *d_rhs, double *d
                  void *stream);
 int xd_slu_resolve(xd_slu *s, const double *d_lu, const double *d_rhs, double *d_x, void *stream);
 int xd_slu_destroy(xd_slu *s);
+/* Whether this handle solves by rounds of independent steps (the default wherever the lists of the
+ * rounds fit in shared memory) or step by step on one warp (on = 0); both give the same bits.
+ * Returns the previous setting, or a negative value on a null handle. */
+int xd_slu_rounds(xd_slu *s, int on);
 
 #ifdef __cplusplus
 }

@@ -137,6 +137,7 @@ SIGNATURES = {
                                      ctypes.POINTER(ctypes.c_void_p)]),
     "xd_slu_solve": (ctypes.c_int, [ctypes.c_void_p] * 7),
     "xd_slu_resolve": (ctypes.c_int, [ctypes.c_void_p] * 5),
+    "xd_slu_rounds": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     "xd_slu_destroy": (ctypes.c_int, [ctypes.c_void_p]),
     "xd_gemm_bf16": (ctypes.c_int, [ctypes.POINTER(XdGemmArgs), ctypes.c_int, ctypes.c_void_p]),
     "xd_mlp_input_layer": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_int,

@@ -44,6 +44,10 @@ struct xd_slu {
   int *d_buf = nullptr;  // all index arrays, one allocation
   int off[12] = {};      // offsets in d_buf: rowptr, colind, pos, lptr, lidx, uptr, uidx, cptr, cidx, cpos, cperm
   int nsched = 0;        // entries of lptr .. cidx
+  bool rounds = false;   // slu_rounds_kernel solves (the round lists fit in shared memory)
+  int entries = 0, factors = 0, n_scale = 0, n_task = 0, n_pair = 0, n_fwd = 0, n_back = 0;  // see SluRounds
+  unsigned char *d_rounds = nullptr;  // the round lists, then src and lupos
+  size_t rounds_bytes = 0;
 };
 
 namespace {
@@ -376,14 +380,16 @@ __global__ void __launch_bounds__(kNormThreads) residual_norm_kernel(int n, cons
 // Static-pivot refactorization of a small system (n <= XD_DENSE_MAX_N). The orders and the fill
 // pattern come from one host factorization (xd_slu_create): a minimum-degree order of A + A^T
 // applied to rows and columns (a supply node's dense row and column go last instead of filling the
-// whole matrix: the ring oscillator's LU has 704 entries instead of 103^2), then row pivoting that
+// whole matrix: the ring oscillator's LU keeps a few hundred of its 103^2 entries), then row pivoting that
 // keeps the diagonal unless it is below 0.1 of its column's largest entry; each
 // Newton matrix is then eliminated in that order over the pattern alone: step k scales the
 // multipliers of the rows that have an entry in column k and updates only the (row, column) pairs
 // of the pattern, the right-hand side carried along as column n. A pivot smaller than tol times an
 // entry below it (the threshold test of circuit solvers such as KLU) stops the solve with info =
-// k + 1, and the pivoting kernel redoes it (xd_tia_dense_solve_fallback). One warp, shared memory,
-// __syncwarp between steps: a few hundred cycles a step where the pivot search costs thousands.
+// k + 1, and the pivoting kernel redoes it (xd_tia_dense_solve_fallback).
+//
+// slu_kernel: one warp, the matrix dense in shared memory, __syncwarp between steps; about 1 us a
+// step. It serves the patterns whose round lists (slu_rounds_kernel) do not fit in shared memory.
 struct SluArgs {
   int n;
   double tol;
@@ -466,6 +472,195 @@ __global__ void __launch_bounds__(32) slu_kernel(SluArgs a, const double *__rest
     }
   }
   if (lane == 0) *info = 0;
+}
+
+// The same elimination by rounds, for a sparse pattern: SluRounds lists, for each round, the
+// entries whose pivot is final (scaled first) and then the updates whose operands are, so all the
+// independent steps of a round run side by side. Every entry still receives its updates one at a
+// time in step order from one thread, so the factors and the solution are bit for bit those of
+// slu_kernel. What bounds it is the length of a round (two barriers, a division, a dependent
+// index-operand-update chain: a few hundred cycles), not work. Entries are stored compactly
+// (pattern only), the lists are copied to shared memory by the whole block. The 103-unknown ring
+// of 51 inverters: 100.7 us by steps on one warp, 17.2 us by rounds (device time, cold caches).
+struct SluRounds {
+  int n, entries, factors;     // entries of the pattern + n of the right-hand side; the pattern's alone
+  int n_scale, n_task, n_pair, n_fwd, n_back, lists;  // list sizes; 16-byte units of all the lists
+  double tol;
+  const uint4 *blob;           // task[n_task], scale[n_scale], pair[n_pair], then the rounds' bounds
+  const int *src;              // [entries] where an entry starts: vals[s], 0 (-1) or rhs[-2 - s]
+  const int *lupos;            // [factors] the entry's place in the n x n output
+  const int *cperm;
+};
+constexpr int kSluThreads = 256;
+constexpr unsigned kSluLast = 0x8000u;  // a back-substitution task that finishes its unknown
+
+__device__ __forceinline__ double slu_updates(double v, const double *M, const unsigned *pair, int count) {
+#pragma unroll 4
+  for (int q = 0; q < count; ++q) {
+    const unsigned ab = pair[q];
+    v = v - M[ab & 0xffffu] * M[ab >> 16];
+  }
+  return v;
+}
+
+__global__ void __launch_bounds__(kSluThreads) slu_rounds_kernel(SluRounds a, const double *__restrict__ vals,
+                                                                 const double *__restrict__ rhs,
+                                                                 double *__restrict__ lu, double *__restrict__ x,
+                                                                 int *info) {
+  extern __shared__ uint4 lists[];
+  __shared__ int bad;
+  const unsigned long long *task = reinterpret_cast<const unsigned long long *>(lists);
+  const unsigned long long *scale = task + a.n_task;
+  const unsigned *pair = reinterpret_cast<const unsigned *>(scale + a.n_scale);
+  const int *scale_at = reinterpret_cast<const int *>(pair + a.n_pair);  // [n_fwd + 1]
+  const int *task_at = scale_at + a.n_fwd + 1;                           // [n_fwd + n_back + 1]
+  double *M = reinterpret_cast<double *>(lists + a.lists), *sinv = M + a.entries;
+  const int tid = threadIdx.x, n = a.n;
+  if (tid == 0) bad = n;
+  for (int e = tid; e < a.entries; e += kSluThreads) {
+    const int s = a.src[e];
+    M[e] = s >= 0 ? vals[s] : s == -1 ? 0.0 : rhs[-2 - s];
+  }
+#pragma unroll 4
+  for (int q = tid; q < a.lists; q += kSluThreads) lists[q] = a.blob[q];
+  __syncthreads();
+  for (int r = 0; r < a.n_fwd; ++r) {
+    for (int t = scale_at[r] + tid; t < scale_at[r + 1]; t += kSluThreads) {
+      const unsigned long long d = scale[t];
+      const int e = (int)(d & 0xffffu), p = (int)(d >> 16 & 0xffffu), k = (int)(d >> 32);
+      const double pv = M[p], v = M[e], inv = 1.0 / pv;
+      if (e == p) {
+        sinv[k] = inv;
+        if (!(fabs(pv) > 0.0)) atomicMin(&bad, k);
+      } else {
+        M[e] = v * inv;
+        if (!(fabs(v) * a.tol <= fabs(pv))) atomicMin(&bad, k);
+      }
+    }
+    __syncthreads();
+    for (int t = task_at[r] + tid; t < task_at[r + 1]; t += kSluThreads) {
+      const unsigned long long d = task[t];
+      const int e = (int)(d & 0xffffu);
+      M[e] = slu_updates(M[e], M, pair + (int)(d >> 32), (int)(d >> 16 & 0xffffu));
+    }
+    __syncthreads();
+  }
+  // A failed step spoils only steps that come after it in the elimination order, so the smallest
+  // failed step is the one that the step order stops at.
+  if (bad < n) {
+    if (tid == 0) *info = bad + 1;
+    return;
+  }
+  if (lu)
+    for (int q = tid; q < n * n; q += kSluThreads) lu[q] = 0.0;
+  for (int r = a.n_fwd; r < a.n_fwd + a.n_back; ++r) {
+    for (int t = task_at[r] + tid; t < task_at[r + 1]; t += kSluThreads) {
+      const unsigned long long d = task[t];
+      const int e = (int)(d & 0xffffu);
+      const unsigned c = (unsigned)(d >> 16) & 0xffffu;
+      const double v = slu_updates(M[e], M, pair + (int)(d >> 32), (int)(c & ~kSluLast));
+      M[e] = (c & kSluLast) ? v * sinv[e - a.factors] : v;
+    }
+    __syncthreads();
+  }
+  for (int j = tid; j < n; j += kSluThreads) x[a.cperm[j]] = M[a.factors + j];
+  if (lu)
+    for (int e = tid; e < a.factors; e += kSluThreads) lu[a.lupos[e]] = M[e];
+  if (tid == 0) *info = 0;
+}
+
+// The rounds of slu_rounds_kernel from the factor pattern S (n x n, in the elimination orders).
+// An entry's updates are taken in step order; each is placed in the first round in which both of
+// its operands are final and the updates before it are done.
+struct SluLists {
+  std::vector<unsigned long long> task, scale;
+  std::vector<unsigned> pair;
+  std::vector<int> scale_at, task_at;
+  int entries = 0, factors = 0, n_fwd = 0, n_back = 0;
+  std::vector<int> id;  // [n * n] the pattern's entries, -1 outside it
+  size_t bytes() const {
+    const size_t b = 8 * (task.size() + scale.size()) + 4 * (pair.size() + scale_at.size() + task_at.size());
+    return (b + 15) / 16 * 16;
+  }
+};
+
+SluLists slu_lists(int n, const std::vector<char> &S) {
+  SluLists L;
+  L.id.assign((size_t)n * n, -1);
+  for (size_t q = 0; q < L.id.size(); ++q)
+    if (S[q]) L.id[q] = L.factors++;
+  L.entries = L.factors + n;
+  auto at = [&](int i, int j) { return j == n ? L.factors + i : L.id[(size_t)i * n + j]; };
+  struct Task {
+    int target;
+    bool last;
+    std::vector<unsigned> pairs;
+  };
+  std::vector<std::vector<Task>> fwd, back;
+  std::vector<std::vector<unsigned long long>> scale;
+  std::vector<int> ready(L.entries, 0), open(L.entries, -1);  // first round that may read; the task being filled
+  auto add = [&](std::vector<std::vector<Task>> &rounds, int t, int e) -> Task & {
+    if ((int)rounds.size() <= t) rounds.resize(t + 1);
+    if (open[e] < 0 || ready[e] != t + 1) {
+      open[e] = (int)rounds[t].size();
+      rounds[t].push_back(Task{e, false, {}});
+      ready[e] = t + 1;
+    }
+    return rounds[t][open[e]];
+  };
+  for (int k = 0; k < n; ++k) {
+    const int p = at(k, k);
+    auto place = [&](int t, int e) {
+      if ((int)scale.size() <= t) scale.resize(t + 1);
+      scale[t].push_back((unsigned)e | (unsigned long long)p << 16 | (unsigned long long)k << 32);
+    };
+    place(ready[p], p);
+    for (int i = k + 1; i < n; ++i) {
+      const int l = at(i, k);
+      if (l < 0) continue;
+      ready[l] = std::max(ready[l], ready[p]);
+      place(ready[l], l);
+      for (int j = k + 1; j <= n; ++j) {
+        const int u = at(k, j);
+        if (u < 0) continue;
+        const int e = at(i, j);
+        const int t = std::max(std::max(ready[l], ready[u]), ready[e] - 1);
+        add(fwd, t, e).pairs.push_back((unsigned)l | (unsigned)u << 16);
+      }
+    }
+  }
+  // Back substitution: unknown k's value reaches row i in the order of falling k.
+  for (int i = 0; i < n; ++i) ready[at(i, n)] = 0, open[at(i, n)] = -1;
+  for (int k = n - 1; k >= 0; --k) {
+    const int e = at(k, n);
+    add(back, std::max(0, ready[e] - 1), e).last = true;
+    for (int i = 0; i < k; ++i) {
+      const int u = at(i, k), y = at(i, n);
+      if (u < 0) continue;
+      add(back, std::max(ready[e], ready[y] - 1), y).pairs.push_back((unsigned)u | (unsigned)e << 16);
+    }
+  }
+  L.n_fwd = (int)std::max(fwd.size(), scale.size());
+  L.n_back = (int)back.size();
+  fwd.resize(L.n_fwd);
+  scale.resize(L.n_fwd);
+  fwd.insert(fwd.end(), back.begin(), back.end());
+  L.scale_at.push_back(0);
+  for (const auto &r : scale) {
+    L.scale.insert(L.scale.end(), r.begin(), r.end());
+    L.scale_at.push_back((int)L.scale.size());
+  }
+  L.task_at.push_back(0);
+  for (auto &r : fwd) {  // the longest tasks of a round first: lanes of a warp run about equally long
+    std::stable_sort(r.begin(), r.end(), [](const Task &x, const Task &y) { return x.pairs.size() > y.pairs.size(); });
+    for (const Task &t : r) {
+      const unsigned c = (unsigned)t.pairs.size() | (t.last ? kSluLast : 0u);
+      L.task.push_back((unsigned)t.target | (unsigned long long)c << 16 | (unsigned long long)L.pair.size() << 32);
+      L.pair.insert(L.pair.end(), t.pairs.begin(), t.pairs.end());
+    }
+    L.task_at.push_back((int)L.task.size());
+  }
+  return L;
 }
 
 // Solve with factors kept from slu_kernel (in its row and column orders): forward substitution
@@ -986,32 +1181,40 @@ int xd_slu_create(int n, const int *rowptr, const int *colind, const double *val
     if (rowptr[r + 1] < rowptr[r]) return xd_internal_fail(-1, "bad CSR pattern");
   for (int k = 0; k < nnz; ++k)
     if (colind[k] < 0 || colind[k] >= n) return xd_internal_fail(-1, "bad CSR pattern");
-  // Minimum-degree order of A + A^T (greedy; ties to the lowest index), applied to rows and
-  // columns: cperm[j] = the unknown eliminated j-th.
+  // Minimum-degree order of A + A^T, applied to rows and columns (cperm[j] = the unknown eliminated
+  // j-th), a pass at a time: a pass takes the unknowns of least degree, lowest index first, and
+  // skips the neighbours of those it has taken (the multiple elimination of Liu, 1985). The steps
+  // of a pass do not depend on one another; one unknown after the other around a ring of inverters
+  // would be a chain as long as the ring.
   std::vector<char> G((size_t)n * n, 0), alive(n, 1);
   for (int r = 0; r < n; ++r)
     for (int k = rowptr[r]; k < rowptr[r + 1]; ++k)
       if (colind[k] != r) G[(size_t)r * n + colind[k]] = G[(size_t)colind[k] * n + r] = 1;
   std::vector<int> cperm(n), cpos(n);
-  for (int step = 0; step < n; ++step) {
-    int v = -1, best = n + 1;
+  for (int step = 0; step < n;) {
+    std::vector<int> degree(n, n + 1);
+    int best = n + 1;
     for (int i = 0; i < n; ++i) {
       if (!alive[i]) continue;
-      int d = 0;
-      for (int j = 0; j < n; ++j) d += (alive[j] && G[(size_t)i * n + j]) ? 1 : 0;
-      if (d < best) {
-        best = d;
-        v = i;
-      }
+      degree[i] = 0;
+      for (int j = 0; j < n; ++j) degree[i] += (alive[j] && G[(size_t)i * n + j]) ? 1 : 0;
+      best = std::min(best, degree[i]);
     }
-    cperm[step] = v;
-    alive[v] = 0;
-    std::vector<int> nb;
-    for (int j = 0; j < n; ++j)
-      if (alive[j] && G[(size_t)v * n + j]) nb.push_back(j);
-    for (int p : nb)
-      for (int q : nb)
-        if (p != q) G[(size_t)p * n + q] = 1;
+    std::vector<char> skip(n, 0);
+    for (int v = 0; v < n; ++v) {
+      if (!alive[v] || skip[v] || degree[v] != best) continue;
+      cperm[step++] = v;
+      alive[v] = 0;
+      std::vector<int> nb;
+      for (int j = 0; j < n; ++j)
+        if (alive[j] && G[(size_t)v * n + j]) {
+          nb.push_back(j);
+          skip[j] = 1;
+        }
+      for (int p : nb)
+        for (int q : nb)
+          if (p != q) G[(size_t)p * n + q] = 1;
+    }
   }
   for (int j = 0; j < n; ++j) cpos[cperm[j]] = j;
   // Host factorization in that order, tracking the pattern: row pivoting that keeps the diagonal
@@ -1086,14 +1289,54 @@ int xd_slu_create(int n, const int *rowptr, const int *colind, const double *val
     h->off[q] = (int)all.size();
     all.insert(all.end(), parts[q]->begin(), parts[q]->end());
   }
+  // The round lists, when they and the entries fit beside each other in shared memory (16-bit entry
+  // numbers: n * (n + 1) is below 65536).
+  const SluLists L = slu_lists(n, S);
+  const size_t lists = L.bytes();
+  h->rounds_bytes = lists + sizeof(double) * (size_t)(L.entries + n);
+  h->rounds = h->rounds_bytes <= 224 * 1024;
+  std::vector<unsigned char> blob;
+  if (h->rounds) {
+    h->entries = L.entries;
+    h->factors = L.factors;
+    h->n_scale = (int)L.scale.size();
+    h->n_task = (int)L.task.size();
+    h->n_pair = (int)L.pair.size();
+    h->n_fwd = L.n_fwd;
+    h->n_back = L.n_back;
+    std::vector<int> src(L.entries, -1), lupos(L.factors);
+    for (int r = 0; r < n; ++r) {
+      for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) src[L.id[(size_t)pos[r] * n + cpos[colind[k]]]] = k;
+      src[L.factors + pos[r]] = -2 - r;
+    }
+    for (int q = 0; q < n * n; ++q)
+      if (L.id[q] >= 0) lupos[L.id[q]] = q;
+    auto put = [&](const void *p, size_t bytes) {
+      blob.insert(blob.end(), (const unsigned char *)p, (const unsigned char *)p + bytes);
+    };
+    put(L.task.data(), 8 * L.task.size());
+    put(L.scale.data(), 8 * L.scale.size());
+    put(L.pair.data(), 4 * L.pair.size());
+    put(L.scale_at.data(), 4 * L.scale_at.size());
+    put(L.task_at.data(), 4 * L.task_at.size());
+    blob.resize(lists, 0);
+    put(src.data(), 4 * src.size());
+    put(lupos.data(), 4 * lupos.size());
+  }
   Guard g(cuda_device);
   cudaError_t e;
-  if ((e = cudaMalloc(&h->d_buf, sizeof(int) * std::max<size_t>(1, all.size()))) != cudaSuccess ||
+  if ((h->rounds && ((e = cudaMalloc(&h->d_rounds, blob.size())) != cudaSuccess ||
+                     (e = cudaMemcpy(h->d_rounds, blob.data(), blob.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
+                     (h->rounds_bytes > 40 * 1024 &&
+                      (e = cudaFuncSetAttribute(slu_rounds_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                224 * 1024)) != cudaSuccess))) ||
+      (e = cudaMalloc(&h->d_buf, sizeof(int) * std::max<size_t>(1, all.size()))) != cudaSuccess ||
       (e = cudaMemcpy(h->d_buf, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (dense_smem_bytes(n) + sizeof(int) * nsched > 48 * 1024 &&
        (e = cudaFuncSetAttribute(slu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(dense_smem_bytes(n) + sizeof(int) * nsched))) != cudaSuccess)) {
     cudaFree(h->d_buf);
+    cudaFree(h->d_rounds);
     delete h;
     return cuda_err(e, "xd_slu_create");
   }
@@ -1112,11 +1355,30 @@ int xd_slu_solve(xd_slu *s, const double *d_vals, const double *d_rhs, double *d
                  void *stream) {
   if (!s || !d_vals || !d_rhs || !d_x || !d_info) return xd_internal_fail(-1, "null argument");
   Guard g(s->device);
+  if (s->rounds) {
+    const size_t lists = s->rounds_bytes - sizeof(double) * (size_t)(s->entries + s->n);
+    const int *src = reinterpret_cast<const int *>(s->d_rounds + lists);
+    slu_rounds_kernel<<<1, kSluThreads, s->rounds_bytes, (cudaStream_t)stream>>>(
+        SluRounds{s->n, s->entries, s->factors, s->n_scale, s->n_task, s->n_pair, s->n_fwd, s->n_back,
+                  (int)(lists / 16), s->tol, reinterpret_cast<const uint4 *>(s->d_rounds), src, src + s->entries,
+                  s->d_buf + s->off[10]},
+        d_vals, d_rhs, d_lu, d_x, d_info);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_err(e, "slu_rounds_kernel launch");
+    return 0;
+  }
   slu_kernel<<<1, 32, dense_smem_bytes(s->n) + sizeof(int) * s->nsched, (cudaStream_t)stream>>>(
       slu_args(s), d_vals, d_rhs, d_lu, d_x, d_info);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(e, "slu_kernel launch");
   return 0;
+}
+
+int xd_slu_rounds(xd_slu *s, int on) {
+  if (!s) return xd_internal_fail(-1, "null argument");
+  const int was = s->rounds;
+  s->rounds = on && s->d_rounds;
+  return was;
 }
 
 int xd_slu_resolve(xd_slu *s, const double *d_lu, const double *d_rhs, double *d_x, void *stream) {
@@ -1132,6 +1394,7 @@ int xd_slu_destroy(xd_slu *s) {
   if (!s) return 0;
   Guard g(s->device);
   cudaFree(s->d_buf);
+  cudaFree(s->d_rounds);
   delete s;
   return 0;
 }
