@@ -29,8 +29,9 @@ int xd_rf_create(int n, int nnz_a, const int *rowptr_a, const int *colind_a, con
                  xd_rf **out);
 
 /* Refactors with new values of A (device, in A's pattern), keeping the pivot order: the library's
- * own elimination (one thread block over the factors' dependency levels, a warp per row, each
- * entry updated in a fixed order, so the factors do not depend on timing). A zero pivot in that
+ * own elimination (the elimination tree's subtrees on independent blocks, the chains above them
+ * eight pivots at a time; small or dense systems level by level on one block; each entry updated in
+ * a fixed order, so the factors do not depend on timing). A zero pivot in that
  * order is an error (< 0, which synchronises the legacy default stream to read); a small one is
  * not detected here, so a caller that cannot bound the growth checks the solution's residual
  * (the transient driver refines and, failing that, makes a new host factorization). */
@@ -50,9 +51,26 @@ int xd_rf_stats(const xd_rf *rf, int *nnz_factors, int *elimination_levels, long
 int xd_rf_copy_factors(const xd_rf *rf, double *h_vals);
 
 /* Solves A x = b in place: d_x holds b on entry and x on return (device, length n). The forward
- * and back substitutions are the library's own kernels (one thread block walking the factors'
- * dependency levels, deterministic sums), ordered on the legacy default stream. */
+ * and back substitutions are the library's own kernels (over the same subtrees and chains; without them
+ * one thread block walking the factors' dependency levels; deterministic sums), ordered on the
+ * legacy default stream. */
 int xd_rf_solve(xd_rf *rf, double *d_x);
+
+/* A solve with its check, the values coming and going on the legacy default stream: refactors first
+ * when refactor is set (a zero pivot is an error, as in xd_rf_refactor), solves into d_x (not d_b),
+ * then refines (r = b - A x, x += A^-1 r) until the componentwise backward error
+ * max_i |r_i| / (|A| |x| + |b|)_i is at most tol, at most max_refine times. d_vals_a: A's values in
+ * A's pattern. The call returns when the outcome is known; every check is one launch and one
+ * synchronisation. */
+enum { XD_RF_WITHIN_TOL = 0, XD_RF_ABOVE_TOL = 1, XD_RF_NOT_FINITE = 2 };
+typedef struct {
+  double first_berr, berr; /* backward error of the first solution, and of d_x */
+  int outcome;             /* XD_RF_... */
+  int solves;              /* triangular solves made, refinement steps included */
+  int checks;              /* solutions that were finite (first_berr holds when at least one was) */
+} xd_rf_check;
+int xd_rf_solve_refined(xd_rf *rf, const double *d_vals_a, const double *d_b, double *d_x, int refactor, double tol,
+                        int max_refine, xd_rf_check *out);
 
 /* The solve through the refactorization library's own triangular solve, with its factors from
  * xd_rf_refactor_library (for comparison). */

@@ -126,7 +126,7 @@ int xd_tia_dense_resolve(xd_tia *t, const double *d_lu, const int *d_piv, const 
 int xd_tia_dense_solve_fallback(xd_tia *t, const double *d_jac, const double *d_rhs, double *d_lu, int *d_piv,
                                 double *d_x, int *d_info, void *stream);
 
-/* Newton's bookkeeping on the device (N_NLS_DampedNewton.C:325-350, 1792-1830), one block each:
+/* Newton's bookkeeping on the device (N_NLS_DampedNewton.C:325-350, 1792-1830), one launch each:
  * xd_tia_newton_update adds the update d_dx to d_x, refreshes the weights d_w = rel_tol *
  * max(|d_xref|, |d_x|) + abs_tol when update_weights is set, and writes the update's weighted RMS
  * norm sqrt(mean((dx / w)^2)) to d_norms[0]; xd_tia_residual_norm writes max |d_rhs| to d_norms[1]

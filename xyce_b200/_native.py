@@ -49,6 +49,16 @@ class XdTiaCoef(ctypes.Structure):
                 ("inv_h", ctypes.c_double), ("hist_scale", ctypes.c_double), ("gshunt", ctypes.c_double)]
 
 
+class XdRfCheck(ctypes.Structure):
+    """Mirror of ``xd_rf_check`` (include/xyce_rf.h)."""
+
+    _fields_ = [("first_berr", ctypes.c_double), ("berr", ctypes.c_double), ("outcome", ctypes.c_int),
+                ("solves", ctypes.c_int), ("checks", ctypes.c_int)]
+
+
+XD_RF_WITHIN_TOL, XD_RF_ABOVE_TOL, XD_RF_NOT_FINITE = 0, 1, 2
+
+
 class XdGemmArgs(ctypes.Structure):
     """Mirror of ``xd_gemm_args`` (include/xyce_surrogate.h)."""
 
@@ -160,6 +170,8 @@ SIGNATURES = {
                                     ctypes.POINTER(ctypes.c_void_p)]),
     "xd_rf_refactor": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
     "xd_rf_solve": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
+    "xd_rf_solve_refined": (ctypes.c_int, [ctypes.c_void_p] * 4 + [ctypes.c_int, ctypes.c_double, ctypes.c_int,
+                                                                   ctypes.POINTER(XdRfCheck)]),
     "xd_rf_solve_library": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
     "xd_rf_refactor_library": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
     "xd_rf_stats": (ctypes.c_int, [ctypes.c_void_p, _ip, _ip, ctypes.POINTER(ctypes.c_longlong)]),

@@ -398,20 +398,27 @@ int xd_lu_copy(XdLu *lu, double *h_vals) {
   return e == cudaSuccess ? 0 : xd_internal_fail(-3, std::string("LU factors: ") + cudaGetErrorString(e));
 }
 
-int xd_lu_info(XdLu *lu, cudaStream_t st, int *info) {
-  if (lu->tree.on) {
-    int c[2] = {0, 0};
-    cudaError_t e = cudaMemcpyAsync(c, lu->tree.d_ctl + kTreeInfo, sizeof(c), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return xd_internal_fail(-3, std::string("LU pivot report: ") + cudaGetErrorString(e));
-    if (c[kTreeExpired - kTreeInfo] != 0) return xd_internal_fail(-3, "LU refactorization: a wait between chains expired");
-    *info = c[0] == 0 ? 0 : lu->n - c[0] + 1;
+const int *xd_lu_status(const XdLu *lu, int *count) {
+  *count = lu->tree.on ? 2 : 1;
+  return lu->tree.on ? lu->tree.d_ctl + kTreeInfo : lu->d_info;
+}
+
+int xd_lu_report(const XdLu *lu, const int *status, int *info) {
+  if (!lu->tree.on) {
+    *info = status[0] == kLuNoZeroPivot ? 0 : status[0];
     return 0;
   }
-  int v = 0;
-  cudaError_t e = cudaMemcpyAsync(&v, lu->d_info, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (status[kTreeExpired - kTreeInfo] != 0)
+    return xd_internal_fail(-3, "LU refactorization: a wait between chains expired");
+  *info = status[0] == 0 ? 0 : lu->n - status[0] + 1;
+  return 0;
+}
+
+int xd_lu_info(XdLu *lu, cudaStream_t st, int *info) {
+  int status[2] = {0, 0}, count = 0;
+  const int *d = xd_lu_status(lu, &count);
+  cudaError_t e = cudaMemcpyAsync(status, d, sizeof(int) * count, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return xd_internal_fail(-3, std::string("LU pivot report: ") + cudaGetErrorString(e));
-  *info = v == kLuNoZeroPivot ? 0 : v;
-  return 0;
+  return xd_lu_report(lu, status, info);
 }

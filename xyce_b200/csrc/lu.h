@@ -56,3 +56,7 @@ int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st);
 int xd_lu_copy(XdLu *lu, double *h_vals);
 // Reads the zero-pivot report (synchronises the stream): 0, or 1 + the first row found.
 int xd_lu_info(XdLu *lu, cudaStream_t st, int *info);
+// The same without a synchronisation of its own: the device words of the report and their number (at
+// most two), and the reading of them once they are on the host.
+const int *xd_lu_status(const XdLu *lu, int *count);
+int xd_lu_report(const XdLu *lu, const int *status, int *info);

@@ -14,6 +14,7 @@
 
 #include "../../include/xyce_rf.h"
 #include "lu.h"
+#include "residual.h"
 #include "sptrsv.h"
 
 int xd_internal_fail(int code, const std::string &msg);
@@ -24,6 +25,7 @@ struct xd_rf {
   int *d_rowptr = nullptr, *d_colind = nullptr, *d_p = nullptr, *d_q = nullptr;
   double *d_temp = nullptr;
   XdLu lu;        // the refactorization
+  XdResidual res; // the check after a solve
   XdSptrsv tri;   // the triangular solves over lu's bundled factors, where lu has no tree plan
   // The comparison library, created on first use from host copies of the set-up inputs.
   cusolverRfHandle_t h = nullptr;
@@ -45,6 +47,7 @@ int cu_fail(cudaError_t e, const char *where) {
 void release(xd_rf *r) {
   if (!r) return;
   if (r->h) cusolverRfDestroy(r->h);
+  xd_residual_free(&r->res);
   xd_sptrsv_free(&r->tri);
   xd_lu_free(&r->lu);
   cudaFree(r->d_rowptr);
@@ -128,6 +131,11 @@ int xd_rf_create(int n, int nnz_a, const int *rowptr_a, const int *colind_a, con
     release(r);
     return rc;
   }
+  rc = xd_residual_init(&r->res, n, rowptr_a, r->d_rowptr, r->d_colind);
+  if (rc != 0) {
+    release(r);
+    return rc;
+  }
   // The set-up factors A's own values.
   double *d_a = nullptr;
   if ((e = cudaMalloc(&d_a, sizeof(double) * (nnz_a > 0 ? nnz_a : 1))) != cudaSuccess ||
@@ -165,6 +173,49 @@ int xd_rf_solve(xd_rf *r, double *d_x) {
   if (!r || !d_x) return xd_internal_fail(-1, "null refactorization argument");
   cudaSetDevice(r->device);
   return r->lu.tree.on ? xd_tree_solve(&r->lu.tree, d_x, 0) : xd_sptrsv_solve(&r->tri, r->lu.d_mx, d_x, 0);
+}
+
+int xd_rf_solve_refined(xd_rf *r, const double *d_vals_a, const double *d_b, double *d_x, int refactor, double tol,
+                        int max_refine, xd_rf_check *out) {
+  if (!r || !d_vals_a || !d_b || !d_x || !out || d_b == d_x || max_refine < 0)
+    return xd_internal_fail(-1, "bad arguments to the refined solve");
+  cudaSetDevice(r->device);
+  *out = xd_rf_check{};
+  out->outcome = XD_RF_ABOVE_TOL;
+  int rc = refactor ? xd_lu_refactor(&r->lu, d_vals_a, 0) : 0;
+  if (rc != 0) return rc;
+  cudaError_t e = cudaMemcpyAsync(d_x, d_b, sizeof(double) * r->n, cudaMemcpyDeviceToDevice, 0);
+  if (e != cudaSuccess) return cu_fail(e, "xd_rf_solve_refined");
+  int nstatus = 0;
+  const int *d_status = xd_lu_status(&r->lu, &nstatus);
+  for (int k = 0;; ++k) {
+    // The solution, then (k > 0) the corrections in d_temp; the refactorization's own report comes
+    // back with the first check, so a zero pivot is found after a solve whose result is dropped.
+    if ((rc = xd_rf_solve(r, k == 0 ? d_x : r->d_temp)) != 0) return rc;
+    if (k > 0 && (rc = xd_residual_add(&r->res, d_x, r->d_temp, 0)) != 0) return rc;
+    if ((rc = xd_residual_check(&r->res, d_vals_a, d_b, d_x, r->d_temp, d_status, nstatus, 0)) != 0) return rc;
+    if ((e = cudaStreamSynchronize(0)) != cudaSuccess) return cu_fail(e, "xd_rf_solve_refined");
+    if (refactor && k == 0) {
+      const int status[2] = {(int)r->res.h_out[2], (int)r->res.h_out[3]};
+      int info = 0;
+      if ((rc = xd_lu_report(&r->lu, status, &info)) != 0) return rc;
+      if (info != 0)
+        return xd_internal_fail(-5, "zero pivot in row " + std::to_string(info - 1) + " of the refactorization");
+    }
+    ++out->solves;
+    if (r->res.h_out[1] != 0.0) {
+      out->outcome = XD_RF_NOT_FINITE;
+      return 0;
+    }
+    out->berr = r->res.h_out[0];
+    if (k == 0) out->first_berr = out->berr;
+    ++out->checks;
+    if (out->berr <= tol) {
+      out->outcome = XD_RF_WITHIN_TOL;
+      return 0;
+    }
+    if (k == max_refine) return 0;
+  }
 }
 
 int xd_rf_levels(const xd_rf *r, int *levels_l, int *levels_u) {

@@ -10,6 +10,7 @@
 // linear devices' F and Q use a fixed shuffle tree, so the results do not vary between runs. Rows
 // of more than kLongRowEntries entries (the supply rail's) are cut into chunks first, a block per
 // chunk, and their warp adds the chunk sums (tia_long.h).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -303,12 +304,24 @@ __global__ void __launch_bounds__(32) dense_resolve_kernel(int n, const double *
 
 size_t dense_smem_bytes(int n) { return sizeof(double) * (size_t)n * (size_t)(n + 1); }
 
-// Newton's bookkeeping between a solve and the next load, one block: x += dx; the update weights
+// Newton's bookkeeping between a solve and the next load: x += dx; the update weights
 // (when refreshed) rel * max(|x_ref|, |x|) + abs; norms[0] = sqrt(mean((dx / w)^2)), the weighted
 // RMS norm of the update (N_NLS_DampedNewton.C's convergence test, :325-350, 1792-1830). Then,
 // after the load, norms[1] = max |rhs| (not finite if any entry is not) and norms[2] = *flag.
-// Sums and maxima use a fixed reduction tree: the same inputs give the same norms.
-constexpr int kNormThreads = 1024;
+// Sums and maxima use a fixed reduction tree: the same inputs give the same norms. One block up to
+// kNormBlock unknowns (a small circuit's launch is all latency); above, one cluster of kNormCluster
+// blocks whose partial results meet in the first one's shared memory, so that the norms need no
+// scratch memory that calls on two streams would share.
+constexpr int kNormThreads = 1024, kNormCluster = 8, kNormBlock = 8 * kNormThreads;
+
+// This block's value (thread 0's) to slot `rank` of the first block's array; complete after the sync.
+template <typename T>
+__device__ __forceinline__ void to_first_block(T v, T *slots) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  if (threadIdx.x == 0) *cl.map_shared_rank(slots + cl.block_rank(), 0) = v;
+  cl.sync();
+}
 
 __device__ __forceinline__ double block_sum(double v, double *red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -329,10 +342,10 @@ __global__ void __launch_bounds__(kNormThreads) newton_update_kernel(int n, doub
                                                                      const double *__restrict__ xref,
                                                                      double *__restrict__ w, double rel, double abs_,
                                                                      int update_w, double *__restrict__ norms) {
-  __shared__ double red[32];
+  __shared__ double red[32], part[kNormCluster];
   double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += kNormThreads) {
-    const double xi = x[i] + dx[i];
+  for (int i = blockIdx.x * kNormThreads + threadIdx.x; i < n; i += gridDim.x * kNormThreads) {
+    const double d = dx[i], xi = x[i] + d;
     x[i] = xi;
     double wi;
     if (update_w) {
@@ -341,40 +354,64 @@ __global__ void __launch_bounds__(kNormThreads) newton_update_kernel(int n, doub
     } else {
       wi = w[i];
     }
-    const double q = dx[i] / wi;
+    const double q = d / wi;
     s += q * q;
   }
   s = block_sum(s, red);
-  if (threadIdx.x == 0) norms[0] = sqrt(s / (double)n);
+  if (gridDim.x > 1) {
+    to_first_block(s, part);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      s = part[0];
+      for (int q = 1; q < kNormCluster; ++q) s += part[q];
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) norms[0] = sqrt(s / (double)n);
 }
 
+// The largest |rhs| by the bits of non-negative doubles: infinity and NaN lie above the finite ones.
 __global__ void __launch_bounds__(kNormThreads) residual_norm_kernel(int n, const double *__restrict__ rhs,
                                                                      const int *__restrict__ flag,
                                                                      double *__restrict__ norms) {
-  __shared__ double red[32];
-  __shared__ int bad;
-  if (threadIdx.x == 0) bad = 0;
-  __syncthreads();
-  double m = 0.0;
-  for (int i = threadIdx.x; i < n; i += kNormThreads) {
-    const double a = fabs(rhs[i]);
-    if (!isfinite(a)) bad = 1;
-    m = fmax(m, a);
-  }
+  __shared__ unsigned long long red[32], part[kNormCluster];
+  unsigned long long m = 0;
+  for (int i = blockIdx.x * kNormThreads + threadIdx.x; i < n; i += gridDim.x * kNormThreads)
+    m = max(m, (unsigned long long)__double_as_longlong(rhs[i]) & 0x7fffffffffffffffull);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
+  for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
   if (lane == 0) red[warp] = m;
   __syncthreads();
   if (warp == 0) {
-    m = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
+    m = red[lane];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
-    if (lane == 0) {
-      norms[1] = bad ? __longlong_as_double(0x7ff8000000000000LL) : m;
-      norms[2] = flag ? (double)*flag : 0.0;
-    }
+    for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
   }
+  if (gridDim.x > 1) {
+    to_first_block(m, part);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      for (int q = 0; q < kNormCluster; ++q) m = max(m, part[q]);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const bool finite = m < 0x7ff0000000000000ull;
+    norms[1] = __longlong_as_double(finite ? (long long)m : 0x7ff8000000000000LL);
+    norms[2] = flag ? (double)*flag : 0.0;
+  }
+}
+
+// One block or one cluster, by the number of unknowns.
+template <typename... P, typename... A>
+cudaError_t launch_norms(void (*kernel)(P...), int n, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n > kNormBlock ? kNormCluster : 1);
+  cfg.blockDim = dim3(kNormThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cfg.gridDim.x;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = cfg.gridDim.x > 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // Static-pivot refactorization of a small system (n <= XD_DENSE_MAX_N). The orders and the fill
@@ -1152,9 +1189,8 @@ int xd_tia_newton_update(xd_tia *t, double *d_x, const double *d_dx, const doubl
   if (!t || !d_x || !d_dx || !d_w || !d_norms || (update_weights && !d_xref)) return xd_internal_fail(-1, "null argument");
   if (t->n_rows == 0) return 0;
   Guard g(t->device);
-  newton_update_kernel<<<1, kNormThreads, 0, (cudaStream_t)stream>>>(t->n_rows, d_x, d_dx, d_xref, d_w, rel_tol, abs_tol,
-                                                                     update_weights, d_norms);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_norms(newton_update_kernel, t->n_rows, (cudaStream_t)stream, t->n_rows, d_x, d_dx, d_xref, d_w,
+                               rel_tol, abs_tol, update_weights, d_norms);
   if (e != cudaSuccess) return cuda_err(e, "newton_update_kernel launch");
   return 0;
 }
@@ -1163,8 +1199,7 @@ int xd_tia_residual_norm(xd_tia *t, const double *d_rhs, const int *d_flag, doub
   if (!t || !d_rhs || !d_norms) return xd_internal_fail(-1, "null argument");
   if (t->n_rows == 0) return 0;
   Guard g(t->device);
-  residual_norm_kernel<<<1, kNormThreads, 0, (cudaStream_t)stream>>>(t->n_rows, d_rhs, d_flag, d_norms);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_norms(residual_norm_kernel, t->n_rows, (cudaStream_t)stream, t->n_rows, d_rhs, d_flag, d_norms);
   if (e != cudaSuccess) return cuda_err(e, "residual_norm_kernel launch");
   return 0;
 }

@@ -29,7 +29,6 @@ from __future__ import annotations
 
 import ctypes
 import math
-import warnings
 import time as _time
 from dataclasses import dataclass, field
 
@@ -665,73 +664,43 @@ class GpuTransient(TransientBase):
         self.stats.factorizations += 1
         self._lu = True
         nan = lambda: torch.full_like(self.rhs, float("nan"))
-        fresh = False
-        if getattr(self, "_rf", None) is None or not self._rf.value:
-            if not self._rf_try_setup():
-                return nan()
-            fresh = True
-        else:
-            torch.cuda.current_stream(self.dev).synchronize()  # values complete before the library reads them
-            rc = self._lib.xd_rf_refactor(self._rf, ctypes.c_void_p(self.jac.data_ptr()))
-            if rc != 0:
-                # A zero pivot in the kept pivot order (the matrices of a DC solve and of a time step
-                # differ in which entries dominate): factor this matrix afresh on the host.
-                if not self._rf_try_setup():
-                    return nan()
-                fresh = True
-        x = self._rf_solve_refined(self.rhs, accept=fresh)
-        if x is None and not fresh:
-            # The kept pivot order does not suit this matrix: factor it afresh on the host.
+        x = None
+        if getattr(self, "_rf", None) is not None and self._rf.value:
+            try:
+                x = self._rf_solve_refined(self.rhs, refactor=True)
+            except _native.NativeError:
+                pass  # a zero pivot in the kept pivot order
+        if x is None:
+            # The first matrix, or one that the kept pivot order does not suit (the matrices of a DC
+            # solve and of a time step differ in which entries dominate): factor it on the host.
             if not self._rf_try_setup():
                 return nan()
             x = self._rf_solve_refined(self.rhs, accept=True)
         return nan() if x is None else x
 
-    def _rf_matrices(self):
-        torch = self.torch
-        if getattr(self, "_rf_crow", None) is None:
-            self._rf_crow = torch.as_tensor(self.rowptr.astype(np.int64), device=self.dev)
-            self._rf_col = torch.as_tensor(self.colind.astype(np.int64), device=self.dev)
-        mk = lambda v: torch.sparse_csr_tensor(self._rf_crow, self._rf_col, v, size=(self.nu, self.nu),
-                                               check_invariants=False)
-        with warnings.catch_warnings():  # torch marks its sparse CSR support as beta
-            warnings.simplefilter("ignore", UserWarning)
-            return mk(self.jac), mk(self.jac.abs())
-
-    def _rf_solve_refined(self, b, tol=1e-10, max_refine=3, accept=False):
-        """Solve with the current factors, then iterative refinement (r = b - J x, x += J^-1 r) until
-        the componentwise backward error max_i |r_i| / (|J| |x| + |b|)_i is at most tol (a stable
-        factorization gives a few ulps after one refinement step), at most max_refine times. Returns
+    def _rf_solve_refined(self, b, refactor=False, tol=1e-10, max_refine=3, accept=False):
+        """Solve with the current factors (after a refactorization with the current matrix, when
+        refactor is set), then iterative refinement (r = b - J x, x += J^-1 r) until the componentwise
+        backward error max_i |r_i| / (|J| |x| + |b|)_i is at most tol (a stable factorization gives a
+        few ulps after one refinement step), at most max_refine times: xd_rf_solve_refined. Returns
         None when the error stays above tol, or the last iterate when accept is set."""
         torch = self.torch
-        J, Ja = self._rf_matrices()
-        x = b.clone()
-        torch.cuda.current_stream(self.dev).synchronize()
-        _native.check(self._lib.xd_rf_solve(self._rf, ctypes.c_void_p(x.data_ptr())), "xd_rf_solve")
-        torch.cuda.synchronize(self.dev)
-        self.stats.solves += 1
-        ab = b.abs()
-        for k in range(max_refine + 1):
-            if not bool(torch.isfinite(x).all()):
-                return None
-            r = b - J @ x
-            den = Ja @ x.abs() + ab
-            err = torch.where(r == 0, torch.zeros_like(r), r.abs() / den.clamp_min(1e-300))
-            e = float(err.max())
-            if k == 0:
-                self.stats.first_solve_berr.append(e)
-            if e <= tol:
-                return x
-            if k == max_refine:
-                return x if accept else None
-            d = r.contiguous()
-            torch.cuda.current_stream(self.dev).synchronize()
-            _native.check(self._lib.xd_rf_solve(self._rf, ctypes.c_void_p(d.data_ptr())), "xd_rf_solve")
-            torch.cuda.synchronize(self.dev)
-            self.stats.solves += 1
-            self.stats.refinements += 1
-            x = x + d
-        return None
+        x = torch.empty_like(b)
+        stream = torch.cuda.current_stream(self.dev)
+        if stream.cuda_stream != 0:  # the library works on the legacy default stream
+            stream.synchronize()
+        check = _native.XdRfCheck()
+        p = self._ptr
+        rc = self._lib.xd_rf_solve_refined(self._rf, p(self.jac), p(b), p(x), int(refactor), tol, max_refine,
+                                           ctypes.byref(check))
+        self.stats.solves += check.solves
+        self.stats.refinements += max(0, check.solves - 1)
+        if check.checks:
+            self.stats.first_solve_berr.append(check.first_berr)
+        _native.check(rc, "xd_rf_solve_refined")
+        if check.outcome == _native.XD_RF_NOT_FINITE:
+            return None
+        return x if accept or check.outcome == _native.XD_RF_WITHIN_TOL else None
 
     def __del__(self):
         try:
@@ -796,6 +765,8 @@ class GpuTransient(TransientBase):
 
     def _newton(self, prm: NewtonParams, flags_for_iter, mode, h=None, order=1, qn0=None, fhist=None):
         self._first_solve = True
+        if self.solver == "rf":
+            return self._newton_rf(prm, flags_for_iter, mode, h, order, qn0, fhist)
         if not self.graphs:
             return super()._newton(prm, flags_for_iter, mode, h, order, qn0, fhist)
         f1, f2 = flags_for_iter(1), flags_for_iter(2)
@@ -818,6 +789,28 @@ class GpuTransient(TransientBase):
             self._lu_from_slu = self._slu is not None and self._g_host[2] == 0
             if self._g_host[2] != 0:
                 self._note_fallback()
+            if not (math.isfinite(max_rhs) and math.isfinite(wrms)):
+                return -1
+            if max_rhs <= prm.rhs_tol and wrms <= prm.delta_x_tol:
+                return it
+        return -1
+
+    def _newton_rf(self, prm, flags_for_iter, mode, h, order, qn0, fhist):
+        """The base class's iteration with the norms on the device: one synchronisation for the checked
+        solve and one for both norms."""
+        if not hasattr(self, "_rf_norms"):
+            self._rf_norms = self.torch.zeros(3, dtype=self.torch.float64, pin_memory=True)
+        x_ref = self.x.clone()
+        w = prm.rel_tol * x_ref.abs() + prm.abs_tol
+        self._load_and_combine(flags_for_iter(0), mode, h, order, qn0, fhist)
+        for it in range(1, prm.max_iter + 1):
+            dx = self._solve()
+            self._device_update(dx, x_ref, w, prm, self._e_norms)
+            self._load_and_combine(flags_for_iter(it), mode, h, order, qn0, fhist)
+            self._device_residual_norm(self._e_norms)
+            self._rf_norms.copy_(self._e_norms, non_blocking=True)
+            self.torch.cuda.current_stream(self.dev).synchronize()
+            wrms, max_rhs = float(self._rf_norms[0]), float(self._rf_norms[1])
             if not (math.isfinite(max_rhs) and math.isfinite(wrms)):
                 return -1
             if max_rhs <= prm.rhs_tol and wrms <= prm.delta_x_tol:
