@@ -19,37 +19,72 @@ int xd_internal_fail(int code, const std::string &msg);
 namespace {
 
 constexpr int kBottomThreads = 512;
+constexpr int kBottomEntries = 13 * 1024;  // a group's entries in shared memory: two blocks to an SM
 constexpr int kSchurLanes = 8;        // threads per top destination
 constexpr int kTopThreads = 256;
 constexpr int kB = kBlockPivots;
 constexpr int kLd = kB + 2;           // row stride of the block's L and U in shared memory: 16-byte reads without conflicts
 constexpr int kSpinLimit = 1 << 24;   // polls of a chain's flag before the wait gives up
 
-// The bottom subtrees: block g walks its own levels, one barrier per level (the schedule of lu.cu's
-// lu_levels_block_kernel: a level's updates form their L factors on the spot, the divisions that
-// store them follow during the next level). A level's pivot updates ancestors only, which sit in
-// later levels of the same block or in the top part.
-__global__ void __launch_bounds__(kBottomThreads) tree_bottom_kernel(
-    const int *__restrict__ glev, const int *__restrict__ ldiv, const int *__restrict__ ldst,
-    const int2 *__restrict__ div, const int4 *__restrict__ dst, const int4 *__restrict__ pairs, double *v) {
-  const int l0 = glev[blockIdx.x], l1 = glev[blockIdx.x + 1], tid = threadIdx.x;
-  int4 ds_next = make_int4(0, 0, 0, 0);
+// One destination's updates, its first two pairs already here (ds.w < 0 and more than one or two: the
+// rest in batches, so that a batch waits for one round of loads).
+__device__ __forceinline__ void bottom_update(int4 ds, int4 p0, int4 p1, const int4 *__restrict__ pairs, double *m) {
+  double acc = m[ds.x];
+  if (ds.w >= 0) {
+    acc = acc - (m[ds.y] / m[ds.w]) * m[ds.z];
+  } else {
+    acc = acc - (m[p0.x] / m[p0.z]) * m[p0.y];
+    if (ds.z > 1) acc = acc - (m[p1.x] / m[p1.z]) * m[p1.y];
+    for (int p = ds.y + 2; p < ds.y + ds.z; p += 4) {
+      int4 lu[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (p + k < ds.y + ds.z) lu[k] = pairs[p + k];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (p + k < ds.y + ds.z) acc = acc - (m[lu[k].x] / m[lu[k].z]) * m[lu[k].y];
+    }
+  }
+  m[ds.x] = acc;
+}
+
+// A block's levels, one barrier per level (the schedule of lu.cu's lu_levels_block_kernel: a level's
+// updates form their L factors on the spot, the divisions that store them follow during the next
+// level). A level's pivot updates ancestors only, which sit in later levels of the same block or in
+// the top part. A level's lists are read two levels ahead, its first pairs one level ahead.
+__device__ __forceinline__ void bottom_levels(int l0, int l1, const int *__restrict__ ldiv,
+                                              const int *__restrict__ ldst, const int2 *__restrict__ div,
+                                              const int4 *__restrict__ dst, const int4 *__restrict__ pairs, double *m) {
+  const int tid = threadIdx.x;
+  const int4 none = make_int4(0, 0, 0, 0);
+  auto list = [&](int l) {  // this thread's destination of level l
+    if (l >= l1) return none;
+    const int b = ldst[l] + tid;
+    return b < ldst[l + 1] ? dst[b] : none;
+  };
+  auto pair = [&](int4 ds, int k) { return ds.w < 0 && ds.z > k ? pairs[ds.y + k] : none; };
+  int4 ds1 = list(l0), ds2 = list(l0 + 1), p0 = pair(ds1, 0), p1 = pair(ds1, 1);
   int2 dv_next = make_int2(0, 0);
   int ub = ldst[l0], ue = l0 < l1 ? ldst[l0 + 1] : ub, db = ldiv[l0], de = db;
-  if (ub + tid < ue) ds_next = dst[ub + tid];
   for (int l = l0; l < l1; ++l) {
-    const int4 ds = ds_next;
+    const int4 ds = ds1, q0 = p0, q1 = p1;
     const int2 dv = dv_next;
     const int ne = l + 1 < l1 ? ldst[l + 2] : ue, nd = ldiv[l + 1];
-    if (ue + tid < ne) ds_next = dst[ue + tid];
+    ds1 = ds2;
+    ds2 = list(l + 2);
+    p0 = pair(ds1, 0);
+    p1 = pair(ds1, 1);
     if (de + tid < nd) dv_next = div[de + tid];
     if (ub + tid < ue) {
-      lu_update_divide(ds, pairs, v);
-      for (int d = ub + tid + kBottomThreads; d < ue; d += kBottomThreads) lu_update_divide(dst[d], pairs, v);
+      bottom_update(ds, q0, q1, pairs, m);
+      for (int d = ub + tid + kBottomThreads; d < ue; d += kBottomThreads) {
+        const int4 more = dst[d];
+        bottom_update(more, pair(more, 0), pair(more, 1), pairs, m);
+      }
     }
     if (db + tid < de) {
-      lu_divide(dv, v);
-      for (int t = db + tid + kBottomThreads; t < de; t += kBottomThreads) lu_divide(div[t], v);
+      lu_divide(dv, m);
+      for (int t = db + tid + kBottomThreads; t < de; t += kBottomThreads) lu_divide(div[t], m);
     }
     __syncthreads();
     ub = ue;
@@ -58,9 +93,32 @@ __global__ void __launch_bounds__(kBottomThreads) tree_bottom_kernel(
     de = nd;
   }
   if (db + tid < de) {
-    lu_divide(dv_next, v);
-    for (int t = db + tid + kBottomThreads; t < de; t += kBottomThreads) lu_divide(div[t], v);
+    lu_divide(dv_next, m);
+    for (int t = db + tid + kBottomThreads; t < de; t += kBottomThreads) lu_divide(div[t], m);
   }
+}
+
+// The bottom subtrees, a block each. What bounds a block is its levels one after the other: quotients,
+// barriers and, in global memory, an L2 round trip of a level's operands. So the group's own entries
+// (gpos: their places in V) come to shared memory first, the lists hold positions there, and the
+// entries go back at the end: refactorization of 4,455 unknowns 149 -> 139 us, of 41k 288 -> 276, of
+// 200k (where the chains wait) the same. A group with more than kBottomEntries entries (gptr: none of
+// them) works in V itself; only systems above a million unknowns have one.
+__global__ void __launch_bounds__(kBottomThreads) tree_bottom_kernel(
+    const int *__restrict__ glev, const int *__restrict__ ldiv, const int *__restrict__ ldst,
+    const int2 *__restrict__ div, const int4 *__restrict__ dst, const int4 *__restrict__ pairs,
+    const int *__restrict__ gptr, const int *__restrict__ gpos, double *v) {
+  extern __shared__ double entries[];
+  const int l0 = glev[blockIdx.x], l1 = glev[blockIdx.x + 1], e0 = gptr[blockIdx.x], ne = gptr[blockIdx.x + 1] - e0;
+  if (ne == 0) {
+    bottom_levels(l0, l1, ldiv, ldst, div, dst, pairs, v);
+    return;
+  }
+  for (int i = threadIdx.x; i < ne; i += kBottomThreads) entries[i] = v[gpos[e0 + i]];
+  __syncthreads();
+  bottom_levels(l0, l1, ldiv, ldst, div, dst, pairs, entries);
+  __syncthreads();
+  for (int i = threadIdx.x; i < ne; i += kBottomThreads) v[gpos[e0 + i]] = entries[i];
 }
 
 // The bottom pivots' updates of top entries, all at once: kSchurLanes threads per destination, fixed
@@ -760,6 +818,65 @@ __global__ void __launch_bounds__(256) tree_tail_kernel(const int4 *__restrict__
   }
 }
 
+// The bottom groups' lists with positions among the group's own entries (gpos, in order of first use)
+// where those fit shared memory, else unchanged.
+struct BottomLists {
+  std::vector<int> gptr, gpos;
+  std::vector<XdPos2> div;
+  std::vector<XdPos4> dst, pairs;
+  size_t most = 0;
+};
+
+BottomLists bottom_lists(const XdTreePlan &p) {
+  BottomLists b;
+  b.gptr.assign(1, 0);
+  b.div = p.div;
+  b.dst = p.dst;
+  b.pairs = p.pairs;
+  std::vector<int> local((size_t)p.nv, -1);
+  for (int g = 0; g < p.ngroups; ++g) {
+    const int l0 = p.glev[g], l1 = p.glev[g + 1];
+    std::vector<int> used;
+    auto at = [&](int &pos, bool set) {
+      if (!set && local[pos] < 0) {
+        local[pos] = (int)used.size();
+        used.push_back(pos);
+      }
+      if (set) pos = local[pos];
+    };
+    auto walk = [&](bool set) {
+      for (int d = p.ldst[l0]; d < p.ldst[l1]; ++d) {
+        XdPos4 &ds = b.dst[d];
+        at(ds.x, set);
+        if (ds.w >= 0) {
+          at(ds.y, set);
+          at(ds.z, set);
+          at(ds.w, set);
+        } else {
+          for (int k = ds.y; k < ds.y + ds.z; ++k) {
+            at(b.pairs[k].x, set);
+            at(b.pairs[k].y, set);
+            at(b.pairs[k].z, set);
+          }
+        }
+      }
+      for (int d = p.ldiv[l0]; d < p.ldiv[l1]; ++d) {
+        at(b.div[d].x, set);
+        at(b.div[d].y, set);
+      }
+    };
+    walk(false);
+    if (used.size() <= (size_t)kBottomEntries) {
+      walk(true);
+      b.gpos.insert(b.gpos.end(), used.begin(), used.end());
+      b.most = std::max(b.most, used.size());
+    }
+    b.gptr.push_back((int)b.gpos.size());
+    for (int pos : used) local[pos] = -1;
+  }
+  return b;
+}
+
 template <class D, class T>
 cudaError_t upload(D **d, const std::vector<T> &h) {
   static_assert(sizeof(D) == sizeof(T), "device and host records match");
@@ -791,6 +908,8 @@ int xd_tree_upload(XdTree *t, const XdTreePlan &p, const int *perm_p, const int 
     bsrc[x] = perm_p[p.order[x]];
     xdst[x] = perm_q[p.order[x]];
   }
+  const BottomLists bottom = bottom_lists(p);
+  t->bottom_smem = sizeof(double) * bottom.most;
   std::vector<int> grow(1, 0);
   size_t most = 0;
   for (int g = 0; g < p.ngroups; ++g) {
@@ -835,8 +954,11 @@ int xd_tree_upload(XdTree *t, const XdTreePlan &p, const int *perm_p, const int 
       (e = cudaMalloc(&t->d_v, sizeof(double) * std::max<long long>(1, p.nv))) != cudaSuccess ||
       (e = upload(&t->d_diag, p.diag)) != cudaSuccess || (e = upload(&t->d_glev, p.glev)) != cudaSuccess ||
       (e = upload(&t->d_ldiv, p.ldiv)) != cudaSuccess || (e = upload(&t->d_ldst, p.ldst)) != cudaSuccess ||
-      (e = upload(&t->d_div, p.div)) != cudaSuccess || (e = upload(&t->d_dst, p.dst)) != cudaSuccess ||
-      (e = upload(&t->d_pairs, p.pairs)) != cudaSuccess || (e = upload(&t->d_sdst, p.sdst)) != cudaSuccess ||
+      (e = upload(&t->d_div, bottom.div)) != cudaSuccess || (e = upload(&t->d_dst, bottom.dst)) != cudaSuccess ||
+      (e = upload(&t->d_gptr, bottom.gptr)) != cudaSuccess || (e = upload(&t->d_gpos, bottom.gpos)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(tree_bottom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(double) * kBottomEntries)) != cudaSuccess ||
+      (e = upload(&t->d_pairs, bottom.pairs)) != cudaSuccess || (e = upload(&t->d_sdst, p.sdst)) != cudaSuccess ||
       (e = upload(&t->d_sptr, p.sptr)) != cudaSuccess || (e = upload(&t->d_spairs, p.spairs)) != cudaSuccess ||
       (e = upload(&t->d_tdiv, p.tdiv)) != cudaSuccess || (e = upload(&t->d_cptr, p.cptr)) != cudaSuccess ||
       (e = upload(&t->d_bptr, p.bptr)) != cudaSuccess || (e = upload(&t->d_blocks, p.blocks)) != cudaSuccess ||
@@ -865,15 +987,16 @@ void xd_tree_free(XdTree *t) {
                   (void *)t->d_bwd.pass, (void *)t->d_bwd.rows, (void *)t->d_bwd.col, (void *)t->d_lptr,
                   (void *)t->d_lcol, (void *)t->d_tcol, (void *)t->d_chunk, (void *)t->d_tail, (void *)t->d_bsrc,
                   (void *)t->d_xdst, (void *)t->d_joined, (void *)t->d_border, (void *)t->d_y, (void *)t->d_x,
-                  (void *)t->d_wbuf, (void *)t->d_part, (void *)t->d_sctl, (void *)t->d_grow})
+                  (void *)t->d_wbuf, (void *)t->d_part, (void *)t->d_sctl, (void *)t->d_grow, (void *)t->d_gptr,
+                  (void *)t->d_gpos})
     cudaFree(p);
   *t = XdTree();
 }
 
 int xd_tree_factor(XdTree *t, cudaStream_t st) {
   if (t->ngroups > 0)
-    tree_bottom_kernel<<<t->ngroups, kBottomThreads, 0, st>>>(t->d_glev, t->d_ldiv, t->d_ldst, t->d_div, t->d_dst,
-                                                              t->d_pairs, t->d_v);
+    tree_bottom_kernel<<<t->ngroups, kBottomThreads, t->bottom_smem, st>>>(
+        t->d_glev, t->d_ldiv, t->d_ldst, t->d_div, t->d_dst, t->d_pairs, t->d_gptr, t->d_gpos, t->d_v);
   if (t->nsd > 0) {
     const long long threads = (long long)t->nsd * kSchurLanes;
     tree_schur_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(t->nsd, t->d_sdst, t->d_sptr, t->d_spairs,

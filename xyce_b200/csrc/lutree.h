@@ -105,6 +105,8 @@ struct XdTree {
   int *d_glev = nullptr, *d_ldiv = nullptr, *d_ldst = nullptr;
   int2 *d_div = nullptr;
   int4 *d_dst = nullptr, *d_pairs = nullptr;
+  int *d_gptr = nullptr, *d_gpos = nullptr;  // the bottom groups' entries (positions in V) in shared memory
+  size_t bottom_smem = 0;
   int *d_sdst = nullptr, *d_sptr = nullptr;
   int2 *d_spairs = nullptr, *d_tdiv = nullptr;
   int *d_cptr = nullptr, *d_bptr = nullptr, *d_blocks = nullptr, *d_jchild = nullptr;
