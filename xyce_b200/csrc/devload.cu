@@ -552,22 +552,26 @@ __device__ __forceinline__ void gather_chunk(int c, const GatherPart &m, const d
   double acc[NOUT];
 #pragma unroll
   for (int o = 0; o < NOUT; ++o) acc[o] = 0.0;
-  // All of a thread's loads are issued before its first add.
-  constexpr int kPer = kChunk / kChunkBlock;
-  size_t s[kPer];
-  double v[kPer][NOUT];
+  // All of a thread's source indices are read first, then kBatch of its sources at a time, loads before
+  // adds.
+  constexpr int kPer = kChunk / kChunkBlock, kBatch = 8 / NOUT;
+  int s[kPer];
 #pragma unroll
-  for (int j = 0; j < kPer; ++j) s[j] = b + tid + j * kChunkBlock < e ? (size_t)m.src[b + tid + j * kChunkBlock] : 0;
+  for (int j = 0; j < kPer; ++j) s[j] = b + tid + j * kChunkBlock < e ? m.src[b + tid + j * kChunkBlock] : -1;
 #pragma unroll
-  for (int j = 0; j < kPer; ++j)
+  for (int j0 = 0; j0 < kPer; j0 += kBatch) {
+    double v[kBatch][NOUT];
 #pragma unroll
-    for (int o = 0; o < NOUT; ++o) v[j][o] = b + tid + j * kChunkBlock < e ? stage[os.base[o] + s[j]] : 0.0;
+    for (int j = 0; j < kBatch; ++j)
 #pragma unroll
-  for (int j = 0; j < kPer; ++j)
-    if (b + tid + j * kChunkBlock < e) {
+      for (int o = 0; o < NOUT; ++o) v[j][o] = s[j0 + j] >= 0 ? stage[os.base[o] + s[j0 + j]] : 0.0;
 #pragma unroll
-      for (int o = 0; o < NOUT; ++o) acc[o] += ABS ? fabs(v[j][o]) : v[j][o];
-    }
+    for (int j = 0; j < kBatch; ++j)
+      if (s[j0 + j] >= 0) {
+#pragma unroll
+        for (int o = 0; o < NOUT; ++o) acc[o] += ABS ? fabs(v[j][o]) : v[j][o];
+      }
+  }
 #pragma unroll
   for (int o = 0; o < NOUT; ++o) red[o][tid] = acc[o];
   block_tree<NOUT>(red, tid);
@@ -605,10 +609,13 @@ __device__ __forceinline__ void gather_chunk(int c, const GatherPart &m, const d
 
 // A load's whole gather in one launch: the chunks of both maps first (the longest blocks), then the
 // vectors' and the matrices' short outputs. Separate launches (two kinds of short outputs, chunks
-// and chunk combinations) left each other's tails and launch gaps idle: of a 1M-instance load they
-// took 0.19 ms, of a 202-instance one 20 us.
+// and chunk combinations) left each other's tails and launch gaps idle: a 202-instance load's took
+// 20 us, now 4. A thread's work is four dependent reads (range, sources, stamps, output), so what bounds
+// it is reads in flight, at 1M instances 1.1 GB of them: 16 blocks of 128 threads to an SM at 32
+// registers, the chunks' batches kept to eight values for that. At 56 registers (9 blocks) it took
+// 207 us at 1M instances, 57 at 300k of level 1, 84 at 60k of the general topology; now 170, 45 and 59.
 template <bool ABS>
-__global__ void __launch_bounds__(kChunkBlock) gather_kernel(GatherPart mv, OutSet<4, ABS> ov, GatherPart mm,
+__global__ void __launch_bounds__(kChunkBlock, 16) gather_kernel(GatherPart mv, OutSet<4, ABS> ov, GatherPart mm,
                                                              OutSet<2, ABS> om, const double *__restrict__ stage,
                                                              int short_v) {
   __shared__ double red[4][kChunkBlock];
