@@ -48,10 +48,11 @@ EVAL_BYTES_PER_INST = 32 + 16 + 4 + 40 + 8 + 384 + 96 + 24 + 8
 # 612 algorithmic bytes.
 EVAL_DRAM_BYTES_PER_INST_NCU = 90 + 326
 SPLIT_DRAM_BYTES_PER_INST_NCU = 362 + 940
-# FP64 operations per instance of one evaluation (ncu thread-instruction counters of the same
-# capture: 2,621 DFMA (2 flops each) + 844 DMUL + 511 DADD per instance), for the evaluation
-# kernel's compute roofline against the FP64 FMA-pipe probe.
-EVAL_FP64_FLOPS_PER_INST = 2 * 2621 + 844 + 511
+# FP64 operations per instance of one evaluation (ncu thread-instruction counters of the fused kernel
+# at 100,060 instances of the same generator: 1,556 DFMA (2 flops each) + 1,138 DMUL + 847 DADD per instance;
+# 2,621 + 844 + 511 while every quotient was the division operator's), for the evaluation kernel's
+# compute roofline against the FP64 FMA-pipe probe.
+EVAL_FP64_FLOPS_PER_INST = 2 * 1556 + 1138 + 847
 
 
 def replica_totals(dist, n, ms, device):

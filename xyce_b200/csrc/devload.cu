@@ -1840,7 +1840,7 @@ static_assert(kRowBlock <= 32 * kFusedWarps, "a thread per row");
 constexpr int kEntryBlock = 256;
 
 // The family's dF/dx and dQ/dx of CSR entry k: its staged sources summed in the matrix map's
-// order (as gather_short_kernel sums them), or the chunked gathers' sum for a long entry.
+// order (as gather_kernel sums them), or the chunked gathers' sum for a long entry.
 template <bool TRAN>
 __device__ __forceinline__ void fused_entry_sums(int k, const int2 *__restrict__ ent, const int *__restrict__ msrc,
                                                  const double *__restrict__ stage, size_t mb_f, size_t mb_q,

@@ -4,7 +4,7 @@
 // 12.6M updates (0.7 us of the FP64 pipe) and 27 MB of values, but 2,888 pivots in a row. On the
 // B200, per refactorization there: 1.09 ms, of which the chains 0.95 ms (0.33 us a pivot), the bottom
 // subtrees 0.09 ms and their updates of top entries 0.03 ms; per solve 0.63 ms: the chains 0.22 ms
-// forward and 0.35 ms backward, the bottom subtrees 0.03 ms each way. At 41k unknowns 0.29 and 0.21
+// forward and 0.35 ms backward, the bottom subtrees 0.03 ms each way. At 41k unknowns 0.28 and 0.21
 // ms. The level lists of lu.cu and sptrsv.cu, with a barrier and a round trip to global memory per
 // level, take 7.32 and 7.25 ms, and 1.40 and 1.56 ms.
 #include <algorithm>
