@@ -1028,12 +1028,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) mlp_train_kernel(xd_mlp_trai
 }
 
 // Adds the blocks' partial gradients in block order and applies Adam, one thread per parameter; the
-// padding (inputs from n_in, outputs from n_out on) stays zero.
+// padding (inputs from n_in, outputs from n_out on) stays zero. What bounds it is the round trips of
+// a thread's reads (27 MB in all from L2, one and a half blocks to an SM), so the sum is unrolled 32
+// times: a step at batch 16,384 took 97 us unrolled 8 times, 93 us now.
 __global__ void __launch_bounds__(256) mlp_apply_kernel(xd_mlp_train_args a, int blocks) {
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= kPartSize) return;
   float gr = 0.0f;
-#pragma unroll 8
+#pragma unroll 32
   for (int k = 0; k < blocks; ++k) gr += a.part[(size_t)k * kPartSize + i];
   int l, r, c = 0;
   bool bias = false, pad = false;
