@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "../../include/xyce_tia.h"
+#include "cluster_meet.h"
 #include "tia_long.h"
 
 int xd_internal_fail(int code, const std::string &msg);
@@ -313,15 +314,7 @@ size_t dense_smem_bytes(int n) { return sizeof(double) * (size_t)n * (size_t)(n 
 // blocks whose partial results meet in the first one's shared memory, so that the norms need no
 // scratch memory that calls on two streams would share.
 constexpr int kNormThreads = 1024, kNormCluster = 8, kNormBlock = 8 * kNormThreads;
-
-// This block's value (thread 0's) to slot `rank` of the first block's array; complete after the sync.
-template <typename T>
-__device__ __forceinline__ void to_first_block(T v, T *slots) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  if (threadIdx.x == 0) *cl.map_shared_rank(slots + cl.block_rank(), 0) = v;
-  cl.sync();
-}
+using NormMeet = ClusterMeet<cooperative_groups::cluster_group>;
 
 __device__ __forceinline__ double block_sum(double v, double *red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -343,6 +336,7 @@ __global__ void __launch_bounds__(kNormThreads) newton_update_kernel(int n, doub
                                                                      double *__restrict__ w, double rel, double abs_,
                                                                      int update_w, double *__restrict__ norms) {
   __shared__ double red[32], part[kNormCluster];
+  NormMeet meet(cooperative_groups::this_cluster(), gridDim.x > 1);
   double s = 0.0;
   for (int i = blockIdx.x * kNormThreads + threadIdx.x; i < n; i += gridDim.x * kNormThreads) {
     const double d = dx[i], xi = x[i] + d;
@@ -359,7 +353,7 @@ __global__ void __launch_bounds__(kNormThreads) newton_update_kernel(int n, doub
   }
   s = block_sum(s, red);
   if (gridDim.x > 1) {
-    to_first_block(s, part);
+    meet.put(s, part, threadIdx.x == 0);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       s = part[0];
       for (int q = 1; q < kNormCluster; ++q) s += part[q];
@@ -373,6 +367,7 @@ __global__ void __launch_bounds__(kNormThreads) residual_norm_kernel(int n, cons
                                                                      const int *__restrict__ flag,
                                                                      double *__restrict__ norms) {
   __shared__ unsigned long long red[32], part[kNormCluster];
+  NormMeet meet(cooperative_groups::this_cluster(), gridDim.x > 1);
   unsigned long long m = 0;
   for (int i = blockIdx.x * kNormThreads + threadIdx.x; i < n; i += gridDim.x * kNormThreads)
     m = max(m, (unsigned long long)__double_as_longlong(rhs[i]) & 0x7fffffffffffffffull);
@@ -387,7 +382,7 @@ __global__ void __launch_bounds__(kNormThreads) residual_norm_kernel(int n, cons
     for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
   }
   if (gridDim.x > 1) {
-    to_first_block(m, part);
+    meet.put(m, part, threadIdx.x == 0);
     if (blockIdx.x == 0 && threadIdx.x == 0)
       for (int q = 0; q < kNormCluster; ++q) m = max(m, part[q]);
   }
