@@ -58,7 +58,8 @@ struct GatherMap {
   int *d_chunk_begin = nullptr;                        // chunk -> [first contribution, next)
   double *d_partial = nullptr;                         // [NOUT][n_chunks] chunk partial sums
   int *d_chunk_long = nullptr;                         // chunk -> its entry
-  int *d_done = nullptr;                               // entry -> chunks summed so far (zero between gathers)
+  int n_multi = 0;
+  int4 *d_multi = nullptr;                             // entries of more than one chunk: (output, first chunk, next)
   int *d_src = nullptr;  // staging index within one output's slot range
   size_t n_src = 0;
 };
@@ -499,11 +500,11 @@ __device__ __forceinline__ void sum_sources(int b, int e, const int *__restrict_
 // rail's row, for instance) are split into fixed chunks of kChunk consecutive contributions, a block
 // each.
 struct GatherPart {
-  int n_short = 0, n_long = 0, n_chunks = 0;
+  int n_short = 0, n_chunks = 0, n_multi = 0;
   const int *short_dst = nullptr, *short_ptr = nullptr, *src = nullptr, *chunk_begin = nullptr,
             *chunk_long = nullptr, *long_dst = nullptr, *long_chunk = nullptr;
+  const int4 *multi = nullptr;
   double *partial = nullptr;
-  int *done = nullptr;
 };
 
 template <int NOUT, bool ABS>
@@ -542,12 +543,11 @@ __device__ __forceinline__ void block_tree(double (*red)[kChunkBlock], int tid) 
   }
 }
 
-// Chunk c: its contributions in a fixed strided split and a fixed tree, into the chunk's partial; the
-// block that finishes an entry's last chunk combines the entry's partials, again in a fixed split
-// and tree, and resets the entry's count. Which block that is does not change the result.
+// Chunk c: its contributions in a fixed strided split and a fixed tree. An entry of one chunk is done
+// with that; of more, the sum goes to the chunk's partial for gather_combine.
 template <int NOUT, bool ABS>
 __device__ __forceinline__ void gather_chunk(int c, const GatherPart &m, const double *__restrict__ stage,
-                                             const OutSet<NOUT, ABS> &os, double (*red)[kChunkBlock], int *last) {
+                                             const OutSet<NOUT, ABS> &os, double (*red)[kChunkBlock]) {
   const int tid = threadIdx.x, b = m.chunk_begin[c], e = m.chunk_begin[c + 1];
   double acc[NOUT];
 #pragma unroll
@@ -575,25 +575,33 @@ __device__ __forceinline__ void gather_chunk(int c, const GatherPart &m, const d
 #pragma unroll
   for (int o = 0; o < NOUT; ++o) red[o][tid] = acc[o];
   block_tree<NOUT>(red, tid);
-  const int t = m.chunk_long[c], c0 = m.long_chunk[t], c1 = m.long_chunk[t + 1];
-  if (tid == 0) {
+  if (tid != 0) return;
 #pragma unroll
-    for (int o = 0; o < NOUT; ++o) __stcg(m.partial + (size_t)o * m.n_chunks + c, red[o][0]);
-    __threadfence();
-    *last = atomicAdd(m.done + t, 1) == c1 - c0 - 1;
+  for (int o = 0; o < NOUT; ++o) acc[o] = red[o][0];
+  const int t = m.chunk_long[c];
+  if (m.long_chunk[t + 1] - m.long_chunk[t] == 1) {
+    put_output<NOUT, ABS>(os, m.long_dst[t], acc);
+  } else {
+#pragma unroll
+    for (int o = 0; o < NOUT; ++o) m.partial[(size_t)o * m.n_chunks + c] = acc[o];
   }
-  __syncthreads();
-  if (!*last) return;
-  __threadfence();
-  // Two strided sums a thread: the split and the tree of a block of 2 kChunkBlock threads.
-  double acc2[NOUT];
+}
+
+// Entry m's partials in a fixed strided split, two sums a thread, and a fixed tree. The partials are the
+// launch before's, which may still run until the wait.
+template <int NOUT, bool ABS>
+__device__ __forceinline__ void gather_combine(int4 m, const GatherPart &g, const OutSet<NOUT, ABS> &os,
+                                               double (*red)[kChunkBlock]) {
+  const int tid = threadIdx.x;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  double acc[NOUT], acc2[NOUT];
 #pragma unroll
   for (int o = 0; o < NOUT; ++o) acc[o] = acc2[o] = 0.0;
-  for (int k = c0 + tid; k < c1; k += 2 * kChunkBlock) {
+  for (int k = m.y + tid; k < m.z; k += 2 * kChunkBlock) {
 #pragma unroll
     for (int o = 0; o < NOUT; ++o) {
-      acc[o] += __ldcg(m.partial + (size_t)o * m.n_chunks + k);
-      if (k + kChunkBlock < c1) acc2[o] += __ldcg(m.partial + (size_t)o * m.n_chunks + k + kChunkBlock);
+      acc[o] += g.partial[(size_t)o * g.n_chunks + k];
+      if (k + kChunkBlock < m.z) acc2[o] += g.partial[(size_t)o * g.n_chunks + k + kChunkBlock];
     }
   }
 #pragma unroll
@@ -602,46 +610,69 @@ __device__ __forceinline__ void gather_chunk(int c, const GatherPart &m, const d
   if (tid == 0) {
 #pragma unroll
     for (int o = 0; o < NOUT; ++o) acc[o] = red[o][0];
-    put_output<NOUT, ABS>(os, m.long_dst[t], acc);
-    m.done[t] = 0;
+    put_output<NOUT, ABS>(os, m.x, acc);
   }
 }
 
-// A load's whole gather in one launch: the chunks of both maps first (the longest blocks), then the
-// vectors' and the matrices' short outputs. Separate launches (two kinds of short outputs, chunks
-// and chunk combinations) left each other's tails and launch gaps idle: a 202-instance load's took
-// 20 us, now 4. A thread's work is four dependent reads (range, sources, stamps, output), so what bounds
-// it is reads in flight, at 1M instances 1.1 GB of them: 16 blocks of 128 threads to an SM at 32
-// registers, the chunks' batches kept to eight values for that. At 56 registers (9 blocks) it took
-// 207 us at 1M instances, 57 at 300k of level 1, 84 at 60k of the general topology; now 170, 45 and 59.
+// Blocks of one launch of a gather: combined entries of both maps, chunks of both, short outputs of both.
+struct GatherBlocks {
+  int combine_v = 0, combine_m = 0, chunks_v = 0, chunks_m = 0, short_v = 0, short_m = 0;
+  int all() const { return combine_v + combine_m + chunks_v + chunks_m + short_v + short_m; }
+};
+
+// A load's gather: the chunks of both maps first (the longest blocks), then the vectors' and the
+// matrices' short outputs. Where no entry has several chunks that is one launch. Else the chunks are
+// a launch of their own, and the entries' combinations go with the short outputs in a second one,
+// which starts while the chunks run (its combining blocks alone wait for them). It is not the block
+// that finishes an entry's last chunk that combines it: that takes a count in memory which all gathers
+// of the map share, and two of them may overlap on two streams (of the same stamps, where they write the
+// same partials). The second launch costs two microseconds: a load of 300k level-1 instances takes
+// 109 us and took 107 with such counts; with the combinations as a launch behind the others, 115.
+//
+// Separate launches for the kinds of outputs, one after the other, left each other's tails and launch
+// gaps idle: a 202-instance load's took 20 us, now 4. A thread's work is four dependent reads (range,
+// sources, stamps, output), so what bounds it is reads in flight, at 1M instances 1.1 GB of them: 16
+// blocks of 128 threads to an SM at 32 registers, the chunks' batches kept to eight values for that. At
+// 56 registers (9 blocks) it took 207 us at 1M instances, 57 at 300k of level 1, 84 at 60k of the
+// general topology; now 170, 45 and 59.
 template <bool ABS>
 __global__ void __launch_bounds__(kChunkBlock, 16) gather_kernel(GatherPart mv, OutSet<4, ABS> ov, GatherPart mm,
                                                              OutSet<2, ABS> om, const double *__restrict__ stage,
-                                                             int short_v) {
+                                                             GatherBlocks n) {
   __shared__ double red[4][kChunkBlock];
-  __shared__ int last;
+  asm volatile("griddepcontrol.launch_dependents;");
   int b = blockIdx.x;
-  if (b < mv.n_chunks) {
-    gather_chunk<4, ABS>(b, mv, stage, ov, red, &last);
+  if (b < n.combine_v) {
+    gather_combine<4, ABS>(mv.multi[b], mv, ov, red);
     return;
   }
-  b -= mv.n_chunks;
-  if (b < mm.n_chunks) {
-    gather_chunk<2, ABS>(b, mm, stage, om, red, &last);
+  b -= n.combine_v;
+  if (b < n.combine_m) {
+    gather_combine<2, ABS>(mm.multi[b], mm, om, red);
     return;
   }
-  b -= mm.n_chunks;
-  if (b < short_v) {
+  b -= n.combine_m;
+  if (b < n.chunks_v) {
+    gather_chunk<4, ABS>(b, mv, stage, ov, red);
+    return;
+  }
+  b -= n.chunks_v;
+  if (b < n.chunks_m) {
+    gather_chunk<2, ABS>(b, mm, stage, om, red);
+    return;
+  }
+  b -= n.chunks_m;
+  if (b < n.short_v) {
     gather_short<4, ABS>(b * kChunkBlock + threadIdx.x, mv, stage, ov);
     return;
   }
-  gather_short<2, ABS>((b - short_v) * kChunkBlock + threadIdx.x, mm, stage, om);
+  gather_short<2, ABS>((b - n.short_v) * kChunkBlock + threadIdx.x, mm, stage, om);
 }
 
 GatherPart gather_part(const GatherMap &m, double *partial = nullptr) {
   GatherPart p;
   p.n_short = m.n_short;
-  p.n_long = m.n_long;
+  p.n_multi = m.n_multi;
   p.n_chunks = m.n_chunks;
   p.short_dst = m.d_short_dst;
   p.short_ptr = m.d_short_ptr;
@@ -650,8 +681,8 @@ GatherPart gather_part(const GatherMap &m, double *partial = nullptr) {
   p.chunk_long = m.d_chunk_long;
   p.long_dst = m.d_long_dst;
   p.long_chunk = m.d_long_chunk;
+  p.multi = m.d_multi;
   p.partial = partial ? partial : m.d_partial;
-  p.done = m.d_done;
   return p;
 }
 
@@ -659,12 +690,28 @@ GatherPart gather_part(const GatherMap &m, double *partial = nullptr) {
 template <bool ABS>
 int run_gather(const GatherPart &mv, const OutSet<4, ABS> &ov, const GatherPart &mm, const OutSet<2, ABS> &om,
                const double *stage, cudaStream_t st) {
-  const int sv = (mv.n_short + kChunkBlock - 1) / kChunkBlock, sm = (mm.n_short + kChunkBlock - 1) / kChunkBlock;
-  const int blocks = mv.n_chunks + mm.n_chunks + sv + sm;
-  if (blocks == 0) return 0;
-  gather_kernel<ABS><<<blocks, kChunkBlock, 0, st>>>(mv, ov, mm, om, stage, sv);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "gather launch");
+  GatherBlocks first, second;
+  GatherBlocks &shorts = mv.n_multi + mm.n_multi > 0 ? second : first;
+  first.chunks_v = mv.n_chunks;
+  first.chunks_m = mm.n_chunks;
+  shorts.short_v = (mv.n_short + kChunkBlock - 1) / kChunkBlock;
+  shorts.short_m = (mm.n_short + kChunkBlock - 1) / kChunkBlock;
+  second.combine_v = mv.n_multi;
+  second.combine_m = mm.n_multi;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kChunkBlock);
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  for (const GatherBlocks &n : {first, second}) {
+    if (n.all() == 0) continue;
+    cfg.gridDim = dim3(n.all());
+    cfg.numAttrs = n.combine_v + n.combine_m > 0;  // the second launch: beside the first
+    if (cudaError_t e = cudaLaunchKernelEx(&cfg, gather_kernel<ABS>, mv, ov, mm, om, stage, n))
+      return cuda_fail(e, "gather launch");
+  }
   return 0;
 }
 
@@ -698,6 +745,7 @@ int build_map(const std::vector<int> &tgt_of, const std::vector<int> &src_of, in
       short_ptr.push_back((int)n_src);
     }
   std::vector<int> long_chunk(1, 0), chunk_begin, chunk_long;
+  std::vector<int4> multi;
   for (int t = 0; t < n_targets; ++t)
     if (count[t] > kLongThreshold) {
       start[t] = (long long)n_src;
@@ -706,6 +754,7 @@ int build_map(const std::vector<int> &tgt_of, const std::vector<int> &src_of, in
         chunk_long.push_back((int)long_dst.size());
       }
       n_src += count[t];
+      if (count[t] > kChunk) multi.push_back(make_int4(t, long_chunk.back(), (int)chunk_begin.size(), 0));
       long_dst.push_back(t);
       long_chunk.push_back((int)chunk_begin.size());
     }
@@ -737,7 +786,11 @@ int build_map(const std::vector<int> &tgt_of, const std::vector<int> &src_of, in
   XD_CUDA(up(&m.d_long_chunk, long_chunk));
   XD_CUDA(up(&m.d_chunk_begin, chunk_begin));
   XD_CUDA(up(&m.d_chunk_long, chunk_long));
-  XD_CUDA(up(&m.d_done, std::vector<int>(long_dst.size(), 0)));
+  m.n_multi = (int)multi.size();
+  if (m.n_multi > 0) {
+    XD_CUDA(cudaMalloc(&m.d_multi, multi.size() * sizeof(int4)));
+    XD_CUDA(cudaMemcpy(m.d_multi, multi.data(), multi.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  }
   if (m.n_chunks > 0) XD_CUDA(cudaMalloc(&m.d_partial, (size_t)4 * m.n_chunks * sizeof(double)));
   XD_CUDA(up(&m.d_src, src));
   return 0;
@@ -751,7 +804,7 @@ void free_map(GatherMap &m) {
   cudaFree(m.d_chunk_begin);
   cudaFree(m.d_partial);
   cudaFree(m.d_chunk_long);
-  cudaFree(m.d_done);
+  cudaFree(m.d_multi);
   cudaFree(m.d_src);
   m = GatherMap();
 }
@@ -1649,7 +1702,7 @@ int xd_launches_per_load(const xd_ctx *ctx) {
   if (!ctx) return -1;
   if (ctx->n == 0) return 0;
   const int eval = (ctx->family == kFamilyBsim4 && kEvalVariants[ctx->eval_variant].split) ? 2 : 1;
-  return eval + (ctx->vmap.n_src + ctx->mmap.n_src > 0);
+  return eval + (ctx->vmap.n_src + ctx->mmap.n_src > 0) + (ctx->vmap.n_multi + ctx->mmap.n_multi > 0);
 }
 
 int xd_eval_launch_shape(const xd_ctx *ctx, int *block, int *min_blocks) {
