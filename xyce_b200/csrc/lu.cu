@@ -353,7 +353,7 @@ void xd_lu_free(XdLu *lu) {
   *lu = XdLu();
 }
 
-int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st) {
+int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st, bool divide) {
   cudaError_t e;
   if (lu->tree.on) {
     XdTree &t = lu->tree;
@@ -362,6 +362,7 @@ int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st) {
       return xd_internal_fail(-3, std::string("LU refactorization: ") + cudaGetErrorString(e));
     if (lu->nnz_a > 0)
       lu_scatter_kernel<<<(lu->nnz_a + 255) / 256, 256, 0, st>>>(lu->nnz_a, lu->d_a2m, d_vals_a, t.d_v);
+    t.divide = divide;
     return xd_tree_factor(&t, st);
   }
   if ((e = cudaMemsetAsync(lu->d_mx, 0, std::max(1, lu->nnz) * sizeof(double), st)) != cudaSuccess ||
@@ -399,11 +400,12 @@ int xd_lu_copy(XdLu *lu, double *h_vals) {
 }
 
 const int *xd_lu_status(const XdLu *lu, int *count) {
-  *count = lu->tree.on ? 2 : 1;
+  *count = lu->tree.on ? kLuStatus : 1;
   return lu->tree.on ? lu->tree.d_ctl + kTreeInfo : lu->d_info;
 }
 
-int xd_lu_report(const XdLu *lu, const int *status, int *info) {
+int xd_lu_report(const XdLu *lu, const int *status, int *info, bool *again) {
+  *again = false;
   if (!lu->tree.on) {
     *info = status[0] == kLuNoZeroPivot ? 0 : status[0];
     return 0;
@@ -411,14 +413,15 @@ int xd_lu_report(const XdLu *lu, const int *status, int *info) {
   if (status[kTreeExpired - kTreeInfo] != 0)
     return xd_internal_fail(-3, "LU refactorization: a wait between chains expired");
   *info = status[0] == 0 ? 0 : lu->n - status[0] + 1;
+  *again = status[kTreeOdd - kTreeInfo] != 0 && !lu->tree.divide;
   return 0;
 }
 
-int xd_lu_info(XdLu *lu, cudaStream_t st, int *info) {
-  int status[2] = {0, 0}, count = 0;
+int xd_lu_info(XdLu *lu, cudaStream_t st, int *info, bool *again) {
+  int status[kLuStatus] = {}, count = 0;
   const int *d = xd_lu_status(lu, &count);
   cudaError_t e = cudaMemcpyAsync(status, d, sizeof(int) * count, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return xd_internal_fail(-3, std::string("LU pivot report: ") + cudaGetErrorString(e));
-  return xd_lu_report(lu, status, info);
+  return xd_lu_report(lu, status, info, again);
 }

@@ -50,13 +50,16 @@ int xd_lu_init(XdLu *lu, int n, int nnz_a, const int *rowptr_a, const int *colin
                const int *colind_l, const int *rowptr_u, const int *colind_u, const int *p, const int *q);
 void xd_lu_free(XdLu *lu);
 // Refactors with A's values d_vals_a (device, A's CSR order): M = P A Q scattered, then
-// eliminated in place. Stream-ordered; the zero-pivot report is left in d_info.
-int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st);
+// eliminated in place. Stream-ordered; its report is left on the device. divide: the chains of a tree
+// plan divide by their pivots instead of multiplying by reciprocals (asked for by the report below).
+int xd_lu_refactor(XdLu *lu, const double *d_vals_a, cudaStream_t st, bool divide = false);
 // Copies M's values to host memory (nnz doubles, M's CSR order).
 int xd_lu_copy(XdLu *lu, double *h_vals);
-// Reads the zero-pivot report (synchronises the stream): 0, or 1 + the first row found.
-int xd_lu_info(XdLu *lu, cudaStream_t st, int *info);
+// Reads the report (synchronises the stream): *info 0, or 1 + the first row with a zero pivot; *again:
+// the matrix has pivots whose reciprocals are no normal numbers, refactor it with divide.
+int xd_lu_info(XdLu *lu, cudaStream_t st, int *info, bool *again);
 // The same without a synchronisation of its own: the device words of the report and their number (at
-// most two), and the reading of them once they are on the host.
+// most kLuStatus), and the reading of them once they are on the host.
+constexpr int kLuStatus = 3;
 const int *xd_lu_status(const XdLu *lu, int *count);
-int xd_lu_report(const XdLu *lu, const int *status, int *info);
+int xd_lu_report(const XdLu *lu, const int *status, int *info, bool *again);

@@ -8,7 +8,6 @@
 // ms. The level lists of lu.cu and sptrsv.cu, with a barrier and a round trip to global memory per
 // level, take 7.32 and 7.25 ms, and 1.40 and 1.56 ms.
 #include <algorithm>
-#include <cfloat>
 #include <string>
 
 #include "lu_updates.cuh"
@@ -143,16 +142,22 @@ __device__ __forceinline__ void cp_async16(void *s, const void *g) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(g) : "memory");
 }
 
-// 1 / x for normal x: the approximate reciprocal instruction and two Newton steps y += y (1 - x y),
-// each squaring its relative error of 2^-20; branch-free, where the division operator's
+// 1 / x for ordinary x (below): the approximate reciprocal instruction and two Newton steps y += y (1 -
+// x y), each squaring its relative error of 2^-20; branch-free, where the division operator's
 // special-case branch would keep the compiler from overlapping a pivot's reciprocal with the
-// block's other updates. Zero and subnormal pivots are reported by tree_finish_kernel.
+// block's other updates.
 __device__ __forceinline__ double reciprocal(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   y = fma(y, fma(-x, y, 1.0), y);
   return fma(y, fma(-x, y, 1.0), y);
 }
+
+// Pivots whose reciprocal and its approximation are normal numbers. The others (subnormal, above 2^1021,
+// zero, not finite) need the division: tree_finish_kernel reports them, and the caller then takes the
+// matrix again with DIVIDE. The chains' kernels do not look for them on their way: a check per pivot
+// and a way round it cost 46 us of the 1.79 ms of a refactorization and solve at 200k unknowns.
+__device__ __forceinline__ bool ordinary(double p) { return fabs(p) >= 0x1p-1021 && fabs(p) <= 0x1p1021; }
 
 // A frame's shared memory: the frame, two blocks' panels, the block's L and U, its diagonal part,
 // two blocks' records and the slots of its pivots.
@@ -238,6 +243,7 @@ __device__ __forceinline__ void rank_update(const Frame &f, int ld, int R, int c
 // A child chain leaves its remaining front in jbuf and its parent adds it at the block where the
 // two paths meet. Chains are taken by ticket, children first, so a chain that waits only waits for
 // blocks already running.
+template <bool DIVIDE>
 __global__ void __launch_bounds__(kTopThreads) tree_top_kernel(int F, const int *__restrict__ cptr,
                                                                const int *__restrict__ bptr,
                                                                const int *__restrict__ blocks,
@@ -332,11 +338,11 @@ __global__ void __launch_bounds__(kTopThreads) tree_top_kernel(int F, const int 
         if (rec[j] == me) mine = j;
 #pragma unroll
       for (int j = 0; j < kB; ++j) {
-        const double rp = reciprocal(d[j][j]);
+        const double pv = d[j][j], rp = DIVIDE ? 0.0 : reciprocal(pv);
 #pragma unroll
-        for (int i = j + 1; i < kB; ++i) d[i][j] *= rp;
+        for (int i = j + 1; i < kB; ++i) d[i][j] = DIVIDE ? d[i][j] / pv : d[i][j] * rp;
         if (lside) {
-          x[j] = j < mine ? x[j] * rp : 0.0;
+          x[j] = j >= mine ? 0.0 : DIVIDE ? x[j] / pv : x[j] * rp;
 #pragma unroll
           for (int i = j + 1; i < kB; ++i) x[i] = fma(-x[j], d[j][i], x[i]);
         } else {
@@ -364,7 +370,7 @@ __global__ void __launch_bounds__(kTopThreads) tree_top_kernel(int F, const int 
       const int i = (tid - (kTopThreads - kB * kB)) / kB, j = tid % kB;
       const double *row = (j >= i ? f.su : f.sl) + (rec[max(i, j)] & 0xff) * kLd;
       double d = i == j ? 1.0 : 0.0;
-      if (i < nb && j < nb) d = i == j ? reciprocal(row[i]) : row[min(i, j)];
+      if (i < nb && j < nb) d = i != j ? row[min(i, j)] : DIVIDE ? row[i] : reciprocal(row[i]);
       panels[t * stride + 2 * kB * F + i * kB + j] = d;
     }
     for (int c0 = 0; c0 < R; c0 += 64) {
@@ -388,15 +394,16 @@ __global__ void __launch_bounds__(kTopThreads) tree_top_kernel(int F, const int 
   if (tid == 0) atomicExch(ctl + kTreeFlags + chain, 1);
 }
 
-// What follows the elimination: the top pivots' column entries outside their panels are divided,
-// and zero pivots (of the top, subnormal ones too) reported: n - k for the first such k.
+// What follows the elimination: the top pivots' column entries outside their panels are divided, zero
+// pivots reported (n - k for the first such k), and whether a top pivot is not an ordinary one.
 __global__ void tree_finish_kernel(int nt, const int2 *__restrict__ tdiv, int n, const int *__restrict__ diag, int p0,
                                    double *v, int *ctl) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < nt) lu_divide(tdiv[k], v);
   if (k < n) {
     const double p = v[diag[k]];
-    if (p == 0.0 || (diag[k] >= p0 && fabs(p) < DBL_MIN)) atomicMax(ctl + kTreeInfo, n - k);
+    if (p == 0.0) atomicMax(ctl + kTreeInfo, n - k);
+    if (diag[k] >= p0 && !ordinary(p)) ctl[kTreeOdd] = 1;
   }
 }
 
@@ -694,6 +701,7 @@ __global__ void __launch_bounds__(kMaxFrame + 32) tree_forward_chain_kernel(
 // Backward chains, parents first: thread r holds the solved value of slot r's variable. Per block:
 // the pivots' row sums over the front, reduced within warps by shuffles and across them through
 // shared memory, then the block's triangle.
+template <bool DIVIDE>
 __global__ void __launch_bounds__(kMaxFrame + 32) tree_backward_chain_kernel(
     int nchains, int F, const int *__restrict__ cptr, const int *__restrict__ bptr, const int *__restrict__ blocks,
     const int *__restrict__ jchild, const int *__restrict__ border, const double *panels, const double *y, int x0,
@@ -766,7 +774,7 @@ __global__ void __launch_bounds__(kMaxFrame + 32) tree_backward_chain_kernel(
         for (int j = 0; j < kB; ++j) v[j] -= red[k * kB + j];
 #pragma unroll
       for (int j = kB - 1; j >= 0; --j) {
-        v[j] = j < nb ? v[j] * g.d[j][j] : 0.0;
+        v[j] = j >= nb ? 0.0 : DIVIDE ? v[j] / g.d[j][j] : v[j] * g.d[j][j];
 #pragma unroll
         for (int i = 0; i < j; ++i) v[i] = fma(-g.d[i][j], v[j], v[i]);
       }
@@ -964,11 +972,15 @@ int xd_tree_upload(XdTree *t, const XdTreePlan &p, const int *perm_p, const int 
       (e = upload(&t->d_bptr, p.bptr)) != cudaSuccess || (e = upload(&t->d_blocks, p.blocks)) != cudaSuccess ||
       (e = upload(&t->d_jchild, p.jchild)) != cudaSuccess || (e = upload(&t->d_jmap, p.jmap)) != cudaSuccess ||
       (e = cudaMalloc(&t->d_jbuf, sizeof(double) * std::max<size_t>(1, (size_t)p.nchains * p.F * p.F))) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(tree_top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      (e = cudaFuncSetAttribute(tree_top_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)Frame::bytes(kMaxFrame))) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(tree_top_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)Frame::bytes(kMaxFrame))) != cudaSuccess ||
       (e = cudaFuncSetAttribute(tree_forward_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)SolveSmem::bytes(kMaxFrame))) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(tree_backward_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      (e = cudaFuncSetAttribute(tree_backward_chain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)SolveSmem::bytes(kMaxFrame))) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(tree_backward_chain_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)SolveSmem::bytes(kMaxFrame))) != cudaSuccess ||
       (e = cudaMalloc(&t->d_ctl, sizeof(int) * (kTreeFlags + p.nchains))) != cudaSuccess) {
     xd_tree_free(t);
@@ -1003,7 +1015,7 @@ int xd_tree_factor(XdTree *t, cudaStream_t st) {
                                                                          t->d_v);
   }
   if (t->nchains > 0) {
-    tree_top_kernel<<<t->nchains, kTopThreads, Frame::bytes(t->F), st>>>(
+    (t->divide ? tree_top_kernel<true> : tree_top_kernel<false>)<<<t->nchains, kTopThreads, Frame::bytes(t->F), st>>>(
         t->F, t->d_cptr, t->d_bptr, t->d_blocks, t->d_jchild, t->d_jmap, t->d_jbuf, t->d_v + t->p0, t->d_ctl);
   }
   const int work = std::max(t->n, t->ntdiv);
@@ -1033,7 +1045,7 @@ int xd_tree_solve(XdTree *t, double *d_x, cudaStream_t st) {
     tree_forward_chain_kernel<<<nc, threads, SolveSmem::bytes(t->F), st>>>(
         t->F, t->d_cptr, t->d_bptr, t->d_blocks, t->d_jchild, t->d_jmap, t->d_wbuf, v + t->p0, t->d_y + t->nbot,
         t->d_sctl, t->d_sctl + 2);
-    tree_backward_chain_kernel<<<nc, threads, SolveSmem::bytes(t->F), st>>>(
+    (t->divide ? tree_backward_chain_kernel<true> : tree_backward_chain_kernel<false>)<<<nc, threads, SolveSmem::bytes(t->F), st>>>(
         nc, t->F, t->d_cptr, t->d_bptr, t->d_blocks, t->d_jchild, t->d_border, v + t->p0, t->d_y, t->nbot, t->d_x,
         t->d_xdst, d_x, t->d_sctl + 1, t->d_sctl + 2 + nc, t->d_joined);
   }

@@ -98,6 +98,7 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
 
 struct XdTree {
   bool on = false;                   // the matrix has a plan
+  bool divide = false;               // V's chain pivots are divided by (their diagonal parts hold no reciprocals)
   int n = 0, F = 0, ntop = 0, ngroups = 0, nchains = 0, nsd = 0, ntdiv = 0, p0 = 0;
   long long nv = 0;
   double *d_v = nullptr;             // V
@@ -112,7 +113,7 @@ struct XdTree {
   int *d_cptr = nullptr, *d_bptr = nullptr, *d_blocks = nullptr, *d_jchild = nullptr;
   unsigned char *d_jmap = nullptr;
   double *d_jbuf = nullptr;          // [nchains][F * F] the fronts that chains hand to their parents
-  int *d_ctl = nullptr;              // zero pivots, expired waits, tickets, chain flags; zeroed by each call
+  int *d_ctl = nullptr;              // the words below; zeroed by each call
   // Solves: rows by position in the plan's order.
   int nbot = 0, ntail = 0, nchunk = 0, l0 = 0, u0 = 0, t0 = 0, d0 = 0;
   struct Passes {
@@ -137,8 +138,10 @@ struct XdTree {
 int xd_tree_upload(XdTree *t, const XdTreePlan &plan, const int *p, const int *q);
 void xd_tree_free(XdTree *t);
 // Eliminates V (holding P A Q, zeros elsewhere) in place; kTreeInfo of d_ctl holds n - k for the first
-// zero pivot k (0: none), kTreeExpired is nonzero when a wait between chains gave up.
-constexpr int kTreeInfo = 0, kTreeExpired = 1, kTreeTicket = 2, kTreeFlags = 4;
+// zero pivot k (0: none), kTreeExpired is nonzero when a wait between chains gave up, kTreeOdd when a
+// chain met a pivot whose reciprocal is not a normal number: without t->divide the factors are then
+// not to be used. (Then the chains' ticket, and a flag for each.)
+constexpr int kTreeInfo = 0, kTreeExpired = 1, kTreeOdd = 2, kTreeTicket = 3, kTreeFlags = 4;
 int xd_tree_factor(XdTree *t, cudaStream_t st);
 // Solves A x = b in place in d_x with V's factors. Stream-ordered.
 int xd_tree_solve(XdTree *t, double *d_x, cudaStream_t st);

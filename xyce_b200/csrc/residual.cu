@@ -180,7 +180,7 @@ int xd_residual_init(XdResidual *r, int n, const int *rowptr, const int *d_rowpt
       (e = cudaMemcpy(r->d_long, rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(r->d_lseg, lseg.data(), sizeof(int) * lseg.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(r->d_seg, seg.data(), sizeof(int2) * seg.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaHostAlloc(&r->h_out, sizeof(double) * 4, cudaHostAllocPortable)) != cudaSuccess) {
+      (e = cudaHostAlloc(&r->h_out, sizeof(double) * (2 + kResidualStatus), cudaHostAllocPortable)) != cudaSuccess) {
     xd_residual_free(r);
     return fail(e, "the residual check's set-up");
   }

@@ -58,6 +58,22 @@ void release(xd_rf *r) {
   delete r;
 }
 
+int zero_pivot(int info) {
+  return xd_internal_fail(-5, "zero pivot in row " + std::to_string(info - 1) + " of the refactorization");
+}
+
+// Refactors and reads the report; once more with divisions where the pivots ask for it.
+int refactor(xd_rf *r, const double *d_vals_a) {
+  int info = 0;
+  bool again = false;
+  for (int pass = 0; pass == 0 || again; ++pass) {
+    int rc = xd_lu_refactor(&r->lu, d_vals_a, 0, pass > 0);
+    if (rc == 0) rc = xd_lu_info(&r->lu, 0, &info, &again);
+    if (rc != 0) return rc;
+  }
+  return info == 0 ? 0 : zero_pivot(info);
+}
+
 bool csr_ok(int n, int nnz, const int *rp, const int *ci) {
   if (!rp || (nnz > 0 && !ci) || rp[0] != 0 || rp[n] != nnz) return false;
   for (int r = 0; r < n; ++r)
@@ -144,12 +160,8 @@ int xd_rf_create(int n, int nnz_a, const int *rowptr_a, const int *colind_a, con
     release(r);
     return cu_fail(e, "xd_rf_create upload");
   }
-  int info = 0;
-  rc = xd_lu_refactor(&r->lu, d_a, 0);
-  if (rc == 0) rc = xd_lu_info(&r->lu, 0, &info);
+  rc = refactor(r, d_a);
   cudaFree(d_a);
-  if (rc == 0 && info != 0)
-    rc = xd_internal_fail(-5, "zero pivot in row " + std::to_string(info - 1) + " of the refactorization");
   if (rc != 0) {
     release(r);
     return rc;
@@ -161,12 +173,7 @@ int xd_rf_create(int n, int nnz_a, const int *rowptr_a, const int *colind_a, con
 int xd_rf_refactor(xd_rf *r, const double *d_vals_a) {
   if (!r || !d_vals_a) return xd_internal_fail(-1, "null refactorization argument");
   cudaSetDevice(r->device);
-  int rc = xd_lu_refactor(&r->lu, d_vals_a, 0);
-  int info = 0;
-  if (rc == 0) rc = xd_lu_info(&r->lu, 0, &info);
-  if (rc == 0 && info != 0)
-    return xd_internal_fail(-5, "zero pivot in row " + std::to_string(info - 1) + " of the refactorization");
-  return rc;
+  return refactor(r, d_vals_a);
 }
 
 int xd_rf_solve(xd_rf *r, double *d_x) {
@@ -182,13 +189,16 @@ int xd_rf_solve_refined(xd_rf *r, const double *d_vals_a, const double *d_b, dou
   cudaSetDevice(r->device);
   *out = xd_rf_check{};
   out->outcome = XD_RF_ABOVE_TOL;
-  int rc = refactor ? xd_lu_refactor(&r->lu, d_vals_a, 0) : 0;
-  if (rc != 0) return rc;
-  cudaError_t e = cudaMemcpyAsync(d_x, d_b, sizeof(double) * r->n, cudaMemcpyDeviceToDevice, 0);
-  if (e != cudaSuccess) return cu_fail(e, "xd_rf_solve_refined");
-  int nstatus = 0;
+  int rc = 0, nstatus = 0;
+  cudaError_t e;
   const int *d_status = xd_lu_status(&r->lu, &nstatus);
+  bool again = false;
   for (int k = 0;; ++k) {
+    if (k == 0) {
+      if (refactor && (rc = xd_lu_refactor(&r->lu, d_vals_a, 0, again)) != 0) return rc;
+      if ((e = cudaMemcpyAsync(d_x, d_b, sizeof(double) * r->n, cudaMemcpyDeviceToDevice, 0)) != cudaSuccess)
+        return cu_fail(e, "xd_rf_solve_refined");
+    }
     // The solution, then (k > 0) the corrections in d_temp; the refactorization's own report comes
     // back with the first check, so a zero pivot is found after a solve whose result is dropped.
     if ((rc = xd_rf_solve(r, k == 0 ? d_x : r->d_temp)) != 0) return rc;
@@ -196,11 +206,15 @@ int xd_rf_solve_refined(xd_rf *r, const double *d_vals_a, const double *d_b, dou
     if ((rc = xd_residual_check(&r->res, d_vals_a, d_b, d_x, r->d_temp, d_status, nstatus, 0)) != 0) return rc;
     if ((e = cudaStreamSynchronize(0)) != cudaSuccess) return cu_fail(e, "xd_rf_solve_refined");
     if (refactor && k == 0) {
-      const int status[2] = {(int)r->res.h_out[2], (int)r->res.h_out[3]};
-      int info = 0;
-      if ((rc = xd_lu_report(&r->lu, status, &info)) != 0) return rc;
-      if (info != 0)
-        return xd_internal_fail(-5, "zero pivot in row " + std::to_string(info - 1) + " of the refactorization");
+      static_assert(kLuStatus <= kResidualStatus, "the check brings the whole report");
+      int status[kLuStatus] = {}, info = 0;
+      for (int q = 0; q < nstatus; ++q) status[q] = (int)r->res.h_out[2 + q];
+      if ((rc = xd_lu_report(&r->lu, status, &info, &again)) != 0) return rc;
+      if (again) {  // the same once more, with divisions
+        k = -1;
+        continue;
+      }
+      if (info != 0) return zero_pivot(info);
     }
     ++out->solves;
     if (r->res.h_out[1] != 0.0) {
