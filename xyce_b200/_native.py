@@ -196,8 +196,15 @@ SIGNATURES = {
 _LIB = None
 
 
+XD_RF_ZERO_PIVOT = -5  # xd_rf_refactor, xd_rf_solve_refined
+
+
 class NativeError(RuntimeError):
-    pass
+    """An entry point's error; ``code`` is what it returned."""
+
+    def __init__(self, message, code=None):
+        super().__init__(message)
+        self.code = code
 
 
 def library_path() -> str:
@@ -223,4 +230,4 @@ def load():
 def check(rc: int, what: str) -> None:
     if rc != 0:
         msg = _LIB.xd_last_error().decode() if _LIB is not None else ""
-        raise NativeError(f"{what} failed ({rc}): {msg}")
+        raise NativeError(f"{what} failed ({rc}): {msg}", rc)

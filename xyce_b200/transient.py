@@ -668,8 +668,9 @@ class GpuTransient(TransientBase):
         if getattr(self, "_rf", None) is not None and self._rf.value:
             try:
                 x = self._rf_solve_refined(self.rhs, refactor=True)
-            except _native.NativeError:
-                pass  # a zero pivot in the kept pivot order
+            except _native.NativeError as e:
+                if e.code != _native.XD_RF_ZERO_PIVOT:  # the kept pivot order's zero pivot is no failure
+                    raise
         if x is None:
             # The first matrix, or one that the kept pivot order does not suit (the matrices of a DC
             # solve and of a time step differ in which entries dominate): factor it on the host.
