@@ -20,6 +20,8 @@ namespace {
 constexpr int kBottomThreads = 512;
 constexpr int kBottomEntries = 13 * 1024;  // a group's entries in shared memory: two blocks to an SM
 constexpr int kSchurLanes = 8;        // threads per top destination
+constexpr int kSchurLong = 512;       // updates of a top destination that these take; more: a block
+constexpr int kTopRowLong = 1024;     // entries of a top row that a warp sums; more: a block
 constexpr int kTopThreads = 256;
 constexpr int kB = kBlockPivots;
 constexpr int kLd = kB + 2;           // row stride of the block's L and U in shared memory: 16-byte reads without conflicts
@@ -47,28 +49,47 @@ __device__ __forceinline__ void bottom_update(int4 ds, int4 p0, int4 p1, const i
   m[ds.x] = acc;
 }
 
+// The same by a warp, for a destination with many updates (a node that everything in its subtree hangs
+// on: a refactorization with a hub of 6,000 leaves took 1,870 us with one thread on its pairs, and takes
+// 153; with 25 hubs of 2,000, 1,200 and 140): strided, fixed tree.
+__device__ __forceinline__ void bottom_update_long(int4 ds, const int4 *__restrict__ pairs, int lane, double *m) {
+  double acc = 0.0;
+#pragma unroll 4
+  for (int p = ds.y + lane; p < ds.y + ds.z; p += 32) {
+    const int4 lu = pairs[p];
+    acc += (m[lu.x] / m[lu.z]) * m[lu.y];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) m[ds.x] -= acc;
+}
+
 // A block's levels, one barrier per level (the schedule of lu.cu's lu_levels_block_kernel: a level's
 // updates form their L factors on the spot, the divisions that store them follow during the next
 // level). A level's pivot updates ancestors only, which sit in later levels of the same block or in
-// the top part. A level's lists are read two levels ahead, its first pairs one level ahead.
+// the top part. A level's lists are read two levels ahead, its first pairs one level ahead. LONG: the
+// destinations from llong on take a warp each.
+template <bool LONG>
 __device__ __forceinline__ void bottom_levels(int l0, int l1, const int *__restrict__ ldiv,
-                                              const int *__restrict__ ldst, const int2 *__restrict__ div,
+                                              const int *__restrict__ ldst, const int *__restrict__ llong,
+                                              const int2 *__restrict__ div,
                                               const int4 *__restrict__ dst, const int4 *__restrict__ pairs, double *m) {
   const int tid = threadIdx.x;
   const int4 none = make_int4(0, 0, 0, 0);
+  auto short_end = [&](int l) { return LONG ? llong[l] : ldst[l + 1]; };
   auto list = [&](int l) {  // this thread's destination of level l
     if (l >= l1) return none;
     const int b = ldst[l] + tid;
-    return b < ldst[l + 1] ? dst[b] : none;
+    return b < short_end(l) ? dst[b] : none;
   };
   auto pair = [&](int4 ds, int k) { return ds.w < 0 && ds.z > k ? pairs[ds.y + k] : none; };
   int4 ds1 = list(l0), ds2 = list(l0 + 1), p0 = pair(ds1, 0), p1 = pair(ds1, 1);
   int2 dv_next = make_int2(0, 0);
-  int ub = ldst[l0], ue = l0 < l1 ? ldst[l0 + 1] : ub, db = ldiv[l0], de = db;
+  int ub = ldst[l0], ue = l0 < l1 ? short_end(l0) : ub, db = ldiv[l0], de = db;
   for (int l = l0; l < l1; ++l) {
     const int4 ds = ds1, q0 = p0, q1 = p1;
     const int2 dv = dv_next;
-    const int ne = l + 1 < l1 ? ldst[l + 2] : ue, nd = ldiv[l + 1];
+    const int ne = l + 1 < l1 ? short_end(l + 1) : ue, nd = ldiv[l + 1], nb = LONG ? ldst[l + 1] : ue;
     ds1 = ds2;
     ds2 = list(l + 2);
     p0 = pair(ds1, 0);
@@ -81,12 +102,14 @@ __device__ __forceinline__ void bottom_levels(int l0, int l1, const int *__restr
         bottom_update(more, pair(more, 0), pair(more, 1), pairs, m);
       }
     }
+    if (LONG)
+      for (int d = ue + tid / 32; d < nb; d += kBottomThreads / 32) bottom_update_long(dst[d], pairs, tid % 32, m);
     if (db + tid < de) {
       lu_divide(dv, m);
       for (int t = db + tid + kBottomThreads; t < de; t += kBottomThreads) lu_divide(div[t], m);
     }
     __syncthreads();
-    ub = ue;
+    ub = nb;
     ue = ne;
     db = de;
     de = nd;
@@ -102,39 +125,71 @@ __device__ __forceinline__ void bottom_levels(int l0, int l1, const int *__restr
 // (gpos: their places in V) come to shared memory first, the lists hold positions there, and the
 // entries go back at the end: refactorization of 4,455 unknowns 149 -> 139 us, of 41k 288 -> 276, of
 // 200k (where the chains wait) the same. A group with more than kBottomEntries entries (gptr: none of
-// them) works in V itself; only systems above a million unknowns have one.
+// them) works in V itself: systems of millions of unknowns have such groups, and a single subtree can be
+// one (the limit on subtrees counts updates, of which a hub of 6,000 leaves has 6,000 for 18,000 entries).
+template <bool LONG>
 __global__ void __launch_bounds__(kBottomThreads) tree_bottom_kernel(
-    const int *__restrict__ glev, const int *__restrict__ ldiv, const int *__restrict__ ldst,
+    const int *__restrict__ glev, const int *__restrict__ ldiv, const int *__restrict__ ldst, const int *__restrict__ llong,
     const int2 *__restrict__ div, const int4 *__restrict__ dst, const int4 *__restrict__ pairs,
     const int *__restrict__ gptr, const int *__restrict__ gpos, double *v) {
   extern __shared__ double entries[];
   const int l0 = glev[blockIdx.x], l1 = glev[blockIdx.x + 1], e0 = gptr[blockIdx.x], ne = gptr[blockIdx.x + 1] - e0;
   if (ne == 0) {
-    bottom_levels(l0, l1, ldiv, ldst, div, dst, pairs, v);
+    bottom_levels<LONG>(l0, l1, ldiv, ldst, llong, div, dst, pairs, v);
     return;
   }
   for (int i = threadIdx.x; i < ne; i += kBottomThreads) entries[i] = v[gpos[e0 + i]];
   __syncthreads();
-  bottom_levels(l0, l1, ldiv, ldst, div, dst, pairs, entries);
+  bottom_levels<LONG>(l0, l1, ldiv, ldst, llong, div, dst, pairs, entries);
   __syncthreads();
   for (int i = threadIdx.x; i < ne; i += kBottomThreads) v[gpos[e0 + i]] = entries[i];
 }
 
-// The bottom pivots' updates of top entries, all at once: kSchurLanes threads per destination, fixed
-// reduction order.
+// The sum of the threads' values over a block of 256, in thread 0, in a fixed order.
+__device__ __forceinline__ double block_sum256(double acc, double *red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = acc;
+  __syncthreads();
+  acc = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < 8; ++w) acc += red[w];
+  __syncthreads();
+  return acc;
+}
+
+// The bottom pivots' updates of top entries, all at once: kSchurLanes threads per destination, and the
+// whole block for one with more than kSchurLong updates (LONG: there are such); fixed reduction order.
+template <bool LONG>
 __global__ void __launch_bounds__(256) tree_schur_kernel(int nd, const int *__restrict__ sdst,
                                                          const int *__restrict__ sptr, const int2 *__restrict__ pairs,
                                                          double *v) {
   const int d = (blockIdx.x * 256 + threadIdx.x) / kSchurLanes, lane = threadIdx.x % kSchurLanes;
   double acc = 0.0;
-  if (d < nd)
-    for (int p = sptr[d] + lane, e = sptr[d + 1]; p < e; p += kSchurLanes) {
+  const int b = d < nd ? sptr[d] : 0, e = d < nd ? sptr[d + 1] : 0;
+  const bool many = LONG && e - b > kSchurLong;
+  if (!many)
+    for (int p = b + lane; p < e; p += kSchurLanes) {
       const int2 lu = pairs[p];
       acc = fma(v[lu.x], v[lu.y], acc);
     }
 #pragma unroll
   for (int o = kSchurLanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (d < nd && lane == 0) v[sdst[d]] -= acc;
+  if (d < nd && lane == 0 && !many) v[sdst[d]] -= acc;
+  if (!LONG || !__syncthreads_or(many)) return;
+  __shared__ double red[8];
+  for (int q = blockIdx.x * (256 / kSchurLanes), qe = min(nd, q + 256 / kSchurLanes); q < qe; ++q) {
+    const int qb = sptr[q], qn = sptr[q + 1];
+    if (qn - qb <= kSchurLong) continue;
+    acc = 0.0;
+#pragma unroll 4
+    for (int p = qb + threadIdx.x; p < qn; p += 256) {
+      const int2 lu = pairs[p];
+      acc = fma(v[lu.x], v[lu.y], acc);
+    }
+    acc = block_sum256(acc, red);
+    if (threadIdx.x == 0) v[sdst[q]] -= acc;
+  }
 }
 
 __device__ __forceinline__ void cp_async16(void *s, const void *g) {
@@ -430,8 +485,9 @@ __global__ void tree_rhs_kernel(int n, const int *__restrict__ bsrc, const doubl
 // with more than kPassRows keeps them in s), and what does not depend on them - columns and values of
 // a pass's first round, its rows and their right-hand sides, solved values of columns outside the
 // group - is loaded a pass ahead, so a level waits for shared memory alone. Forward: s[row] =
-// rhs[row] - sum, in place; backward: divided by the diagonal, and scattered to the solution.
-template <bool BACKWARD>
+// rhs[row] - sum, in place; backward: divided by the diagonal, and scattered to the solution. LONG:
+// there are rows of several warps.
+template <bool BACKWARD, bool LONG>
 __global__ void __launch_bounds__(kPassThreads) tree_pass_kernel(const int *__restrict__ gptr,
                                                                  const int4 *__restrict__ pass,
                                                                  const int *__restrict__ rows,
@@ -441,6 +497,7 @@ __global__ void __launch_bounds__(kPassThreads) tree_pass_kernel(const int *__re
                                                                  double *s, const int *__restrict__ xdst, double *out,
                                                                  const int *__restrict__ grow) {
   extern __shared__ __align__(16) double smem[];
+  __shared__ double red[kPassThreads / 32];
   const int tid = threadIdx.x, base = grow[blockIdx.x], size = grow[blockIdx.x + 1] - base;
   const bool fits = size <= kPassRows;
   double *loc = fits ? smem : s + base;
@@ -511,7 +568,14 @@ __global__ void __launch_bounds__(kPassThreads) tree_pass_kernel(const int *__re
         const int at = f.m.z + k * width + tid, c = col[at - off0];
         if (c >= 0) acc += v[at] * (own(c) ? loc[c - base] : s[c]);
       }
-    for (int o = 1 << lg >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    for (int o = LONG ? min(16, 1 << lg >> 1) : 1 << lg >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (LONG && lg > 5) {
+      if (tid % 32 == 0) red[tid / 32] = acc;
+      __syncthreads();
+      if (f.x >= 0)
+        for (int w = 1; w < 1 << (lg - 5); ++w) acc += red[tid / 32 + w];
+      __syncthreads();
+    }
     if (f.x >= 0) {
       const double r = BACKWARD ? (q.b - acc) / q.d : q.b - acc;
       s[f.x] = r;
@@ -522,17 +586,31 @@ __global__ void __launch_bounds__(kPassThreads) tree_pass_kernel(const int *__re
   }
 }
 
-// Rows [x0, n): the top rows' sums over columns outside their panels, a warp each.
+// Rows [x0, n): the top rows' sums over columns outside their panels, a warp each, the block for a row of
+// more than kTopRowLong entries (LONG: there are such).
+template <bool LONG>
 __global__ void __launch_bounds__(256) tree_top_rows_kernel(int x0, int n, const int *__restrict__ lptr,
                                                             const int *__restrict__ lcol, const double *v, double *y) {
-  const int r = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x % 32;
-  if (x0 + r >= n) return;
-  const int b = lptr[r], end = lptr[r + 1];
+  const int r = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x % 32, rows = n - x0;
+  const int b = r < rows ? lptr[r] : 0, end = r < rows ? lptr[r + 1] : 0;
+  const bool many = LONG && end - b > kTopRowLong;
   double acc = 0.0;
-  for (int e = b + lane; e < end; e += 32) acc += v[e] * y[lcol[e]];
+  if (!many)
+    for (int e = b + lane; e < end; e += 32) acc += v[e] * y[lcol[e]];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0 && end > b) y[x0 + r] -= acc;
+  if (lane == 0 && end > b && !many) y[x0 + r] -= acc;
+  if (!LONG || !__syncthreads_or(many)) return;
+  __shared__ double red[8];
+  for (int q = blockIdx.x * 8, qe = min(rows, q + 8); q < qe; ++q) {
+    const int qb = lptr[q], qn = lptr[q + 1];
+    if (qn - qb <= kTopRowLong) continue;
+    acc = 0.0;
+#pragma unroll 4
+    for (int e = qb + threadIdx.x; e < qn; e += 256) acc += v[e] * y[lcol[e]];
+    acc = block_sum256(acc, red);
+    if (threadIdx.x == 0) y[x0 + q] -= acc;
+  }
 }
 
 __device__ __forceinline__ void cp_async8(void *s, const void *g) {
@@ -935,6 +1013,13 @@ int xd_tree_upload(XdTree *t, const XdTreePlan &p, const int *perm_p, const int 
     tail.push_back({x, p.diag[p.order[x]], first, (int)chunk.size() - first});
   }
   t->nchunk = (int)chunk.size();
+  for (size_t k = 0; k + 1 < p.sptr.size(); ++k) t->schur_long = t->schur_long || p.sptr[k + 1] - p.sptr[k] > kSchurLong;
+  for (size_t k = 0; k + 1 < p.lptr.size(); ++k) t->row_long = t->row_long || p.lptr[k + 1] - p.lptr[k] > kTopRowLong;
+  for (int u = 0; u < 2; ++u)
+    for (const XdPos4 &q : (u ? p.bwd : p.fwd).pass) t->pass_long[u] = t->pass_long[u] || (q.y >> 16 & 0xff) > 5;
+  auto pass_attribute = [](auto *kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(double) * kPassRows);
+  };
   for (int c : p.jchild) joined[c] = 1;
   cudaError_t e;
   auto upload_passes = [](XdTree::Passes &d, const XdPasses &h) {
@@ -950,10 +1035,10 @@ int xd_tree_upload(XdTree *t, const XdTreePlan &p, const int *perm_p, const int 
       (e = upload(&t->d_tail, tail)) != cudaSuccess || (e = upload(&t->d_bsrc, bsrc)) != cudaSuccess ||
       (e = upload(&t->d_xdst, xdst)) != cudaSuccess || (e = upload(&t->d_joined, joined)) != cudaSuccess ||
       (e = upload(&t->d_border, p.border)) != cudaSuccess || (e = upload(&t->d_grow, grow)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(tree_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(double) * kPassRows)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(tree_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(double) * kPassRows)) != cudaSuccess ||
+      (e = pass_attribute(tree_pass_kernel<false, false>)) != cudaSuccess ||
+      (e = pass_attribute(tree_pass_kernel<true, false>)) != cudaSuccess ||
+      (e = pass_attribute(tree_pass_kernel<false, true>)) != cudaSuccess ||
+      (e = pass_attribute(tree_pass_kernel<true, true>)) != cudaSuccess ||
       (e = cudaMalloc(&t->d_y, sizeof(double) * std::max(1, p.n))) != cudaSuccess ||
       (e = cudaMalloc(&t->d_x, sizeof(double) * std::max(1, p.n))) != cudaSuccess ||
       (e = cudaMalloc(&t->d_wbuf, sizeof(double) * std::max<size_t>(1, (size_t)p.nchains * p.F))) != cudaSuccess ||
@@ -964,7 +1049,10 @@ int xd_tree_upload(XdTree *t, const XdTreePlan &p, const int *perm_p, const int 
       (e = upload(&t->d_ldiv, p.ldiv)) != cudaSuccess || (e = upload(&t->d_ldst, p.ldst)) != cudaSuccess ||
       (e = upload(&t->d_div, bottom.div)) != cudaSuccess || (e = upload(&t->d_dst, bottom.dst)) != cudaSuccess ||
       (e = upload(&t->d_gptr, bottom.gptr)) != cudaSuccess || (e = upload(&t->d_gpos, bottom.gpos)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(tree_bottom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      (p.any_long && (e = upload(&t->d_llong, p.llong)) != cudaSuccess) ||
+      (e = cudaFuncSetAttribute(tree_bottom_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(double) * kBottomEntries)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(tree_bottom_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(double) * kBottomEntries)) != cudaSuccess ||
       (e = upload(&t->d_pairs, bottom.pairs)) != cudaSuccess || (e = upload(&t->d_sdst, p.sdst)) != cudaSuccess ||
       (e = upload(&t->d_sptr, p.sptr)) != cudaSuccess || (e = upload(&t->d_spairs, p.spairs)) != cudaSuccess ||
@@ -1000,18 +1088,18 @@ void xd_tree_free(XdTree *t) {
                   (void *)t->d_lcol, (void *)t->d_tcol, (void *)t->d_chunk, (void *)t->d_tail, (void *)t->d_bsrc,
                   (void *)t->d_xdst, (void *)t->d_joined, (void *)t->d_border, (void *)t->d_y, (void *)t->d_x,
                   (void *)t->d_wbuf, (void *)t->d_part, (void *)t->d_sctl, (void *)t->d_grow, (void *)t->d_gptr,
-                  (void *)t->d_gpos})
+                  (void *)t->d_gpos, (void *)t->d_llong})
     cudaFree(p);
   *t = XdTree();
 }
 
 int xd_tree_factor(XdTree *t, cudaStream_t st) {
   if (t->ngroups > 0)
-    tree_bottom_kernel<<<t->ngroups, kBottomThreads, t->bottom_smem, st>>>(
-        t->d_glev, t->d_ldiv, t->d_ldst, t->d_div, t->d_dst, t->d_pairs, t->d_gptr, t->d_gpos, t->d_v);
+    (t->d_llong ? tree_bottom_kernel<true> : tree_bottom_kernel<false>)<<<t->ngroups, kBottomThreads, t->bottom_smem, st>>>(
+        t->d_glev, t->d_ldiv, t->d_ldst, t->d_llong, t->d_div, t->d_dst, t->d_pairs, t->d_gptr, t->d_gpos, t->d_v);
   if (t->nsd > 0) {
     const long long threads = (long long)t->nsd * kSchurLanes;
-    tree_schur_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(t->nsd, t->d_sdst, t->d_sptr, t->d_spairs,
+    (t->schur_long ? tree_schur_kernel<true> : tree_schur_kernel<false>)<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(t->nsd, t->d_sdst, t->d_sptr, t->d_spairs,
                                                                          t->d_v);
   }
   if (t->nchains > 0) {
@@ -1036,12 +1124,12 @@ int xd_tree_solve(XdTree *t, double *d_x, cudaStream_t st) {
     return xd_internal_fail(-3, std::string("triangular solve: ") + cudaGetErrorString(e));
   tree_rhs_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, t->d_bsrc, d_x, t->d_y);
   if (t->ngroups > 0)
-    tree_pass_kernel<false><<<t->ngroups, kPassThreads, t->pass_smem, st>>>(t->d_fwd.gptr, t->d_fwd.pass, t->d_fwd.rows,
+    (t->pass_long[0] ? tree_pass_kernel<false, true> : tree_pass_kernel<false, false>)<<<t->ngroups, kPassThreads, t->pass_smem, st>>>(t->d_fwd.gptr, t->d_fwd.pass, t->d_fwd.rows,
                                                                  t->d_fwd.col, 0, v, nullptr, t->d_y, t->d_y, nullptr,
                                                                  nullptr, t->d_grow);
   if (nc > 0) {
     const int threads = (t->F + 31) / 32 * 32 + 32;
-    tree_top_rows_kernel<<<(t->ntop + 7) / 8, 256, 0, st>>>(t->nbot, n, t->d_lptr, t->d_lcol, v + t->l0, t->d_y);
+    (t->row_long ? tree_top_rows_kernel<true> : tree_top_rows_kernel<false>)<<<(t->ntop + 7) / 8, 256, 0, st>>>(t->nbot, n, t->d_lptr, t->d_lcol, v + t->l0, t->d_y);
     tree_forward_chain_kernel<<<nc, threads, SolveSmem::bytes(t->F), st>>>(
         t->F, t->d_cptr, t->d_bptr, t->d_blocks, t->d_jchild, t->d_jmap, t->d_wbuf, v + t->p0, t->d_y + t->nbot,
         t->d_sctl, t->d_sctl + 2);
@@ -1050,7 +1138,7 @@ int xd_tree_solve(XdTree *t, double *d_x, cudaStream_t st) {
         t->d_xdst, d_x, t->d_sctl + 1, t->d_sctl + 2 + nc, t->d_joined);
   }
   if (t->ngroups > 0)
-    tree_pass_kernel<true><<<t->ngroups, kPassThreads, t->pass_smem, st>>>(t->d_bwd.gptr, t->d_bwd.pass, t->d_bwd.rows,
+    (t->pass_long[1] ? tree_pass_kernel<true, true> : tree_pass_kernel<true, false>)<<<t->ngroups, kPassThreads, t->pass_smem, st>>>(t->d_bwd.gptr, t->d_bwd.pass, t->d_bwd.rows,
                                                                 t->d_bwd.col, t->u0, v, v + t->d0, t->d_y, t->d_x,
                                                                 t->d_xdst, d_x, t->d_grow);
   if (t->nchunk > 0)

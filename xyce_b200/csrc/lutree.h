@@ -29,6 +29,7 @@ constexpr int kBlockPivots = 8;      // pivots a chain eliminates at a time
 constexpr int kBlockInts = 12;       // a block's record: its pivots' slots (kNoPivot past the last), the
                                      // frame's live slots, the first and last child chain that joins
 constexpr int kNoPivot = (int)0x80000000;
+constexpr int kLongPairs = 32;       // updates of a bottom destination that a thread takes; more: a warp
 #ifdef __CUDACC__
 #define XD_TREE_FN __host__ __device__
 #else
@@ -72,6 +73,8 @@ struct XdTreePlan {
   // lrow[l + 1]), its divisions and its update destinations.
   int ngroups = 0;
   std::vector<int> glev, lrow, ldiv, ldst;
+  std::vector<int> llong;            // [levels] the first of a level's destinations with more than kLongPairs updates
+  bool any_long = false;
   std::vector<XdPos2> div;           // (position of L(i, k), position of U(k, k))
   std::vector<XdPos4> dst, pairs;    // as in lu.cu: one update inline, or a range of pairs
   // Updates of top entries by bottom pivots: destination sdst[d], pairs (L, U) sptr[d] .. sptr[d + 1].
@@ -104,6 +107,7 @@ struct XdTree {
   double *d_v = nullptr;             // V
   int *d_diag = nullptr;             // [n]
   int *d_glev = nullptr, *d_ldiv = nullptr, *d_ldst = nullptr;
+  int *d_llong = nullptr;            // null: no destination has more than kLongPairs updates
   int2 *d_div = nullptr;
   int4 *d_dst = nullptr, *d_pairs = nullptr;
   int *d_gptr = nullptr, *d_gpos = nullptr;  // the bottom groups' entries (positions in V) in shared memory
@@ -122,6 +126,7 @@ struct XdTree {
   } d_fwd, d_bwd;
   int *d_grow = nullptr;             // [ngroups + 1] first row of each group
   size_t pass_smem = 0;
+  bool schur_long = false, row_long = false, pass_long[2] = {};  // lists that a block takes (lutree.cu)
   int *d_lptr = nullptr, *d_lcol = nullptr, *d_tcol = nullptr;
   int4 *d_chunk = nullptr;           // chunks of the rows solved last: (row, first entry, end, chunk of the row)
   int4 *d_tail = nullptr;            // those rows: (position in order, V position of its pivot, first chunk, chunks)

@@ -15,6 +15,7 @@ namespace {
 // at 200k (12.6M); a matrix with few updates has no use for tall subtrees.
 constexpr double kTopWork = 30000, kTopWorkSmall = 10000, kSmallMatrix = 300000, kNoPlan = 5000;
 constexpr int kTopHeight = 64;  // nor with more levels than this
+constexpr size_t kLongRow = 256;  // entries of a bottom row that one warp sums in a solve
 constexpr int kGroups = 296;  // two blocks per SM walk the bottom subtrees
 
 }  // namespace
@@ -300,7 +301,12 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
         for (size_t r = 0; r < rows.size();) {
           int lg = 0;
           while (lg < 5 && (1u << lg) < ents[rows[r]].size()) ++lg;
+          // A long row takes up to the whole block, in passes with its like (a hub's row of 6,000 entries
+          // by 32 lanes: 78 us a solve; by 512: 24).
+          const bool longer = ents[rows[r]].size() > kLongRow;
+          while (longer && (1u << lg) < (unsigned)kPassThreads && ents[rows[r]].size() > (8u << lg)) ++lg;
           size_t count = std::min(rows.size() - r, (size_t)(kPassThreads >> lg));
+          while (!longer && ents[rows[r + count - 1]].size() > kLongRow) --count;
           size_t most = ents[rows[r + count - 1]].size();
           while (lg < 5 && most > (1u << lg) && (count << (lg + 1)) <= (size_t)kPassThreads) ++lg;
           const int lanes = 1 << lg, rounds = std::max(1, (int)((most + lanes - 1) / lanes)), width = (int)count * lanes;
@@ -414,16 +420,23 @@ bool xd_tree_plan(int n, const std::vector<int> &mp, const std::vector<int> &mi,
       std::vector<int> f(start.begin(), start.end());
       for (size_t x = 0; x < lv.size(); ++x) sorted[f[upd[x]]++] = lv[x];
     }
+    std::vector<XdPos4> longer;
     for (size_t d = 0; d < touched.size(); ++d) {
       const int b = start[d], c = cnt[d + 1], dp = t.pos[touched[d]];
       slot_of[touched[d]] = -1;
-      if (c == 1) {
+      if (c > kLongPairs) {
+        longer.push_back({dp, (int)t.pairs.size(), c, -1});
+        t.pairs.insert(t.pairs.end(), sorted.begin() + b, sorted.begin() + b + c);
+      } else if (c == 1) {
         t.dst.push_back({dp, sorted[b].x, sorted[b].y, sorted[b].z});
       } else {
         t.dst.push_back({dp, (int)t.pairs.size(), c, -1});
         t.pairs.insert(t.pairs.end(), sorted.begin() + b, sorted.begin() + b + c);
       }
     }
+    t.llong.push_back((int)t.dst.size());
+    t.any_long = t.any_long || !longer.empty();
+    t.dst.insert(t.dst.end(), longer.begin(), longer.end());
     t.ldiv.push_back((int)t.div.size());
     t.ldst.push_back((int)t.dst.size());
     if (t.pairs.size() > (size_t)INT_MAX || sv.size() > (size_t)INT_MAX) return false;
