@@ -502,7 +502,6 @@ struct FusedSmem {
   float b[4 * kHid + kOutPad];           // biases of layers 1..5
   uint64_t bar[kFwdGroups];
   uint32_t tmem;
-  int failed[kFwdGroups];                // a wait of the group expired
 };
 static_assert(sizeof(FusedSmem) <= 227 * 1024, "one block's shared memory");
 
@@ -558,7 +557,6 @@ __global__ void __launch_bounds__(kFwdGroups *kFusedThreads, 1) mlp_forward_fuse
   if (threadIdx.x < 32) tmem_alloc(&S.tmem, 512);
   if (threadIdx.x < kFwdGroups) {
     mbar_init(&S.bar[threadIdx.x], 1);
-    S.failed[threadIdx.x] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc_fence_before();
@@ -574,8 +572,21 @@ __global__ void __launch_bounds__(kFwdGroups *kFusedThreads, 1) mlp_forward_fuse
   const int row = quarter * 32 + lane;    // the tile row this thread owns in the epilogues
   const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
   uint32_t phase = 0;
-  bool ok = true;
-  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kFusedThreads) : "memory"); };
+  // The group's barrier, which also tells every thread whether all waits so far were in time: the
+  // threads of a group leave their loop together, or one would be left at a barrier of its own.
+  bool ok = true, mine = true;
+  auto group_sync = [&]() {
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all)
+        : "r"((uint32_t)mine), "r"(1 + group), "n"(kFusedThreads)
+        : "memory");
+    return all != 0;
+  };
   const int tiles = (n + kTileM - 1) / kTileM, stride = gridDim.x * kFwdGroups;
   bool staged = false;
   float xi[8];
@@ -606,9 +617,8 @@ __global__ void __launch_bounds__(kFwdGroups *kFusedThreads, 1) mlp_forward_fuse
     for (int l = 0; l < 4; ++l) {
       fence_proxy_async_smem();
       tc_fence_before();
-      group_sync();
+      ok = group_sync();
       tc_fence_after();
-      ok = *(volatile int *)&S.failed[group] == 0;
       if (!ok) break;
       const bool last = (l == 3);
       if (tid == 0) {
@@ -618,7 +628,7 @@ __global__ void __launch_bounds__(kFwdGroups *kFusedThreads, 1) mlp_forward_fuse
                    last ? idesc_o : idesc_h, s > 0 ? 1u : 0u);
         mma_commit(bar);
       }
-      if (!mbar_wait(bar, phase)) S.failed[group] = 1;
+      mine = mbar_wait(bar, phase) && mine;
       phase ^= 1u;
       tc_fence_after();
       if (!last) {
@@ -653,8 +663,7 @@ __global__ void __launch_bounds__(kFwdGroups *kFusedThreads, 1) mlp_forward_fuse
     fence_proxy_async_smem();
     asm volatile("bar.sync 0;" ::: "memory");
   }
-  group_sync();
-  if (S.failed[group]) {  // an expired wait: record it and drain (bounded) before tensor memory goes
+  if (!group_sync()) {  // an expired wait: record it and drain (bounded) before tensor memory goes
     if (tid == 0) atomicExch(err, 1);
     mbar_wait(bar, phase ^ 1u);
   }
