@@ -274,12 +274,12 @@ class SurrogateMLP:
         torch = self.torch
         n, _ = self._load_inputs(X)
         self.T[:n] = torch.as_tensor(T, dtype=torch.float32, device=self.dev)
-        self.step_count += 1
-        t = self.step_count
+        t = self.step_count + 1
         a = self._train_args()
         a.n, a.scale = n, 2.0 / (n * N_OUT)
         a.adam = _native.XdAdamArgs(cfg.lr, cfg.beta1, cfg.beta2, cfg.eps, 1 - cfg.beta1 ** t, 1 - cfg.beta2 ** t)
         _native.check(self.k.lib.xd_mlp_train_step(ctypes.byref(a), self.k.stream()), "xd_mlp_train_step")
+        self.step_count = t
         return self.sq[:n].mean() / N_OUT
 
     def _train_args(self):
