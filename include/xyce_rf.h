@@ -32,8 +32,8 @@ int xd_rf_create(int n, int nnz_a, const int *rowptr_a, const int *colind_a, con
  * own elimination (the elimination tree's subtrees on independent blocks, the chains above them
  * eight pivots at a time; small or dense systems level by level on one block; each entry updated in
  * a fixed order, so the factors do not depend on timing). A zero pivot in that
- * order is an error (< 0, which synchronises the legacy default stream to read); a small one is
- * not detected here, so a caller that cannot bound the growth checks the solution's residual
+ * order is an error (-5; the call synchronises the legacy default stream to read it); a small one,
+ * down to subnormal ones, is accepted, so a caller that cannot bound the growth checks the solution's residual
  * (the transient driver refines and, failing that, makes a new host factorization). */
 int xd_rf_refactor(xd_rf *rf, const double *d_vals_a);
 

@@ -465,9 +465,9 @@ __global__ void tree_finish_kernel(int nt, const int2 *__restrict__ tdiv, int n,
 // ---- solves --------------------------------------------------------------------------------------
 // Forward: the bottom subtrees' rows level by level, the top rows' sums over bottom columns in one
 // pass, then the chains; backward the other way round. As in the factorization, a chain's pivots
-// are the serial part: one warp per chain takes kB of them at a time, every lane solving the
-// block's small triangle redundantly in registers, so that consecutive pivots cost a
-// multiply-add's latency.
+// are the serial part: a block per chain takes kB of them at a time, a thread per slot of the frame and
+// one more warp that streams the panels in; every thread solves the block's small triangle redundantly
+// in registers, so that consecutive pivots cost a multiply-add's latency.
 
 constexpr int kSolveAhead = 4;        // blocks in flight in a chain's solve
 constexpr int kPassRows = 24 * 1024;  // rows of a group whose values fit shared memory

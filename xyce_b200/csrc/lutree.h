@@ -5,14 +5,14 @@
 // struct(k) (the rows of L's column k and the columns of U's row k, closed under elimination), all
 // of which are ancestors of k. Two facts about circuit factors shape the plan:
 //   * the tree is a wide forest of small subtrees under a few long paths. At 200k unknowns (the
-//     placed 100k-MOSFET netlist) 4,374 subtrees of at most 36 levels hang off 61 paths, the
-//     longest of 2,890 pivots whose fronts have 24 to 64 variables;
+//     placed 100k-MOSFET netlist) 4,212 subtrees of at most 40 levels hang off 56 paths, the
+//     longest of 2,888 pivots, in frames of 35 to 71 slots;
 //   * a few pivots (a supply's branch equation and current) have an empty row of U or an empty
 //     column of L and so make no updates, however long their other side is; their adjacency must
 //     not be counted as a front (the rail's 90k-entry row would make one front of 90k variables).
 // So the pivots are split in two: the BOTTOM subtrees, of at most kTopWork updates each, are spread
 // over thread blocks that walk their levels independently; the TOP pivots are eliminated path by
-// path ("chains"), one thread block per chain, with the front held densely in registers
+// path ("chains"), one thread block per chain, with the front held densely in shared memory
 // (lutree.cu). A matrix whose structure does not fit (frame over kMaxFrame, fill of the symmetrised
 // pattern, an update-free pivot that others wait for) has no plan, and the level-by-level
 // kernels of lu.cu and sptrsv.cu take it.

@@ -9,14 +9,22 @@
 namespace {
 
 // A subtree with at most this many updates is a bottom subtree. Larger: fewer and shorter chains and
-// fewer joins, but taller subtrees, whose levels cost a block barrier each. Refactorization at 1,000
-// / 3,000 / 10,000 / 30,000 / 100,000 updates: 106 / 95 / 99 / 120 / 183 us at 2.8k unknowns (74k
-// updates in all), 442 / 409 / 309 / 309 / 355 us at 41k (2M), 1.87 / 1.80 / 1.44 / 1.16 / 1.15 ms
-// at 200k (12.6M); a matrix with few updates has no use for tall subtrees.
+// fewer joins, but taller subtrees, whose levels cost a block barrier each. Refactorization + solve in
+// us at 3,000 / 10,000 / 30,000 / 100,000 updates:
+//     2.8k unknowns,  74k updates in all    90+60    90+65   102+82   188+149
+//     7.8k           252k                  131+97   110+92   143+138  193+156
+//     4.5k (any net) 413k                  164+82   162+84   139+83   170+106
+//     12k            518k                  202+134  148+112  176+152  242+193
+//     24k            1.2M                  367+225  265+175  254+185  319+230
+//     41k            2.0M                  398+237  281+181  275+211  348+246
+//     200k           12.6M                1732+916 1350+740 1088+630 1085+638
+// A matrix with few updates has no use for tall subtrees. The line at 300k is right for what lies below
+// it and for netlists wired any to any; placed ones between it and a million updates would be up to a
+// fifth faster with the smaller limit.
 constexpr double kTopWork = 30000, kTopWorkSmall = 10000, kSmallMatrix = 300000, kNoPlan = 5000;
 constexpr int kTopHeight = 64;  // nor with more levels than this
 constexpr size_t kLongRow = 256;  // entries of a bottom row that one warp sums in a solve
-constexpr int kGroups = 296;  // two blocks per SM walk the bottom subtrees
+constexpr int kGroups = 296;  // two blocks for each of 148 SMs walk the bottom subtrees
 
 }  // namespace
 

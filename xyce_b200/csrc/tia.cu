@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(32) slu_kernel(SluArgs a, const double *__rest
 // slu_kernel. What bounds it is the length of a round (two barriers, a division, a dependent
 // index-operand-update chain: a few hundred cycles), not work. Entries are stored compactly
 // (pattern only), the lists are copied to shared memory by the whole block. The 103-unknown ring
-// of 51 inverters: 100.7 us by steps on one warp, 17.2 us by rounds (device time, cold caches).
+// of 101 inverters: 100.7 us by steps on one warp, 17.2 us by rounds (device time, cold caches).
 struct SluRounds {
   int n, entries, factors;     // entries of the pattern + n of the right-hand side; the pattern's alone
   int n_scale, n_task, n_pair, n_fwd, n_back, lists;  // list sizes; 16-byte units of all the lists

@@ -8,8 +8,11 @@ compressed scale, y = asinh(x / s) per output, so that relative accuracy holds a
 decades a MOSFET current spans.
 
 Weights of the 128-wide layers are BF16 for the matrix products (FP32 master copies and Adam
-moments), accumulation is FP32; those products run in ``xd_gemm_bf16`` (tcgen05 tensor cores,
-include/xyce_surrogate.h) with the bias / SiLU / SiLU-derivative work fused into the epilogue. The
+moments), accumulation is FP32. A training step is one call, ``xd_mlp_train_step`` (include/
+xyce_surrogate.h: forward, backward and Adam on the tcgen05 tensor cores in two launches), and
+``forward_fused`` is ``xd_mlp_forward``; ``forward``, ``backward`` and ``adam_step`` make the same
+passes layer by layer, their products in ``xd_gemm_bf16``. The bias / SiLU / SiLU-derivative work is
+fused into the products' epilogues. The
 first layer (5 -> 128, 0.5% of the FLOPs) runs in FP32 on the CUDA cores so that the bias inputs
 keep full precision (BF16 would round 1 V to ~4 mV, a 10% step of a subthreshold current). The
 loss gradient, bias gradients, split-K reductions and the Adam update are the library's own
