@@ -152,3 +152,14 @@ def test_long_lists(name):
     assert (np.abs(b - B @ x) / (abs(B) @ np.abs(x) + np.abs(b))).max() < 2.2e-12
     assert rf.refactor(B.data) == 0 and np.array_equal(rf.factors(), f1) and np.array_equal(rf.solve(b), x)
     rf.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", tree.CASES)
+def test_factors_of_the_other_tests_are_compared(name):
+    """The factor check of test_rf_tree_gpu reads the library's factors through the pattern of L's and U's
+    entries, where both have as many: they have."""
+    rf = tree.Rf(matrix(name))
+    pat = sp.csr_matrix(abs(sp.tril(rf.L, -1)) + abs(rf.U))
+    assert rf.factors().shape[0] == pat.nnz
+    rf.close()
